@@ -1,6 +1,7 @@
-"""ctypes binding of libflashmoba_b200.so (the C ABI declared in include/flash_moba_b200.h).
+"""Loads the compiled parts: libflashmoba_b200.so (ctypes binding of the C ABI declared in
+include/flash_moba_b200.h) and _fmb_torch.so (the native host path of the PyTorch front end).
 
-There is no fallback: if the library has not been built, importing this module raises.
+There is no fallback: if they have not been built, importing this module raises.
 """
 import ctypes
 import os
@@ -24,6 +25,13 @@ if not os.path.exists(LIB_PATH):
     )
 
 lib = ctypes.CDLL(LIB_PATH)
+
+# the C++ host path of the PyTorch front end (csrc/fmb_torch.cpp); it links against the library above
+if not os.path.exists(os.path.join(HERE, "_fmb_torch.so")):
+    raise ImportError(f"{os.path.join(HERE, '_fmb_torch.so')} is missing: build it with `python flash_moba_b200/build.py`.")
+import torch  # noqa: E402,F401  (its libraries have to be loaded first)
+
+from . import _fmb_torch as native  # noqa: E402,F401
 
 _SIGS = {
     "fmb_version": (i32, []),

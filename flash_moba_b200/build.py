@@ -1,9 +1,10 @@
-"""In-tree build of libflashmoba_b200.so with nvcc for sm_100a (no torch headers involved).
+"""In-tree build of libflashmoba_b200.so with nvcc for sm_100a (no torch headers involved) and of
+_fmb_torch.so, the C++ host path of the PyTorch front end, with the host compiler.
 
     python flash_moba_b200/build.py [--force]
 
-Objects go to flash_moba_b200/_build/, the library next to this file, so that the built
-library travels with a snapshot of the source tree.
+Objects go to flash_moba_b200/_build/, the libraries next to this file, so that the built
+libraries travel with a snapshot of the source tree.
 """
 import concurrent.futures
 import os
@@ -15,6 +16,8 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 BUILD = os.path.join(HERE, "_build")
 LIB = os.path.join(HERE, "libflashmoba_b200.so")
+TORCH_EXT = os.path.join(HERE, "_fmb_torch.so")
+TORCH_SRC = os.path.join(CSRC, "fmb_torch.cpp")
 INCLUDE = os.path.join(os.path.dirname(HERE), "include")
 
 NVCC_FLAGS = [
@@ -55,6 +58,28 @@ def _compile(nvcc, src, obj, log):
     return obj
 
 
+def _build_torch_ext(log):
+    """_fmb_torch.so: links against the torch libraries of the running interpreter and against
+    libflashmoba_b200.so (found beside it at run time)."""
+    import sysconfig
+
+    import torch
+    from torch.utils import cpp_extension
+    cuda = os.path.dirname(os.path.dirname(_nvcc()))
+    torch_lib = os.path.join(os.path.dirname(torch.__file__), "lib")
+    cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", "-DTORCH_EXTENSION_NAME=_fmb_torch"]
+    for d in cpp_extension.include_paths() + [sysconfig.get_path("include"), os.path.join(cuda, "include")]:
+        cmd += ["-isystem", d]
+    cmd += [TORCH_SRC, "-o", TORCH_EXT, "-L", HERE, "-lflashmoba_b200", "-L", torch_lib, "-ltorch_python", "-ltorch",
+            "-ltorch_cpu", "-lc10", "-lc10_cuda", "-L", os.path.join(cuda, "lib64"), "-lcudart", "-Wl,-rpath,$ORIGIN"]
+    r = subprocess.run(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
+    with open(log, "w") as f:
+        f.write(" ".join(cmd) + "\n" + r.stdout)
+    if r.returncode != 0:
+        raise RuntimeError("g++ failed on fmb_torch.cpp:\n" + r.stdout[-4000:])
+
+
 def build(force: bool = False, verbose: bool = False) -> str:
     """Compile what is out of date and link the shared library; returns its path."""
     nvcc = _nvcc()
@@ -80,6 +105,11 @@ def build(force: bool = False, verbose: bool = False) -> str:
             raise RuntimeError("link failed:\n" + r.stdout[-4000:])
         if verbose:
             print("linked", LIB)
+    header_t = max(os.path.getmtime(os.path.join(INCLUDE, f)) for f in os.listdir(INCLUDE))
+    if force or not os.path.exists(TORCH_EXT) or os.path.getmtime(TORCH_EXT) < max(os.path.getmtime(TORCH_SRC), header_t):
+        _build_torch_ext(os.path.join(BUILD, "fmb_torch.log"))
+        if verbose:
+            print("linked", TORCH_EXT)
     return LIB
 
 

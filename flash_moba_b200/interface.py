@@ -19,6 +19,7 @@ from typing import Optional, Tuple
 import torch
 
 from . import ops
+from ._lib import native
 
 
 def round_multiple(x: int, m: int) -> int:
@@ -50,6 +51,14 @@ def _reject_unsupported(dropout_p, softcap, alibi_slopes):
         raise RuntimeError("FlashMoBA does not support ALiBi (alibi_slopes must be None)")
 
 
+def _check_attention_arguments(lg_block_m, lg_block_n, dropout_p, softcap, alibi_slopes):
+    _reject_unsupported(dropout_p, softcap, alibi_slopes)
+    if lg_block_n % 64 != 0:
+        raise RuntimeError("lg_block_n must be divisible by 64")
+    if lg_block_m % 64 != 0 or not (128 <= lg_block_m <= 1024):
+        raise RuntimeError("lg_block_m must be divisible by 64 and within [128, 1024]")
+
+
 # ======================================================================================
 # custom ops (same names and schemas as the reference)
 # ======================================================================================
@@ -66,11 +75,8 @@ def _moba_fused_topk(
     moba_chunk_size: int,
     causal: bool = True,
 ) -> Tuple[torch.Tensor, torch.Tensor, torch.Tensor]:
-    q, km = _fix_last_stride(q), km.contiguous()
-    idx, _ = ops.gate_topk(q, km, cu_seqlens_q, cu_seqlens_k, cu_seqlens_km, max_seqlen_q, max_seqlen_k,
-                           moba_topk, moba_chunk_size, causal)
-    ncol = (max_seqlen_k + moba_chunk_size - 1) // moba_chunk_size
-    return ops.build_csc(idx, cu_seqlens_q, max_seqlen_q, ncol, keep_rows=True)
+    return native.fused_topk(q, km, cu_seqlens_q, cu_seqlens_k, cu_seqlens_km, int(max_seqlen_q), int(max_seqlen_k),
+                             int(moba_topk), int(moba_chunk_size), bool(causal))
 
 
 @torch.library.register_fake("flash_moba::_moba_fused_topk")
@@ -119,11 +125,7 @@ def _flash_moba_attn_varlen_forward(
     seqused_k: Optional[torch.Tensor] = None,
     zero_tensors: bool = False,
 ) -> Tuple[torch.Tensor, torch.Tensor, torch.Tensor, torch.Tensor]:
-    _reject_unsupported(dropout_p, softcap, alibi_slopes)
-    if lg_block_n % 64 != 0:
-        raise RuntimeError("lg_block_n must be divisible by 64")
-    if lg_block_m % 64 != 0 or not (128 <= lg_block_m <= 1024):
-        raise RuntimeError("lg_block_m must be divisible by 64 and within [128, 1024]")
+    _check_attention_arguments(lg_block_m, lg_block_n, dropout_p, softcap, alibi_slopes)
     q, k, v = [_fix_last_stride(x) for x in (q, k, v)]
     out, lse = ops.attn_fwd(q, k, v, moba_col_offsets.contiguous(), moba_col_nnz.contiguous(),
                             moba_row_indices.contiguous(), cu_seqlens_q, cu_seqlens_k, max_seqlen_q,
@@ -191,15 +193,11 @@ def _flash_moba_attn_varlen_backward_fake(dout, q, k, v, out, softmax_lse, dq, d
     return torch.empty((heads, total_q), device=q.device, dtype=torch.float32)
 
 
-def _op(name: str):
-    """The callable behind one of the four custom ops.  Eager callers run the op's plain Python
-    body: the dispatcher's per-call work (schema checks, aliasing checks of every output) costs
-    about 0.1 ms per op on the host, a third of the whole step's enqueue time at 4 heads per GPU.
-    Under torch.compile the registered op is used, so that traced graphs hold `flash_moba::` nodes
-    as they do with the reference."""
-    if torch.compiler.is_compiling():
-        return getattr(torch.ops.flash_moba, name)
-    return globals()[name]._init_fn
+def _compiling() -> bool:
+    """Eager callers run the native host path (csrc/fmb_torch.cpp) from end to end.  Under
+    torch.compile the registered ops are used, so that traced graphs hold `flash_moba::` nodes as
+    they do with the reference."""
+    return torch.compiler.is_compiling()
 
 
 def _attention_head_dim(d: int) -> int:
@@ -216,6 +214,9 @@ def _attention_head_dim(d: int) -> int:
 # autograd
 # ======================================================================================
 class FlashMobaAttnVarlenFunc(torch.autograd.Function):
+    """The autograd node in terms of the registered ops, for traced graphs; eager calls are recorded by
+    its native counterpart (MobaAttention in csrc/fmb_torch.cpp)."""
+
     @staticmethod
     def forward(ctx, q, k, v, cu_seqlens_q, cu_seqlens_k, max_seqlen_q, max_seqlen_k, moba_col_offsets,
                 moba_col_nnz, moba_row_indices, lg_block_m, lg_block_n, dropout_p, softmax_scale, causal, softcap,
@@ -228,7 +229,7 @@ class FlashMobaAttnVarlenFunc(torch.autograd.Function):
         if d_pad != d_og:      # zero columns change neither the scores nor the first d_og outputs
             pad = [0, d_pad - d_og]
             q, k, v = (torch.nn.functional.pad(x, pad) for x in (q, k, v))
-        out_padded, lse, s_dmask, rng_state = _op("_flash_moba_attn_varlen_forward")(
+        out_padded, lse, s_dmask, rng_state = torch.ops.flash_moba._flash_moba_attn_varlen_forward(
             q, k, v, cu_seqlens_q, cu_seqlens_k, max_seqlen_q, max_seqlen_k, moba_col_offsets, moba_col_nnz,
             moba_row_indices, lg_block_m, lg_block_n, dropout_p, softmax_scale, causal=causal, softcap=softcap,
             alibi_slopes=alibi_slopes, return_softmax=return_softmax and dropout_p > 0)
@@ -251,7 +252,7 @@ class FlashMobaAttnVarlenFunc(torch.autograd.Function):
         d_og = dout.size(2)
         dout_padded = dout if q.size(2) == d_og else torch.nn.functional.pad(dout, [0, q.size(2) - d_og])
         ops.offer_lists(getattr(ctx, "lists", None))
-        _op("_flash_moba_attn_varlen_backward")(
+        torch.ops.flash_moba._flash_moba_attn_varlen_backward(
             dout_padded, q, k, v, out, lse, dq, dk, dv, cu_seqlens_q, cu_seqlens_k, max_seqlen_q, max_seqlen_k,
             col_offsets, col_nnz, row_indices, lg_block_m, lg_block_n, dropout_p, softmax_scale, causal, softcap,
             alibi_slopes, deterministic, rng_state=rng_state)
@@ -281,13 +282,16 @@ def flash_topk_varlen_func(q, k, cu_seqlens_q, cu_seqlens_k, max_seqlen_q, max_s
 
     q: (total_q, nheads, d); k: (total_k, nheads_k, d); cu_seqlens_*: int32 (batch+1,).
     Note the argument order (top-k, then chunk size), as in the reference."""
+    if not _compiling():
+        return native.topk_varlen(q, k, cu_seqlens_q, cu_seqlens_k, int(max_seqlen_q), int(max_seqlen_k), int(moba_topk),
+                                  int(moba_chunk_size), bool(causal))
     d_og = q.size(2)
     d_pad = _attention_head_dim(d_og)      # zero columns change no score; 64 / 128 / 256 run on tensor cores
     if d_pad != d_og:
         pad = [0, d_pad - d_og]
         q, k = torch.nn.functional.pad(q, pad), torch.nn.functional.pad(k, pad)
     km, cu_seqlens_km = ops.mean_pool(_fix_last_stride(k), cu_seqlens_k, max_seqlen_k, moba_chunk_size)
-    return _op("_moba_fused_topk")(q, km, cu_seqlens_q, cu_seqlens_k, cu_seqlens_km, max_seqlen_q,
+    return torch.ops.flash_moba._moba_fused_topk(q, km, cu_seqlens_q, cu_seqlens_k, cu_seqlens_km, max_seqlen_q,
                                                  max_seqlen_k, moba_topk, moba_chunk_size, causal=causal)
 
 
@@ -299,6 +303,12 @@ def flash_moba_attn_varlen_func(q, k, v, cu_seqlens_q, cu_seqlens_k, max_seqlen_
     heads, bottom-right aligned causal mask).  `lg_block_n` is the key chunk size of the
     pattern.  Returns out (total_q, nheads, d), or (out, softmax_lse (nheads, total_q), S_dmask)
     when `return_attn_probs`.  Rows that see no key produce zeros."""
+    if not _compiling():
+        _check_attention_arguments(lg_block_m, lg_block_n, dropout_p, softcap, alibi_slopes)
+        out, lse = native.attn_varlen(q, k, v, cu_seqlens_q, cu_seqlens_k, int(max_seqlen_q), int(max_seqlen_k),
+                                      moba_col_offsets, moba_col_nnz, moba_row_indices, int(lg_block_n), softmax_scale,
+                                      bool(causal))
+        return (out, lse, torch.empty((0,), dtype=q.dtype, device=q.device)) if return_attn_probs else out
     return FlashMobaAttnVarlenFunc.apply(q, k, v, cu_seqlens_q, cu_seqlens_k, max_seqlen_q, max_seqlen_k,
                                          moba_col_offsets, moba_col_nnz, moba_row_indices, lg_block_m, lg_block_n,
                                          dropout_p, softmax_scale, causal, softcap, alibi_slopes, deterministic,
@@ -308,6 +318,11 @@ def flash_moba_attn_varlen_func(q, k, v, cu_seqlens_q, cu_seqlens_k, max_seqlen_
 def flash_moba_varlen_func(q, k, v, cu_seqlens_q, cu_seqlens_k, max_seqlen_q, max_seqlen_k, moba_chunk_size,
                            moba_topk, causal=True):
     """End-to-end MoBA attention: gating pattern, then block-sparse attention with it."""
+    if not _compiling():
+        if moba_chunk_size % 64 != 0:
+            raise RuntimeError("lg_block_n must be divisible by 64")
+        return native.moba_varlen(q, k, v, cu_seqlens_q, cu_seqlens_k, int(max_seqlen_q), int(max_seqlen_k),
+                                  int(moba_chunk_size), int(moba_topk), bool(causal))
     col_offsets, col_nnz, indices = flash_topk_varlen_func(q, k, cu_seqlens_q, cu_seqlens_k, max_seqlen_q,
                                                            max_seqlen_k, moba_topk, moba_chunk_size, causal=causal)
     lg_block_m = decide_lg_block_m(moba_topk, moba_chunk_size, max_seqlen_k, causal)

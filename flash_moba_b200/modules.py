@@ -18,6 +18,7 @@ import torch
 from torch import nn
 
 from . import ops
+from ._lib import native
 from .interface import decide_lg_block_m, flash_moba_attn_varlen_func, flash_moba_varlen_func
 
 
@@ -112,6 +113,9 @@ class CentroidCache:
 
     def attend(self, q, k, v, cu_seqlens_q, cu_seqlens_k, max_seqlen_q: int, max_seqlen_k: int, topk: int):
         """Gating against the cache, then block-sparse attention: the decode step."""
+        if not torch.compiler.is_compiling():
+            return native.moba_cached(q, k, v, self.km, self.cu_seqlens_km, cu_seqlens_q, cu_seqlens_k, int(max_seqlen_q),
+                                      int(max_seqlen_k), int(topk), self.chunk)
         pattern = self.pattern(q, cu_seqlens_q, cu_seqlens_k, max_seqlen_q, max_seqlen_k, topk)
         lg_m = decide_lg_block_m(topk, self.chunk, max_seqlen_k, True)
         return flash_moba_attn_varlen_func(q, k, v, cu_seqlens_q, cu_seqlens_k, max_seqlen_q, max_seqlen_k, *pattern,
