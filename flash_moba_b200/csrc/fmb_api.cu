@@ -365,6 +365,46 @@ int fmb_attn_key_spans(const int32_t* k_begin, const int32_t* k_end) {
   return FMB_OK;
 }
 
+int fmb_decode_preferred(int64_t total_q, int64_t total_k, int batch, int heads, int heads_k, int head_dim,
+                         int max_seqlen_k, int topk, int chunk) {
+  if (g_engine != 1 || total_q <= 0 || batch <= 0 || heads <= 0 || heads_k <= 0 || heads % heads_k != 0 || topk < 1 ||
+      chunk <= 0 || chunk % 64 != 0 || head_dim <= 0 || max_seqlen_k <= 0)
+    return 0;
+  return decode_preferred(total_q, total_k, batch, heads, heads_k, head_dim, max_seqlen_k, topk, chunk) ? 1 : 0;
+}
+
+int fmb_decode_fwd(const void* q, int64_t q_row_stride, int64_t q_head_stride, const void* k, int64_t k_row_stride,
+                   int64_t k_head_stride, const void* v, int64_t v_row_stride, int64_t v_head_stride, const void* km,
+                   void* out, int64_t o_row_stride, int64_t o_head_stride, const int32_t* cu_seqlens_q,
+                   const int32_t* cu_seqlens_k, const int32_t* cu_seqlens_km, int batch, int heads, int heads_k,
+                   int head_dim, int64_t total_q, int max_seqlen_k, int topk, int chunk, float softmax_scale, int causal,
+                   int dtype, fmb_stream_t stream) {
+  int rc = check_common("decode_fwd", heads, heads_k, head_dim, dtype);
+  if (rc) return rc;
+  FMB_CHECK_ARG(topk >= 1 && topk <= 64, "decode_fwd: moba_topk must be in [1, 64], got %d", topk);
+  FMB_CHECK_ARG(chunk > 0 && chunk % 64 == 0, "decode_fwd: chunk must be a multiple of 64, got %d", chunk);
+  FMB_CHECK_ARG(batch >= 0 && total_q >= 0 && max_seqlen_k >= 0, "decode_fwd: bad sizes");
+  FMB_CHECK_ARG(cu_seqlens_q && cu_seqlens_k && cu_seqlens_km, "decode_fwd: null cu_seqlens");
+  if (batch == 0 || total_q == 0) return FMB_OK;
+  FMB_CHECK_ARG(decode_supported(total_q, heads, heads_k, head_dim, max_seqlen_k, topk, chunk),
+                "decode_fwd: too many rows, heads or chunks for the row-major kernel");
+  if ((rc = check_tensor("decode_fwd: q", q, q_row_stride, q_head_stride, head_dim))) return rc;
+  if ((rc = check_tensor("decode_fwd: out", out, o_row_stride, o_head_stride, head_dim))) return rc;
+  if (max_seqlen_k > 0) {
+    if ((rc = check_tensor("decode_fwd: k", k, k_row_stride, k_head_stride, head_dim))) return rc;
+    if ((rc = check_tensor("decode_fwd: v", v, v_row_stride, v_head_stride, head_dim))) return rc;
+    FMB_CHECK_ARG(km && aligned16(km), "decode_fwd: km must be non-null and 16-byte aligned");
+  }
+  DecodeArgs a;
+  a.q = q; a.k = k; a.v = v; a.km = km; a.o = out;
+  a.q_rs = q_row_stride; a.q_hs = q_head_stride; a.k_rs = k_row_stride; a.k_hs = k_head_stride;
+  a.v_rs = v_row_stride; a.v_hs = v_head_stride; a.o_rs = o_row_stride; a.o_hs = o_head_stride;
+  a.cu_q = cu_seqlens_q; a.cu_k = cu_seqlens_k; a.cu_km = cu_seqlens_km;
+  a.batch = batch; a.heads = heads; a.heads_k = heads_k; a.d = head_dim; a.total_q = total_q; a.max_k = max_seqlen_k;
+  a.topk = topk; a.chunk = chunk; a.scale = softmax_scale; a.causal = causal; a.dtype = dtype;
+  return launch_decode(a, (cudaStream_t)stream);
+}
+
 int fmb_attn_fwd(const void* q, int64_t q_row_stride, int64_t q_head_stride, const void* k,
                  int64_t k_row_stride, int64_t k_head_stride, const void* v, int64_t v_row_stride,
                  int64_t v_head_stride, void* out, int64_t o_row_stride, int64_t o_head_stride, float* lse,

@@ -115,6 +115,17 @@ struct GateArgs {
 };
 int launch_gate_topk(const GateArgs& a, cudaStream_t s);
 void set_gate_engine(int e);
+
+struct DecodeArgs {
+  const void *q, *k, *v, *km; void* o;
+  int64_t q_rs, q_hs, k_rs, k_hs, v_rs, v_hs, o_rs, o_hs;
+  const int32_t *cu_q, *cu_k, *cu_km;
+  int batch, heads, heads_k, d; int64_t total_q; int max_k, topk, chunk;
+  float scale; int causal, dtype;
+};
+bool decode_supported(int64_t total_q, int heads, int heads_k, int d, int max_k, int topk, int chunk);
+bool decode_preferred(int64_t total_q, int64_t total_k, int batch, int heads, int heads_k, int d, int max_k, int topk, int chunk);
+int launch_decode(const DecodeArgs& a, cudaStream_t s);
 bool gate_tc_supported(int d, int topk);
 int read_gate_status(int* out);
 

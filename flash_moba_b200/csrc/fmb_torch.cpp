@@ -516,6 +516,37 @@ Pattern moba_pattern(const Tensor& q0, const Tensor& k0, const Tensor& cu_q, con
   return pattern_from_centroids(q, km, cu_q, cu_k, cu_km, max_q, max_k, topk, chunk, causal);
 }
 
+// A call with few query rows and no gradients to record: one launch for gating and attention
+// (fmb_decode_fwd); undefined where the general path is to run.
+Tensor try_decode(const Tensor& q0, const Tensor& k0, const Tensor& v0, const OptTensor& km0, const OptTensor& cu_km0,
+                  const Tensor& cu_q, const Tensor& cu_k, int64_t max_k, int64_t topk, int64_t chunk, bool causal) {
+  if (at::GradMode::is_enabled() && (q0.requires_grad() || k0.requires_grad() || v0.requires_grad())) return {};
+  if (q0.dim() != 3 || k0.dim() != 3 || v0.dim() != 3 || q0.size(2) % 8 != 0) return {};
+  const int64_t total_q = q0.size(0), h = q0.size(1), d = q0.size(2), hk = k0.size(1), batch = cu_q.numel() - 1;
+  if (!fmb_decode_preferred(total_q, k0.size(0), (int)batch, (int)h, (int)hk, (int)d, (int)max_k, (int)topk, (int)chunk)) return {};
+  at::NoGradGuard no_grad;
+  Tensor q = fix_last_stride(q0), k = fix_last_stride(k0), v = fix_last_stride(v0), km, cu_km;
+  for (const Tensor* t : {(const Tensor*)&q, (const Tensor*)&k, (const Tensor*)&v, &cu_q, &cu_k}) require_cuda(*t);
+  TORCH_CHECK(q.scalar_type() == k.scalar_type() && k.scalar_type() == v.scalar_type(),
+              "query, key and value must have the same dtype");
+  if (km0) {
+    km = km0->contiguous();
+    cu_km = *cu_km0;
+    TORCH_CHECK(km.dim() == 3 && km.size(1) == hk && km.size(2) == d && km.scalar_type() == q.scalar_type(),
+                "the centroids must have the keys' heads, head_dim and dtype");
+  } else {
+    std::tie(km, cu_km) = mean_pool(k, cu_k, max_k, chunk);
+  }
+  c10::cuda::CUDAGuard guard(q.device());
+  Tensor out = at::empty_like(q);
+  check(fmb_decode_fwd(q.data_ptr(), q.stride(0), q.stride(1), k.data_ptr(), k.stride(0), k.stride(1), v.data_ptr(), v.stride(0),
+                       v.stride(1), km.data_ptr(), out.data_ptr(), out.stride(0), out.stride(1), i32c(cu_q, "cu_seqlens_q"),
+                       i32c(cu_k, "cu_seqlens_k"), i32c(cu_km, "cu_seqlens_km"), (int)batch, (int)h, (int)hk, (int)d, total_q,
+                       (int)max_k, (int)topk, (int)chunk, (float)(1.0 / std::sqrt((double)d)), causal ? 1 : 0, dtype_code(q),
+                       current_stream()));
+  return out;
+}
+
 using Triple = std::tuple<Tensor, Tensor, Tensor>;
 Triple shown(const Pattern& p) {
   remember(p);
@@ -542,11 +573,13 @@ std::tuple<Tensor, Tensor> py_attn_varlen(const Tensor& q, const Tensor& k, cons
 }
 Tensor py_moba_varlen(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& cu_q, const Tensor& cu_k, int64_t max_q,
                       int64_t max_k, int64_t chunk, int64_t topk, bool causal) {
+  if (Tensor out = try_decode(q, k, v, {}, {}, cu_q, cu_k, max_k, topk, chunk, causal); out.defined()) return out;
   Pattern p = moba_pattern(q, k, cu_q, cu_k, max_q, max_k, topk, chunk, causal);
   return std::get<0>(attention(q, k, v, std::move(p), cu_q, cu_k, max_q, max_k, chunk, std::nullopt, causal));
 }
 Tensor py_moba_cached(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& km, const Tensor& cu_km, const Tensor& cu_q,
                       const Tensor& cu_k, int64_t max_q, int64_t max_k, int64_t topk, int64_t chunk) {
+  if (Tensor out = try_decode(q, k, v, km, cu_km, cu_q, cu_k, max_k, topk, chunk, true); out.defined()) return out;
   Pattern p;
   {
     at::NoGradGuard no_grad;

@@ -186,6 +186,28 @@ size_t fmb_attn_bwd_workspace_bytes(int64_t total_q, int heads, int heads_k, int
                                     int64_t n_indices, int batch, int max_seqlen_k, int chunk,
                                     int heads_per_pass);
 
+/* ------------------------------------------------- few query rows: gating + attention in one launch
+ * out[row,h] as fmb_attn_fwd gives it for the pattern that fmb_gate_topk + fmb_build_csc would build
+ * from the same centroids, without building one: for decoding and short blocks of new rows, where
+ * the columns of the pattern hold a row or two each.  The same selection rule; fp32 throughout (no
+ * rounding of the probabilities or of partial results), so results agree with fmb_attn_fwd's to the
+ * latter's rounding.  km: (km_rows, heads_k, head_dim) contiguous, sequence b's centroids from row
+ * cu_seqlens_km[b] on.  No gradients (no log-sum-exp is written).  head_dim: any multiple of 8 up to
+ * 256; chunk: a multiple of 64; topk <= 64.
+ *
+ * fmb_decode_preferred: 1 where this entry point serves the shape and is the faster one (a rule on
+ * the sizes the host knows: total_q rows against total_k keys in `batch` sequences), else 0. */
+int fmb_decode_preferred(int64_t total_q, int64_t total_k, int batch, int heads, int heads_k,
+                         int head_dim, int max_seqlen_k, int topk, int chunk);
+int fmb_decode_fwd(const void* q, int64_t q_row_stride, int64_t q_head_stride,
+                   const void* k, int64_t k_row_stride, int64_t k_head_stride,
+                   const void* v, int64_t v_row_stride, int64_t v_head_stride, const void* km,
+                   void* out, int64_t o_row_stride, int64_t o_head_stride,
+                   const int32_t* cu_seqlens_q, const int32_t* cu_seqlens_k,
+                   const int32_t* cu_seqlens_km, int batch, int heads, int heads_k, int head_dim,
+                   int64_t total_q, int max_seqlen_k, int topk, int chunk, float softmax_scale,
+                   int causal, int dtype, fmb_stream_t stream);
+
 /* out[row,h] = softmax over the visible keys (scale * q.k) . v, where key col of the row's
  * sequence is visible iff chunk col/chunk is in the row's pattern, col < len_k and, if
  * causal, col <= row + len_k - len_q.  lse float (heads, total_q) = log-sum-exp of the
