@@ -55,6 +55,8 @@ _SIGS = {
     "fmb_mean_pool_offsets": (i32, [c_ptr, i64, i64, c_ptr, c_ptr, c_ptr, i32, i32, i32, i32, i32, i32, c_ptr]),
     "fmb_gate_topk": (i32, [c_ptr, i64, i64, c_ptr, c_ptr, c_ptr, c_ptr, c_ptr, c_ptr, i64, i64,
                             i32, i32, i32, i32, i32, i32, i32, i32, i32, i32, c_ptr]),
+    "fmb_gate_topk_sized": (i32, [c_ptr, i64, i64, i64, c_ptr, i64, c_ptr, c_ptr, c_ptr, c_ptr, c_ptr, i64, i64,
+                                  i32, i32, i32, i32, i32, i32, i32, i32, i32, i32, c_ptr]),
     "fmb_build_csc_workspace_bytes": (sz, [i32, i32, i32, i32]),
     "fmb_build_csc": (i32, [c_ptr, i64, i64, c_ptr, c_ptr, c_ptr, c_ptr, c_ptr, sz, i32, i32, i32, i32, i32, c_ptr]),
     "fmb_build_csc_rows": (i32, [c_ptr, i64, i64, c_ptr, c_ptr, c_ptr, c_ptr, c_ptr, c_ptr, sz, i32, i32, i32, i64, i32, i32,

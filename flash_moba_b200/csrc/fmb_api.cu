@@ -208,11 +208,11 @@ int fmb_mean_pool_offsets(const void* k, int64_t k_row_stride, int64_t k_head_st
                           max_seqlen_k, chunk, dtype, (cudaStream_t)stream, true);
 }
 
-int fmb_gate_topk(const void* q, int64_t q_row_stride, int64_t q_head_stride, const void* km,
-                  const int32_t* cu_seqlens_q, const int32_t* cu_seqlens_k, const int32_t* cu_seqlens_km,
-                  int32_t* topk_idx, float* topk_val, int64_t topk_row_stride, int64_t topk_head_stride,
-                  int batch, int heads, int heads_k, int head_dim, int max_seqlen_q, int max_seqlen_k,
-                  int topk, int chunk, int causal, int dtype, fmb_stream_t stream) {
+int fmb_gate_topk_sized(const void* q, int64_t q_row_stride, int64_t q_head_stride, int64_t total_q, const void* km,
+                        int64_t km_rows, const int32_t* cu_seqlens_q, const int32_t* cu_seqlens_k,
+                        const int32_t* cu_seqlens_km, int32_t* topk_idx, float* topk_val, int64_t topk_row_stride,
+                        int64_t topk_head_stride, int batch, int heads, int heads_k, int head_dim, int max_seqlen_q,
+                        int max_seqlen_k, int topk, int chunk, int causal, int dtype, fmb_stream_t stream) {
   int rc = check_common("gate_topk", heads, heads_k, head_dim, dtype);
   if (rc) return rc;
   FMB_CHECK_ARG(topk >= 1 && topk <= 64, "gate_topk: moba_topk must be in [1, 64], got %d", topk);
@@ -229,7 +229,18 @@ int fmb_gate_topk(const void* q, int64_t q_row_stride, int64_t q_head_stride, co
   a.topk_idx = topk_idx; a.topk_val = topk_val; a.t_rs = topk_row_stride; a.t_hs = topk_head_stride;
   a.batch = batch; a.heads = heads; a.heads_k = heads_k; a.d = head_dim; a.max_q = max_seqlen_q;
   a.max_k = max_seqlen_k; a.topk = topk; a.chunk = chunk; a.causal = causal; a.dtype = dtype;
+  a.total_q = total_q; a.km_rows = km_rows;
   return launch_gate_topk(a, (cudaStream_t)stream);
+}
+
+int fmb_gate_topk(const void* q, int64_t q_row_stride, int64_t q_head_stride, const void* km,
+                  const int32_t* cu_seqlens_q, const int32_t* cu_seqlens_k, const int32_t* cu_seqlens_km,
+                  int32_t* topk_idx, float* topk_val, int64_t topk_row_stride, int64_t topk_head_stride,
+                  int batch, int heads, int heads_k, int head_dim, int max_seqlen_q, int max_seqlen_k,
+                  int topk, int chunk, int causal, int dtype, fmb_stream_t stream) {
+  return fmb_gate_topk_sized(q, q_row_stride, q_head_stride, 0, km, 0, cu_seqlens_q, cu_seqlens_k, cu_seqlens_km, topk_idx,
+                             topk_val, topk_row_stride, topk_head_stride, batch, heads, heads_k, head_dim, max_seqlen_q,
+                             max_seqlen_k, topk, chunk, causal, dtype, stream);
 }
 
 size_t fmb_build_csc_workspace_bytes(int batch, int heads, int max_seqlen_q, int ncol) {

@@ -112,6 +112,7 @@ struct GateArgs {
   const int32_t *cu_q, *cu_k, *cu_km;
   int32_t* topk_idx; float* topk_val; int64_t t_rs, t_hs;
   int batch, heads, heads_k, d, max_q, max_k, topk, chunk, causal, dtype;
+  int64_t total_q, km_rows;      // rows of q and of km; 0: not known
 };
 int launch_gate_topk(const GateArgs& a, cudaStream_t s);
 void set_gate_engine(int e);

@@ -10,10 +10,14 @@
 //     shared memory, a warp per row, the list distributed over the lanes.
 // Ordering rule = the reference's: descending score, and on equal scores the higher chunk id
 // first (csrc/flash_topk/src/flash_topk_kernel.h:261-285).
+#include <type_traits>
+
 #include "fmb_common.cuh"
-#include "fmb_tc.cuh"
+#include "fmb_tma.cuh"
 
 namespace fmb {
+
+int sm_count();   // SMs of the current device (fmb_attn_common.cu)
 
 constexpr int kGateM = 128;          // query rows per CTA
 constexpr int kGateN = 128;          // centroids per score tile
@@ -589,6 +593,422 @@ __global__ void __launch_bounds__(128 * NQ) gate_topk_tc_kernel(GateParams p) {
   }
 }
 
+// ---------------------------------------------------------------------------------------
+// Two-sweep selection (top-k <= 16, sizes of q and km known): the kernel of the usual shapes.
+//
+// What bounds gating is the selection on the CUDA cores, not the score product: with a list kept while
+// the scores stream by (the kernel above) a thread handled some 33 insertions per row of 512
+// candidates, each a divergent loop of 40-odd instructions: 65 instructions per score.  Here the scores are
+// looked at twice instead, straight-line both times:
+//   sweep 1  only keeps maxima of groups of scores (strided groups: neighbouring chunks may score
+//            alike) and, every few tiles, merges them into a sorted list of the K largest by a sorting network.
+//            Group maxima are different candidates' scores, so the k-th largest of them is a floor no
+//            member of the row's top-k lies under; only some 9 scores of a row (k = 8) reach it;
+//   sweep 2  appends the scores that reach the floor to a short queue in shared memory (predicated
+//            stores, no branch).  A candidate's place in the list is then the number of the row's
+//            candidates ahead of it, counted by comparing all with all; the two threads of a row share
+//            the row's candidates evenly, however they were distributed over the columns.
+// The score tiles of sweep 2 are those of sweep 1, still in TMEM, for up to 256 candidates; beyond that the
+// products are computed again (the tensor pipe is idle otherwise).  A queue that runs full (masses of
+// equal scores) is cut down to its k best, the last of which then is the floor.
+// Persistent CTAs, two per SM.  Warp 8 loads Q and the centroid tiles by TMA and issues the MMAs, running
+// ahead into the next item (row tile, head, sequence) while warps 0-7 (two threads per row, alternate halves of a
+// tile's columns) are still in sweep 2: with a CTA per item, start-up and Q's way from HBM were a third of its time.
+// Measured (B200, d 128, the kernel above / this one): 64K tokens, 32 heads, chunk 128, top-k 8 1.02 / 0.65 ms;
+// 8 x 8K tokens 0.58 / 0.28 ms; 32K tokens, 16 heads 185 / 104 us; 317K tokens in 16 sequences, chunk 64, top-k 16
+// 7.4 / 3.7 ms; d 256, 16K tokens, 16 heads 141 / 59 us.  Now: 15,500 instructions per row tile and head at 61 % issue
+// (fixed-latency dependencies and the shared min / max pipe), 30 instructions per score.
+// ---------------------------------------------------------------------------------------
+constexpr int kSelN = 64;            // centroids per score tile
+constexpr int kSelBufs = 4;          // score tiles in TMEM
+constexpr int kSelRing = 2;          // centroid tiles in shared memory
+constexpr int kSelThreads = 256 + 32;
+
+// descending sorting networks on registers: 8 values in 19 compare-exchanges; 16 as two sorted eights
+// and a bitonic merge
+__device__ __forceinline__ void sel_ce(float& a, float& b) {
+  const float hi = fmaxf(a, b), lo = fminf(a, b);
+  a = hi;
+  b = lo;
+}
+__device__ __forceinline__ void sel_sort8(float* x) {
+  sel_ce(x[0], x[1]); sel_ce(x[2], x[3]); sel_ce(x[4], x[5]); sel_ce(x[6], x[7]);
+  sel_ce(x[0], x[2]); sel_ce(x[1], x[3]); sel_ce(x[4], x[6]); sel_ce(x[5], x[7]);
+  sel_ce(x[1], x[2]); sel_ce(x[5], x[6]); sel_ce(x[0], x[4]); sel_ce(x[3], x[7]);
+  sel_ce(x[1], x[5]); sel_ce(x[2], x[6]);
+  sel_ce(x[1], x[4]); sel_ce(x[3], x[6]);
+  sel_ce(x[2], x[4]); sel_ce(x[3], x[5]);
+  sel_ce(x[3], x[4]);
+}
+// x bitonic -> descending
+template <int N>
+__device__ __forceinline__ void sel_bitonic(float* x) {
+#pragma unroll
+  for (int o = N / 2; o; o >>= 1)
+#pragma unroll
+    for (int i = 0; i < N; ++i)
+      if ((i & o) == 0) sel_ce(x[i], x[i + o]);
+}
+template <int N>
+__device__ __forceinline__ void sel_sort(float* x) {
+  if constexpr (N == 8) {
+    sel_sort8(x);
+  } else {
+    static_assert(N == 16, "8 or 16");
+    sel_sort8(x);
+    sel_sort8(x + 8);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) sel_ce(x[i], x[15 - i]);
+    sel_bitonic<8>(x);
+    sel_bitonic<8>(x + 8);
+  }
+}
+
+// candidate as one number: descending score, on equal scores the higher chunk id first
+__device__ __forceinline__ uint64_t sel_key(float2 c) { return ((uint64_t)score_to_ordered(c.x) << 32) | (uint32_t)__float_as_int(c.y); }
+
+// A thread's queue (entries 64 apart) cut down to its `keep` best, in order.  Rare (see above) and long:
+// kept out of line.
+__device__ __noinline__ void sel_compact(float2* queue, int cnt, int keep) {
+  for (int i = 0; i < keep; ++i) {
+    int best = i;
+    uint64_t kb = sel_key(queue[i * 64]);
+    for (int j = i + 1; j < cnt; ++j) {
+      const uint64_t kj = sel_key(queue[j * 64]);
+      if (kj > kb) { kb = kj; best = j; }
+    }
+    const float2 x = queue[i * 64];
+    queue[i * 64] = queue[best * 64];
+    queue[best * 64] = x;
+  }
+}
+
+// n / d for 0 <= n < 2^31: one multiplication with a reciprocal from the host, rounded up, which is exact
+// for these n (d = 1 is its own case)
+struct FastDiv {
+  uint32_t mul, shift, d;
+};
+__device__ __forceinline__ int fast_div(int n, const FastDiv& f) {
+  return f.d == 1 ? n : (int)(__umulhi((uint32_t)n, f.mul) >> f.shift);
+}
+
+// Queue entries per thread: what two CTAs per SM leave room for.  A row has some 9 (k = 8) or 19 (k = 16)
+// candidates, a thread half of them on average; more than 12 or 18 in one thread's queue are rare (with room
+// for 16 the queues ran full all the time: 0.82 ms instead of 0.65 at 64K).
+template <int KMAX> __host__ __device__ constexpr int sel_cap() { return KMAX == 8 ? 20 : 22; }
+
+constexpr int kSelSeqs = 64;         // sequences whose bounds are kept in shared memory
+
+template <typename T, int D, int KMAX>
+__global__ void __launch_bounds__(kSelThreads, D <= 128 ? 2 : 1)
+gate_select_kernel(GateParams p, const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_km,
+                   int batch, int row_tiles, FastDiv by_chunk) {
+  using namespace tc;
+  constexpr uint32_t kQTile = kGateM * D * 2, kKTile = kSelN * D * 2;
+  constexpr int CAP = sel_cap<KMAX>();                   // queue entries per thread
+  constexpr int STEP = KMAX == 8 ? 8 : 4;                // scores between two looks at the queue's length
+  constexpr int OWN = KMAX == 8 ? 6 : 12;                // candidates of a row that each of its two threads ranks at a time
+  extern __shared__ unsigned char smem_raw[];
+  __shared__ uint64_t bar_q, bar_qfree, bar_kfull[kSelRing], bar_kfree[kSelRing], bar_tfull[kSelBufs], bar_tfree[kSelBufs];
+  __shared__ uint32_t tmem_base_s;
+  __shared__ int sCount[256];
+  __shared__ int sCu[3][kSelSeqs + 1];
+  unsigned char* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
+  unsigned char* sQ = smem;
+  unsigned char* sKM = sQ + kQTile;
+  unsigned char* sQueue = sKM + kSelRing * kKTile;       // per warp pair [CAP][64] (score, chunk); also the pair's exchange area
+
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int topk = p.topk;
+  const bool small_batch = batch <= kSelSeqs;
+  if (small_batch)
+    for (int i = tid; i <= batch; i += kSelThreads) { sCu[0][i] = p.cu_q[i]; sCu[1][i] = p.cu_k[i]; sCu[2][i] = p.cu_km[i]; }
+  if (warp == 0) tmem_alloc(&tmem_base_s, kSelBufs * kSelN);
+  if (tid == 0) {
+    mbar_init(&bar_q, 1);
+    mbar_init(&bar_qfree, 1);
+    for (int i = 0; i < kSelRing; ++i) { mbar_init(&bar_kfull[i], 1); mbar_init(&bar_kfree[i], 1); }
+    for (int i = 0; i < kSelBufs; ++i) { mbar_init(&bar_tfull[i], 1); mbar_init(&bar_tfree[i], 8); }
+    mbar_fence_init();
+  }
+  tc_fence_before_sync();
+  __syncthreads();
+  tc_fence_after_sync();
+  const uint32_t tmem_base = tmem_base_s;
+
+  // items: the last row tiles (most candidates under a causal mask) first, all heads and sequences of a
+  // row tile before the next, so that the CTAs running at the same time have equally long items
+  const int per_tile = p.heads * batch, n_items = row_tiles * per_tile;
+  struct Item { int h, r0, q0, rows, shift, km0, nchunks, nt; };
+  auto decode = [&](int item, Item& I) -> bool {
+    const int x = item / per_tile, y = item - x * per_tile, b = y / p.heads;
+    int len_k, km1;
+    I.h = y - b * p.heads;
+    I.r0 = (row_tiles - 1 - x) * kGateM;
+    if (small_batch) {
+      I.q0 = sCu[0][b]; I.rows = sCu[0][b + 1]; len_k = sCu[1][b + 1] - sCu[1][b]; I.km0 = sCu[2][b]; km1 = sCu[2][b + 1];
+    } else {
+      I.q0 = p.cu_q[b]; I.rows = p.cu_q[b + 1]; len_k = p.cu_k[b + 1] - p.cu_k[b]; I.km0 = p.cu_km[b]; km1 = p.cu_km[b + 1];
+    }
+    const int len_q = I.rows - I.q0;
+    I.rows = min(kGateM, len_q - I.r0);
+    if (I.rows <= 0) return false;                       // past the sequence's last row
+    I.shift = len_k - len_q;
+    I.nchunks = km1 - I.km0;
+    int n_end = I.nchunks;                               // candidates of any row of the tile: n < n_end
+    if (p.causal) {
+      const int pmax = I.r0 + I.rows - 1 + I.shift;
+      n_end = pmax < 0 ? 0 : min(I.nchunks, fast_div(pmax, by_chunk));
+    }
+    I.nt = (n_end + kSelN - 1) / kSelN;
+    return true;
+  };
+
+  if (warp == 8) {
+    // =============================================================== loads and MMAs
+    if (lane == 0) {
+      constexpr uint32_t idesc = make_idesc(FmtOf<T>::v, kGateM, kSelN, 0, 0);
+      const uint32_t hi = desc_hi_sw128(1024), q_km = desc_lo_sw128(smem_u32(sQ), 16);
+      const int group = p.heads / p.heads_k;
+      uint32_t gs = 0, qn = 0;                           // steps and items with candidates so far
+      bool ok = true;
+#pragma unroll 1
+      for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
+        Item I;
+        if (!decode(item, I) || I.nt == 0) continue;
+        const int nt = I.nt, steps = nt <= kSelBufs ? nt : 2 * nt, hk = I.h / group;
+        auto load_km = [&](int s) {                      // centroid tile of step s into its ring slot
+          const uint32_t n = gs + s, slot = n % kSelRing;
+          if (n >= kSelRing) ok = ok && mbar_wait(&bar_kfree[slot], (n / kSelRing - 1) & 1, &g_gate_status, 2);
+          if (!ok) return;
+          const int row = I.km0 + (s < nt ? s : s - nt) * kSelN;
+          mbar_expect_tx(&bar_kfull[slot], kKTile);
+#pragma unroll
+          for (int hb = 0; hb < D / 64; ++hb)
+            tma_load_3d(sKM + slot * kKTile + hb * (kSelN * 128), &map_km, hb * 64, hk, row, &bar_kfull[slot]);
+        };
+        if (qn > 0) ok = mbar_wait(&bar_qfree, (qn - 1) & 1, &g_gate_status, 2);   // the last item's MMAs have read Q
+        if (!ok) break;
+        mbar_expect_tx(&bar_q, kQTile);
+#pragma unroll
+        for (int hb = 0; hb < D / 64; ++hb) tma_load_3d(sQ + hb * (kGateM * 128), &map_q, hb * 64, I.h, I.q0 + I.r0, &bar_q);
+        load_km(0);
+        if (steps > 1) load_km(1);
+        ok = ok && mbar_wait(&bar_q, qn & 1, &g_gate_status, 2);
+#pragma unroll 1
+        for (int s = 0; s < steps && ok; ++s) {
+          const uint32_t n = gs + s, slot = n % kSelRing, buf = n % kSelBufs;
+          ok = mbar_wait(&bar_kfull[slot], (n / kSelRing) & 1, &g_gate_status, 2);
+          if (ok && n >= kSelBufs) ok = mbar_wait(&bar_tfree[buf], (n / kSelBufs - 1) & 1, &g_gate_status, 2);
+          if (!ok) break;
+          tc_fence_after_sync();
+          umma_gemm<D / 16>(tmem_base + buf * kSelN, q_km, hi, 2, (kGateM * 128) >> 4,
+                            desc_lo_sw128(smem_u32(sKM) + slot * kKTile, 16), hi, 2, (kSelN * 128) >> 4, idesc, 0);
+          umma_commit(&bar_tfull[buf]);
+          umma_commit(&bar_kfree[slot]);
+          if (s >= 1 && s + 1 < steps) load_km(s + 1);   // into the slot of the step before this one
+        }
+        umma_commit(&bar_qfree);
+        gs += steps;
+        ++qn;
+      }
+    }
+  } else {
+    // =============================================================== selection
+    const int lt = tid & 127, qd = (tid >> 7) & 1;       // row, and which half of a tile's columns
+    const int pair = 1 + (warp & 3);                     // barrier of warps w and w + 4, which hold the same rows
+    const uint32_t lane_sel = (uint32_t)((warp & 3) * 32) << 16;
+    unsigned char* mine = sQueue + (warp & 3) * (CAP * 64 * 8);   // the pair's own part of the area
+    float2* queue = reinterpret_cast<float2*>(mine) + qd * 32 + lane;
+    bool good = true;
+    uint32_t gs = 0;
+#pragma unroll 1
+    for (int item = blockIdx.x; item < n_items && good; item += gridDim.x) {
+      Item I;
+      if (!decode(item, I)) continue;
+      const int nt = I.nt;
+      const bool resident = nt <= kSelBufs;              // sweep 2 finds every score tile where sweep 1 left it
+      const int pos = I.r0 + lt + I.shift;
+      const bool row_ok = lt < I.rows;
+      int nlim = I.nchunks;                              // candidate chunks of the row: n < nlim
+      const int pos_chunk = pos < 0 ? 0 : fast_div(pos, by_chunk);
+      if (p.causal) nlim = min(I.nchunks, pos_chunk);
+      if (!row_ok) nlim = 0;
+      const bool own = p.causal && row_ok && pos >= 0 && I.nchunks > 0;
+      const int need = topk - (own ? 1 : 0);
+      const int nlim_warp = __reduce_max_sync(0xffffffffu, nlim);
+
+      // this thread's 32 scores of score tile s; columns at or past the row's limit read as -inf
+      auto fetch = [&](uint32_t n, int s, bool wait, bool release, float (&v)[32]) {
+        const int buf = n % kSelBufs;
+        if (wait && good) good = mbar_wait(&bar_tfull[buf], (n / kSelBufs) & 1, &g_gate_status, 1);
+        good = __all_sync(0xffffffffu, good);
+        tc_fence_after_sync();
+        tmem_ld16(tmem_base + buf * kSelN + qd * 16 + lane_sel, v);          // columns 0-15 and 32-47, or 16-31 and 48-63
+        tmem_ld16(tmem_base + buf * kSelN + 32 + qd * 16 + lane_sel, v + 16);
+        tmem_ld_wait();
+        if (release) {
+          tc_fence_before_sync();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&bar_tfree[buf]);
+        }
+        const int left = nlim - (s * kSelN + qd * 16);
+        if (__any_sync(0xffffffffu, left < 48)) {
+#pragma unroll
+          for (int j = 0; j < 32; ++j) v[j] = j + (j & 16) < left ? v[j] : -CUDART_INF_F;
+        }
+      };
+      // ---- sweep 1: the KMAX largest group maxima of this thread's columns
+      float top[KMAX];
+      {
+        float gm[KMAX];
+        const int period = max(1, nt / 2);
+        int since = 0;
+#pragma unroll
+        for (int j = 0; j < KMAX; ++j) { top[j] = -CUDART_INF_F; gm[j] = -CUDART_INF_F; }
+#pragma unroll 1
+        for (int s = 0; s < nt; ++s) {
+          float v[32];
+          fetch(gs + s, s, true, !resident, v);
+#pragma unroll
+          for (int j = 0; j < 32; ++j) gm[j % KMAX] = fmaxf(gm[j % KMAX], v[j]);   // (fmaxf drops NaN operands)
+          if (++since == period || s + 1 == nt) {
+            since = 0;
+            sel_sort<KMAX>(gm);
+#pragma unroll
+            for (int j = 0; j < KMAX; ++j) top[j] = fmaxf(top[j], gm[KMAX - 1 - j]);
+            sel_bitonic<KMAX>(top);
+#pragma unroll
+            for (int j = 0; j < KMAX; ++j) gm[j] = -CUDART_INF_F;
+          }
+        }
+      }
+      // floor: the need-th largest of the two threads' lists together (both sorted: min over i of
+      // max(a[i], b[need - 1 - i]))
+      float thr = CUDART_INF_F;
+      {
+        float* sX = reinterpret_cast<float*>(mine);
+#pragma unroll
+        for (int j = 0; j < KMAX; ++j) sX[(qd * KMAX + j) * 32 + lane] = top[j];
+        bar_sync(pair, 64);
+#pragma unroll
+        for (int j = 0; j < KMAX; ++j)
+          if (j < need) thr = fminf(thr, fmaxf(top[j], sX[((qd ^ 1) * KMAX + need - 1 - j) * 32 + lane]));
+        thr = fmaxf(thr, -3.402823466e38f);              // a score of -inf is no candidate
+        bar_sync(pair, 64);                              // both have read before the queue is written
+      }
+
+      // ---- sweep 2
+      const uint32_t q_first = smem_u32(queue);
+      uint32_t q_next = q_first;                         // where the next candidate goes
+#pragma unroll 1
+      for (int s = 0; s < nt; ++s) {
+        float v[32];
+        fetch(resident ? gs + s : gs + nt + s, s, !resident, true, v);
+        const int nb = s * kSelN + qd * 16;
+#pragma unroll
+        for (int js = 0; js < 32; js += STEP) {
+          if (nb + js + (js & 16) >= nlim_warp) break;   // warp-uniform
+          if (__any_sync(0xffffffffu, q_next > q_first + (CAP - STEP) * 512)) {
+            const int cnt = (q_next - q_first) / 512;
+            if (cnt > need) {
+              sel_compact(queue, cnt, need);
+              q_next = q_first + need * 512;
+              if (need > 0) thr = fmaxf(thr, queue[(need - 1) * 64].x);
+            }
+            __syncwarp();
+          }
+#pragma unroll
+          for (int j = js; j < js + STEP; ++j)
+            asm volatile(
+                "{\n\t.reg .pred p;\n\t"
+                "setp.ge.f32 p, %1, %2;\n\t"
+                "@p st.shared.v2.b32 [%0], {%3, %4};\n\t"
+                "@p add.u32 %0, %0, 512;\n\t}"
+                : "+r"(q_next)
+                : "f"(v[j]), "f"(thr), "r"(__float_as_uint(v[j])), "r"(nb + j + (j & 16))
+                : "memory");
+        }
+      }
+      gs += resident ? nt : 2 * nt;
+      const int cnt = (q_next - q_first) / 512;
+      sCount[tid] = cnt;
+      bar_sync(pair, 64);                                // both queues are complete
+      {
+        // ---- ranks: this thread takes every second one of the row's candidates
+        const int other = sCount[tid ^ 128];
+        const float2* q_lo = reinterpret_cast<const float2*>(mine) + lane;
+        const int c0 = qd == 0 ? cnt : other, c = cnt + other;
+        const int most = __reduce_max_sync(0xffffffffu, c);      // (the same for both warps of the pair)
+        const bool staged = most <= 2 * OWN && p.t_rs == topk;   // one round, and the pair's lists are contiguous in memory
+        int* sOut = reinterpret_cast<int*>(mine) + lane * topk;
+        const int64_t row_at = (int64_t)(I.q0 + I.r0 + lt) * p.t_rs + (int64_t)I.h * p.t_hs;
+        int* out = staged ? sOut : p.topk_idx + row_at;
+        float* val = p.topk_val ? p.topk_val + row_at : nullptr;
+#pragma unroll 1
+        for (int first = qd; first < most; first += 2 * OWN) {
+          uint64_t key[OWN];
+          int rank[OWN];
+#pragma unroll
+          for (int m = 0; m < OWN; ++m) {
+            const int i = first + 2 * m;
+            rank[m] = topk;
+            key[m] = ~0ull;
+            if (i < c) {
+              key[m] = sel_key(q_lo[i < c0 ? i * 64 : (i - c0) * 64 + 32]);
+              rank[m] = own ? 1 : 0;
+            }
+          }
+          const float2* at = q_lo;
+          for (int i = 0; i < most; ++i) {
+            if (i == c0) at = q_lo + 32;
+            const uint64_t k = i < c ? sel_key(*at) : 0ull;
+            at += 64;
+#pragma unroll
+            for (int m = 0; m < OWN; ++m) rank[m] += k > key[m] ? 1 : 0;
+          }
+          if (staged) bar_sync(pair, 64);                // both have read the queues: their place takes the lists
+#pragma unroll
+          for (int m = 0; m < OWN; ++m) {
+            if (rank[m] < topk) {
+              out[rank[m]] = (int)(uint32_t)key[m];
+              if (val) val[rank[m]] = ordered_to_score((uint32_t)(key[m] >> 32));
+            }
+          }
+        }
+        if (staged && qd >= most) bar_sync(pair, 64);    // (most is 0, or 1 for the second thread: no round above)
+        if (qd == 0 && row_ok) {                         // the row's own chunk first, nothing after the last candidate
+          if (own) {
+            out[0] = pos_chunk;
+            if (val) val[0] = CUDART_INF_F;
+          }
+          for (int j = c + (own ? 1 : 0); j < topk; ++j) {
+            out[j] = -1;
+            if (val) val[j] = -CUDART_INF_F;
+          }
+        }
+        if (staged) {
+          bar_sync(pair, 64);                            // the pair's 32 lists are complete
+          const int first = (warp & 3) * 32, n_out = max(0, min(32, I.rows - first)) * topk;
+          int32_t* dst = p.topk_idx + (int64_t)(I.q0 + I.r0 + first) * p.t_rs + (int64_t)I.h * p.t_hs;
+          const int* src = reinterpret_cast<const int*>(mine);
+          if ((topk & 3) == 0 && (reinterpret_cast<uintptr_t>(dst) & 15) == 0) {
+            for (int i = qd * 32 + lane; i < n_out / 4; i += 64)
+              reinterpret_cast<int4*>(dst)[i] = reinterpret_cast<const int4*>(src)[i];
+          } else {
+            for (int i = qd * 32 + lane; i < n_out; i += 64) dst[i] = src[i];
+          }
+        }
+      }
+      good = bar_and(pair, 64, good);                    // the pair goes on, or leaves, together; its areas are free
+    }
+  }
+  tc_fence_before_sync();
+  __syncthreads();
+  tc_fence_after_sync();
+  if (warp == 0) tmem_dealloc(tmem_base, kSelBufs * kSelN);
+}
+
 static int g_gate_engine = 1;
 void set_gate_engine(int e) { g_gate_engine = e; }
 bool gate_tc_supported(int d, int topk) { return (d == 64 || d == 128 || d == 256) && topk <= 32; }
@@ -624,8 +1044,52 @@ static int gate_tc_pick(const GateParams& p, int batch, int max_q, cudaStream_t 
   return gate_tc_launch<T, D, 32, 1>(p, batch, max_q, s);
 }
 
+template <typename T, int D, int KMAX>
+static int gate_select_launch(const GateParams& p, const CUtensorMap& mq, const CUtensorMap& mk, int batch, int max_q, cudaStream_t s) {
+  constexpr int kCap = sel_cap<KMAX>();
+  const size_t smem = 1024 + (size_t)kGateM * D * 2 + (size_t)kSelRing * kSelN * D * 2 + (size_t)kCap * 256 * 8;
+  static_assert(2 * KMAX * 32 * 4 <= kCap * 64 * 8, "a pair's exchange area fits its queues");
+  FastDiv fd{0, 0, (uint32_t)p.chunk};
+  if (p.chunk > 1) {                   // 2^(32 + shift) / chunk rounded up, shift = ceil(log2(chunk)) - 1
+    while ((2u << fd.shift) < fd.d) ++fd.shift;
+    fd.mul = (uint32_t)((((uint64_t)1 << (32 + fd.shift)) + fd.d - 1) / fd.d);
+  }
+  auto kern = gate_select_kernel<T, D, KMAX>;
+  FMB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  const int row_tiles = ceil_div(max_q, kGateM);
+  const int64_t items = (int64_t)row_tiles * p.heads * batch;
+  const int64_t ctas = (int64_t)sm_count() * (D <= 128 ? 2 : 1);
+  kern<<<(unsigned)(items < ctas ? items : ctas), kSelThreads, smem, s>>>(p, mq, mk, batch, row_tiles, fd);
+  FMB_LAUNCH_CHECK("gate_select_kernel");
+  return FMB_OK;
+}
+// The two-sweep kernel where its tensor maps can be made; *done = false: left to the other kernels
 template <typename T>
-static int gate_dispatch(const GateParams& p, int batch, int max_q, cudaStream_t s) {
+static int gate_select_try(const GateParams& p, int batch, int max_q, int64_t total_q, int64_t km_rows, cudaStream_t s, bool* done) {
+  *done = false;
+  if (total_q <= 0 || km_rows <= 0 || p.topk > 16 || p.q_rs <= 0 || p.q_hs <= 0) return FMB_OK;
+  if ((int64_t)ceil_div(max_q, kGateM) * p.heads * batch >= (1 << 30)) return FMB_OK;
+  CUtensorMap mq, mk;
+  const int dt = std::is_same<T, __nv_bfloat16>::value ? FMB_BF16 : FMB_FP16;
+  if (make_tmap_3d(&mq, p.q, dt, p.d, p.heads, total_q, (uint64_t)p.q_hs * 2, (uint64_t)p.q_rs * 2, kGateM) != FMB_OK ||
+      make_tmap_3d(&mk, p.km, dt, p.d, p.heads_k, km_rows, (uint64_t)p.d * 2, (uint64_t)p.heads_k * p.d * 2, kSelN) != FMB_OK)
+    return FMB_OK;
+  *done = true;
+#define FMB_SEL(D_) \
+  return p.topk <= 8 ? gate_select_launch<T, D_, 8>(p, mq, mk, batch, max_q, s) : gate_select_launch<T, D_, 16>(p, mq, mk, batch, max_q, s)
+  if (p.d <= 64) FMB_SEL(64);
+  if (p.d <= 128) FMB_SEL(128);
+  FMB_SEL(256);
+#undef FMB_SEL
+}
+
+template <typename T>
+static int gate_dispatch(const GateParams& p, int batch, int max_q, int64_t total_q, int64_t km_rows, cudaStream_t s) {
+  if (g_gate_engine == 1) {
+    bool done = false;
+    const int rc = gate_select_try<T>(p, batch, max_q, total_q, km_rows, s, &done);
+    if (done) return rc;
+  }
   const size_t smem = (size_t)kGateDSlab * (kGateM + kGateN) * sizeof(T) +
                       (size_t)kGateM * kGateSStride * sizeof(float) + (size_t)kGateM * p.topk * 8;
   dim3 grid(ceil_div(max_q, kGateM), p.heads, batch);
@@ -655,8 +1119,8 @@ int launch_gate_topk(const GateArgs& a, cudaStream_t s) {
   p.topk_idx = a.topk_idx; p.topk_val = a.topk_val; p.t_rs = a.t_rs; p.t_hs = a.t_hs;
   p.heads = a.heads; p.heads_k = a.heads_k; p.d = a.d; p.topk = a.topk; p.chunk = a.chunk; p.causal = a.causal;
   prof_begin(2, s);
-  const int rc = a.dtype == FMB_BF16 ? gate_dispatch<__nv_bfloat16>(p, a.batch, a.max_q, s)
-                                     : gate_dispatch<__half>(p, a.batch, a.max_q, s);
+  const int rc = a.dtype == FMB_BF16 ? gate_dispatch<__nv_bfloat16>(p, a.batch, a.max_q, a.total_q, a.km_rows, s)
+                                     : gate_dispatch<__half>(p, a.batch, a.max_q, a.total_q, a.km_rows, s);
   prof_end(2, s);
   return rc;
 }

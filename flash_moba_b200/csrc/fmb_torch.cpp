@@ -180,7 +180,7 @@ std::tuple<Tensor, OptTensor> gate_topk(const Tensor& q, const Tensor& km, const
   Tensor idx = at::empty({h, total_q, topk}, q.options().dtype(at::kInt));
   OptTensor val;
   if (return_values) val = at::empty({h, total_q, topk}, q.options().dtype(at::kFloat));
-  check(fmb_gate_topk(q.data_ptr(), q.stride(0), q.stride(1), km.data_ptr(), i32c(cu_q, "cu_seqlens_q"),
+  check(fmb_gate_topk_sized(q.data_ptr(), q.stride(0), q.stride(1), total_q, km.data_ptr(), km.size(0), i32c(cu_q, "cu_seqlens_q"),
                       i32c(cu_k, "cu_seqlens_k"), i32c(cu_km, "cu_seqlens_km"), static_cast<int32_t*>(idx.data_ptr()),
                       val ? static_cast<float*>(val->data_ptr()) : nullptr, topk, total_q * topk, (int)batch, (int)h, (int)hk,
                       (int)d, (int)max_q, (int)max_k, (int)topk, (int)chunk, causal ? 1 : 0, dtype_code(q),

@@ -106,6 +106,15 @@ int fmb_gate_topk(const void* q, int64_t q_row_stride, int64_t q_head_stride,
                   int batch, int heads, int heads_k, int head_dim, int max_seqlen_q,
                   int max_seqlen_k, int topk, int chunk, int causal, int dtype,
                   fmb_stream_t stream);
+/* The same with the number of rows of q (total_q) and of km (km_rows) stated, so that both can be
+ * read through tensor maps: the faster kernel for topk <= 16 and positive strides; other shapes and
+ * sizes given as 0 run what fmb_gate_topk runs.  Results are the same. */
+int fmb_gate_topk_sized(const void* q, int64_t q_row_stride, int64_t q_head_stride, int64_t total_q,
+                        const void* km, int64_t km_rows, const int32_t* cu_seqlens_q,
+                        const int32_t* cu_seqlens_k, const int32_t* cu_seqlens_km, int32_t* topk_idx,
+                        float* topk_val, int64_t topk_row_stride, int64_t topk_head_stride, int batch,
+                        int heads, int heads_k, int head_dim, int max_seqlen_q, int max_seqlen_k,
+                        int topk, int chunk, int causal, int dtype, fmb_stream_t stream);
 
 /* ------------------------------------------------------------------ stages O/E/S: pattern
  * Bytes of scratch `fmb_build_csc` needs. */

@@ -1,0 +1,46 @@
+"""The two-sweep gating kernel at the sizes where it can go wrong: candidate counts around its 64-column
+score tiles and the four tiles that stay in TMEM, many tiles, lists shorter than the kernel's 8 or 16
+places, masses of equal scores (its queues run full), rows without candidates, ragged row tiles.
+
+Integer-valued queries and centroids make every fp32 score exact, so the lists must equal the oracle's
+entry by entry, ties (the higher chunk id first) included."""
+import os
+import sys
+
+import pytest
+import torch
+
+from conftest import cu_of
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+sys.path.insert(0, ROOT)
+from oracle import moba_oracle as O  # noqa: E402
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+@pytest.mark.parametrize("spread", [0, 1, 6])       # 0: every score is the same
+@pytest.mark.parametrize("lens_q,lens_k,H,Hk,d,topk,causal", [
+    ([130], [130], 2, 2, 64, 8, True),              # candidates 0 ... 129: one to three tiles, two row tiles
+    ([1, 63, 64], [65, 128, 256], 4, 2, 128, 5, True),
+    ([128], [257], 2, 1, 128, 8, False),            # five tiles: the products are computed twice
+    ([20, 7], [256, 255], 2, 2, 128, 16, False),    # four tiles, lists of 16
+    ([40], [1500], 2, 1, 64, 11, True),             # 24 tiles, lists of 11
+    ([3, 0, 30], [640, 10, 2111], 2, 2, 128, 1, True),
+    ([9], [700], 2, 2, 256, 13, False),
+    ([50], [20], 2, 2, 64, 4, True),                # more rows than keys
+    ([2] * 70, [90 + i for i in range(70)], 6, 2, 96, 7, True),   # more sequences than are kept in shared memory
+])
+def test_gate_select_exact(lens_q, lens_k, H, Hk, d, topk, causal, spread):
+    from flash_moba_b200 import ops
+    g = torch.Generator().manual_seed(d + topk)
+    q = torch.randint(-2, 3, (sum(lens_q), H, d), generator=g).to(torch.bfloat16) if spread else torch.ones(sum(lens_q), H, d).bfloat16()
+    km = torch.randint(-spread, spread + 1, (sum(lens_k), Hk, d), generator=g).to(torch.bfloat16)
+    cq, ck = cu_of(lens_q), cu_of(lens_k)            # chunks of one key: the centroids are the keys
+    for values in (True, False):
+        idx, val = ops.gate_topk(q.to(DEV), km.to(DEV), cq.to(DEV), ck.to(DEV), ck.to(DEV), max(lens_q), max(lens_k), topk, 1,
+                                 causal, return_values=values)
+        ref_idx, ref_val = O.gate_topk(q, km, cq, ck, ck, topk, 1, causal)
+        assert torch.equal(idx.cpu(), ref_idx)
+        assert val is None or torch.equal(val.cpu(), ref_val)
