@@ -5,19 +5,20 @@
 // atomics (unordered) and then runs a segmented sort
 // (csrc/flash_topk/src/flash_topk_kernel.h:303-312, 376-402, 407-478;
 //  csrc/flash_topk/src/varlen_sort.cu:29-124).  Here:
-//   1. tile_hist : a CTA takes kTileRows query rows of one (b,h) and a range of columns,
-//                  marks (column,row) bits in a shared-memory bitmap and pop-counts each
-//                  column -> hist[bh][tile][col]
-//   2. col_scan  : per (b,h): running sum over tiles per column (hist becomes the tile's
-//                  write cursor), col_nnz, exclusive scan over columns -> col_offsets,
-//                  zero of the region's unused tail
-//   3. scatter   : rebuild the bitmap; a half-warp per column walks its bits in row
-//                  order and writes them at col_offsets + cursor -> columns come out
-//                  ascending, bit-exact and run-to-run deterministic.  On request the same
-//                  kernel also writes, for entry j of every row's top-k list, the position
-//                  in `indices` where that (row, chunk) pair landed (row_slots): the
-//                  row-major view of the pattern that the attention kernels' combine pass
+//   1. tile_hist : a CTA takes kTileRows query rows of one (b,h) and counts its entries per column
+//                  in shared memory -> hist[bh][tile][col]
+//   2. tile_scan : per (b,h) and group of columns: running sum over tiles per column (hist becomes the
+//                  tile's write cursor), col_nnz.  Left out for sequences of few tiles, whose scatter
+//                  CTAs sum the tiles before their own themselves
+//   3. scatter   : the column offsets (a scan over col_nnz, repeated by every CTA: a few hundred numbers);
+//                  a bitmap (column x row) of the tile in shared memory with a running count per 32 rows, from
+//                  which every entry's place in its column follows directly: columns come out ascending,
+//                  bit-exact and run-to-run deterministic, entries are written where the row stands.
+//                  On request the same thread also writes the row's places in `indices`, in ascending
+//                  order (row_slots): the row-major view of the pattern that the attention kernels' merge
 //                  needs, so that an attention call on this pattern builds no lists of its own.
+// Measured (B200, three kernels with bitmap walks before / now): 64K tokens x 32 heads, 512 columns 297 / 192 us; 32K x 16
+// 71 / 45; 317K tokens, lists of 16 2.19 / 1.63 ms; 512K x 4 heads, 2,048 columns 1.49 / 0.84 ms.
 // HBM bound.  Algorithmic bytes: 4*nnz read + 4*nnz written + 12*B*H*ncol.
 #include <mutex>
 
@@ -28,7 +29,9 @@ namespace fmb {
 constexpr int kTileRows = 512;                 // query rows per tile
 constexpr int kTileWords = kTileRows / 32;     // bitmap words per column
 constexpr int kBmStride = kTileWords + 1;      // padded: conflict-free column walks
-constexpr int kMaxColsPerCta = 1024;
+constexpr int kMaxHistCols = 8192;             // columns per CTA of the histogram (32 KB of counters)
+constexpr int kMaxColsPerCta = 1024;           // columns per CTA of the scatter
+constexpr int kColBytes = kBmStride * 4 + kTileWords * 2 + 4;   // shared memory of the scatter per column
 constexpr int kCscThreads = 512;
 
 struct CscParams {
@@ -36,162 +39,280 @@ struct CscParams {
   const int32_t* cu_q;
   int64_t* col_offsets; int32_t* col_nnz; int32_t* indices;
   int32_t* hist;                                      // [B*H][ntiles][ncol]
-  uint32_t* row_slots;                                // optional: [(h*total_q + token)*topk + j], 0xffffffff = no entry
+  uint32_t* row_slots;                                // optional: [(h*total_q + token)*topk + ...], ascending, 0xffffffff = no entry
   int64_t total_q;
   int heads, topk, ncol, ntiles, cols_per_cta;
+  int scanned;                                        // 1: hist holds cursors (tile_scan has run), 0: counts
 };
 
-// marks the bits of this CTA's (tile, column range); returns through smem `bm`
-__device__ __forceinline__ void build_bitmap(const CscParams& p, uint32_t* bm, int b, int h, int tile,
-                                             int c0, int ncols, int len_q, int seq0) {
-  const int words = ncols * kBmStride;
-  for (int i = threadIdx.x; i < words; i += blockDim.x) bm[i] = 0u;
-  __syncthreads();
-  const int r0 = tile * kTileRows;
-  const int rows = min(kTileRows, len_q - r0);
-  const int n = rows * p.topk;
-  const int32_t* src = p.topk_idx + (int64_t)(seq0 + r0) * p.idx_rs + (int64_t)h * p.idx_hs;
-  for (int e = threadIdx.x; e < n; e += blockDim.x) {
-    const int r = e / p.topk, s = e - r * p.topk;
-    const int c = src[(int64_t)r * p.idx_rs + s] - c0;
-    if (c >= 0 && c < ncols) atomicOr(&bm[c * kBmStride + (r >> 5)], 1u << (r & 31));
-  }
-  __syncthreads();
+// ascending sorting networks on 8 and 16 ids
+__device__ __forceinline__ void csc_ce(int& a, int& b) {
+  const int lo = min(a, b), hi = max(a, b);
+  a = lo;
+  b = hi;
+}
+template <int N>
+__device__ __forceinline__ void csc_sort(int* x) {
+#pragma unroll
+  for (int k = 2; k <= N; k <<= 1)
+#pragma unroll
+    for (int j = k >> 1; j >= 1; j >>= 1)
+#pragma unroll
+      for (int i = 0; i < N; ++i) {
+        const int l = j == (k >> 1) ? (i ^ (k - 1)) : (i ^ j);
+        if (l > i) csc_ce(x[i], x[l]);
+      }
 }
 
+constexpr int kCscNone = 0x7fffffff;
+// the list of row `r` of a tile (src: the tile's first row), places without a chunk of the pattern as kCscNone
+template <int KMAX>
+__device__ __forceinline__ void csc_load_row(const CscParams& p, const int32_t* src, int r, int (&id)[KMAX]) {
+  const int32_t* mine = src + (int64_t)r * p.idx_rs;
+  if (p.topk == KMAX && (p.idx_rs & 3) == 0 && (reinterpret_cast<uintptr_t>(src) & 15) == 0) {
+#pragma unroll
+    for (int j = 0; j < KMAX; j += 4) {
+      const int4 q = *reinterpret_cast<const int4*>(mine + j);
+      id[j] = q.x; id[j + 1] = q.y; id[j + 2] = q.z; id[j + 3] = q.w;
+    }
+  } else {
+#pragma unroll
+    for (int j = 0; j < KMAX; ++j) id[j] = j < p.topk ? mine[j] : kCscNone;
+  }
+#pragma unroll
+  for (int j = 0; j < KMAX; ++j)
+    if (id[j] < 0 || id[j] >= p.ncol) id[j] = kCscNone;
+}
+
+// KMAX as for the scatter kernel below.  A chunk that a row names twice counts once.
+template <int KMAX>
 __global__ void __launch_bounds__(kCscThreads) csc_tile_hist_kernel(CscParams p) {
-  extern __shared__ uint32_t bm[];
+  extern __shared__ uint32_t sm[];
   const int bh = blockIdx.x, tile = blockIdx.y, c0 = blockIdx.z * p.cols_per_cta;
   const int b = bh / p.heads, h = bh - b * p.heads;
   const int seq0 = p.cu_q[b], len_q = p.cu_q[b + 1] - seq0;
   const int ncols = min(p.cols_per_cta, p.ncol - c0);
   int32_t* hist = p.hist + ((int64_t)bh * p.ntiles + tile) * p.ncol + c0;
-  if (tile * kTileRows >= len_q) {   // tile beyond this sequence: empty counts
-    for (int c = threadIdx.x; c < ncols; c += blockDim.x) hist[c] = 0;
+  const int r0 = tile * kTileRows, rows = min(kTileRows, len_q - r0);
+  if (rows <= 0) {   // tile beyond this sequence: empty counts
+    for (int c = threadIdx.x; c < ncols; c += kCscThreads) hist[c] = 0;
     return;
   }
-  build_bitmap(p, bm, b, h, tile, c0, ncols, len_q, seq0);
-  for (int c = threadIdx.x; c < ncols; c += blockDim.x) {
-    int cnt = 0;
+  for (int c = threadIdx.x; c < ncols; c += kCscThreads) sm[c] = 0u;
+  __syncthreads();
+  const int32_t* src = p.topk_idx + (int64_t)(seq0 + r0) * p.idx_rs + (int64_t)h * p.idx_hs;
+  auto count = [&](int c) {
+    c -= c0;
+    if (c >= 0 && c < ncols) atomicAdd(&sm[c], 1u);
+  };
+  if constexpr (KMAX > 0) {
+    if ((int)threadIdx.x < rows) {
+      int id[KMAX];
+      csc_load_row<KMAX>(p, src, threadIdx.x, id);
+      csc_sort<KMAX>(id);
 #pragma unroll
-    for (int w = 0; w < kTileWords; ++w) cnt += __popc(bm[c * kBmStride + w]);
-    hist[c] = cnt;
+      for (int j = 0; j < KMAX; ++j)
+        if (id[j] != kCscNone && (j == 0 || id[j] != id[j > 0 ? j - 1 : 0])) count(id[j]);
+    }
+  } else {
+    for (int e = threadIdx.x; e < rows * p.topk; e += kCscThreads) {
+      const int r = e / p.topk, j = e - r * p.topk;
+      const int32_t* list = src + (int64_t)r * p.idx_rs;
+      const int c = list[j];
+      bool again = false;
+      for (int i = 0; i < j; ++i) again = again || list[i] == c;
+      if (!again) count(c);
+    }
   }
+  __syncthreads();
+  for (int c = threadIdx.x; c < ncols; c += kCscThreads) hist[c] = (int)sm[c];
 }
 
-__global__ void __launch_bounds__(1024) csc_col_scan_kernel(CscParams p) {
-  __shared__ int64_t warp_sums[32];
-  __shared__ int64_t carry_s;
-  const int bh = blockIdx.x;
+// grid (b*h, groups of 32 columns): 32 warps, lane = column; the tiles are cut into 32 runs, one per warp
+__global__ void __launch_bounds__(1024) csc_tile_scan_kernel(CscParams p) {
+  __shared__ int run_sum[32][33];
+  const int bh = blockIdx.x, b = bh / p.heads;
+  const int ntiles_b = (p.cu_q[b + 1] - p.cu_q[b] + kTileRows - 1) / kTileRows;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int c = blockIdx.y * 32 + lane;
+  const int per = (ntiles_b + 31) / 32, t0 = warp * per, t1 = min(ntiles_b, t0 + per);
+  int32_t* hist = p.hist + (int64_t)bh * p.ntiles * p.ncol + c;
+  int sum = 0;
+  if (c < p.ncol) {
+#pragma unroll 4
+    for (int t = t0; t < t1; ++t) sum += hist[(int64_t)t * p.ncol];
+  }
+  run_sum[warp][lane] = sum;
+  __syncthreads();
+  int before = 0, total = 0;
+  for (int w = 0; w < 32; ++w) {
+    const int x = run_sum[w][lane];
+    before += w < warp ? x : 0;
+    total += x;
+  }
+  if (c >= p.ncol) return;
+  for (int t = t0; t < t1; ++t) {
+    const int x = hist[(int64_t)t * p.ncol];
+    hist[(int64_t)t * p.ncol] = before;
+    before += x;
+  }
+  if (warp == 0) p.col_nnz[(int64_t)bh * p.ncol + c] = total;
+}
+
+// KMAX: 8 or 16: lists of at most that many ids are sorted in registers by one thread per row; 0: any length,
+// a thread per entry
+template <int KMAX>
+__global__ void __launch_bounds__(kCscThreads) csc_scatter_kernel(CscParams p) {
+  extern __shared__ uint32_t sm[];
+  __shared__ int64_t warp_sums[kCscThreads / 32];
+  const int bh = blockIdx.x, tile = blockIdx.y, c0 = blockIdx.z * p.cols_per_cta;
   const int b = bh / p.heads, h = bh - b * p.heads;
   const int seq0 = p.cu_q[b], len_q = p.cu_q[b + 1] - seq0;
+  const int r0 = tile * kTileRows, rows = min(kTileRows, len_q - r0);
+  if (rows <= 0 && tile > 0) return;            // (the first tile of an empty sequence still writes its columns)
+  const int ncols = min(p.cols_per_cta, p.ncol - c0);
   const int ntiles_b = (len_q + kTileRows - 1) / kTileRows;
-  const int64_t base = ((int64_t)seq0 * p.heads + (int64_t)len_q * h) * p.topk;
-  int32_t* hist = p.hist + (int64_t)bh * p.ntiles * p.ncol;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  if (threadIdx.x == 0) carry_s = 0;
-  __syncthreads();
-  for (int c0 = 0; c0 < p.ncol; c0 += blockDim.x) {
-    const int c = c0 + threadIdx.x;
-    int run = 0;
+  uint32_t* bm = sm;                                              // [ncols][kBmStride] bit (row) of every column
+  uint16_t* before = reinterpret_cast<uint16_t*>(bm + ncols * kBmStride);   // [ncols][kTileWords] rows ahead of each 32
+  uint32_t* base = reinterpret_cast<uint32_t*>(before + ncols * kTileWords);   // [ncols] first place of the tile's entries
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int64_t region = ((int64_t)seq0 * p.heads + (int64_t)len_q * h) * p.topk;   // first place of this (b, h) in `indices`
+  for (int i = tid; i < ncols * kBmStride; i += kCscThreads) bm[i] = 0u;
+
+  // ---- column offsets (places inside the region) and this tile's cursor in every column
+  const int32_t* hist = p.hist + (int64_t)bh * p.ntiles * p.ncol;
+  int64_t carry = 0;
+  for (int g0 = 0; g0 < p.ncol; g0 += kCscThreads) {
+    const int c = g0 + tid;
+    int nnz = 0, cursor = 0;
     if (c < p.ncol) {
-      // tiles beyond the sequence hold zeros.  Sixteen counters are fetched at a time so that the
-      // loads overlap: one dependent load-add-store chain per tile would cost a memory latency each
-      for (int t0 = 0; t0 < ntiles_b; t0 += 16) {
-        int x[16];
-#pragma unroll
-        for (int u = 0; u < 16; ++u) x[u] = (t0 + u < ntiles_b) ? hist[(int64_t)(t0 + u) * p.ncol + c] : 0;
-#pragma unroll
-        for (int u = 0; u < 16; ++u) {
-          if (t0 + u < ntiles_b) hist[(int64_t)(t0 + u) * p.ncol + c] = run;
-          run += x[u];
+      if (p.scanned) {
+        nnz = p.col_nnz[(int64_t)bh * p.ncol + c];
+        cursor = tile < ntiles_b ? hist[(int64_t)tile * p.ncol + c] : 0;
+      } else {
+#pragma unroll 4
+        for (int t = 0; t < ntiles_b; ++t) {
+          const int x = hist[(int64_t)t * p.ncol + c];
+          cursor += t < tile ? x : 0;
+          nnz += x;
         }
       }
     }
-    // block-wide exclusive scan of `run` over this group of columns
-    int64_t x = run;
+    int64_t x = nnz;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-      int64_t y = __shfl_up_sync(0xffffffffu, x, o);
+      const int64_t y = __shfl_up_sync(0xffffffffu, x, o);
       if (lane >= o) x += y;
     }
     if (lane == 31) warp_sums[warp] = x;
     __syncthreads();
-    if (warp == 0) {
-      int64_t w = warp_sums[lane];
+    int64_t ahead = carry, total = 0;
 #pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        int64_t y = __shfl_up_sync(0xffffffffu, w, o);
-        if (lane >= o) w += y;
-      }
-      warp_sums[lane] = w;   // inclusive over warps
+    for (int w = 0; w < kCscThreads / 32; ++w) {
+      const int64_t y = warp_sums[w];
+      ahead += w < warp ? y : 0;
+      total += y;
     }
-    __syncthreads();
-    const int64_t carry = carry_s;
-    const int64_t excl = carry + (warp ? warp_sums[warp - 1] : 0) + x - run;
     if (c < p.ncol) {
-      p.col_offsets[(int64_t)bh * p.ncol + c] = base + excl;
-      p.col_nnz[(int64_t)bh * p.ncol + c] = run;
+      const int64_t off = ahead + x - nnz;
+      if (c >= c0 && c < c0 + ncols) base[c - c0] = (uint32_t)(off + cursor);
+      if (tile == 0 && blockIdx.z == 0) {
+        p.col_offsets[(int64_t)bh * p.ncol + c] = region + off;
+        if (!p.scanned) p.col_nnz[(int64_t)bh * p.ncol + c] = nnz;
+      }
     }
-    __syncthreads();
-    if (threadIdx.x == blockDim.x - 1) carry_s = carry + warp_sums[31];
+    carry += total;
     __syncthreads();
   }
-  // unused tail of this (b,h) region stays zero, as in the reference's zero-initialised
-  // buffer (csrc/flash_topk/flash_topk_api.cpp:217)
-  const int64_t total = carry_s, region = (int64_t)len_q * p.topk;
-  for (int64_t i = total + threadIdx.x; i < region; i += blockDim.x) p.indices[base + i] = 0;
-}
+  // the unused tail of the region stays zero, as in the reference's zero-initialised buffer
+  // (csrc/flash_topk/flash_topk_api.cpp:217); its tiles share it
+  if (blockIdx.z == 0 && ntiles_b > 0)
+    for (int64_t i = carry + (int64_t)tile * kCscThreads + tid; i < (int64_t)len_q * p.topk; i += (int64_t)ntiles_b * kCscThreads)
+      p.indices[region + i] = 0;
+  if (rows <= 0) return;
 
-__global__ void __launch_bounds__(kCscThreads) csc_scatter_kernel(CscParams p) {
-  extern __shared__ uint32_t bm[];
-  const int bh = blockIdx.x, tile = blockIdx.y, c0 = blockIdx.z * p.cols_per_cta;
-  const int b = bh / p.heads, h = bh - b * p.heads;
-  const int seq0 = p.cu_q[b], len_q = p.cu_q[b + 1] - seq0;
-  if (tile * kTileRows >= len_q) return;
-  const int ncols = min(p.cols_per_cta, p.ncol - c0);
-  build_bitmap(p, bm, b, h, tile, c0, ncols, len_q, seq0);
-  const int32_t* cursor = p.hist + ((int64_t)bh * p.ntiles + tile) * p.ncol + c0;
-  const int64_t* offs = p.col_offsets + (int64_t)bh * p.ncol + c0;
-  // a half-warp per column: lane w of the half owns bitmap word w (32 rows)
-  static_assert(kTileWords == 16, "half-warp mapping assumes 16 words per column");
-  const int half = threadIdx.x >> 4, hl = threadIdx.x & 15;
-  const int nhalves = blockDim.x >> 4;
-  const unsigned hmask = 0xffffu << (threadIdx.x & 16);
-  for (int c = half; c < ncols; c += nhalves) {
-    uint32_t bits = bm[c * kBmStride + hl];
-    int cnt = __popc(bits), x = cnt;
+  // ---- bitmap of the tile
+  const int32_t* src = p.topk_idx + (int64_t)(seq0 + r0) * p.idx_rs + (int64_t)h * p.idx_hs;
+  static_assert(kTileRows == kCscThreads, "a thread per row");
+  int id[KMAX > 0 ? KMAX : 1];
+  if constexpr (KMAX > 0) {
+    if (tid < rows) {
+      csc_load_row<KMAX>(p, src, tid, id);
 #pragma unroll
-    for (int o = 1; o < 16; o <<= 1) {
-      int y = __shfl_up_sync(hmask, x, o, 16);
-      if (hl >= o) x += y;
+      for (int j = 0; j < KMAX; ++j) {
+        const int c = id[j] - c0;
+        if (c >= 0 && c < ncols) atomicOr(&bm[c * kBmStride + (tid >> 5)], 1u << (tid & 31));
+      }
     }
-    int32_t* dst = p.indices + offs[c] + cursor[c] + (x - cnt);
-    const int rbase = tile * kTileRows + hl * 32;
-    while (bits) {
-      const int bit = __ffs(bits) - 1;
-      bits &= bits - 1;
-      *dst++ = rbase + bit;
+  } else {
+    for (int e = tid; e < rows * p.topk; e += kCscThreads) {
+      const int r = e / p.topk, c = src[(int64_t)r * p.idx_rs + (e - r * p.topk)] - c0;
+      if (c >= 0 && c < ncols) atomicOr(&bm[c * kBmStride + (r >> 5)], 1u << (r & 31));
     }
   }
-  if (p.row_slots == nullptr) return;
-  // Row-major pass: entry (row r, list place j) with chunk c in this CTA's column range sits at
-  // col_offsets[c] + cursor[c] + (rows of this tile below r that also selected c).
-  const int r0 = tile * kTileRows;
-  const int rows = min(kTileRows, len_q - r0);
-  const int32_t* src = p.topk_idx + (int64_t)(seq0 + r0) * p.idx_rs + (int64_t)h * p.idx_hs;
-  uint32_t* out = p.row_slots + ((int64_t)h * p.total_q + seq0 + r0) * p.topk;
-  for (int e = threadIdx.x; e < rows * p.topk; e += blockDim.x) {
-    const int r = e / p.topk, j = e - r * p.topk;
-    const int cg = src[(int64_t)r * p.idx_rs + j];
-    const int c = cg - c0;
-    if (c >= 0 && c < ncols) {
-      const uint32_t* col = bm + c * kBmStride;
-      int below = __popc(col[r >> 5] & ((1u << (r & 31)) - 1u));
-      for (int w = 0; w < (r >> 5); ++w) below += __popc(col[w]);
-      out[e] = (uint32_t)(offs[c] + cursor[c] + below);
-    } else if (blockIdx.z == 0 && (cg < 0 || cg >= p.ncol)) {
-      out[e] = 0xffffffffu;     // empty place of the list (or a chunk id outside the pattern)
+  __syncthreads();
+  for (int c = tid; c < ncols; c += kCscThreads) {
+    int run = 0;
+#pragma unroll
+    for (int w = 0; w < kTileWords; ++w) {
+      before[c * kTileWords + w] = (uint16_t)run;
+      run += __popc(bm[c * kBmStride + w]);
+    }
+  }
+  __syncthreads();
+
+  // ---- places: first place of the column's entries in this tile, plus its rows ahead of this one
+  auto place = [&](int c, int r) {
+    return base[c] + before[c * kTileWords + (r >> 5)] + (uint32_t)__popc(bm[c * kBmStride + (r >> 5)] & ((1u << (r & 31)) - 1u));
+  };
+  if constexpr (KMAX > 0) {
+    if (tid >= rows) return;
+    if (p.row_slots != nullptr) csc_sort<KMAX>(id);               // ascending columns are ascending places
+    uint32_t at[KMAX];
+#pragma unroll
+    for (int j = 0; j < KMAX; ++j) {
+      const int c = id[j] - c0;
+      at[j] = 0xffffffffu;
+      if (c >= 0 && c < ncols) {
+        const uint32_t x = place(c, tid);
+        p.indices[region + x] = r0 + tid;
+        at[j] = (uint32_t)region + x;                             // (row_slots are kept for fewer than 2^32 entries only)
+      }
+    }
+    if (p.row_slots != nullptr) {
+      uint32_t* out = p.row_slots + ((int64_t)h * p.total_q + seq0 + r0 + tid) * p.topk;
+      if (p.topk == KMAX && gridDim.z == 1) {
+#pragma unroll
+        for (int j = 0; j < KMAX; j += 4) *reinterpret_cast<uint4*>(out + j) = make_uint4(at[j], at[j + 1], at[j + 2], at[j + 3]);
+      } else {                                                    // a CTA writes the entries of its own columns
+#pragma unroll
+        for (int j = 0; j < KMAX; ++j)
+          if (j < p.topk && (at[j] != 0xffffffffu || (id[j] == kCscNone && blockIdx.z == 0))) out[j] = at[j];
+      }
+    }
+  } else {
+    uint32_t* out = p.row_slots ? p.row_slots + ((int64_t)h * p.total_q + seq0 + r0) * p.topk : nullptr;
+    for (int e = tid; e < rows * p.topk; e += kCscThreads) {
+      const int r = e / p.topk, j = e - r * p.topk;
+      const int32_t* list = src + (int64_t)r * p.idx_rs;
+      const int cg = list[j];
+      const bool used = cg >= 0 && cg < p.ncol;
+      const int c = cg - c0;
+      const bool here = used && c >= 0 && c < ncols;
+      uint32_t x = 0;
+      if (here) {
+        x = place(c, r);
+        p.indices[region + x] = r0 + r;
+      }
+      if (out != nullptr && (here || (!used && blockIdx.z == 0))) {
+        int rank = 0;                                             // places in ascending order, empty ones last
+        for (int i = 0; i < p.topk; ++i) {
+          const int o = list[i];
+          const bool o_used = o >= 0 && o < p.ncol;
+          rank += (used ? (o_used && o < cg) : (o_used || i < j)) ? 1 : 0;
+        }
+        out[(int64_t)r * p.topk + rank] = here ? (uint32_t)region + x : 0xffffffffu;
+      }
     }
   }
 }
@@ -217,21 +338,26 @@ int launch_build_csc(const int32_t* topk_idx, int64_t idx_rs, int64_t idx_hs, co
   p.hist = static_cast<int32_t*>(ws);
   p.row_slots = row_slots; p.total_q = total_q;
   p.heads = heads; p.topk = topk; p.ncol = ncol; p.ntiles = csc_ntiles(max_q);
-  p.cols_per_cta = min(kMaxColsPerCta, ncol);
-  const int ncr = ceil_div(ncol, p.cols_per_cta);
-  const size_t smem = (size_t)p.cols_per_cta * kBmStride * sizeof(uint32_t);
-  // the attribute belongs to the current device: set on every call (cheap, idempotent, thread-safe)
-  FMB_CUDA(cudaFuncSetAttribute(csc_tile_hist_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                kMaxColsPerCta * kBmStride * 4));
-  FMB_CUDA(cudaFuncSetAttribute(csc_scatter_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                kMaxColsPerCta * kBmStride * 4));
-  dim3 grid(batch * heads, p.ntiles, ncr);
+  // few tiles: their scatter CTAs add up the counts of the tiles before their own (at most 16 numbers per
+  // column) instead of waiting for one more launch
+  p.scanned = p.ntiles > 16 ? 1 : 0;
   prof_begin(6, s);
-  csc_tile_hist_kernel<<<grid, kCscThreads, smem, s>>>(p);
+  p.cols_per_cta = min(kMaxHistCols, ncol);
+  auto count = topk <= 8 ? csc_tile_hist_kernel<8> : topk <= 16 ? csc_tile_hist_kernel<16> : csc_tile_hist_kernel<0>;
+  count<<<dim3(batch * heads, p.ntiles, ceil_div(ncol, p.cols_per_cta)), kCscThreads,
+                         (size_t)p.cols_per_cta * sizeof(uint32_t), s>>>(p);
   FMB_LAUNCH_CHECK("csc_tile_hist_kernel");
-  csc_col_scan_kernel<<<batch * heads, 1024, 0, s>>>(p);
-  FMB_LAUNCH_CHECK("csc_col_scan_kernel");
-  csc_scatter_kernel<<<grid, kCscThreads, smem, s>>>(p);
+  if (p.scanned) {
+    csc_tile_scan_kernel<<<dim3(batch * heads, ceil_div(ncol, 32)), 1024, 0, s>>>(p);
+    FMB_LAUNCH_CHECK("csc_tile_scan_kernel");
+  }
+  p.cols_per_cta = min(kMaxColsPerCta, ncol);
+  const dim3 grid(batch * heads, p.ntiles, ceil_div(ncol, p.cols_per_cta));
+  const size_t smem = (size_t)p.cols_per_cta * kColBytes;
+  auto scatter = topk <= 8 ? csc_scatter_kernel<8> : topk <= 16 ? csc_scatter_kernel<16> : csc_scatter_kernel<0>;
+  // the attribute belongs to the current device: set on every call (cheap, idempotent, thread-safe)
+  FMB_CUDA(cudaFuncSetAttribute(scatter, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxColsPerCta * kColBytes));
+  scatter<<<grid, kCscThreads, smem, s>>>(p);
   prof_end(6, s);
   FMB_LAUNCH_CHECK("csc_scatter_kernel");
   return FMB_OK;
