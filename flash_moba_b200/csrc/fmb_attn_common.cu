@@ -120,6 +120,43 @@ __global__ void __launch_bounds__(256) row_list_kernel(RowListParams p) {
   }
 }
 
+// The atomics of the fill leave a row's list in no particular order: put it in ascending slot order,
+// which is the order of the merge.  A warp per row; lists of up to 32 by counting, longer ones by a
+// direction-free bitonic network in place (every compare-exchange puts the smaller slot at the lower place).
+__global__ void __launch_bounds__(256) sort_rows_kernel(const uint32_t* __restrict__ row_ptr, uint32_t* row_pos, int64_t rows) {
+  const int64_t r = ((int64_t)blockIdx.x * 256 + threadIdx.x) >> 5;
+  const int lane = threadIdx.x & 31;
+  if (r >= rows) return;
+  uint32_t* a = row_pos + row_ptr[r];
+  const int n = (int)(row_ptr[r + 1] - row_ptr[r]);
+  if (n <= 32) {
+    const uint32_t x = lane < n ? a[lane] : 0xffffffffu;
+    int rank = 0;
+#pragma unroll
+    for (int i = 0; i < 32; ++i) {
+      const uint32_t y = __shfl_sync(0xffffffffu, x, i);
+      rank += (y < x || (y == x && i < lane)) ? 1 : 0;
+    }
+    if (lane < n) a[rank] = x;
+    return;
+  }
+  int N = 64;
+  while (N < n) N <<= 1;
+  for (int k = 2; k <= N; k <<= 1) {
+    for (int j = k >> 1; j >= 1; j >>= 1) {
+      const bool flip = j == (k >> 1);
+      for (int i = lane; i < N; i += 32) {
+        const int l = flip ? (i ^ (k - 1)) : (i ^ j);
+        if (l > i && l < n) {
+          const uint32_t x = a[i], y = a[l];
+          if (x > y) { a[i] = y; a[l] = x; }
+        }
+      }
+      __syncwarp();
+    }
+  }
+}
+
 // inclusive scan of u32 in place, three phases, 4096 items per block
 constexpr int kScanItems = 4096;
 __global__ void __launch_bounds__(1024) scan_block_kernel(uint32_t* data, int64_t n, uint32_t* block_sums) {
@@ -230,476 +267,147 @@ int build_row_lists(const AttnArgs& a, const AttnWorkspace& w, const PassParams&
   if (rc) return rc;
   row_list_kernel<true><<<grid, 256, 0, s>>>(p);
   FMB_LAUNCH_CHECK("row_list_kernel<fill>");
+  sort_rows_kernel<<<(unsigned)ceil_div64(rows, 8), 256, 0, s>>>(w.row_ptr, w.row_pos, rows);
+  FMB_LAUNCH_CHECK("sort_rows_kernel");
   return FMB_OK;
 }
 
-// ------------------------------------------------------------------ combine kernels
-// What a combine kernel needs to know about the pass
-struct CombineParams {
+// ------------------------------------------------------------------ merge of a row's partials
+// What the merge kernel needs to know about the pass
+struct MergeParams {
   const uint32_t* row_ptr; const uint32_t* row_pos;
   int64_t total_q, cap;
-  int heads_out;   // heads of the output tensor's row (for nothing but documentation)
-  int h0, nh, nsub, d;
+  int h0, nh, nsub;
   int fixed_k;     // > 0: row lists handed over by the pattern builder: row `rid` owns the fixed_k places
-                   // row_pos[rid*fixed_k ..], empty places hold 0xffffffff; row_ptr is not used
+                   // row_pos[rid*fixed_k ..], empty places last (0xffffffff); row_ptr is not used
   int64_t slot_shift;               // handed-over rows hold positions in `indices`: slot = position - slot_shift
-  const int* status; int* mirror;   // mirror != nullptr: the first combine kernel of the call's last pass copies
-                                    // the call's status word there (see attn_status_mirror)
+  const int* status; int* mirror;   // mirror != nullptr: the merge kernel of the call's last pass copies the
+                                    // call's status word there (see attn_status_mirror)
 };
-// The main kernels, which set the status word, have completed when a combine kernel starts.
-__device__ __forceinline__ void mirror_status(const CombineParams& c) {
-  if (c.mirror != nullptr && blockIdx.x == 0 && threadIdx.x == 0) *c.mirror = *c.status;
-}
-// first place and number of places of row `rid` in row_pos
-__device__ __forceinline__ void row_span(const CombineParams& c, int64_t rid, int64_t& p0, int& n) {
-  if (c.fixed_k > 0) {
-    p0 = rid * c.fixed_k;
-    n = c.fixed_k;
-  } else {
-    p0 = c.row_ptr[rid];
-    n = (int)(c.row_ptr[rid + 1] - (uint32_t)p0);
-  }
-}
 constexpr uint32_t kNoSlot = 0xffffffffu;
+constexpr int kMergeThreads = 256;
+constexpr int kMergeBatch = 8;      // partial rows in flight per row
 
-// Generic kernel: a warp per (token, head of the pass).  The row's partials are visited plane by
-// plane, inside a plane in ascending slot order = ascending (sb*cap + slot).
-// next_slot(): smallest slot of the row that is greater than `last` (-1 first).
-__device__ __forceinline__ int64_t next_slot(const uint32_t* rp, int n, int64_t last, int lane) {
-  int64_t best = INT64_MAX;
-  for (int j = lane; j < n; j += 32) {
-    const int64_t x = rp[j];
-    if (x > last && x < best) best = x;
-  }
-#pragma unroll
-  for (int o = 16; o; o >>= 1) {
-    const int64_t y = __shfl_xor_sync(0xffffffffu, best, o);
-    best = y < best ? y : best;
-  }
-  return best;
-}
+// Row lists are in ascending slot order (the pattern builder writes them so; sort_rows_kernel puts the
+// lists of other patterns in order), so a row's partials are taken as they come: D/8 lanes per
+// (head, token) row, one 16-byte chunk of every partial each, eight partials requested before anything
+// waits, the next row's list requested before this row is worked on.  Merge order: plane by plane,
+// ascending slots, whatever made the lists: results do not depend on it.  FWD weights the partials by
+// exp(lse_j - max lse) and writes the row's log-sum-exp; the backward form is a plain sum.
+// Bound: HBM (random 256-byte rows at d = 128), rows taken head by head.  With lists in the order of the
+// gating lists, every lane group had to rank its row's places first and short lists left lanes idle; measured
+// (B200, before / now, forward and backward): 64K tokens x 32 heads, top-k 8 1.19 / 0.94 and 0.93 / 0.79 ms (5.4 GB and
+// 4.8 GB: 5.7 and 6.1 TB/s); 317K tokens, chunk 64, top-k 16 9.6 / 7.7 and 9.8 / 6.8 ms; 512K tokens x 4 heads, chunk 256,
+// top-k 16 5.3 / 3.3 and 3.3 / 2.7 ms; d 64, 9,391 tokens x 12 heads 64 / 27 and 57 / 24 us.
+template <typename T, int D, bool FWD>
+__global__ void __launch_bounds__(kMergeThreads, 3) merge_kernel(const T* __restrict__ part, const float* __restrict__ part_lse,
+                                                              MergeParams c, T* out, int64_t rs, int64_t hs, float* lse) {
+  constexpr int LPR = D / 8, RPW = 32 / LPR, B = kMergeBatch;
+  if (c.mirror != nullptr && blockIdx.x == 0 && threadIdx.x == 0) *c.mirror = *c.status;   // (the main kernel has completed)
+  const int lane = threadIdx.x & 31, gl = lane % LPR;
+  const int64_t n_rows = c.total_q * c.nh, stride = (int64_t)gridDim.x * (kMergeThreads / 32) * RPW;
+  int64_t rid = ((int64_t)blockIdx.x * (kMergeThreads / 32) + (threadIdx.x >> 5)) * RPW + lane / LPR;
+  const int64_t warp_first = rid - lane / LPR;
 
-// The combine kernels walk "virtual blocks" of 256 threads with a grid-stride loop, so that the
-// later stages of the cascade can be launched with a small grid: they usually find their flag
-// clear and must cost microseconds, not a scan of the whole block range.
-template <typename T>
-__device__ __forceinline__ void fwd_combine_body(int64_t vblock, const T* __restrict__ part_o,
-                                                 const float* __restrict__ part_lse, const CombineParams& c,
-                                                 T* out, int64_t o_rs, int64_t o_hs, float* lse, int min_n) {
-  using T2 = typename Elem<T>::T2;
-  const int64_t wid = (vblock * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  if (wid >= c.total_q * c.nh) return;
-  const int64_t t = wid / c.nh;
-  const int hr = (int)(wid - t * c.nh);
-  const int64_t rid = (int64_t)hr * c.total_q + t;
+  // list of row r: its first place and length (an upper bound with empty places)
+  auto span = [&](int64_t r, int64_t& p0, int& n) {
+    p0 = 0;
+    n = 0;
+    if (r >= n_rows) return;
+    if (c.fixed_k > 0) {
+      p0 = r * c.fixed_k;
+      n = c.fixed_k;
+    } else {
+      p0 = c.row_ptr[r];
+      n = (int)(c.row_ptr[r + 1] - (uint32_t)p0);
+    }
+  };
+  auto place = [&](int64_t p0, int n, int j) -> uint32_t { return j < n ? c.row_pos[p0 + j] : kNoSlot; };
   int64_t p0;
   int n;
-  row_span(c, rid, p0, n);
-  if (n * c.nsub < min_n) return;
-  const uint32_t* rp = c.row_pos + p0;
-  float m = -CUDART_INF_F;
-  for (int sb = 0; sb < c.nsub; ++sb)
-    for (int j = lane; j < n; j += 32)
-      if (rp[j] != kNoSlot) m = fmaxf(m, part_lse[(int64_t)sb * c.cap + rp[j] - c.slot_shift]);
+  span(rid, p0, n);
+  uint32_t slot_n = place(p0, n, gl);           // this lane's place of the list, a row ahead
+#pragma unroll 1
+  for (int64_t w0 = warp_first; w0 < n_rows; w0 += stride, rid += stride) {
+    const int64_t q0 = p0;
+    const int nr = n;
+    uint32_t slot = slot_n;
+    span(rid + stride, p0, n);
+    slot_n = place(p0, n, gl);
+    const int n_warp = __reduce_max_sync(0xffffffffu, nr);
+
+    float m = -CUDART_INF_F, ssum = 0.f, acc[8];
 #pragma unroll
-  for (int o = 16; o; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-  float2 acc[4];
+    for (int e = 0; e < 8; ++e) acc[e] = 0.f;
+    // places [b0, b0 + B) of the block of LPR places this lane's `s` belongs to, plane sb
+    auto request = [&](uint32_t s, int sb, int b0, uint4 (&x)[B]) {
 #pragma unroll
-  for (int i = 0; i < 4; ++i) acc[i] = make_float2(0.f, 0.f);
-  float ssum = 0.f;
-  if (m > -CUDART_INF_F) {
+      for (int k = 0; k < B; ++k) {
+        const uint32_t sk = __shfl_sync(0xffffffffu, s, b0 + k, LPR);
+        if (sk == kNoSlot) {
+          x[k] = make_uint4(0, 0, 0, 0);
+        } else {
+          const int64_t at = (int64_t)(sk - (uint32_t)c.slot_shift);
+          x[k] = ldg_nc_16(part + ((int64_t)sb * c.cap + at) * D + ((gl ^ (int)(at & 7)) * 8));
+        }
+      }
+    };
+    auto lse_of = [&](uint32_t s, int sb) {
+      return s == kNoSlot ? -CUDART_INF_F : part_lse[(int64_t)sb * c.cap + (int64_t)(s - (uint32_t)c.slot_shift)];
+    };
+    // the first batch is requested before the weights are known
+    uint4 x[B];
+    float l = FWD ? lse_of(slot, 0) : 0.f;
+    request(slot, 0, 0, x);
+    if (FWD) {
+      m = l;
+      for (int sb = 0; sb < c.nsub; ++sb)       // (longer lists and further planes)
+        for (int j0 = sb == 0 ? LPR : 0; j0 < n_warp; j0 += LPR)
+          m = fmaxf(m, lse_of(j0 == 0 ? slot : place(q0, nr, j0 + gl), sb));
+#pragma unroll
+      for (int o = LPR / 2; o; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+    }
     for (int sb = 0; sb < c.nsub; ++sb) {
-      int64_t last = -1;
-      for (int r = 0; r < n; ++r) {
-        const int64_t raw = next_slot(rp, n, last, lane);
-        if (raw >= (int64_t)kNoSlot) break;      // the remaining places of the row are empty
-        last = raw;
-        const int64_t slot = raw - c.slot_shift;
-        const int64_t pp = (int64_t)sb * c.cap + slot;
-        const float wgt = __expf(part_lse[pp] - m);
-        ssum += wgt;
-        const T* src = part_o + pp * c.d;
+      for (int j0 = 0; j0 < n_warp; j0 += LPR) {
+        const uint32_t s = j0 == 0 ? slot : place(q0, nr, j0 + gl);
+        float w = 1.f;
+        if (FWD) {
+          if (sb > 0 || j0 > 0) l = lse_of(s, sb);
+          w = (s != kNoSlot && m > -CUDART_INF_F) ? __expf(l - m) : 0.f;
+        }
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const int col = lane * 2 + i * 64;
-          if (col < c.d) {
-            const float2 x = Elem<T>::to_f2(*reinterpret_cast<const T2*>(src + part_col(slot, col, 8)));
-            acc[i].x = fmaf(wgt, x.x, acc[i].x);
-            acc[i].y = fmaf(wgt, x.y, acc[i].y);
+        for (int b0 = 0; b0 < LPR; b0 += B) {
+          if (j0 + b0 >= n_warp) break;         // warp-uniform
+          if (sb > 0 || j0 > 0 || b0 > 0) request(s, sb, b0, x);
+#pragma unroll
+          for (int k = 0; k < B; ++k) {
+            float f[8];
+            unpack8<T>(x[k], f);
+            if (FWD) {
+              const float wk = __shfl_sync(0xffffffffu, w, b0 + k, LPR);
+              ssum += wk;
+#pragma unroll
+              for (int e = 0; e < 8; ++e) acc[e] = fmaf(wk, f[e], acc[e]);
+            } else {
+#pragma unroll
+              for (int e = 0; e < 8; ++e) acc[e] += f[e];
+            }
           }
         }
       }
     }
-  }
-  const float inv = ssum > 0.f ? 1.f / ssum : 0.f;
-  const int h = c.h0 + hr;
-  T* dst = out + t * o_rs + (int64_t)h * o_hs;
+    if (rid < n_rows) {
+      const int hr = (int)(rid / c.total_q);
+      const int64_t t = rid - (int64_t)hr * c.total_q;
+      if (FWD) {
+        const float inv = ssum > 0.f ? 1.f / ssum : 0.f;
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int col = lane * 2 + i * 64;
-    if (col < c.d) *reinterpret_cast<T2*>(dst + col) = Elem<T>::from_f2(acc[i].x * inv, acc[i].y * inv);
-  }
-  if (lane == 0) lse[(int64_t)h * c.total_q + t] = ssum > 0.f ? m + logf(ssum) : CUDART_INF_F;
-}
-template <typename T>
-__global__ void __launch_bounds__(256) fwd_combine_kernel(const T* __restrict__ part_o,
-                                                          const float* __restrict__ part_lse, CombineParams c,
-                                                          T* out, int64_t o_rs, int64_t o_hs, float* lse,
-                                                          const int* only_if, int min_n, int64_t nvb) {
-  mirror_status(c);
-  if (only_if && *only_if == 0) return;   // the earlier stages met no row they had to leave
-  for (int64_t vb = blockIdx.x; vb < nvb; vb += gridDim.x)
-    fwd_combine_body<T>(vb, part_o, part_lse, c, out, o_rs, o_hs, lse, min_n);
-}
-
-template <typename T>
-__device__ __forceinline__ void bwd_combine_body(int64_t vblock, const T* __restrict__ part_dq, const CombineParams& c,
-                                                 T* dq, int64_t rs, int64_t hs, int min_n) {
-  using T2 = typename Elem<T>::T2;
-  const int64_t wid = (vblock * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  if (wid >= c.total_q * c.nh) return;
-  const int64_t t = wid / c.nh;
-  const int hr = (int)(wid - t * c.nh);
-  const int64_t rid = (int64_t)hr * c.total_q + t;
-  int64_t p0;
-  int n;
-  row_span(c, rid, p0, n);
-  if (n * c.nsub < min_n) return;
-  const uint32_t* rp = c.row_pos + p0;
-  float2 acc[4];
-#pragma unroll
-  for (int i = 0; i < 4; ++i) acc[i] = make_float2(0.f, 0.f);
-  for (int sb = 0; sb < c.nsub; ++sb) {
-    int64_t last = -1;
-    for (int r = 0; r < n; ++r) {
-      const int64_t raw = next_slot(rp, n, last, lane);
-      if (raw >= (int64_t)kNoSlot) break;        // the remaining places of the row are empty
-      last = raw;
-      const int64_t slot = raw - c.slot_shift;
-      const T* src = part_dq + ((int64_t)sb * c.cap + slot) * c.d;
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const int col = lane * 2 + i * 64;
-        if (col < c.d) {
-          const float2 x = Elem<T>::to_f2(*reinterpret_cast<const T2*>(src + part_col(slot, col, 8)));
-          acc[i].x += x.x;
-          acc[i].y += x.y;
-        }
+        for (int e = 0; e < 8; ++e) acc[e] *= inv;
+        if (gl == 0) lse[(int64_t)c.h0 * c.total_q + rid] = ssum > 0.f ? m + logf(ssum) : CUDART_INF_F;
       }
+      *reinterpret_cast<uint4*>(out + t * rs + (int64_t)(c.h0 + hr) * hs + gl * 8) = pack8<T>(acc);
     }
   }
-  T* dst = dq + t * rs + (int64_t)(c.h0 + hr) * hs;
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int col = lane * 2 + i * 64;
-    if (col < c.d) *reinterpret_cast<T2*>(dst + col) = Elem<T>::from_f2(acc[i].x, acc[i].y);
-  }
-}
-template <typename T>
-__global__ void __launch_bounds__(256) bwd_combine_kernel(const T* __restrict__ part_dq, CombineParams c, T* dq,
-                                                          int64_t rs, int64_t hs, const int* only_if, int min_n,
-                                                          int64_t nvb) {
-  mirror_status(c);
-  if (only_if && *only_if == 0) return;
-  for (int64_t vb = blockIdx.x; vb < nvb; vb += gridDim.x) bwd_combine_body<T>(vb, part_dq, c, dq, rs, hs, min_n);
-}
-
-// ------------------------------------------------------------------ fast combine (rows of <= G partials)
-// G lanes per (token, head) row, 32/G rows per warp.  Lane j of a group first fetches the plane
-// position (sb*cap + slot) and log-sum-exp of the row's j-th partial; the group ranks the positions
-// (merge order = ascending position, whatever order the atomics of the row-list build produced);
-// then every lane fetches its d/G elements of ALL the row's partial rows before the ordered
-// accumulation.  Several rows per warp and all loads of a row in flight at once hide the chain of
-// dependent, scattered reads.  Rows with more than G partials set *overflow and are left to the
-// next kernel (larger G, finally the generic one).
-template <int G>
-__device__ __forceinline__ unsigned group_mask(int lane) {
-  return G == 32 ? 0xffffffffu : (((1u << G) - 1u) << (lane & ~(G - 1)));
-}
-
-// common prologue: the row of this lane group and the plane position held by this lane
-struct GroupRow {
-  int64_t t; int hr; int64_t rid; int n; bool mine; bool valid; uint32_t pos; uint32_t slot;
-};
-template <int G>
-__device__ __forceinline__ GroupRow group_row(int64_t vblock, const CombineParams& c, int min_n, int* overflow) {
-  GroupRow g;
-  const int lane = threadIdx.x & 31, gl = lane & (G - 1);
-  const int64_t gid = ((vblock * blockDim.x + threadIdx.x) >> 5) * (32 / G) + (lane / G);
-  const bool row_ok = gid < c.total_q * c.nh;
-  g.t = row_ok ? gid / c.nh : 0;
-  g.hr = row_ok ? (int)(gid - g.t * c.nh) : 0;
-  g.rid = (int64_t)g.hr * c.total_q + g.t;
-  int64_t p0 = 0;
-  int n_e = 0;
-  if (row_ok) row_span(c, g.rid, p0, n_e);
-  g.n = n_e * c.nsub;                       // partials of the row
-  g.mine = row_ok && g.n >= min_n;          // rows below min_n were done by the previous kernel
-  if (g.n > G) {
-    if (gl == 0) *overflow = 1;
-    g.mine = false;
-  }
-  if (!g.mine) g.n = 0;
-  g.valid = gl < g.n;
-  g.slot = g.valid ? c.row_pos[p0 + gl / c.nsub] : 0u;
-  if (g.slot == kNoSlot) g.valid = false;      // an empty place of a handed-over row list
-  else g.slot -= (uint32_t)c.slot_shift;
-  g.pos = g.valid ? (uint32_t)((gl % c.nsub) * c.cap) + g.slot : 0xffffffffu;
-  return g;
-}
-
-template <typename T, int G, int EPL>
-__device__ __forceinline__ void fwd_combine_group_body(int64_t vblock, const T* __restrict__ part_o,
-                                                       const float* __restrict__ part_lse, const CombineParams& c,
-                                                       T* out, int64_t o_rs, int64_t o_hs, float* lse, int min_n,
-                                                       int* overflow) {
-  constexpr int d = G * EPL;
-  constexpr int NV = EPL / 8;                 // 16-byte loads per partial row per lane
-  static_assert(EPL % 8 == 0, "a lane owns whole 16-byte chunks");
-  const int lane = threadIdx.x & 31, gl = lane & (G - 1);
-  const unsigned gm = group_mask<G>(lane);
-  const GroupRow g = group_row<G>(vblock, c, min_n, overflow);
-  // the log-sum-exp of this lane's partial: requested first, used last (the partial rows are
-  // requested before anything waits for it, so that there is ONE round trip to memory, not two)
-  const float l = g.valid ? part_lse[g.pos] : -CUDART_INF_F;
-  int rank = 0;
-#pragma unroll
-  for (int i = 0; i < G; ++i) rank += (__shfl_sync(gm, g.pos, i, G) < g.pos) ? 1 : 0;
-  float acc[EPL];
-#pragma unroll
-  for (int i = 0; i < EPL; ++i) acc[i] = 0.f;
-  float ssum = 0.f;
-  float m = -CUDART_INF_F, w = 0.f;
-  constexpr int B = G < 8 ? G : 8;            // partial rows in flight per step
-#pragma unroll
-  for (int r0 = 0; r0 < G; r0 += B) {
-    uint4 x[B][NV];
-    int srcs[B];
-#pragma unroll
-    for (int k = 0; k < B; ++k) {
-      // the lane of this group whose partial has rank r0+k (none if the row is shorter).  Every
-      // partial row of a listed slot has been written (zeros for a row that saw no key), so it is
-      // fetched whatever its weight turns out to be.
-      const unsigned hit = __ballot_sync(0xffffffffu, g.valid && rank == r0 + k) & gm;
-      const int src = hit ? (__ffs(hit) - 1) : lane;
-      srcs[k] = hit ? src : -1;
-      const uint32_t pk = __shfl_sync(0xffffffffu, g.pos, src);
-      const uint32_t sk = __shfl_sync(0xffffffffu, g.slot, src);
-      if (hit) {
-        const T* row = part_o + (int64_t)pk * d;
-#pragma unroll
-        for (int v = 0; v < NV; ++v) x[k][v] = *reinterpret_cast<const uint4*>(row + part_col(sk, gl * EPL + 8 * v, 8));
-      } else {
-#pragma unroll
-        for (int v = 0; v < NV; ++v) x[k][v] = make_uint4(0, 0, 0, 0);
-      }
-    }
-    if (r0 == 0) {   // weights: the row maximum of the partial log-sum-exps
-      m = l;
-#pragma unroll
-      for (int o = G / 2; o; o >>= 1) m = fmaxf(m, __shfl_xor_sync(gm, m, o, G));
-      w = (g.valid && m > -CUDART_INF_F) ? __expf(l - m) : 0.f;
-    }
-#pragma unroll
-    for (int k = 0; k < B; ++k) {
-      // executed by every lane: groups of one warp differ in srcs[k] when their rows have
-      // different numbers of partials
-      const float w_src = __shfl_sync(0xffffffffu, w, srcs[k] < 0 ? lane : srcs[k]);
-      const float wk = srcs[k] < 0 ? 0.f : w_src;
-      ssum += wk;
-#pragma unroll
-      for (int v = 0; v < NV; ++v) {
-        float f[8];
-        unpack8<T>(x[k][v], f);
-#pragma unroll
-        for (int e = 0; e < 8; ++e) acc[8 * v + e] = fmaf(wk, f[e], acc[8 * v + e]);
-      }
-    }
-  }
-  if (g.mine) {
-    const float inv = ssum > 0.f ? 1.f / ssum : 0.f;
-    const int h = c.h0 + g.hr;
-    T* dst = out + g.t * o_rs + (int64_t)h * o_hs + gl * EPL;
-#pragma unroll
-    for (int v = 0; v < NV; ++v) {
-#pragma unroll
-      for (int e = 0; e < 8; ++e) acc[8 * v + e] *= inv;
-      *reinterpret_cast<uint4*>(dst + 8 * v) = pack8<T>(acc + 8 * v);
-    }
-    if (gl == 0) lse[(int64_t)h * c.total_q + g.t] = ssum > 0.f ? m + logf(ssum) : CUDART_INF_F;
-  }
-}
-template <typename T, int G, int EPL>
-__global__ void __launch_bounds__(256, EPL <= 8 ? 3 : 2) fwd_combine_group_kernel(const T* __restrict__ part_o,
-                                                                const float* __restrict__ part_lse,
-                                                                CombineParams c, T* out, int64_t o_rs, int64_t o_hs,
-                                                                float* lse, int min_n, const int* only_if,
-                                                                int* overflow, int64_t nvb) {
-  mirror_status(c);
-  if (only_if && *only_if == 0) return;
-  for (int64_t vb = blockIdx.x; vb < nvb; vb += gridDim.x)
-    fwd_combine_group_body<T, G, EPL>(vb, part_o, part_lse, c, out, o_rs, o_hs, lse, min_n, overflow);
-}
-
-template <typename T, int G, int EPL>
-__device__ __forceinline__ void bwd_combine_group_body(int64_t vblock, const T* __restrict__ part_dq,
-                                                       const CombineParams& c, T* dq, int64_t rs, int64_t hs,
-                                                       int min_n, int* overflow) {
-  constexpr int d = G * EPL;
-  constexpr int NV = EPL / 8;                 // 16-byte loads per partial row per lane
-  static_assert(EPL % 8 == 0, "a lane owns whole 16-byte chunks");
-  const int lane = threadIdx.x & 31, gl = lane & (G - 1);
-  const unsigned gm = group_mask<G>(lane);
-  const GroupRow g = group_row<G>(vblock, c, min_n, overflow);
-  int rank = 0;
-#pragma unroll
-  for (int i = 0; i < G; ++i) rank += (__shfl_sync(gm, g.pos, i, G) < g.pos) ? 1 : 0;
-  float acc[EPL];
-#pragma unroll
-  for (int i = 0; i < EPL; ++i) acc[i] = 0.f;
-  constexpr int B = G < 8 ? G : 8;            // partial rows in flight per step
-#pragma unroll
-  for (int r0 = 0; r0 < G; r0 += B) {
-    uint4 x[B][NV];
-#pragma unroll
-    for (int k = 0; k < B; ++k) {
-      const unsigned hit = __ballot_sync(0xffffffffu, g.valid && rank == r0 + k) & gm;
-      const int src = hit ? (__ffs(hit) - 1) : lane;
-      const uint32_t pk = __shfl_sync(0xffffffffu, g.pos, src);
-      const uint32_t sk = __shfl_sync(0xffffffffu, g.slot, src);
-      if (hit) {
-        const T* row = part_dq + (int64_t)pk * d;
-#pragma unroll
-        for (int v = 0; v < NV; ++v) x[k][v] = *reinterpret_cast<const uint4*>(row + part_col(sk, gl * EPL + 8 * v, 8));
-      } else {
-#pragma unroll
-        for (int v = 0; v < NV; ++v) x[k][v] = make_uint4(0, 0, 0, 0);
-      }
-    }
-#pragma unroll
-    for (int k = 0; k < B; ++k) {
-#pragma unroll
-      for (int v = 0; v < NV; ++v) {
-        float f[8];
-        unpack8<T>(x[k][v], f);
-#pragma unroll
-        for (int e = 0; e < 8; ++e) acc[8 * v + e] += f[e];
-      }
-    }
-  }
-  if (g.mine) {
-    T* dst = dq + g.t * rs + (int64_t)(c.h0 + g.hr) * hs + gl * EPL;
-#pragma unroll
-    for (int v = 0; v < NV; ++v) *reinterpret_cast<uint4*>(dst + 8 * v) = pack8<T>(acc + 8 * v);
-  }
-}
-template <typename T, int G, int EPL>
-__global__ void __launch_bounds__(256) bwd_combine_group_kernel(const T* __restrict__ part_dq, CombineParams c,
-                                                                T* dq, int64_t rs, int64_t hs, int min_n,
-                                                                const int* only_if, int* overflow, int64_t nvb) {
-  mirror_status(c);
-  if (only_if && *only_if == 0) return;
-  for (int64_t vb = blockIdx.x; vb < nvb; vb += gridDim.x)
-    bwd_combine_group_body<T, G, EPL>(vb, part_dq, c, dq, rs, hs, min_n, overflow);
-}
-
-// ------------------------------------------------------------------ wide combine (rows of <= 32 partials)
-// A warp per (token, head) row.  Lane j fetches the position and log-sum-exp of the row's j-th
-// partial and the warp ranks the positions, as above.  A partial row is D/8 16-byte chunks, so D/8
-// lanes fetch one partial row and the warp fetches 32/(D/8) partial rows per step, eight steps in
-// flight; lane group s accumulates the partials of rank s, s + 32/(D/8), ... in ascending order and
-// the groups are added at the end in a fixed order.  FWD weights the partials by
-// exp(lse_j - max lse) and writes the row's log-sum-exp; the backward form is a plain sum.
-template <typename T, int D, bool FWD>
-__device__ __forceinline__ void combine_wide_body(int64_t vblock, const T* __restrict__ part,
-                                                  const float* __restrict__ part_lse, const CombineParams& c,
-                                                  T* out, int64_t rs, int64_t hs, float* lse, int min_n,
-                                                  int* overflow) {
-  constexpr int LPR = D / 8;                  // lanes per partial row
-  constexpr int PPS = 32 / LPR;               // partial rows per step
-  constexpr int B = 8;                        // steps in flight
-  static_assert(D == 64 || D == 128 || D == 256, "a partial row is 8, 16 or 32 chunks");
-  const int lane = threadIdx.x & 31, sub = lane / LPR, ch = lane % LPR;
-  const GroupRow g = group_row<32>(vblock, c, min_n, overflow);
-  if (!g.mine) return;                        // the same for every lane of the warp
-  float l = -CUDART_INF_F;
-  if (FWD && g.valid) l = part_lse[g.pos];
-  int rank = 0;
-#pragma unroll
-  for (int i = 0; i < 32; ++i) rank += (__shfl_sync(0xffffffffu, g.pos, i) < g.pos) ? 1 : 0;
-  // the row's partials in use (a handed-over row list may have empty places: they rank last)
-  const int nv = __popc(__ballot_sync(0xffffffffu, g.valid));
-  int inv = 0;                                // the lane that holds the partial of rank `lane`
-#pragma unroll
-  for (int i = 0; i < 32; ++i) {
-    const int ri = __shfl_sync(0xffffffffu, rank, i);
-    const bool vi = (__shfl_sync(0xffffffffu, (int)g.valid, i) != 0);
-    if (vi && ri == lane) inv = i;
-  }
-  float m = 0.f, w = 1.f, ssum = 1.f;
-  if (FWD) {
-    m = l;
-#pragma unroll
-    for (int o = 16; o; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-    w = (g.valid && m > -CUDART_INF_F) ? __expf(l - m) : 0.f;
-    // summed with the weights in rank order: the order in which the row's partials sit in the
-    // lanes is that of the row list, which the atomics of its build leave undefined
-    const float w_ranked = __shfl_sync(0xffffffffu, w, inv);
-    ssum = lane < nv ? w_ranked : 0.f;
-#pragma unroll
-    for (int o = 16; o; o >>= 1) ssum += __shfl_xor_sync(0xffffffffu, ssum, o);
-  }
-  float acc[8];
-#pragma unroll
-  for (int e = 0; e < 8; ++e) acc[e] = 0.f;
-  for (int r0 = 0; r0 < nv; r0 += PPS * B) {
-    uint4 x[B];
-    float wk[B];
-#pragma unroll
-    for (int k = 0; k < B; ++k) {
-      const int want = r0 + k * PPS + sub;
-      const bool hit = want < nv;
-      const int src = __shfl_sync(0xffffffffu, inv, want & 31);
-      const uint32_t pk = __shfl_sync(0xffffffffu, g.pos, src);
-      const uint32_t sk = __shfl_sync(0xffffffffu, g.slot, src);
-      const float ws = __shfl_sync(0xffffffffu, w, src);
-      wk[k] = hit ? ws : 0.f;
-      x[k] = hit ? *reinterpret_cast<const uint4*>(part + (int64_t)pk * D + part_col(sk, ch * 8, 8))
-                 : make_uint4(0, 0, 0, 0);
-    }
-#pragma unroll
-    for (int k = 0; k < B; ++k) {
-      float f[8];
-      unpack8<T>(x[k], f);
-#pragma unroll
-      for (int e = 0; e < 8; ++e) acc[e] = FWD ? fmaf(wk[k], f[e], acc[e]) : acc[e] + f[e];   // x is 0 past the row's end
-    }
-  }
-#pragma unroll
-  for (int o = LPR; o < 32; o <<= 1) {
-#pragma unroll
-    for (int e = 0; e < 8; ++e) acc[e] += __shfl_xor_sync(0xffffffffu, acc[e], o);
-  }
-  const int h = c.h0 + g.hr;
-  if (sub == 0) {
-    const float inv_s = FWD ? (ssum > 0.f ? 1.f / ssum : 0.f) : 1.f;
-#pragma unroll
-    for (int e = 0; e < 8; ++e) acc[e] *= inv_s;
-    *reinterpret_cast<uint4*>(out + g.t * rs + (int64_t)h * hs + ch * 8) = pack8<T>(acc);
-  }
-  if (FWD && lane == 0) lse[(int64_t)h * c.total_q + g.t] = ssum > 0.f ? m + logf(ssum) : CUDART_INF_F;
-}
-template <typename T, int D, bool FWD>
-__global__ void __launch_bounds__(256) combine_wide_kernel(const T* __restrict__ part,
-                                                           const float* __restrict__ part_lse, CombineParams c,
-                                                           T* out, int64_t rs, int64_t hs, float* lse, int min_n,
-                                                           const int* only_if, int* overflow, int64_t nvb) {
-  mirror_status(c);
-  if (only_if && *only_if == 0) return;
-  for (int64_t vb = blockIdx.x; vb < nvb; vb += gridDim.x)
-    combine_wide_body<T, D, FWD>(vb, part, part_lse, c, out, rs, hs, lse, min_n, overflow);
 }
 
 // D[h, t] = sum_d dO.O.  LPR lanes per row, each with one 16-byte load of dO and of O (LPR = d / 8
@@ -751,11 +459,6 @@ __global__ void __launch_bounds__(256) dot_do_o_kernel(const T* __restrict__ dou
 }
 
 static int64_t warp_grid(int64_t warps) { return ceil_div64(warps, 8); }
-
-// Cascade: lane groups of 8 (rows of <= 8 partials), of 16 (<= 16, head dims of 128 and more), the
-// warp-per-row wide kernel (<= 32), then the generic kernel; each later stage runs only the rows the earlier ones left and exits at once if
-// there were none.
-static int64_t group_grid(int64_t rows, int G) { return ceil_div64(ceil_div64(rows, 32 / G), 8); }
 int sm_count() {
   int dev = 0, n = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0)
@@ -763,183 +466,37 @@ int sm_count() {
   return n;
 }
 
-// First cascade stage: persistent CTAs, as many as are resident (2 per SM at 128 registers); measured
-// at 64K tokens 0.24 ms per step faster than one CTA per block of rows (65,536 short-lived CTAs).
-// (Prefetching the next blocks' row lists inside the loop was tried and lost 0.7 ms to spills; with the
-// pattern builder's fixed-stride rows the prefetch is one register and changed nothing: 0.94 against
-// 0.92 ms in the backward combine, which reads its 4.8 GB at 80 % of the measured copy bandwidth.)
-static unsigned first_grid(int64_t nvb, int ctas_per_sm = 2) {
-  const int64_t cap = (int64_t)sm_count() * ctas_per_sm;
-  return (unsigned)(nvb < cap ? nvb : cap);
-}
-// grid of a later cascade stage: enough CTAs to fill the GPU if it does have work
-static unsigned late_grid(int64_t nvb) {
-  const int64_t cap = (int64_t)sm_count() * 8;
-  return (unsigned)(nvb < cap ? (nvb > 0 ? nvb : 1) : cap);
-}
-
-static CombineParams make_combine(const AttnArgs& a, const AttnWorkspace& w, const PassParams& ps) {
-  CombineParams c;
-  c.row_ptr = w.row_ptr; c.row_pos = w.row_pos; c.total_q = a.total_q; c.cap = w.cap; c.heads_out = a.heads;
-  c.h0 = ps.h0; c.nh = ps.nh; c.nsub = w.nsub; c.d = a.d;
+template <typename T, int D, bool FWD>
+static int merge_launch(const AttnArgs& a, const AttnWorkspace& w, const PassParams& ps, cudaStream_t s) {
+  MergeParams c;
+  c.row_ptr = w.row_ptr; c.row_pos = w.row_pos; c.total_q = a.total_q; c.cap = w.cap;
+  c.h0 = ps.h0; c.nh = ps.nh; c.nsub = w.nsub;
   c.fixed_k = w.fixed_k;
   c.slot_shift = ps.slot_shift;
   if (w.fixed_k > 0) c.row_pos = w.row_pos + (int64_t)ps.h0 * a.total_q * w.fixed_k;   // the pass's heads
   c.status = w.status;
   c.mirror = (ps.h0 + ps.nh >= a.heads) ? w.mirror : nullptr;   // the call's last pass
-  return c;
-}
-
-template <typename T, int D>
-static int fwd_combine_dispatch(const AttnArgs& a, const AttnWorkspace& w, const PassParams& ps, cudaStream_t s) {
-  const int64_t rows = a.total_q * ps.nh;
-  const CombineParams c = make_combine(a, w, ps);
-  int* ovf = w.status + 1;   // words 1..3 of the status block, zeroed with it
-  const T* po = (const T*)w.part_o;
-  T* out = (T*)a.o;
-  const int64_t nb8 = group_grid(rows, 8), nbw = warp_grid(rows);
-  if (c.fixed_k > 0) {   // every row has fixed_k * nsub places: the stage is known on the host, one launch
-    const int places = c.fixed_k * c.nsub;
-    // 8 lanes per row while a lane's share of a partial row is at most 32 bytes (at d = 128, 16 lanes
-    // for these rows: 1.57 ms against 1.21 ms at 64K; at d = 256, 8 lanes would hold 128 registers of
-    // loads in flight each: 3.5 ms against the 16-lane form's time for the same bytes)
-    if (places <= 8 && D <= 128) {
-      fwd_combine_group_kernel<T, 8, D / 8><<<first_grid(nb8), 256, 0, s>>>(po, w.part_lse, c, out, a.o_rs, a.o_hs, a.lse,
-                                                                          0, nullptr, ovf, nb8);
-      FMB_LAUNCH_CHECK("fwd_combine_group_kernel<8>");
-    } else if (D >= 128 && places <= 16) {
-      if constexpr (D >= 128) {
-        const int64_t nb16 = group_grid(rows, 16);
-        fwd_combine_group_kernel<T, 16, D / 16><<<first_grid(nb16, D / 16 <= 8 ? 3 : 2), 256, 0, s>>>(
-            po, w.part_lse, c, out, a.o_rs, a.o_hs, a.lse, 0, nullptr, ovf, nb16);
-        FMB_LAUNCH_CHECK("fwd_combine_group_kernel<16>");
-      }
-    } else if (places <= 32) {
-      combine_wide_kernel<T, D, true><<<late_grid(nbw), 256, 0, s>>>(po, w.part_lse, c, out, a.o_rs, a.o_hs, a.lse, 0,
-                                                                     nullptr, ovf, nbw);
-      FMB_LAUNCH_CHECK("combine_wide_kernel<fwd>");
-    } else {
-      fwd_combine_kernel<T><<<late_grid(nbw), 256, 0, s>>>(po, w.part_lse, c, out, a.o_rs, a.o_hs, a.lse, nullptr, 0, nbw);
-      FMB_LAUNCH_CHECK("fwd_combine_kernel");
-    }
-    return FMB_OK;
-  }
-  int* left = ovf;            // flag set by the stage before; rows of at least min_n partials are left
-  int min_n = 9;
-  if constexpr (D <= 128) {
-    fwd_combine_group_kernel<T, 8, D / 8><<<first_grid(nb8), 256, 0, s>>>(po, w.part_lse, c, out, a.o_rs, a.o_hs, a.lse, 0,
-                                                                        nullptr, ovf, nb8);
-    FMB_LAUNCH_CHECK("fwd_combine_group_kernel<8>");
-  }
-  if constexpr (D >= 128) {   // 16 lanes of a row own whole 16-byte chunks: two rows per warp
-    const int64_t nb16 = group_grid(rows, 16);
-    if constexpr (D <= 128)
-      fwd_combine_group_kernel<T, 16, D / 16><<<late_grid(nb16), 256, 0, s>>>(po, w.part_lse, c, out, a.o_rs, a.o_hs,
-                                                                             a.lse, 9, ovf, ovf + 1, nb16);
-    else                      // d = 256: the first stage
-      fwd_combine_group_kernel<T, 16, D / 16><<<first_grid(nb16), 256, 0, s>>>(po, w.part_lse, c, out, a.o_rs, a.o_hs,
-                                                                              a.lse, 0, nullptr, ovf + 1, nb16);
-    FMB_LAUNCH_CHECK("fwd_combine_group_kernel<16>");
-    left = ovf + 1;
-    min_n = 17;
-  }
-  combine_wide_kernel<T, D, true><<<late_grid(nbw), 256, 0, s>>>(po, w.part_lse, c, out, a.o_rs, a.o_hs, a.lse, min_n,
-                                                                 left, ovf + 2, nbw);
-  FMB_LAUNCH_CHECK("combine_wide_kernel<fwd>");
-  fwd_combine_kernel<T><<<late_grid(nbw), 256, 0, s>>>(po, w.part_lse, c, out, a.o_rs, a.o_hs, a.lse, ovf + 2, 33, nbw);
-  FMB_LAUNCH_CHECK("fwd_combine_kernel");
+  // persistent CTAs, as many as are resident
+  const int64_t ctas = ceil_div64(a.total_q * ps.nh, (kMergeThreads / 32) * (32 / (D / 8))), most = (int64_t)sm_count() * 3;
+  const unsigned grid = (unsigned)(ctas < most ? ctas : most);
+  if (FWD) merge_kernel<T, D, true><<<grid, kMergeThreads, 0, s>>>((const T*)w.part_o, w.part_lse, c, (T*)const_cast<void*>(a.o), a.o_rs, a.o_hs, a.lse);
+  else merge_kernel<T, D, false><<<grid, kMergeThreads, 0, s>>>((const T*)w.part_o, nullptr, c, (T*)a.dq, a.dq_rs, a.dq_hs, nullptr);
+  FMB_LAUNCH_CHECK(FWD ? "merge_kernel<fwd>" : "merge_kernel<bwd>");
   return FMB_OK;
 }
-
-template <typename T>
-static int fwd_combine_any(const AttnArgs& a, const AttnWorkspace& w, const PassParams& ps, cudaStream_t s) {
-  if (a.d == 64) return fwd_combine_dispatch<T, 64>(a, w, ps, s);
-  if (a.d == 128) return fwd_combine_dispatch<T, 128>(a, w, ps, s);
-  if (a.d == 256) return fwd_combine_dispatch<T, 256>(a, w, ps, s);
-  const int64_t rows = a.total_q * ps.nh;
-  fwd_combine_kernel<T><<<warp_grid(rows), 256, 0, s>>>((const T*)w.part_o, w.part_lse, make_combine(a, w, ps),
-                                                        (T*)a.o, a.o_rs, a.o_hs, a.lse, nullptr, 0, warp_grid(rows));
-  FMB_LAUNCH_CHECK("fwd_combine_kernel");
-  return FMB_OK;
-}
-
-int launch_fwd_combine(const AttnArgs& a, const AttnWorkspace& w, const PassParams& ps, cudaStream_t s) {
+template <bool FWD>
+static int launch_merge(const AttnArgs& a, const AttnWorkspace& w, const PassParams& ps, cudaStream_t s) {
   if (a.total_q * ps.nh == 0) return FMB_OK;
-  return a.dtype == FMB_BF16 ? fwd_combine_any<__nv_bfloat16>(a, w, ps, s) : fwd_combine_any<__half>(a, w, ps, s);
+  const bool bf = a.dtype == FMB_BF16;
+#define FMB_MERGE(D_) return bf ? merge_launch<__nv_bfloat16, D_, FWD>(a, w, ps, s) : merge_launch<__half, D_, FWD>(a, w, ps, s)
+  if (a.d == 64) FMB_MERGE(64);
+  if (a.d == 128) FMB_MERGE(128);
+  if (a.d == 256) FMB_MERGE(256);
+#undef FMB_MERGE
+  return fail(FMB_ERR_UNSUPPORTED, "attention: head_dim %d not built (64, 128 or 256)", a.d);
 }
-
-template <typename T, int D>
-static int bwd_combine_dispatch(const AttnArgs& a, const AttnWorkspace& w, const PassParams& ps, cudaStream_t s) {
-  const int64_t rows = a.total_q * ps.nh;
-  const CombineParams c = make_combine(a, w, ps);
-  int* ovf = w.status + 1;
-  const T* pd = (const T*)w.part_o;
-  T* dq = (T*)a.dq;
-  const int64_t nb8 = group_grid(rows, 8), nbw = warp_grid(rows);
-  if (c.fixed_k > 0) {   // every row has fixed_k * nsub places: the stage is known on the host, one launch
-    const int places = c.fixed_k * c.nsub;
-    if (places <= 8 && D <= 128) {
-      bwd_combine_group_kernel<T, 8, D / 8><<<first_grid(nb8), 256, 0, s>>>(pd, c, dq, a.dq_rs, a.dq_hs, 0, nullptr, ovf, nb8);
-      FMB_LAUNCH_CHECK("bwd_combine_group_kernel<8>");
-    } else if (D >= 128 && places <= 16) {
-      if constexpr (D >= 128) {
-        const int64_t nb16 = group_grid(rows, 16);
-        bwd_combine_group_kernel<T, 16, D / 16><<<first_grid(nb16), 256, 0, s>>>(pd, c, dq, a.dq_rs, a.dq_hs, 0, nullptr,
-                                                                                ovf, nb16);
-        FMB_LAUNCH_CHECK("bwd_combine_group_kernel<16>");
-      }
-    } else if (places <= 32) {
-      combine_wide_kernel<T, D, false><<<late_grid(nbw), 256, 0, s>>>(pd, nullptr, c, dq, a.dq_rs, a.dq_hs, nullptr, 0,
-                                                                      nullptr, ovf, nbw);
-      FMB_LAUNCH_CHECK("combine_wide_kernel<bwd>");
-    } else {
-      bwd_combine_kernel<T><<<late_grid(nbw), 256, 0, s>>>(pd, c, dq, a.dq_rs, a.dq_hs, nullptr, 0, nbw);
-      FMB_LAUNCH_CHECK("bwd_combine_kernel");
-    }
-    return FMB_OK;
-  }
-  int* left = ovf;
-  int min_n = 9;
-  if constexpr (D <= 128) {
-    bwd_combine_group_kernel<T, 8, D / 8><<<first_grid(nb8), 256, 0, s>>>(pd, c, dq, a.dq_rs, a.dq_hs, 0, nullptr, ovf, nb8);
-    FMB_LAUNCH_CHECK("bwd_combine_group_kernel<8>");
-  }
-  if constexpr (D >= 128) {
-    const int64_t nb16 = group_grid(rows, 16);
-    if constexpr (D <= 128)
-      bwd_combine_group_kernel<T, 16, D / 16><<<late_grid(nb16), 256, 0, s>>>(pd, c, dq, a.dq_rs, a.dq_hs, 9, ovf, ovf + 1,
-                                                                             nb16);
-    else
-      bwd_combine_group_kernel<T, 16, D / 16><<<first_grid(nb16), 256, 0, s>>>(pd, c, dq, a.dq_rs, a.dq_hs, 0, nullptr,
-                                                                              ovf + 1, nb16);
-    FMB_LAUNCH_CHECK("bwd_combine_group_kernel<16>");
-    left = ovf + 1;
-    min_n = 17;
-  }
-  combine_wide_kernel<T, D, false><<<late_grid(nbw), 256, 0, s>>>(pd, nullptr, c, dq, a.dq_rs, a.dq_hs, nullptr, min_n,
-                                                                  left, ovf + 2, nbw);
-  FMB_LAUNCH_CHECK("combine_wide_kernel<bwd>");
-  bwd_combine_kernel<T><<<late_grid(nbw), 256, 0, s>>>(pd, c, dq, a.dq_rs, a.dq_hs, ovf + 2, 33, nbw);
-  FMB_LAUNCH_CHECK("bwd_combine_kernel");
-  return FMB_OK;
-}
-
-template <typename T>
-static int bwd_combine_any(const AttnArgs& a, const AttnWorkspace& w, const PassParams& ps, cudaStream_t s) {
-  if (a.d == 64) return bwd_combine_dispatch<T, 64>(a, w, ps, s);
-  if (a.d == 128) return bwd_combine_dispatch<T, 128>(a, w, ps, s);
-  if (a.d == 256) return bwd_combine_dispatch<T, 256>(a, w, ps, s);
-  const int64_t rows = a.total_q * ps.nh;
-  bwd_combine_kernel<T><<<warp_grid(rows), 256, 0, s>>>((const T*)w.part_o, make_combine(a, w, ps), (T*)a.dq,
-                                                        a.dq_rs, a.dq_hs, nullptr, 0, warp_grid(rows));
-  FMB_LAUNCH_CHECK("bwd_combine_kernel");
-  return FMB_OK;
-}
-
-int launch_bwd_combine(const AttnArgs& a, const AttnWorkspace& w, const PassParams& ps, cudaStream_t s) {
-  if (a.total_q * ps.nh == 0) return FMB_OK;
-  return a.dtype == FMB_BF16 ? bwd_combine_any<__nv_bfloat16>(a, w, ps, s) : bwd_combine_any<__half>(a, w, ps, s);
-}
+int launch_fwd_combine(const AttnArgs& a, const AttnWorkspace& w, const PassParams& ps, cudaStream_t s) { return launch_merge<true>(a, w, ps, s); }
+int launch_bwd_combine(const AttnArgs& a, const AttnWorkspace& w, const PassParams& ps, cudaStream_t s) { return launch_merge<false>(a, w, ps, s); }
 
 template <typename T>
 static int dot_do_o_dispatch(const AttnArgs& a, cudaStream_t s) {
