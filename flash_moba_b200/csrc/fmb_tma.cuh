@@ -8,12 +8,6 @@
 
 namespace fmb {
 
-// 2-D tensor map over a row-major matrix of 16-bit elements: `cols` contiguous elements per
-// row, `rows` rows, rows `row_stride_bytes` apart; box = box_cols x box_rows; 128-byte swizzle
-// (box_cols must be 64); out-of-range elements read as zero.  Returns FMB_OK or an error.
-int make_tmap_2d(CUtensorMap* map, const void* base, int dtype, uint64_t cols, uint64_t rows,
-                 uint64_t row_stride_bytes, uint32_t box_cols, uint32_t box_rows);
-
 // 3-D tensor map over a (tokens, heads, d) tensor with arbitrary (16-byte aligned) token and head
 // strides: box = 64 elements of d x 1 head x box_rows tokens, 128-byte swizzle; elements past d and
 // tokens past `rows` read as zero.
@@ -27,16 +21,7 @@ __device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
                : "memory");
 }
 
-// box (box_cols x box_rows) whose first element is (x, y) -> shared memory
-__device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, int x, int y, uint64_t* bar) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
-      :
-      : "r"(smem_u32(dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(smem_u32(bar)), "r"(x), "r"(y)
-      : "memory");
-}
-
-// the same for a 3-D map: box at (x, head, row)
+// box whose first element is (x, head, row) -> shared memory
 __device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, int x, int head, int row, uint64_t* bar) {
   asm volatile(
       "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"

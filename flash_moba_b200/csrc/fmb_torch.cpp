@@ -18,6 +18,7 @@
 #include <cstring>
 #include <mutex>
 #include <optional>
+#include <string>
 #include <tuple>
 
 #include "../../include/flash_moba_b200.h"
@@ -27,10 +28,12 @@ namespace {
 using at::Tensor;
 using OptTensor = std::optional<Tensor>;
 
+// (Numbers in messages go through std::to_string: the streams behind TORCH_CHECK may be another C++
+// library's than this file's, and formatting an integer through them has crashed.)
 void check(int rc) {
   if (rc == FMB_OK) return;
   const char* msg = fmb_last_error();
-  if (msg == nullptr || msg[0] == 0) TORCH_CHECK(false, "flash_moba_b200 error ", rc);
+  if (msg == nullptr || msg[0] == 0) TORCH_CHECK(false, "flash_moba_b200 error ", std::to_string(rc));
   TORCH_CHECK(false, msg);
 }
 
@@ -87,7 +90,7 @@ StatusRing& ring() {
 void raise_for_status(int code, const char* what) {
   TORCH_CHECK(code != 7, "flash_moba_b200: ", what,
               ": the pattern does not fit the slots of a pass (overlapping columns, or raise FMB_WORKSPACE_GB)");
-  TORCH_CHECK(code == 0, "flash_moba_b200: ", what, ": a bounded device-side wait expired (code ", code, ")");
+  TORCH_CHECK(code == 0, "flash_moba_b200: ", what, ": a bounded device-side wait expired (code ", std::to_string(code), ")");
 }
 
 // looks at the words that have arrived; block: waits for all of them.  Called with the lock held.
@@ -344,8 +347,8 @@ std::tuple<Tensor, Tensor, OptTensor> attn_fwd(const Tensor& q, const Tensor& k,
   const int64_t total_q = q.size(0), h = q.size(1), d = q.size(2), hk = k.size(1), batch = cu_q.numel() - 1;
   TORCH_CHECK(p.col_offsets.size(0) == batch && p.col_offsets.size(1) == h, "pattern shape does not match (batch, heads)");
   const int64_t ncol = (max_k + chunk - 1) / chunk;
-  TORCH_CHECK(p.col_offsets.size(2) == ncol, "pattern has ", p.col_offsets.size(2),
-              " columns, expected ceil(max_seqlen_k/lg_block_n) = ", ncol);
+  TORCH_CHECK(p.col_offsets.size(2) == ncol, "pattern has ", std::to_string(p.col_offsets.size(2)),
+              " columns, expected ceil(max_seqlen_k/lg_block_n) = ", std::to_string(ncol));
   const int32_t* cuq = i32c(cu_q, "cu_seqlens_q");
   const int32_t* cuk = i32c(cu_k, "cu_seqlens_k");
   c10::cuda::CUDAGuard guard(q.device());
