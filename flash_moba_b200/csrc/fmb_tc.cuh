@@ -278,28 +278,30 @@ __device__ __forceinline__ void gather_cp_async(int t, unsigned char* tile, uint
   }
 }
 
-// 32 rows of NCHUNK*16 bytes gathered by one warp: this lane holds the element offset of row `lane` from
-// `base` (-1 = zero fill); tile: the first of the 32 rows (a multiple of 8) in the swizzled tile.  The offsets of four passes
+// 32 rows of NCHUNK*16 bytes gathered by one warp: this lane holds the offset of row `lane` from
+// `base` in units of 16 bytes (kNoRow = zero fill); tile: the first of the 32 rows (a multiple of 8) in the swizzled tile.  The offsets of four passes
 // are exchanged before the four copies are issued: shuffles and copies keep their order in the program, and a
 // shuffle's latency in front of every copy held a warp to 92 cycles per copy (5.3 B/clk) whatever else the SM
 // did; measured for whole tiles of 128 rows, B200.  The loop stays rolled: code size counts in these kernels.
-template <typename T, int NCHUNK>
-__device__ __forceinline__ void gather_rows32(int lane, unsigned char* tile, uint32_t block_stride, const T* base, int64_t off) {
+constexpr uint32_t kNoRow = 0xffffffffu;
+template <int NCHUNK>
+__device__ __forceinline__ void gather_rows32(int lane, unsigned char* tile, uint32_t block_stride, const void* base, uint32_t off) {
   constexpr int RPP = 32 / NCHUNK;           // rows per pass
   constexpr int GB = 4;                      // copies per turn of the loop
   const int j = lane % NCHUNK, rsub = lane / NCHUNK;
   const uint32_t dst = smem_u32(tile + (j >> 3) * block_stride) + rsub * 128;
-  const T* src = base + j * 8;
+  const char* src = static_cast<const char*>(base) + j * 16;
 #pragma unroll 1
   for (int i0 = 0; i0 < NCHUNK; i0 += GB) {
-    int64_t o[GB];
+    uint32_t o[GB];
 #pragma unroll
     for (int i = 0; i < GB; ++i) o[i] = __shfl_sync(0xffffffffu, off, (i0 + i) * RPP + rsub);
 #pragma unroll
     for (int i = 0; i < GB; ++i) {
       const int r = (i0 + i) * RPP;          // plus rsub
       const uint32_t d = dst + r * 128 + ((((uint32_t)j & 7) ^ ((r + rsub) & 7)) << 4);
-      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src + (o[i] < 0 ? 0 : o[i])), "r"(o[i] < 0 ? 0u : 16u)
+      const bool ok = o[i] != kNoRow;
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src + (size_t)(ok ? o[i] : 0u) * 16), "r"(ok ? 16u : 0u)
                    : "memory");
     }
   }
