@@ -2,27 +2,17 @@
 //
 // The kernels of fmb_attn_tc.cu keep dK and dV of a 128-key block in the SM's 512 TMEM columns,
 // which a head dim of 128 already fills, and their shared-memory tiles assume d <= 128.  Wider heads
-// run here (forward: key blocks of 128 keys where the chunk allows, else 64; backward: 64), in a
-// simpler shape: one CTA of 256 threads per work item (key block, head or kv head, sequence), every
-// thread takes part in every phase, one thread issues the MMAs, and the only overlap is the
-// cp.async gather of the next tile's rows under the rest of the current tile's work (the row
-// gathers, 512 bytes per row, bound these kernels).  Same workspace contract (slots, per-entry
-// partials) and the same merge kernels as the other engines.  Every mbarrier wait is bounded
-// (status word of the workspace).
+// run here (forward: key blocks of 128 keys where the chunk allows, else 64; backward: 64): one CTA per
+// work item (key block, head or kv head, sequence), described at each kernel.  Same workspace
+// contract (slots, per-entry partials) and the same merge kernels as the other engines.  Every mbarrier
+// wait is bounded (status word of the workspace).
 //
-// Forward, per tile of 128 gathered query rows:
-//     S = Q.K^T (K dimension d)  ->  the Q tile is refilled with the next tile's rows
-//     chunk-local softmax in one pass (32 or 64 scores per thread), P (I/O dtype) to shared memory
-//     O = P.V  (N = d)           ->  O / l written from registers (256 contiguous bytes per thread)
-// Backward (head dim 256), work item = key block of one kv head, tiles = the q heads of its group
-// times the 128-row tiles of each head's column.  dK and dV are accumulated TRANSPOSED (TMEM lane =
-// head-dim index, two halves of 128; column = key), which takes 2 x 128 columns instead of the
-// 2 x 256 of a key-per-lane layout; S | dP share 128 columns with the two halves of dQ, which are
-// computed and written one after the other:
-//     S = Q.K^T, dP = dO.V^T -> P = exp2(S.scale - LSE), dS = P o (dP - D) to shared memory
-//     dV^T += dO^T.P, dK^T += Q^T.dS (Q, dO as M-major A operands), dQ = dS.K per half
-//     once those have completed the Q and dO tiles are refilled with the next tile's rows while the
-//     dQ halves are read out and written from registers
+// dK and dV are accumulated TRANSPOSED (TMEM lane = head-dim index, two halves of 128; column = key), which takes
+// 2 x 128 columns instead of the 2 x 256 of a key-per-lane layout.
+// Measured (B200, 16K tokens in three sequences, 16 / 4 heads, chunk 128, top-k 8; the kernels before, in which every
+// thread took part in every phase / these): backward 1830 / 1120 us.  Of that: gathers that read their
+// row numbers ahead of the copies 3 - 5 %; long columns first 5 - 7 %; MMA issue in turns of four instructions, not
+// fully unrolled, 17 % of the backward (sixteen unrolled ones took 2850 cycles to issue, in turns 1050).
 #include "fmb_attn.cuh"
 #include "fmb_tc.cuh"
 
@@ -47,10 +37,59 @@ struct WideParams {
   void* part_o; float* part_lse; int* status;
   int heads, heads_k; int64_t total_q;
   float scale; int causal;
+  // one CTA per item (key block, head or kv head, sequence); the first `items_heavy` key blocks of every head (under a
+  // causal mask the longest columns) come before all others, which follow one head after the other
+  int items_x, items_y, items_z, items_heavy;
 };
+
+struct WideItem { int c, sb, y, b; };           // chunk, key block in it, head or kv head of the pass, sequence
+__device__ __forceinline__ WideItem wide_item(const WideParams& p) {
+  const int yz = p.items_y * p.items_z, heavy = p.items_heavy * yz, item = blockIdx.x;
+  int bx, rem;
+  if (item < heavy) {
+    bx = item / yz;
+    rem = item - bx * yz;
+  } else {
+    const int rest = p.items_x - p.items_heavy;
+    rem = (item - heavy) / rest;
+    bx = p.items_heavy + (item - heavy - rem * rest);
+  }
+  return WideItem{bx / p.ps.nsub, bx % p.ps.nsub, rem % p.items_y, rem / p.items_y};
+}
 
 // threads that take part in the 16-byte copies of rows of D elements: eight rows per pass
 template <int D> struct Copiers { static constexpr int n = (D / 8) * 8; };
+
+// 16 rows of NCHUNK*16 bytes gathered by one warp: lanes 0-15 (and again 16-31) hold the rows' numbers (-1 = zero fill);
+// see gather_rows32()
+template <int NCHUNK, typename T>
+__device__ __forceinline__ void gather_rows16(int lane, unsigned char* tile, uint32_t block_stride, const T* base, int64_t rs, int row) {
+  static_assert(NCHUNK == 32, "a warp copies a row at a time");
+  constexpr int GB = 4;                         // copies per turn of the loop
+  const uint32_t dst = smem_u32(tile + (lane >> 3) * block_stride);
+  const T* src = base + lane * 8;
+#pragma unroll 1
+  for (int i0 = 0; i0 < 16; i0 += GB) {
+    int o[GB];
+#pragma unroll
+    for (int i = 0; i < GB; ++i) o[i] = __shfl_sync(0xffffffffu, row, i0 + i);
+#pragma unroll
+    for (int i = 0; i < GB; ++i) {
+      const int r = i0 + i;
+      const uint32_t d = dst + r * 128 + ((((uint32_t)lane & 7) ^ (r & 7)) << 4);
+      const bool ok = o[i] >= 0;
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src + (int64_t)(ok ? o[i] : 0) * rs), "r"(ok ? 16u : 0u)
+                   : "memory");
+    }
+  }
+}
+
+// 32 bytes (aligned to 32) in one store: a lane that writes a row of its own then fills whole sectors
+__device__ __forceinline__ void st_global_32(void* dst, uint4 a, uint4 b) {
+  asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(dst), "r"(a.x), "r"(a.y), "r"(a.z), "r"(a.w),
+               "r"(b.x), "r"(b.y), "r"(b.z), "r"(b.w)
+               : "memory");
+}
 
 template <typename T, int C, int D>
 __global__ void __launch_bounds__(kThreads) fwd_wide_tc_kernel(WideParams p) {
@@ -79,7 +118,8 @@ __global__ void __launch_bounds__(kThreads) fwd_wide_tc_kernel(WideParams p) {
 
   const int tid = threadIdx.x, warp = tid >> 5;
   const int lt = tid & (kM - 1), hf = tid >> 7;
-  const int c = blockIdx.x / p.ps.nsub, sb = blockIdx.x % p.ps.nsub, h = p.ps.h0 + blockIdx.y, b = blockIdx.z;
+  const WideItem item = wide_item(p);
+  const int c = item.c, sb = item.sb, h = p.ps.h0 + item.y, b = item.b;
   const ColRef col = column_of(p.ps, b, h, c);
   if (col.nnz <= 0) return;                     // CTA-uniform
   const int64_t slot0 = (int64_t)sb * p.ps.cap + col.slot;
@@ -225,19 +265,34 @@ __global__ void __launch_bounds__(kThreads) fwd_wide_tc_kernel(WideParams p) {
   if (warp == 0) tmem_dealloc(tmem_base, 512);
 }
 
+// ---- backward
+// Work item = key block of 64 keys of one (sequence, kv head); one CTA per item; 768 threads, warp-specialised:
+//   warps 0-7    compute: TMEM lane = gathered row, warps w and w + 4 split the keys in halves.  P and dS of a tile; at
+//                the end the item's dK and dV.
+//   warps 8-11   drain: the tile's two dQ halves from TMEM to the entries' slots, from registers, 32 bytes a store.
+//   warp 12      one thread issues every MMA.
+//   warps 16-23  loaders: each fetches 16 of a tile's Q rows and 16 of its dO rows.
+// Q and dO of one tile, K, V, P and dS fill the shared memory, so a tile's rows can only be fetched once the GEMMs that
+// read the tile before have completed: dK^T += Q^T.dS is issued first (Q is what the next tile starts with), dV^T += dO^T.P
+// behind it, then dQ, whose two halves share 128 TMEM columns: the second is issued behind the next tile's dP.
+// What bounds it is that cycle: gather of Q, S, P (dP beside it), dS, dK.
+constexpr int kBwDrainWarp = 8, kBwIssuerWarp = 12, kBwLoadWarp = 16, kBwLoaders = 8, kBwThreads = 768;
+// registers per thread: launched with 80 (65536 / 768 rounded down to a multiple of 8)
+constexpr int kBwRegsLaunch = 80, kBwRegsCompute = 112, kBwRegsOther = 64;
+static_assert(2 * (kBwRegsCompute - kBwRegsLaunch) <= 4 * (kBwRegsLaunch - kBwRegsOther), "registers requested <= registers released");
+
 template <typename T, int D>
-__global__ void __launch_bounds__(kThreads) bwd_wide_tc_kernel(WideParams p) {
+__global__ void __launch_bounds__(kBwThreads, 1) bwd_wide_tc_kernel(WideParams p) {
   static_assert(D == 256, "two head-dim halves of 128 TMEM lanes");
   constexpr int NCH = D / 8;
-  constexpr int NT = Copiers<D>::n;
   constexpr uint32_t kKBlock = kC * 128;
   constexpr uint32_t kQBlock = kM * 128;
   constexpr uint32_t kQTile = kM * D * 2;
   extern __shared__ __align__(1024) unsigned char smem_raw[];
-  __shared__ uint64_t bar_a, bar_b, bar_c;
+  __shared__ uint64_t bar_fullq, bar_fulldo, bar_s, bar_p, bar_ds, bar_dk, bar_dv, bar_dq[2], bar_dqfree, bar_fin;
   __shared__ uint32_t tmem_base_s;
-  __shared__ int sRow[kM];
-  __shared__ float sLse[kM], sDsum[kM];
+  __shared__ int sRow[kM];                      // query rows of the tile
+  __shared__ float sLse[kM], sDsum[kM];         // their log-sum-exps and dO.O sums
 
   // the tiles fill the 227 KB together with the static arrays above: no room for alignment padding
   unsigned char* smem = smem_raw;
@@ -252,10 +307,10 @@ __global__ void __launch_bounds__(kThreads) bwd_wide_tc_kernel(WideParams p) {
   unsigned char* sP = sdO + kQTile;             // [128][64]
   unsigned char* sdS = sP + kM * kC * 2;        // [128][64]
 
-  const int tid = threadIdx.x, warp = tid >> 5;
-  const int lt = tid & (kM - 1), hf = tid >> 7;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int group = p.heads / p.heads_k;
-  const int c = blockIdx.x / p.ps.nsub, sb = blockIdx.x % p.ps.nsub, hk = p.ps.h0 / group + blockIdx.y, b = blockIdx.z;
+  const WideItem item = wide_item(p);
+  const int c = item.c, sb = item.sb, hk = p.ps.h0 / group + item.y, b = item.b;
   const int64_t plane = (int64_t)sb * p.ps.cap;
   const int q0 = p.cu_q[b], len_q = p.cu_q[b + 1] - q0;
   const int k0 = p.k_begin[b], len_k = p.k_end[b] - k0;
@@ -267,42 +322,32 @@ __global__ void __launch_bounds__(kThreads) bwd_wide_tc_kernel(WideParams p) {
   }
   const int keys_valid = min(kC, len_k - key0);
   const int shift = len_k - len_q;
-  const float scale_log2 = p.scale * kLog2e;
 
   if (warp == 0) tmem_alloc(&tmem_base_s, 512);
   if (tid == 0) {
-    mbar_init(&bar_a, 1);
-    mbar_init(&bar_b, 1);
-    mbar_init(&bar_c, 1);
+    mbar_init(&bar_fullq, kBwLoaders); mbar_init(&bar_fulldo, kBwLoaders);   // one arrival per loader warp
+    mbar_init(&bar_s, 1); mbar_init(&bar_p, 1); mbar_init(&bar_dk, 1); mbar_init(&bar_dv, 1);
+    mbar_init(&bar_dq[0], 1); mbar_init(&bar_dq[1], 1); mbar_init(&bar_fin, 1);
+    mbar_init(&bar_ds, 8);                      // one arrival per compute warp
+    mbar_init(&bar_dqfree, 4);                  // one arrival per drain warp
     mbar_fence_init();
   }
-  if (tid < NT) {
+  if (tid < 512) {
     const T* kbase = static_cast<const T*>(p.k) + (int64_t)(k0 + key0) * p.k_rs + (int64_t)hk * p.k_hs;
     const T* vbase = static_cast<const T*>(p.v) + (int64_t)(k0 + key0) * p.v_rs + (int64_t)hk * p.v_hs;
-    dense_cp_async<T, NCH, kC, NT>(tid, sK, kKBlock, kbase, p.k_rs, keys_valid);
-    dense_cp_async<T, NCH, kC, NT>(tid, sV, kKBlock, vbase, p.v_rs, keys_valid);
+    dense_cp_async<T, NCH, kC, 512>(tid, sK, kKBlock, kbase, p.k_rs, keys_valid);
+    dense_cp_async<T, NCH, kC, 512>(tid, sV, kKBlock, vbase, p.v_rs, keys_valid);
+    cp_async_wait_all();
+    fence_async_smem();
   }
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = tmem_base_s;
-  const uint32_t tS = tmem_base, tdP = tmem_base + 64, tdQ = tmem_base;      // dQ halves over S | dP
-  const uint32_t tdK = tmem_base + 128, tdV = tmem_base + 256;                // [half][64 keys]
-  const uint32_t lane_sel = (uint32_t)((warp & 3) * 32) << 16;
-  constexpr uint32_t idesc_s = make_idesc(FmtOf<T>::v, kM, kC, 0, 0);         // rows x keys
-  constexpr uint32_t idesc_t = make_idesc(FmtOf<T>::v, 128, kC, 1, 1);        // head-dim half x keys, both M/N-major
-  constexpr uint32_t idesc_dq = make_idesc(FmtOf<T>::v, kM, 128, 0, 1);       // rows x head-dim half
-  const uint32_t hi = desc_hi_sw128(1024);
-  const uint32_t k_km = desc_lo_sw128(smem_u32(sK), 16), v_km = desc_lo_sw128(smem_u32(sV), 16);
-  const uint32_t q_km = desc_lo_sw128(smem_u32(sQ), 16), do_km = desc_lo_sw128(smem_u32(sdO), 16);
-  const uint32_t ds_km = desc_lo_sw128(smem_u32(sdS), 16);
-  const uint32_t p_mn = desc_lo_sw128(smem_u32(sP), kQBlock), ds_mn = desc_lo_sw128(smem_u32(sdS), kQBlock);
-  bool good = true;
-  uint32_t g = 0;                               // tiles so far (phase of the three barriers)
+  const uint32_t tS = tmem_base, tdP = tmem_base + 64, tdQ = tmem_base + 128;
+  const uint32_t tdK = tmem_base + 256, tdV = tmem_base + 384;                // [half][64 keys]
 
-  // The item's tiles as one sequence over the q heads of the group and the 128-row tiles of each
-  // head's column: `cur` is the tile being worked on, `nxt` the one whose rows are gathered under
-  // the end of it.
+  // The item's tiles as one sequence over the q heads of the group and the 128-row tiles of each head's column
   struct Tile { int hg, t0, nnz; int64_t off, slot; bool valid; };
   auto seek = [&](Tile& t) {                    // first head >= t.hg with a column; t.t0 = 0
     t.valid = false;
@@ -311,171 +356,228 @@ __global__ void __launch_bounds__(kThreads) bwd_wide_tc_kernel(WideParams p) {
       if (col.nnz > 0) { t.nnz = col.nnz; t.off = col.off; t.slot = col.slot; t.t0 = 0; t.valid = true; return; }
     }
   };
-  auto advance = [&](Tile t) {
-    t.t0 += kM;
-    if (t.t0 >= t.nnz) { ++t.hg; seek(t); }
+  auto first = [&] {
+    Tile t{0, 0, 0, 0, 0, false};
+    seek(t);
     return t;
   };
-  // row ids, log-sum-exps and dO.O sums of a tile into shared memory (the first 128 threads)
-  auto load_rows = [&](const Tile& t) {
-    if (tid < kM) {
-      int r = -1;
+  auto advance = [&](Tile& t) {
+    t.t0 += kM;
+    if (t.t0 >= t.nnz) { ++t.hg; seek(t); }
+  };
+  auto count = [&] {                            // tiles of the item
+    int n = 0;
+    for (int hg = 0; hg < group; ++hg) n += (column_of(p.ps, b, hk * group + hg, c).nnz + kM - 1) / kM;
+    return n;
+  };
+  auto wait_all = [&](uint64_t* bar, uint32_t parity, int where) -> bool {   // the same answer for the whole warp
+    return __all_sync(0xffffffffu, mbar_wait(bar, parity & 1u, p.status, where));
+  };
+
+  if (warp >= kBwLoadWarp) {
+    // =============================================================== loaders
+    reg_dec<kBwRegsOther>();
+    const int row0 = (warp - kBwLoadWarp) * 16, i = row0 + (lane & 15);   // this lane's row (lanes in pairs)
+    uint32_t g = 0;
+    Tile t = first();
+    auto entry = [&](const Tile& x) { return x.valid && x.t0 + i < x.nnz ? ldg_s32_here(p.ps.indices + x.off + x.t0 + i) : -1; };
+    int raw = entry(t);
+#pragma unroll 1
+    for (; t.valid; ++g) {
+      const int r = (raw < 0 || raw >= len_q) ? -1 : raw, h = hk * group + t.hg;
+      const T* qbase = static_cast<const T*>(p.q) + (int64_t)q0 * p.q_rs + (int64_t)h * p.q_hs;
+      const T* obase = static_cast<const T*>(p.dout) + (int64_t)q0 * p.do_rs + (int64_t)h * p.do_hs;
       float l = CUDART_INF_F, dd = 0.f;
-      if (t.valid && t.t0 + tid < t.nnz) {
-        r = p.ps.indices[t.off + t.t0 + tid];
-        if (r < 0 || r >= len_q) r = -1;
-        else {
-          const int64_t at = (int64_t)(hk * group + t.hg) * p.total_q + q0 + r;
-          l = p.lse[at];
-          dd = p.softmax_d[at];
+      if (r >= 0) {
+        const int64_t at = (int64_t)h * p.total_q + q0 + r;
+        l = p.lse[at];
+        dd = p.softmax_d[at];
+      }
+      advance(t);
+      raw = entry(t);                           // the next tile's, in flight meanwhile
+      // dK of the tile before has read the Q tile (and, before that, the compute warps the row data)
+      if (g > 0 && !wait_all(&bar_dk, g - 1, 5)) break;
+      gather_rows16<NCH>(lane, sQ + row0 * 128, kQBlock, qbase, p.q_rs, r);
+      asm volatile("cp.async.commit_group;" ::: "memory");
+      if (lane < 16) { sRow[i] = r; sLse[i] = l; sDsum[i] = dd; }
+      if (g > 0 && !wait_all(&bar_dv, g - 1, 5)) break;   // dV has read the dO tile
+      gather_rows16<NCH>(lane, sdO + row0 * 128, kQBlock, obase, p.do_rs, r);
+      asm volatile("cp.async.commit_group;" ::: "memory");
+      asm volatile("cp.async.wait_group 1;" ::: "memory");
+      fence_async_smem();                       // the copies are generic-proxy writes; the MMAs read through the async proxy
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&bar_fullq);
+      asm volatile("cp.async.wait_group 0;" ::: "memory");
+      fence_async_smem();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&bar_fulldo);
+    }
+    cp_async_wait_all();
+  } else if (warp >= kBwIssuerWarp) {
+    // =============================================================== MMA issuer
+    reg_dec<kBwRegsOther>();
+    if (warp == kBwIssuerWarp && lane == 0) {
+      constexpr uint32_t idesc_s = make_idesc(FmtOf<T>::v, kM, kC, 0, 0);         // rows x keys
+      constexpr uint32_t idesc_t = make_idesc(FmtOf<T>::v, 128, kC, 1, 1);        // head-dim half x keys, both M/N-major
+      constexpr uint32_t idesc_dq = make_idesc(FmtOf<T>::v, kM, 128, 0, 1);       // rows x head-dim half
+      const uint32_t hi = desc_hi_sw128(1024);
+      const uint32_t k_km = desc_lo_sw128(smem_u32(sK), 16), v_km = desc_lo_sw128(smem_u32(sV), 16);
+      const uint32_t k_mn = desc_lo_sw128(smem_u32(sK), kKBlock);
+      const uint32_t q_km = desc_lo_sw128(smem_u32(sQ), 16), do_km = desc_lo_sw128(smem_u32(sdO), 16);
+      const uint32_t q_mn = desc_lo_sw128(smem_u32(sQ), kQBlock), do_mn = desc_lo_sw128(smem_u32(sdO), kQBlock);
+      const uint32_t ds_km = desc_lo_sw128(smem_u32(sdS), 16);
+      const uint32_t p_mn = desc_lo_sw128(smem_u32(sP), kQBlock), ds_mn = desc_lo_sw128(smem_u32(sdS), kQBlock);
+      const uint32_t ntiles = (uint32_t)count();
+      bool ok = true;
+      // the second dQ half of tile g, once the first has been read out
+      auto dq_second = [&] {
+        if (!mbar_wait(&bar_dqfree, 0, p.status, 6)) return false;   // phase 2 g: the first half of tile g
+        tc_fence_after_sync();
+        umma_gemm<kC / 16>(tdQ, ds_km, hi, 2, 0, k_mn + (2 * kKBlock >> 4), hi, 128, 512, idesc_dq, 0);
+        umma_commit(&bar_dq[1]);
+        return true;
+      };
+#pragma unroll 1
+      for (uint32_t g = 0; g <= ntiles && ok; ++g) {
+        if (g < ntiles) {
+          // S(g) and dP(g): their columns were read before dS(g - 1) was ready
+          if (!(ok = mbar_wait(&bar_fullq, g & 1, p.status, 6))) break;
+          tc_fence_after_sync();
+          umma_gemm<D / 16>(tS, q_km, hi, 2, kQBlock >> 4, k_km, hi, 2, kKBlock >> 4, idesc_s, 0);
+          umma_commit(&bar_s);
+          if (!(ok = mbar_wait(&bar_fulldo, g & 1, p.status, 6))) break;
+          tc_fence_after_sync();
+          umma_gemm<D / 16>(tdP, do_km, hi, 2, kQBlock >> 4, v_km, hi, 2, kKBlock >> 4, idesc_s, 0);
+          umma_commit(&bar_p);
+        }
+        if (g > 0 && !(ok = dq_second())) break;
+        if (g == ntiles) break;
+        if (!(ok = mbar_wait(&bar_ds, g & 1, p.status, 6))) break;
+        tc_fence_after_sync();
+        const uint32_t acc = g > 0 ? 1u : 0u;   // the item's first tile starts the accumulators
+        // dK^T[half] += Q^T.dS, dV^T[half] += dO^T.P : M = 128 head-dim columns, N = keys, K = the rows
+#pragma unroll
+        for (int hh = 0; hh < 2; ++hh)
+          umma_gemm<kM / 16>(tdK + hh * 64, q_mn + hh * (2 * kQBlock >> 4), hi, 128, 512, ds_mn, hi, 128, 512, idesc_t, acc);
+        umma_commit(&bar_dk);
+#pragma unroll
+        for (int hh = 0; hh < 2; ++hh)
+          umma_gemm<kM / 16>(tdV + hh * 64, do_mn + hh * (2 * kQBlock >> 4), hi, 128, 512, p_mn, hi, 128, 512, idesc_t, acc);
+        umma_commit(&bar_dv);
+        // first half of dQ = dS.K, once the second half of the tile before has been read out (phase 2 g - 1 of bar_dqfree)
+        if (g > 0 && !(ok = mbar_wait(&bar_dqfree, 1, p.status, 6))) break;
+        tc_fence_after_sync();
+        umma_gemm<kC / 16>(tdQ, ds_km, hi, 2, 0, k_mn, hi, 128, 512, idesc_dq, 0);
+        umma_commit(&bar_dq[0]);
+      }
+      if (ok) umma_commit(&bar_fin);
+    }
+  } else if (warp >= kBwDrainWarp) {
+    // =============================================================== drain warps
+    reg_dec<kBwRegsOther>();
+    const uint32_t at = (uint32_t)((warp & 3) * 32) << 16;
+    const int lt = tid & (kM - 1);
+    bool good = true;
+    uint32_t g = 0;
+#pragma unroll 1
+    for (Tile t = first(); t.valid && good; advance(t), ++g) {
+      const bool mine = lt < t.nnz - t.t0;
+      const int64_t slot = plane + t.slot + t.t0 + lt;
+      const int key = (int)(slot & 7);
+      T* dst = part_dq + slot * D;
+      // ---- dQ partial of row `lt`: scaled, rounded, 16-byte chunks permuted like every partial; a 32-byte store takes
+      // a pair of neighbouring chunks
+#pragma unroll 1
+      for (int hh = 0; hh < 2; ++hh) {
+        if (!(good = wait_all(&bar_dq[hh], g, 4))) break;
+        tc_fence_after_sync();
+#pragma unroll 1
+        for (int i2 = 0; i2 < 4; ++i2) {
+          float o[32];
+          tmem_ld32(tdQ + at + i2 * 32, o);
+          tmem_ld_wait();
+          if (i2 == 3) {
+            tc_fence_before_sync();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&bar_dqfree);
+          }
+#pragma unroll
+          for (int e = 0; e < 32; ++e) o[e] *= p.scale;
+#pragma unroll
+          for (int jj = 0; jj < 4; jj += 2) {
+            const uint4 u = pack8<T>(o + jj * 8), v = pack8<T>(o + jj * 8 + 8);
+            const int ch = hh * 16 + i2 * 4 + jj;
+            if (mine) st_global_32(dst + (((ch ^ key) & ~1) << 3), (key & 1) ? v : u, (key & 1) ? u : v);
+          }
         }
       }
-      sRow[tid] = r; sLse[tid] = l; sDsum[tid] = dd;
     }
-  };
-  auto gather = [&](const Tile& t) {
-    if (tid < NT) {
-      const int h = hk * group + t.hg;
-      gather_cp_async<T, NCH, NT>(tid, sQ, kQBlock, static_cast<const T*>(p.q) + (int64_t)q0 * p.q_rs + (int64_t)h * p.q_hs,
-                                  p.q_rs, sRow);
-      gather_cp_async<T, NCH, NT>(tid, sdO, kQBlock,
-                                  static_cast<const T*>(p.dout) + (int64_t)q0 * p.do_rs + (int64_t)h * p.do_hs, p.do_rs, sRow);
-    }
-  };
-  Tile cur{0, 0, 0, 0, 0, false};
-  seek(cur);
-  if (cur.valid) {
-    load_rows(cur);
-    __syncthreads();
-    gather(cur);
-  }
+  } else {
+    // =============================================================== compute warps
+    reg_inc<kBwRegsCompute>();
+    const int lt = tid & (kM - 1), hf = tid >> 7;
+    const uint32_t lane_sel = (uint32_t)((warp & 3) * 32) << 16;
+    const float scale_log2 = p.scale * kLog2e;
+    const uint32_t ntiles = (uint32_t)count();
+    bool good = true;
 #pragma unroll 1
-  for (; cur.valid; ++g) {
-    const int rows = min(kM, cur.nnz - cur.t0);
-    const int64_t slot0 = plane + cur.slot + cur.t0;
-    cp_async_wait_all();                        // Q and dO rows of the tile (and K, V on the item's first)
-    fence_async_smem();
-    tc_fence_before_sync();
-    good = __syncthreads_and(good);             // (a wait that gave up in the tile before ends the loop for every thread)
-    if (!good) break;
-    tc_fence_after_sync();
-    if (tid == 0) {
-      umma_gemm<D / 16>(tS, q_km, hi, 2, kQBlock >> 4, k_km, hi, 2, kKBlock >> 4, idesc_s, 0);
-      umma_gemm<D / 16>(tdP, do_km, hi, 2, kQBlock >> 4, v_km, hi, 2, kKBlock >> 4, idesc_s, 0);
-      umma_commit(&bar_a);
-    }
-    const Tile nxt = advance(cur);              // (global loads of the next column's header, under the MMAs)
-    good = mbar_wait(&bar_a, g & 1, p.status, 3);
-    tc_fence_after_sync();
-
-    // ---- P and dS of row `lt`, this thread's 32 keys
-    {
+    for (uint32_t g = 0; g < ntiles; ++g) {
+      // ---- P of row `lt`, this thread's 32 keys (Q's barrier: for the row data)
+      if (!(good = wait_all(&bar_fullq, g, 3) && wait_all(&bar_s, g, 3))) break;
+      tc_fence_after_sync();
       const int r = sRow[lt];
       const float lse2 = sLse[lt] * kLog2e, dd = sDsum[lt];
-      const int lim = r < 0 ? 0 : (p.causal ? min(keys_valid, r + shift - key0 + 1) : keys_valid);
+      const int lim = (r < 0 ? 0 : (p.causal ? min(keys_valid, r + shift - key0 + 1) : keys_valid)) - hf * 32;
       float pr[32], dp[32];
       tmem_ld32(tS + lane_sel + hf * 32, pr);
+      tmem_ld_wait();
+#pragma unroll
+      for (int jj = 0; jj < 32; ++jj) pr[jj] = jj < lim ? exp2f(pr[jj] * scale_log2 - lse2) : 0.f;
+      if (g > 0 && !(good = wait_all(&bar_dv, g - 1, 3))) break;    // dV of the tile before has read P
+#pragma unroll
+      for (int jj = 0; jj < 4; ++jj)
+        *reinterpret_cast<uint4*>(sP + sw128_offset(lt, hf * 4 + jj, kQBlock)) = pack8<T>(pr + jj * 8);
+      // ---- dS
+      if (!(good = wait_all(&bar_p, g, 3))) break;
+      tc_fence_after_sync();
       tmem_ld32(tdP + lane_sel + hf * 32, dp);
       tmem_ld_wait();
       tc_fence_before_sync();
 #pragma unroll
-      for (int jj = 0; jj < 32; ++jj) {
-        pr[jj] = (hf * 32 + jj < lim) ? exp2f(pr[jj] * scale_log2 - lse2) : 0.f;
-        dp[jj] = pr[jj] * (dp[jj] - dd);
-      }
+      for (int jj = 0; jj < 32; ++jj) dp[jj] = pr[jj] * (dp[jj] - dd);
+      if (g > 0 && !(good = wait_all(&bar_dq[1], g - 1, 3))) break;   // dQ of the tile before has read dS
 #pragma unroll
-      for (int jj = 0; jj < 4; ++jj) {
-        *reinterpret_cast<uint4*>(sP + sw128_offset(lt, hf * 4 + jj, kQBlock)) = pack8<T>(pr + jj * 8);
+      for (int jj = 0; jj < 4; ++jj)
         *reinterpret_cast<uint4*>(sdS + sw128_offset(lt, hf * 4 + jj, kQBlock)) = pack8<T>(dp + jj * 8);
-      }
+      fence_async_smem();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&bar_ds);      // S, dP and the row data have been read, P and dS are in shared memory
     }
-    fence_async_smem();
-    tc_fence_before_sync();
-    good = __syncthreads_and(good);             // P, dS complete; S, dP and the row data have been read by every thread
-    if (!good) break;
-    tc_fence_after_sync();
-    if (tid == 0) {
-      const uint32_t acc = g > 0 ? 1u : 0u;     // the item's first tile starts the accumulators
-#pragma unroll
-      for (int hh = 0; hh < 2; ++hh) {
-        // dV^T[half] += dO^T.P, dK^T[half] += Q^T.dS : M = 128 head-dim columns, N = keys, K = the rows
-        umma_gemm<kM / 16>(tdV + hh * 64, desc_lo_sw128(smem_u32(sdO) + hh * 2 * kQBlock, kQBlock), hi, 128, 512,
-                           p_mn, hi, 128, 512, idesc_t, acc);
-        umma_gemm<kM / 16>(tdK + hh * 64, desc_lo_sw128(smem_u32(sQ) + hh * 2 * kQBlock, kQBlock), hi, 128, 512,
-                           ds_mn, hi, 128, 512, idesc_t, acc);
-      }
-      // dQ[first half of the head dim] = dS.K over the columns S and dP occupied
-      umma_gemm<kC / 16>(tdQ, ds_km, hi, 2, 0, desc_lo_sw128(smem_u32(sK), kKBlock), hi, 128, 512, idesc_dq, 0);
-      umma_commit(&bar_b);
-    }
-    load_rows(nxt);                             // the next tile's row data, under these MMAs
-    good = mbar_wait(&bar_b, g & 1, p.status, 4);
-    good = __syncthreads_and(good);             // (also publishes the row data)
-    if (!good) break;
-    tc_fence_after_sync();
-    // dV^T, dK^T and the first dQ half are complete: the Q and dO tiles are free, and the next
-    // tile's rows are gathered while dQ is read out (the gathers bound this kernel)
-    if (nxt.valid) gather(nxt);
-    // ---- dQ partial of row `lt`: per head-dim half, this thread's 64 columns (128 contiguous bytes
-    // of the row's slot): scaled, rounded, written from registers, 16-byte chunks permuted like every partial
-    const int key = (int)((slot0 + lt) & 7);
-    T* dst = part_dq + (slot0 + lt) * D;
+    // ---- dK (scaled) and dV of this key block: TMEM lane = head-dim index of this thread's half,
+    // column = key; consecutive lanes write consecutive elements of a key's row
+    if (good) good = wait_all(&bar_fin, 0, 4);
+    if (good) {
+      tc_fence_after_sync();
+      T* dkp = static_cast<T*>(p.dk) + (int64_t)(k0 + key0) * p.dk_rs + (int64_t)hk * p.dk_hs + hf * 128 + lt;
+      T* dvp = static_cast<T*>(p.dv) + (int64_t)(k0 + key0) * p.dv_rs + (int64_t)hk * p.dv_hs + hf * 128 + lt;
 #pragma unroll 1
-    for (int hh = 0; hh < 2; ++hh) {
-#pragma unroll
       for (int i2 = 0; i2 < 2; ++i2) {
-        float o[32];
-        tmem_ld32(tdQ + lane_sel + hf * 64 + i2 * 32, o);
-        tmem_ld_wait();
-        if (lt < rows) {
+        float a[32], bq[32];
+        if (ntiles > 0) {
+          tmem_ld32(tdK + hf * 64 + lane_sel + i2 * 32, a);
+          tmem_ld32(tdV + hf * 64 + lane_sel + i2 * 32, bq);
+          tmem_ld_wait();
+        } else {                                 // no tile at all: the gradients of these keys are zero
 #pragma unroll
-          for (int jj = 0; jj < 4; ++jj) {
+          for (int jj = 0; jj < 32; ++jj) { a[jj] = 0.f; bq[jj] = 0.f; }
+        }
 #pragma unroll
-            for (int e = 0; e < 8; ++e) o[jj * 8 + e] *= p.scale;
-            *reinterpret_cast<uint4*>(dst + (((hh * 16 + hf * 8 + i2 * 4 + jj) ^ key) << 3)) = pack8<T>(o + jj * 8);
+        for (int jj = 0; jj < 32; ++jj) {
+          const int kk = i2 * 32 + jj;
+          if (kk < keys_valid) {
+            dkp[(int64_t)kk * p.dk_rs] = Elem<T>::from_f(a[jj] * p.scale);
+            dvp[(int64_t)kk * p.dv_rs] = Elem<T>::from_f(bq[jj]);
           }
-        }
-      }
-      tc_fence_before_sync();
-      if (hh == 0) {
-        __syncthreads();                        // the first half has been read out of TMEM
-        tc_fence_after_sync();
-        if (tid == 0) {
-          umma_gemm<kC / 16>(tdQ, ds_km, hi, 2, 0, desc_lo_sw128(smem_u32(sK) + 2 * kKBlock, kKBlock), hi, 128, 512,
-                             idesc_dq, 0);
-          umma_commit(&bar_c);
-        }
-        good = mbar_wait(&bar_c, g & 1, p.status, 4);
-        tc_fence_after_sync();
-      }
-    }
-    cur = nxt;
-    // (the barrier at the top of the next tile keeps its S and dP, which overwrite dQ, behind these reads)
-  }
-  cp_async_wait_all();                          // (K and V of an item without tiles)
-  // ---- dK (scaled) and dV of this key block: TMEM lane = head-dim index of this thread's half,
-  // column = key; consecutive lanes write consecutive elements of a key's row
-  if (good) {
-    tc_fence_after_sync();
-    T* dkp = static_cast<T*>(p.dk) + (int64_t)(k0 + key0) * p.dk_rs + (int64_t)hk * p.dk_hs + hf * 128 + lt;
-    T* dvp = static_cast<T*>(p.dv) + (int64_t)(k0 + key0) * p.dv_rs + (int64_t)hk * p.dv_hs + hf * 128 + lt;
-#pragma unroll 1
-    for (int i2 = 0; i2 < 2; ++i2) {
-      float a[32], bq[32];
-      if (g > 0) {
-        tmem_ld32(tdK + hf * 64 + lane_sel + i2 * 32, a);
-        tmem_ld32(tdV + hf * 64 + lane_sel + i2 * 32, bq);
-        tmem_ld_wait();
-      } else {                                   // no tile at all: the gradients of these keys are zero
-#pragma unroll
-        for (int jj = 0; jj < 32; ++jj) { a[jj] = 0.f; bq[jj] = 0.f; }
-      }
-#pragma unroll
-      for (int jj = 0; jj < 32; ++jj) {
-        const int kk = i2 * 32 + jj;
-        if (kk < keys_valid) {
-          dkp[(int64_t)kk * p.dk_rs] = Elem<T>::from_f(a[jj] * p.scale);
-          dvp[(int64_t)kk * p.dv_rs] = Elem<T>::from_f(bq[jj]);
         }
       }
     }
@@ -486,7 +588,7 @@ __global__ void __launch_bounds__(kThreads) bwd_wide_tc_kernel(WideParams p) {
   if (warp == 0) tmem_dealloc(tmem_base, 512);
 }
 
-WideParams make_wide_params(const AttnArgs& a, const AttnWorkspace& w, const PassParams& ps) {
+WideParams make_wide_params(const AttnArgs& a, const AttnWorkspace& w, const PassParams& ps, int nchunk, int items_y) {
   WideParams p;
   p.q = a.q; p.k = a.k; p.v = a.v; p.dout = a.dout;
   p.q_rs = a.q_rs; p.q_hs = a.q_hs; p.k_rs = a.k_rs; p.k_hs = a.k_hs; p.v_rs = a.v_rs; p.v_hs = a.v_hs;
@@ -498,29 +600,37 @@ WideParams make_wide_params(const AttnArgs& a, const AttnWorkspace& w, const Pas
   p.part_o = w.part_o; p.part_lse = w.part_lse; p.status = w.status;
   p.heads = a.heads; p.heads_k = a.heads_k; p.total_q = a.total_q;
   p.scale = a.scale; p.causal = a.causal;
+  p.items_x = nchunk * ps.nsub; p.items_y = items_y; p.items_z = a.batch;
+  p.items_heavy = a.causal ? min(p.items_x, 16 * ps.nsub) : 0;
   return p;
 }
 
 template <typename T, int C, int D>
 int fwd_wide_launch(const AttnArgs& a, const AttnWorkspace& w, const PassParams& ps, cudaStream_t s) {
-  const WideParams p = make_wide_params(a, w, ps);
+  const WideParams p = make_wide_params(a, w, ps, a.ncol, ps.nh);
   const size_t smem = (size_t)2 * C * D * 2 + (size_t)kM * D * 2 + (size_t)kM * C * 2;   // K, V, Q, P
   auto kern = fwd_wide_tc_kernel<T, C, D>;
   FMB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  kern<<<dim3(a.ncol * ps.nsub, ps.nh, a.batch), kThreads, smem, s>>>(p);
+  kern<<<p.items_x * p.items_y * p.items_z, kThreads, smem, s>>>(p);
   FMB_LAUNCH_CHECK("fwd_wide_tc_kernel");
   return FMB_OK;
 }
 
 template <typename T, int D>
 int bwd_wide_launch(const AttnArgs& a, const AttnWorkspace& w, const PassParams& ps, cudaStream_t s) {
-  const WideParams p = make_wide_params(a, w, ps);
+  const WideParams p = make_wide_params(a, w, ps, max(a.ncol, ceil_div(a.max_k, a.chunk)), ps.nh / (a.heads / a.heads_k));
   // K, V, Q, dO, P, dS: with d = 256 that and the kernel's static arrays are the 227 KB a CTA may have
   const size_t smem = (size_t)2 * kC * D * 2 + (size_t)2 * kM * D * 2 + (size_t)2 * kM * kC * 2;
   auto kern = bwd_wide_tc_kernel<T, D>;
+  // the hand-over of registers inside the kernel counts on the launch's share per thread
+  static const int regs = [kern] {
+    cudaFuncAttributes at;
+    return cudaFuncGetAttributes(&at, kern) == cudaSuccess ? at.numRegs : 0;
+  }();
+  if (regs != kBwRegsLaunch)
+    return fail(FMB_ERR_CUDA, "wide-head backward: built with %d registers per thread (%d expected)", regs, kBwRegsLaunch);
   FMB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  const int nchunk = max(a.ncol, ceil_div(a.max_k, a.chunk));
-  kern<<<dim3(nchunk * ps.nsub, ps.nh / (a.heads / a.heads_k), a.batch), kThreads, smem, s>>>(p);
+  kern<<<p.items_x * p.items_y * p.items_z, kBwThreads, smem, s>>>(p);
   FMB_LAUNCH_CHECK("bwd_wide_tc_kernel");
   return FMB_OK;
 }
