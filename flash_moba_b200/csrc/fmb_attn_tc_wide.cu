@@ -3,14 +3,14 @@
 // The kernels of fmb_attn_tc.cu keep dK and dV of a 128-key block in the SM's 512 TMEM columns,
 // which a head dim of 128 already fills, and their shared-memory tiles assume d <= 128.  Wider heads
 // run here (forward: key blocks of 128 keys where the chunk allows, else 64; backward: 64): one CTA per
-// work item (key block, head or kv head, sequence), described at each kernel.  Same workspace
+// work item (key block, head or kv head, sequence), warp-specialised, described at each kernel.  Same workspace
 // contract (slots, per-entry partials) and the same merge kernels as the other engines.  Every mbarrier
 // wait is bounded (status word of the workspace).
 //
 // dK and dV are accumulated TRANSPOSED (TMEM lane = head-dim index, two halves of 128; column = key), which takes
 // 2 x 128 columns instead of the 2 x 256 of a key-per-lane layout.
 // Measured (B200, 16K tokens in three sequences, 16 / 4 heads, chunk 128, top-k 8; the kernels before, in which every
-// thread took part in every phase / these): backward 1830 / 1120 us.  Of that: gathers that read their
+// thread took part in every phase / these): forward 790 / 446 us, backward 1830 / 1120 us.  Of that: gathers that read their
 // row numbers ahead of the copies 3 - 5 %; long columns first 5 - 7 %; MMA issue in turns of four instructions, not
 // fully unrolled, 17 % of the backward (sixteen unrolled ones took 2850 cycles to issue, in turns 1050).
 #include "fmb_attn.cuh"
@@ -24,7 +24,6 @@ namespace {
 
 constexpr int kM = 128;               // gathered rows per tile = TMEM lanes
 constexpr int kC = 64;                // keys per block
-constexpr int kThreads = 256;         // two threads per row: each owns half of the columns
 constexpr float kLog2e = 1.4426950408889634f;
 
 struct WideParams {
@@ -40,6 +39,7 @@ struct WideParams {
   // one CTA per item (key block, head or kv head, sequence); the first `items_heavy` key blocks of every head (under a
   // causal mask the longest columns) come before all others, which follow one head after the other
   int items_x, items_y, items_z, items_heavy;
+  int item_heads;                               // forward: q heads per item
 };
 
 struct WideItem { int c, sb, y, b; };           // chunk, key block in it, head or kv head of the pass, sequence
@@ -56,9 +56,6 @@ __device__ __forceinline__ WideItem wide_item(const WideParams& p) {
   }
   return WideItem{bx / p.ps.nsub, bx % p.ps.nsub, rem % p.items_y, rem / p.items_y};
 }
-
-// threads that take part in the 16-byte copies of rows of D elements: eight rows per pass
-template <int D> struct Copiers { static constexpr int n = (D / 8) * 8; };
 
 // 16 rows of NCHUNK*16 bytes gathered by one warp: lanes 0-15 (and again 16-31) hold the rows' numbers (-1 = zero fill);
 // see gather_rows32()
@@ -91,19 +88,29 @@ __device__ __forceinline__ void st_global_32(void* dst, uint4 a, uint4 b) {
                : "memory");
 }
 
+// ---- forward
+// Work item = key block of one (sequence, several q heads of a kv head); one CTA per item, which walks the 128-row tiles
+// of the heads' columns; 768 threads, warp-specialised:
+//   warps 0-7    compute: two groups of 4 warps take the tiles in turn, a thread per row (TMEM lane): row maximum in one
+//                pass over the scores in TMEM, P in a second one.
+//   warps 8-11   drain: O / l of the tile from TMEM to the entries' slots, from registers, 32 bytes a store.
+//   warp 12      one thread issues every MMA.
+//   warps 16-23  loaders: each fetches 16 of a tile's Q rows as soon as S of the tile before has completed.
+// S is double-buffered in TMEM, O is not: its two halves of the head dim are computed and drained one after the other.
+// K, V, one Q tile and one P tile fill the shared memory at 128 keys.  What bounds it is the drain (stores of a row per
+// lane) beside the row gathers, both through the same load / store unit.
+constexpr int kFwDrainWarp = 8, kFwIssuerWarp = 12, kFwLoadWarp = 16, kFwLoaders = 8, kFwThreads = 768;
+
 template <typename T, int C, int D>
-__global__ void __launch_bounds__(kThreads) fwd_wide_tc_kernel(WideParams p) {
+__global__ void __launch_bounds__(kFwThreads, 1) fwd_wide_tc_kernel(WideParams p) {
+  static_assert(D == 256 && (C == 64 || C == 128), "head dim 256, key blocks of 64 or 128");
   constexpr int NCH = D / 8;                    // 16-byte chunks of a row
-  constexpr int NT = Copiers<D>::n;             // copying threads
   constexpr uint32_t kKBlock = C * 128;         // bytes between 64-element blocks of the K / V tiles
   constexpr uint32_t kQBlock = kM * 128;        // same for the 128-row Q and P tiles
-  constexpr int CH = C / 2, DH = D / 2;         // keys / head-dim columns per thread
-  static_assert(D == 256 && (C == 64 || C == 128), "head dim 256, key blocks of 64 or 128");
   extern __shared__ __align__(1024) unsigned char smem_raw[];
-  __shared__ uint64_t bar_s, bar_o;
+  __shared__ uint64_t bar_fullq, bar_k, bar_v, bar_s[2], bar_pready[2], bar_o[2][2], bar_ofree[2];
   __shared__ uint32_t tmem_base_s;
-  __shared__ int sRow[kM];
-  __shared__ float sMax[2][kM], sSum[2][kM];
+  __shared__ float sInv[2][kM];                 // 1 / l of the tile's rows, per group
 
   // with 128-key blocks the tiles and the arrays above fill the 227 KB: no room for alignment padding
   unsigned char* smem = smem_raw;
@@ -113,150 +120,222 @@ __global__ void __launch_bounds__(kThreads) fwd_wide_tc_kernel(WideParams p) {
   }
   unsigned char* sK = smem;                     // [C][D]
   unsigned char* sV = sK + C * D * 2;           // [C][D]
-  unsigned char* sQ = sV + C * D * 2;           // [128][D]: refilled as soon as the tile's S has been computed
+  unsigned char* sQ = sV + C * D * 2;           // [128][D]
   unsigned char* sP = sQ + kM * D * 2;          // [128][C]
 
-  const int tid = threadIdx.x, warp = tid >> 5;
-  const int lt = tid & (kM - 1), hf = tid >> 7;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const WideItem item = wide_item(p);
-  const int c = item.c, sb = item.sb, h = p.ps.h0 + item.y, b = item.b;
-  const ColRef col = column_of(p.ps, b, h, c);
-  if (col.nnz <= 0) return;                     // CTA-uniform
-  const int64_t slot0 = (int64_t)sb * p.ps.cap + col.slot;
+  const int c = item.c, h0 = p.ps.h0 + item.y * p.item_heads, b = item.b;
+  // The item's tiles as one sequence over its heads and the 128-row tiles of each head's column
+  struct Tile { int hg, t0, nnz; int64_t off, slot; bool valid; };
+  auto seek = [&](Tile& t) {                    // first head >= t.hg with a column; t.t0 = 0
+    t.valid = false;
+    for (; t.hg < p.item_heads; ++t.hg) {
+      const ColRef col = column_of(p.ps, b, h0 + t.hg, c);
+      if (col.nnz > 0) { t.nnz = col.nnz; t.off = col.off; t.slot = col.slot; t.t0 = 0; t.valid = true; return; }
+    }
+  };
+  auto first = [&] {
+    Tile t{0, 0, 0, 0, 0, false};
+    seek(t);
+    return t;
+  };
+  auto advance = [&](Tile& t) {
+    t.t0 += kM;
+    if (t.t0 >= t.nnz) { ++t.hg; seek(t); }
+  };
+  uint32_t ntiles = 0;
+  for (int hg = 0; hg < p.item_heads; ++hg) ntiles += (uint32_t)((column_of(p.ps, b, h0 + hg, c).nnz + kM - 1) / kM);
+  if (ntiles == 0) return;                      // CTA-uniform
+  const int64_t plane = (int64_t)item.sb * p.ps.cap;
   const int q0 = p.cu_q[b], len_q = p.cu_q[b + 1] - q0;
   const int k0 = p.k_begin[b], len_k = p.k_end[b] - k0;
-  const int key0 = c * p.ps.chunk + sb * C;
+  const int key0 = c * p.ps.chunk + item.sb * C;
   const int keys_valid = max(0, min(C, len_k - key0));
-  const int hk = h / (p.heads / p.heads_k);
+  const int hk = h0 / (p.heads / p.heads_k);
   const int shift = len_k - len_q;
-  const float scale_log2 = p.scale * kLog2e;
-  const int ntiles = (col.nnz + kM - 1) / kM;
-  const T* qbase = static_cast<const T*>(p.q) + (int64_t)q0 * p.q_rs + (int64_t)h * p.q_hs;
-  T* part_o = static_cast<T*>(p.part_o);
 
   if (warp == 0) tmem_alloc(&tmem_base_s, 512);
   if (tid == 0) {
-    mbar_init(&bar_s, 1);
-    mbar_init(&bar_o, 1);
+    mbar_init(&bar_fullq, kFwLoaders);          // one arrival per loader warp
+    mbar_init(&bar_k, 8); mbar_init(&bar_v, 8); // one arrival per warp that copies
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(&bar_s[i], 1);                  // per group
+      mbar_init(&bar_pready[i], 4);
+      mbar_init(&bar_o[i][0], 1); mbar_init(&bar_o[i][1], 1);   // per group and half of the head dim
+      mbar_init(&bar_ofree[i], 4);              // per half
+    }
     mbar_fence_init();
   }
-  // row ids of tile t (-1 = none)
-  auto load_rows = [&](int t) {
-    if (tid < kM) {
-      int r = -1;
-      if (t < ntiles && t * kM + tid < col.nnz) {
-        r = p.ps.indices[col.off + t * kM + tid];
-        if (r < 0 || r >= len_q) r = -1;
-      }
-      sRow[tid] = r;
-    }
-  };
-  load_rows(0);
-  if (tid < NT) {
-    const T* kbase = static_cast<const T*>(p.k) + (int64_t)(k0 + key0) * p.k_rs + (int64_t)hk * p.k_hs;
-    const T* vbase = static_cast<const T*>(p.v) + (int64_t)(k0 + key0) * p.v_rs + (int64_t)hk * p.v_hs;
-    dense_cp_async<T, NCH, C, NT>(tid, sK, kKBlock, kbase, p.k_rs, keys_valid);
-    dense_cp_async<T, NCH, C, NT>(tid, sV, kKBlock, vbase, p.v_rs, keys_valid);
-  }
   tc_fence_before_sync();
-  __syncthreads();                              // row ids of tile 0, the TMEM base, the barriers
+  __syncthreads();
   tc_fence_after_sync();
-  if (tid < NT) gather_cp_async<T, NCH, NT>(tid, sQ, kQBlock, qbase, p.q_rs, sRow);
   const uint32_t tmem_base = tmem_base_s;
-  const uint32_t tS = tmem_base, tO = tmem_base + 256;
-  const uint32_t lane_sel = (uint32_t)((warp & 3) * 32) << 16;
-  constexpr uint32_t idesc_s = make_idesc(FmtOf<T>::v, kM, C, 0, 0);
-  constexpr uint32_t idesc_o = make_idesc(FmtOf<T>::v, kM, D, 0, 1);
-  const uint32_t hi = desc_hi_sw128(1024);
-  const uint32_t q_km = desc_lo_sw128(smem_u32(sQ), 16), k_km = desc_lo_sw128(smem_u32(sK), 16);
-  const uint32_t v_mn = desc_lo_sw128(smem_u32(sV), kKBlock), p_km = desc_lo_sw128(smem_u32(sP), 16);
-  bool good = true;
+  const uint32_t tO = tmem_base + 256;          // S of group i at columns 128 i
+  auto wait_all = [&](uint64_t* bar, uint32_t parity, int where) -> bool {   // the same answer for the whole warp
+    return __all_sync(0xffffffffu, mbar_wait(bar, parity & 1u, p.status, where));
+  };
 
-#pragma unroll 1
-  for (int i = 0; i < ntiles && good; ++i) {
-    const int t0 = i * kM;
-    const int rows = min(kM, col.nnz - t0);
-    // Q(i) (with K and V on the first tile) has landed
-    const int r = sRow[lt];                     // this tile's row, before the next tile's ids replace it
+  // K is copied by the drain and issuer warpgroups, V by the compute warps, each on its way to its role
+  auto stage = [&](unsigned char* tile, const void* src, int64_t rs, int64_t hs, int t, uint64_t* bar) {
+    dense_cp_async<T, NCH, C, 256>(t, tile, kKBlock, static_cast<const T*>(src) + (int64_t)(k0 + key0) * rs + (int64_t)hk * hs, rs,
+                                   keys_valid);
     cp_async_wait_all();
     fence_async_smem();
-    tc_fence_before_sync();
-    __syncthreads();
-    tc_fence_after_sync();
-    if (tid == 0) {
-      umma_gemm<D / 16>(tS, q_km, hi, 2, kQBlock >> 4, k_km, hi, 2, kKBlock >> 4, idesc_s, 0);
-      umma_commit(&bar_s);
-    }
-    load_rows(i + 1);                           // (every thread has read its row id above)
-    good = mbar_wait(&bar_s, i & 1, p.status, 1);
-    __syncthreads();                            // the next tile's row ids
-    tc_fence_after_sync();
-    // S is complete, so the Q tile is free: the next tile's rows are gathered under the rest of this
-    // tile's work (the row gather, not the arithmetic, is what bounds these kernels)
-    if (i + 1 < ntiles && tid < NT) gather_cp_async<T, NCH, NT>(tid, sQ, kQBlock, qbase, p.q_rs, sRow);
+    __syncwarp();
+    if (lane == 0) mbar_arrive(bar);
+  };
+  if (warp < kFwDrainWarp) stage(sV, p.v, p.v_rs, p.v_hs, tid, &bar_v);
+  else if (warp < kFwLoadWarp) stage(sK, p.k, p.k_rs, p.k_hs, tid - kFwDrainWarp * 32, &bar_k);
 
-    // ---- chunk-local softmax of row `lt`, this thread's half of the keys, in one pass over the scores
-    const int lim = r < 0 ? 0 : (p.causal ? min(keys_valid, r + shift - key0 + 1) : keys_valid);
-    float s[CH];
-#pragma unroll
-    for (int q4 = 0; q4 < CH / 32; ++q4) tmem_ld32(tS + lane_sel + hf * CH + q4 * 32, s + q4 * 32);
-    tmem_ld_wait();
-    tc_fence_before_sync();
-    float mx = -CUDART_INF_F;
-#pragma unroll
-    for (int jj = 0; jj < CH; ++jj) mx = fmaxf(mx, hf * CH + jj < lim ? s[jj] : -CUDART_INF_F);
-    sMax[hf][lt] = mx;
-    good = __syncthreads_and(good);
-    if (!good) break;
-    mx = fmaxf(mx, sMax[hf ^ 1][lt]);
-    const float mref = lim > 0 ? mx * scale_log2 : 0.f;
-    float sum = 0.f;
-#pragma unroll
-    for (int jj = 0; jj < CH; ++jj) {
-      const float e = exp2f(s[jj] * scale_log2 - mref);
-      s[jj] = (hf * CH + jj < lim) ? e : 0.f;
-      sum += s[jj];
+  if (warp >= kFwLoadWarp) {
+    // =============================================================== loaders
+    const int row0 = (warp - kFwLoadWarp) * 16, i = row0 + (lane & 15);   // this lane's row (lanes in pairs)
+    uint32_t g = 0;
+    Tile t = first();
+    auto entry = [&](const Tile& x) { return x.valid && x.t0 + i < x.nnz ? ldg_s32_here(p.ps.indices + x.off + x.t0 + i) : -1; };
+    int raw = entry(t);
+#pragma unroll 1
+    for (; t.valid; ++g) {
+      const int r = (raw < 0 || raw >= len_q) ? -1 : raw;
+      const T* qbase = static_cast<const T*>(p.q) + (int64_t)q0 * p.q_rs + (int64_t)(h0 + t.hg) * p.q_hs;
+      advance(t);
+      raw = entry(t);                           // the next tile's, in flight meanwhile
+      if (g > 0 && !wait_all(&bar_s[(g - 1) & 1], (g - 1) >> 1, 5)) break;   // S of the tile before has read the Q tile
+      gather_rows16<NCH>(lane, sQ + row0 * 128, kQBlock, qbase, p.q_rs, r);
+      cp_async_wait_all();
+      fence_async_smem();                       // the copies are generic-proxy writes; the MMAs read through the async proxy
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&bar_fullq);
     }
-#pragma unroll
-    for (int jj = 0; jj < CH / 8; ++jj)
-      *reinterpret_cast<uint4*>(sP + sw128_offset(lt, hf * (CH / 8) + jj, kQBlock)) = pack8<T>(s + jj * 8);
-    sSum[hf][lt] = sum;
-    fence_async_smem();
-    tc_fence_before_sync();
-    __syncthreads();                            // P complete; S has been read by every thread
-    tc_fence_after_sync();
-    if (tid == 0) {
-      umma_gemm<C / 16>(tO, p_km, hi, 2, kQBlock >> 4, v_mn, hi, 128, 512, idesc_o, 0);
-      umma_commit(&bar_o);
-    }
-    sum += sSum[hf ^ 1][lt];
-    const float inv = sum > 0.f ? 1.f / sum : 0.f;
-    if (hf == 0 && lt < rows) p.part_lse[slot0 + t0 + lt] = sum > 0.f ? mx * p.scale + logf(sum) : -CUDART_INF_F;
-    good = mbar_wait(&bar_o, i & 1, p.status, 2);
-    tc_fence_after_sync();
-
-    // ---- normalised partial O of row `lt`, this thread's half of the head dim (256 contiguous
-    // bytes of the row's slot), written from registers; 16-byte chunks permuted like every partial
-    {
-      const int key = (int)((slot0 + t0 + lt) & 7);
-      T* dst = part_o + (slot0 + t0 + lt) * D;
-#pragma unroll
-      for (int q4 = 0; q4 < DH / 32; ++q4) {
-        float o[32];
-        tmem_ld32(tO + lane_sel + hf * DH + q4 * 32, o);
-        tmem_ld_wait();
-        if (lt < rows) {
-#pragma unroll
-          for (int jj = 0; jj < 4; ++jj) {
-#pragma unroll
-            for (int e = 0; e < 8; ++e) o[jj * 8 + e] *= inv;
-            *reinterpret_cast<uint4*>(dst + (((hf * (DH / 8) + q4 * 4 + jj) ^ key) << 3)) = pack8<T>(o + jj * 8);
-          }
+  } else if (warp >= kFwIssuerWarp) {
+    // =============================================================== MMA issuer
+    if (warp == kFwIssuerWarp && lane == 0) {
+      constexpr uint32_t idesc_s = make_idesc(FmtOf<T>::v, kM, C, 0, 0);
+      constexpr uint32_t idesc_o = make_idesc(FmtOf<T>::v, kM, 128, 0, 1);
+      const uint32_t hi = desc_hi_sw128(1024);
+      const uint32_t q_km = desc_lo_sw128(smem_u32(sQ), 16), k_km = desc_lo_sw128(smem_u32(sK), 16);
+      const uint32_t v_mn = desc_lo_sw128(smem_u32(sV), kKBlock), p_km = desc_lo_sw128(smem_u32(sP), 16);
+      bool ok = mbar_wait(&bar_k, 0, p.status, 6);
+#pragma unroll 1
+      for (uint32_t g = 0; g <= ntiles && ok; ++g) {
+        if (g < ntiles) {                       // S(g); its columns were read before P(g - 2) was ready
+          if (!(ok = mbar_wait(&bar_fullq, g & 1, p.status, 6))) break;
+          tc_fence_after_sync();
+          umma_gemm<D / 16>(tmem_base + (g & 1) * 128, q_km, hi, 2, kQBlock >> 4, k_km, hi, 2, kKBlock >> 4, idesc_s, 0);
+          umma_commit(&bar_s[g & 1]);
+        }
+        if (g == 0) {
+          ok = mbar_wait(&bar_v, 0, p.status, 6);
+          continue;
+        }
+        const uint32_t m = g - 1;               // O(m) = P.V per half of the head dim, once O(m - 1) has been read out
+        if (!(ok = mbar_wait(&bar_pready[m & 1], (m >> 1) & 1, p.status, 6))) break;
+#pragma unroll 1
+        for (int hh = 0; hh < 2; ++hh) {
+          if (m > 0 && !(ok = mbar_wait(&bar_ofree[hh], (m - 1) & 1, p.status, 6))) break;
+          tc_fence_after_sync();
+          umma_gemm<C / 16>(tO + hh * 128, p_km, hi, 2, kQBlock >> 4, v_mn + hh * (2 * kKBlock >> 4), hi, 128, 512, idesc_o, 0);
+          umma_commit(&bar_o[m & 1][hh]);
         }
       }
-      tc_fence_before_sync();
     }
-    // (the barrier at the top of the next tile keeps its P.V, which overwrites O, behind these reads)
+  } else if (warp >= kFwDrainWarp) {
+    // =============================================================== drain warps
+    const uint32_t at = (uint32_t)((warp & 3) * 32) << 16;
+    const int lt = tid & (kM - 1);
+    T* part_o = static_cast<T*>(p.part_o);
+    bool good = true;
+    uint32_t g = 0;
+#pragma unroll 1
+    for (Tile t = first(); t.valid && good; advance(t), ++g) {
+      const bool mine = lt < t.nnz - t.t0;
+      const int64_t slot = plane + t.slot + t.t0 + lt;
+      const int key = (int)(slot & 7);
+      T* dst = part_o + slot * D;
+      if (!(good = wait_all(&bar_pready[g & 1], g >> 1, 4))) break;   // (for 1 / l)
+      const float inv = sInv[g & 1][lt];
+      // ---- normalised partial O of row `lt`; 16-byte chunks permuted like every partial, a 32-byte store takes a pair
+      // of neighbouring chunks
+#pragma unroll 1
+      for (int q4 = 0; q4 < D / 32; ++q4) {
+        if ((q4 & 3) == 0) {
+          if (!(good = wait_all(&bar_o[g & 1][q4 >> 2], g >> 1, 4))) break;
+          tc_fence_after_sync();
+        }
+        float o[32];
+        tmem_ld32(tO + at + q4 * 32, o);
+        tmem_ld_wait();
+        if ((q4 & 3) == 3) {
+          tc_fence_before_sync();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&bar_ofree[q4 >> 2]);
+        }
+#pragma unroll
+        for (int e = 0; e < 32; ++e) o[e] *= inv;
+#pragma unroll
+        for (int jj = 0; jj < 4; jj += 2) {
+          const uint4 u = pack8<T>(o + jj * 8), v = pack8<T>(o + jj * 8 + 8);
+          if (mine) st_global_32(dst + ((((q4 * 4 + jj) ^ key) & ~1) << 3), (key & 1) ? v : u, (key & 1) ? u : v);
+        }
+      }
+    }
+  } else {
+    // =============================================================== compute groups
+    const int grp = warp >> 2, lt = tid & (kM - 1);
+    const uint32_t tS = tmem_base + grp * 128 + ((uint32_t)((warp & 3) * 32) << 16);
+    const float scale_log2 = p.scale * kLog2e;
+    uint32_t g = 0;
+    Tile t = first();
+    if (grp == 1 && t.valid) { advance(t); ++g; }
+    auto entry = [&](const Tile& x) { return x.valid && x.t0 + lt < x.nnz ? ldg_s32_here(p.ps.indices + x.off + x.t0 + lt) : -1; };
+    int raw = entry(t);
+#pragma unroll 1
+    for (; t.valid; g += 2) {
+      const int lim = (raw < 0 || raw >= len_q) ? 0 : (p.causal ? min(keys_valid, raw + shift - key0 + 1) : keys_valid);
+      const bool mine = lt < t.nnz - t.t0;
+      const int64_t slot = plane + t.slot + t.t0 + lt;
+      advance(t);
+      if (t.valid) advance(t);
+      raw = entry(t);                           // the group's next tile's, in flight meanwhile
+      if (!wait_all(&bar_s[grp], g >> 1, 1)) break;
+      tc_fence_after_sync();
+      // ---- chunk-local softmax of row `lt`
+      float mx = -CUDART_INF_F;
+#pragma unroll 1
+      for (int q4 = 0; q4 < C / 32; ++q4) {
+        float s[32];
+        tmem_ld32(tS + q4 * 32, s);
+        tmem_ld_wait();
+#pragma unroll
+        for (int jj = 0; jj < 32; ++jj) mx = fmaxf(mx, q4 * 32 + jj < lim ? s[jj] : -CUDART_INF_F);
+      }
+      const float mref = lim > 0 ? mx * scale_log2 : 0.f;
+      // P.V of the tile before (the other group's) has read the P tile
+      if (g > 0 && !wait_all(&bar_o[grp ^ 1][1], (g - 1) >> 1, 1)) break;
+      float sum = 0.f;
+#pragma unroll 1
+      for (int q4 = 0; q4 < C / 32; ++q4) {
+        float s[32];
+        tmem_ld32(tS + q4 * 32, s);
+        tmem_ld_wait();
+#pragma unroll
+        for (int jj = 0; jj < 32; ++jj) {
+          const float e = exp2f(s[jj] * scale_log2 - mref);
+          s[jj] = q4 * 32 + jj < lim ? e : 0.f;
+          sum += s[jj];
+        }
+#pragma unroll
+        for (int jj = 0; jj < 4; ++jj)
+          *reinterpret_cast<uint4*>(sP + sw128_offset(lt, q4 * 4 + jj, kQBlock)) = pack8<T>(s + jj * 8);
+      }
+      sInv[grp][lt] = sum > 0.f ? 1.f / sum : 0.f;
+      if (mine) p.part_lse[slot] = sum > 0.f ? mx * p.scale + logf(sum) : -CUDART_INF_F;
+      fence_async_smem();
+      tc_fence_before_sync();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&bar_pready[grp]);   // S has been read, P is in shared memory
+    }
   }
   cp_async_wait_all();
   tc_fence_before_sync();
@@ -607,11 +686,18 @@ WideParams make_wide_params(const AttnArgs& a, const AttnWorkspace& w, const Pas
 
 template <typename T, int C, int D>
 int fwd_wide_launch(const AttnArgs& a, const AttnWorkspace& w, const PassParams& ps, cudaStream_t s) {
-  const WideParams p = make_wide_params(a, w, ps, a.ncol, ps.nh);
+  WideParams p = make_wide_params(a, w, ps, a.ncol, ps.nh);
+  // q heads per item: a divisor of the kv head's group.  More of them share the staging of K and V and the start of
+  // the pipeline, but a small problem needs its items to fill the SMs evenly.
+  const int group = a.heads / a.heads_k;
+  const int64_t cols = (int64_t)p.items_x * ps.nh * a.batch;
+  for (p.item_heads = group; p.item_heads > 1; --p.item_heads)
+    if (group % p.item_heads == 0 && cols >= (int64_t)p.item_heads * 8 * sm_count()) break;
+  p.items_y = ps.nh / p.item_heads;
   const size_t smem = (size_t)2 * C * D * 2 + (size_t)kM * D * 2 + (size_t)kM * C * 2;   // K, V, Q, P
   auto kern = fwd_wide_tc_kernel<T, C, D>;
   FMB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  kern<<<p.items_x * p.items_y * p.items_z, kThreads, smem, s>>>(p);
+  kern<<<p.items_x * p.items_y * p.items_z, kFwThreads, smem, s>>>(p);
   FMB_LAUNCH_CHECK("fwd_wide_tc_kernel");
   return FMB_OK;
 }

@@ -263,29 +263,6 @@ __device__ __forceinline__ void cp_async_wait_all() {
   asm volatile("cp.async.commit_group;" ::: "memory");
   asm volatile("cp.async.wait_group 0;" ::: "memory");
 }
-// one 128-row x NCHUNK*16-byte tile gathered by a group of NT threads (t = index in the group);
-// rows[] holds the source row of each tile row, -1 = zero fill.  The row ids of GB copies are read before the
-// copies are issued, for the reason given at gather_rows32().
-template <typename T, int NCHUNK, int NT = 128>
-__device__ __forceinline__ void gather_cp_async(int t, unsigned char* tile, uint32_t block_stride, const T* base,
-                                                int64_t row_stride, const int* rows) {
-  static_assert(NT % NCHUNK == 0 && 128 % (NT / NCHUNK) == 0, "a thread keeps one 16-byte chunk column");
-  constexpr int RPP = NT / NCHUNK;           // rows per pass
-  constexpr int PASSES = 128 / RPP, GB = PASSES % 8 == 0 ? 8 : 4;
-  static_assert(PASSES % GB == 0, "whole turns");
-  const int j = t % NCHUNK, rb = t / NCHUNK;
-#pragma unroll 1
-  for (int i0 = 0; i0 < PASSES; i0 += GB) {
-    int src[GB];
-#pragma unroll
-    for (int i = 0; i < GB; ++i) src[i] = rows[rb + RPP * (i0 + i)];
-#pragma unroll
-    for (int i = 0; i < GB; ++i)
-      cp_async_16(tile + sw128_offset(rb + RPP * (i0 + i), j, block_stride),
-                  base + (int64_t)(src[i] < 0 ? 0 : src[i]) * row_stride + j * 8, src[i] >= 0);
-  }
-}
-
 // 32 rows of NCHUNK*16 bytes gathered by one warp: this lane holds the offset of row `lane` from
 // `base` in units of 16 bytes (kNoRow = zero fill); tile: the first of the 32 rows (a multiple of 8) in the swizzled tile.  The offsets of four passes
 // are exchanged before the four copies are issued: shuffles and copies keep their order in the program, and a
