@@ -61,7 +61,7 @@ def _load_accounting():
 
 
 ACC = _load_accounting()
-BWD_MAIN_DRAM_BYTES_PER_ENTRY = 575.2
+BWD_MAIN_DRAM_BYTES_PER_ENTRY = 534.7
 
 
 class ClockSampler:
@@ -577,7 +577,7 @@ def main():
         roof = {"bound": "tensor", "kernel": dom, "achieved": ach, "peak": peak_tf, "unit": "TFLOP/s",
                 "frac": ach / peak_tf, "frac_of_burst": ach / peak_burst, "frac_of_sustained": ach / peak_sust,
                 "traffic": (entry_bytes * entries if entry_bytes else None),
-                "traffic_source": "ncu dram bytes of a 32K-token x 32-head case of this build, scaled by (row, chunk) entries" if entry_bytes else None,
+                "traffic_source": "ncu dram bytes of a 64K-token x 32-head launch, scaled by (row, chunk) entries" if entry_bytes else None,
                 "peak_source": peak_src,
                 "launch_ms": kern_ms[dom], "flops_per_launch": dom_flops,
                 "other_kernels_ms": {k_: v_ for k_, v_ in kern_ms.items() if k_ != dom}}

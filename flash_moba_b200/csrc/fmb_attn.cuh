@@ -7,7 +7,7 @@
 //   forward : part_o[pos][d]  (chunk-local softmax(QK^T)V, normalised, in the I/O dtype)
 //             part_lse[pos]   (chunk-local log-sum-exp, natural log, of the scaled scores)
 //   backward: part_dq[pos][d] (softmax_scale * dS.K of that chunk, in the I/O dtype)
-// A row-major "combine" kernel then merges the partials of each row in ascending `pos`
+// A row-major merge kernel then merges the partials of each row in ascending `pos`
 // order, found through a CSR transpose of the pattern (row_ptr / row_pos) that is rebuilt
 // per call with integer atomics; the merge order is fixed by sorting, so results are
 // run-to-run deterministic and no floating-point atomics are used anywhere.
@@ -20,7 +20,7 @@ namespace fmb {
 // `pos` sits at chunk (c ^ (pos & 7)).  The tensor-core kernels stage a tile of partial rows
 // in shared memory before one bulk copy per warp; with this permutation the 32 lanes of a
 // warp (consecutive positions) write their rows without bank conflicts, and the linear copy
-// preserves it.  Writers and the combine kernels use part_col() for the element index.
+// preserves it.  Writers and the merge kernel use part_col() for the element index.
 __host__ __device__ __forceinline__ int part_col(int64_t pos, int col, int elems_per_chunk) {
   const int chunk = col / elems_per_chunk;
   return ((chunk ^ (int)(pos & 7)) * elems_per_chunk) + (col % elems_per_chunk);
@@ -85,7 +85,7 @@ __device__ __forceinline__ ColRef column_of(const PassParams& r, int b, int h, i
 }
 
 // A key block that starts beyond the sequence's keys contributes nothing: its dQ partials are
-// zero (the combine still reads them).  Called by a whole CTA of the backward kernels (or, _by, by `nthreads` threads numbered `tid`).
+// zero (the merge still reads them).  Called by a whole CTA of the backward kernels (or, _by, by `nthreads` threads numbered `tid`).
 template <typename T>
 __device__ __forceinline__ void zero_dq_partials_by(const PassParams& r, T* part_dq, int64_t plane, int b, int hk,
                                                     int group, int c, int d, int tid, int nthreads) {
