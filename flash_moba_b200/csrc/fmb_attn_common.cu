@@ -1,5 +1,5 @@
-// Pass planning, slot and row lists (CSR transpose of the pattern), the row-major combine
-// kernels and the forward / backward drivers shared by both attention engines.
+// Pass planning, slot and row lists (CSR transpose of the pattern), the row-major merge
+// kernel and the forward / backward drivers shared by both attention engines.
 #include "fmb_attn.cuh"
 
 namespace fmb {
@@ -296,9 +296,10 @@ constexpr int kMergeBatch = 8;      // partial rows in flight per row
 // exp(lse_j - max lse) and writes the row's log-sum-exp; the backward form is a plain sum.
 // Bound: HBM (random 256-byte rows at d = 128), rows taken head by head.  With lists in the order of the
 // gating lists, every lane group had to rank its row's places first and short lists left lanes idle; measured
-// (B200, before / now, forward and backward): 64K tokens x 32 heads, top-k 8 1.19 / 0.94 and 0.93 / 0.79 ms (5.4 GB and
-// 4.8 GB: 5.7 and 6.1 TB/s); 317K tokens, chunk 64, top-k 16 9.6 / 7.7 and 9.8 / 6.8 ms; 512K tokens x 4 heads, chunk 256,
-// top-k 16 5.3 / 3.3 and 3.3 / 2.7 ms; d 64, 9,391 tokens x 12 heads 64 / 27 and 57 / 24 us.
+// (B200, before / now, forward and backward): 64K tokens x 32 heads, top-k 8 1.19 / 0.82 and 0.93 / 0.78 ms (4.9 GB and
+// 4.8 GB: 5.9 and 6.1 TB/s); 317K tokens, chunk 64, top-k 16 9.6 / 7.3 and 9.8 / 6.8 ms; 512K tokens x 4 heads, chunk 256,
+// top-k 16 5.3 / 3.1 and 3.3 / 2.7 ms; d 64, 9,391 tokens x 12 heads 64 / 25 and 57 / 24 us.  Requesting a row's
+// log-sum-exps before the output of the row before, not with its partials, is 10 % of the forward merge (0.915 -> 0.823).
 template <typename T, int D, bool FWD>
 __global__ void __launch_bounds__(kMergeThreads, 3) merge_kernel(const T* __restrict__ part, const float* __restrict__ part_lse,
                                                               MergeParams c, T* out, int64_t rs, int64_t hs, float* lse) {
@@ -323,10 +324,14 @@ __global__ void __launch_bounds__(kMergeThreads, 3) merge_kernel(const T* __rest
     }
   };
   auto place = [&](int64_t p0, int n, int j) -> uint32_t { return j < n ? c.row_pos[p0 + j] : kNoSlot; };
+  auto lse_of = [&](uint32_t s, int sb) {
+    return s == kNoSlot ? -CUDART_INF_F : part_lse[(int64_t)sb * c.cap + (int64_t)(s - (uint32_t)c.slot_shift)];
+  };
   int64_t p0;
   int n;
   span(rid, p0, n);
   uint32_t slot_n = place(p0, n, gl);           // this lane's place of the list, a row ahead
+  float l_n = FWD ? lse_of(slot_n, 0) : 0.f;    // its log-sum-exp: requested ahead of the row before's output
 #pragma unroll 1
   for (int64_t w0 = warp_first; w0 < n_rows; w0 += stride, rid += stride) {
     const int64_t q0 = p0;
@@ -352,12 +357,9 @@ __global__ void __launch_bounds__(kMergeThreads, 3) merge_kernel(const T* __rest
         }
       }
     };
-    auto lse_of = [&](uint32_t s, int sb) {
-      return s == kNoSlot ? -CUDART_INF_F : part_lse[(int64_t)sb * c.cap + (int64_t)(s - (uint32_t)c.slot_shift)];
-    };
     // the first batch is requested before the weights are known
     uint4 x[B];
-    float l = FWD ? lse_of(slot, 0) : 0.f;
+    float l = l_n;
     request(slot, 0, 0, x);
     if (FWD) {
       m = l;
@@ -396,6 +398,7 @@ __global__ void __launch_bounds__(kMergeThreads, 3) merge_kernel(const T* __rest
         }
       }
     }
+    if (FWD) l_n = lse_of(slot_n, 0);
     if (rid < n_rows) {
       const int hr = (int)(rid / c.total_q);
       const int64_t t = rid - (int64_t)hr * c.total_q;
