@@ -138,7 +138,11 @@ __global__ void __launch_bounds__(kDecThreads, DecGeo<D>::CTAS) decode_kernel(De
     b = lo;
   }
   const int q0 = p.cu_q[b], len_q = p.cu_q[b + 1] - q0;
-  if (t < q0 || t >= q0 + len_q) return;        // a row of no sequence (uniform over the cluster)
+  if (t < q0 || t >= q0 + len_q) {              // a row of no sequence (uniform over the cluster) sees no key
+    for (int i = rank * kDecThreads + tid; i < HG * p.d; i += S * kDecThreads)
+      static_cast<T*>(p.out)[(int64_t)t * p.o_rs + (int64_t)(h0 + i / p.d) * p.o_hs + i % p.d] = Elem<T>::from_f(0.f);
+    return;
+  }
   const int k0 = p.cu_k[b], len_k = p.cu_k[b + 1] - k0;
   const int km0 = p.cu_km[b];
   const int nchunks = min((len_k + p.chunk - 1) / p.chunk, p.ncap);

@@ -202,7 +202,7 @@ size_t fmb_attn_bwd_workspace_bytes(int64_t total_q, int heads, int heads_k, int
  * rounding of the probabilities or of partial results), so results agree with fmb_attn_fwd's to the
  * latter's rounding.  km: (km_rows, heads_k, head_dim) contiguous, sequence b's centroids from row
  * cu_seqlens_km[b] on.  No gradients (no log-sum-exp is written).  head_dim: any multiple of 8 up to
- * 256; chunk: a multiple of 64; topk <= 64.
+ * 256; chunk: a multiple of 64; topk <= 64.  Rows of q that belong to no sequence get zeros.
  *
  * fmb_decode_preferred: 1 where this entry point serves the shape and is the faster one (a rule on
  * the sizes the host knows: total_q rows against total_k keys in `batch` sequences), else 0. */
