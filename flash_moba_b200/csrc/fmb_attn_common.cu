@@ -324,21 +324,25 @@ __global__ void __launch_bounds__(kMergeThreads, 3) merge_kernel(const T* __rest
     }
   };
   auto place = [&](int64_t p0, int n, int j) -> uint32_t { return j < n ? c.row_pos[p0 + j] : kNoSlot; };
-  auto lse_of = [&](uint32_t s, int sb) {
-    return s == kNoSlot ? -CUDART_INF_F : part_lse[(int64_t)sb * c.cap + (int64_t)(s - (uint32_t)c.slot_shift)];
+  // slot in the pass of a place's content; kNoSlot also for what is no slot of this pass: nothing else is ever read.
+  // (Applied at the use, not at the load, which is a row ahead.)
+  auto slot_of = [&](uint32_t x) -> uint32_t {
+    const uint32_t at = x - (uint32_t)c.slot_shift;
+    return x != kNoSlot && at < c.cap ? at : kNoSlot;
   };
+  auto lse_of = [&](uint32_t s, int sb) { return s == kNoSlot ? -CUDART_INF_F : part_lse[(int64_t)sb * c.cap + s]; };
   int64_t p0;
   int n;
   span(rid, p0, n);
-  uint32_t slot_n = place(p0, n, gl);           // this lane's place of the list, a row ahead
-  float l_n = FWD ? lse_of(slot_n, 0) : 0.f;    // its log-sum-exp: requested ahead of the row before's output
+  uint32_t next = place(p0, n, gl);             // this lane's place of the list, a row ahead
+  float l_n = FWD ? lse_of(slot_of(next), 0) : 0.f;    // its log-sum-exp: requested ahead of the row before's output
 #pragma unroll 1
   for (int64_t w0 = warp_first; w0 < n_rows; w0 += stride, rid += stride) {
     const int64_t q0 = p0;
     const int nr = n;
-    uint32_t slot = slot_n;
+    const uint32_t slot = slot_of(next);
     span(rid + stride, p0, n);
-    slot_n = place(p0, n, gl);
+    next = place(p0, n, gl);
     const int n_warp = __reduce_max_sync(0xffffffffu, nr);
 
     float m = -CUDART_INF_F, ssum = 0.f, acc[8];
@@ -352,8 +356,7 @@ __global__ void __launch_bounds__(kMergeThreads, 3) merge_kernel(const T* __rest
         if (sk == kNoSlot) {
           x[k] = make_uint4(0, 0, 0, 0);
         } else {
-          const int64_t at = (int64_t)(sk - (uint32_t)c.slot_shift);
-          x[k] = ldg_nc_16(part + ((int64_t)sb * c.cap + at) * D + ((gl ^ (int)(at & 7)) * 8));
+          x[k] = ldg_nc_16(part + ((int64_t)sb * c.cap + sk) * D + ((gl ^ (int)(sk & 7)) * 8));
         }
       }
     };
@@ -365,13 +368,13 @@ __global__ void __launch_bounds__(kMergeThreads, 3) merge_kernel(const T* __rest
       m = l;
       for (int sb = 0; sb < c.nsub; ++sb)       // (longer lists and further planes)
         for (int j0 = sb == 0 ? LPR : 0; j0 < n_warp; j0 += LPR)
-          m = fmaxf(m, lse_of(j0 == 0 ? slot : place(q0, nr, j0 + gl), sb));
+          m = fmaxf(m, lse_of(j0 == 0 ? slot : slot_of(place(q0, nr, j0 + gl)), sb));
 #pragma unroll
       for (int o = LPR / 2; o; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
     }
     for (int sb = 0; sb < c.nsub; ++sb) {
       for (int j0 = 0; j0 < n_warp; j0 += LPR) {
-        const uint32_t s = j0 == 0 ? slot : place(q0, nr, j0 + gl);
+        const uint32_t s = j0 == 0 ? slot : slot_of(place(q0, nr, j0 + gl));
         float w = 1.f;
         if (FWD) {
           if (sb > 0 || j0 > 0) l = lse_of(s, sb);
@@ -398,7 +401,7 @@ __global__ void __launch_bounds__(kMergeThreads, 3) merge_kernel(const T* __rest
         }
       }
     }
-    if (FWD) l_n = lse_of(slot_n, 0);
+    if (FWD) l_n = lse_of(slot_of(next), 0);
     if (rid < n_rows) {
       const int hr = (int)(rid / c.total_q);
       const int64_t t = rid - (int64_t)hr * c.total_q;

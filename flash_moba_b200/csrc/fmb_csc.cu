@@ -41,7 +41,7 @@ struct CscParams {
   int32_t* hist;                                      // [B*H][ntiles][ncol]
   uint32_t* row_slots;                                // optional: [(h*total_q + token)*topk + ...], ascending, 0xffffffff = no entry
   int64_t total_q;
-  int heads, topk, ncol, ntiles, cols_per_cta;
+  int batch, heads, topk, ncol, ntiles, cols_per_cta;
   int scanned;                                        // 1: hist holds cursors (tile_scan has run), 0: counts
 };
 
@@ -167,7 +167,7 @@ __global__ void __launch_bounds__(kCscThreads) csc_scatter_kernel(CscParams p) {
   __shared__ int64_t warp_sums[kCscThreads / 32];
   const int bh = blockIdx.x, tile = blockIdx.y, c0 = blockIdx.z * p.cols_per_cta;
   const int b = bh / p.heads, h = bh - b * p.heads;
-  const int seq0 = p.cu_q[b], len_q = p.cu_q[b + 1] - seq0;
+  const int lead = p.cu_q[0], seq0 = p.cu_q[b], len_q = p.cu_q[b + 1] - seq0;
   const int r0 = tile * kTileRows, rows = min(kTileRows, len_q - r0);
   if (rows <= 0 && tile > 0) return;            // (the first tile of an empty sequence still writes its columns)
   const int ncols = min(p.cols_per_cta, p.ncol - c0);
@@ -229,6 +229,13 @@ __global__ void __launch_bounds__(kCscThreads) csc_scatter_kernel(CscParams p) {
   if (blockIdx.z == 0 && ntiles_b > 0)
     for (int64_t i = carry + (int64_t)tile * kCscThreads + tid; i < (int64_t)len_q * p.topk; i += (int64_t)ntiles_b * kCscThreads)
       p.indices[region + i] = 0;
+  // rows of no sequence (q padded to a fixed size): their lists are empty.  The merge goes over all rows of q
+  if (p.row_slots != nullptr && b == p.batch - 1 && blockIdx.z == 0 && (lead > 0 || seq0 + len_q < p.total_q)) {
+    uint32_t* lists = p.row_slots + (int64_t)h * p.total_q * p.topk;
+    const int64_t first = (int64_t)tile * kCscThreads + tid, step = (int64_t)max(1, ntiles_b) * kCscThreads;
+    for (int64_t i = first; i < (int64_t)lead * p.topk; i += step) lists[i] = 0xffffffffu;
+    for (int64_t i = (int64_t)(seq0 + len_q) * p.topk + first; i < p.total_q * p.topk; i += step) lists[i] = 0xffffffffu;
+  }
   if (rows <= 0) return;
 
   // ---- bitmap of the tile
@@ -337,7 +344,7 @@ int launch_build_csc(const int32_t* topk_idx, int64_t idx_rs, int64_t idx_hs, co
   p.cu_q = cu_q; p.col_offsets = col_offsets; p.col_nnz = col_nnz; p.indices = indices;
   p.hist = static_cast<int32_t*>(ws);
   p.row_slots = row_slots; p.total_q = total_q;
-  p.heads = heads; p.topk = topk; p.ncol = ncol; p.ntiles = csc_ntiles(max_q);
+  p.batch = batch; p.heads = heads; p.topk = topk; p.ncol = ncol; p.ntiles = csc_ntiles(max_q);
   // few tiles: their scatter CTAs add up the counts of the tiles before their own (at most 16 numbers per
   // column) instead of waiting for one more launch
   p.scanned = p.ntiles > 16 ? 1 : 0;

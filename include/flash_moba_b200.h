@@ -135,9 +135,9 @@ int fmb_build_csc(const int32_t* topk_idx, int64_t topk_row_stride, int64_t topk
 /* fmb_build_csc that also writes the row-major view of the pattern it builds: row_slots
  * (uint32, total_q*heads*topk, topk places from (h*total_q + token)*topk on) receives, for every chunk
  * in the top-k list of (token, head h), the position in `indices` where that (row, chunk) pair was
- * put, in ascending order; 0xffffffff fills the places left (chunk ids < 0 or >= ncol).  Rows of sequences shorter than
- * max_seqlen_q and all tokens of the batch are covered; a list must not name a chunk twice (the
- * lists of fmb_gate_topk never do).  fmb_attn_rows_offer hands row_slots to the next fmb_attn_fwd
+ * put, in ascending order; 0xffffffff fills the places left (chunk ids < 0 or >= ncol), and all
+ * places of tokens that belong to no sequence.  Rows of sequences shorter than max_seqlen_q and all tokens of
+ * the batch are covered; a list must not name a chunk twice (the lists of fmb_gate_topk never do).  fmb_attn_rows_offer hands row_slots to the next fmb_attn_fwd
  * or fmb_attn_bwd call made by the same host thread: if that call's geometry matches (total_q,
  * heads, n_indices = total_q*heads*topk) and its workspace holds all heads in one pass, it uses an
  * entry's position in `indices` as its partial-result slot and these row lists, and launches none

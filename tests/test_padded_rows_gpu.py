@@ -34,3 +34,45 @@ def test_decode_kernel_writes_zeros(lens_q, H, Hk, d, pad):
     assert torch.equal(got[n:], torch.zeros_like(got[n:]))
     # (the split of a row's keys over CTAs goes by the number of rows: fp32 sums in another order, then one rounding)
     torch.testing.assert_close(got[:n].float(), decode(q[:n]).float(), rtol=2 ** -7, atol=1e-4)
+
+
+@pytest.mark.parametrize("lens,topk,pad,lead", [([512, 100], 4, 700, 0), ([300], 8, 1, 0), ([40, 0], 16, 600, 0), ([100, 60], 20, 30, 0),
+                                                ([50, 0, 9], 3, 5, 7)])
+def test_row_lists_of_such_rows_are_empty(lens, topk, pad, lead):
+    from flash_moba_b200 import _lib
+    H, ncol, n = 2, 11, sum(lens)
+    T, mx = lead + n + pad, max(lens)
+    cu = (cu_of(lens) + lead).to(torch.int32).to(DEV)
+    lists = torch.randint(0, ncol, (H, T, topk), dtype=torch.int32, device=DEV)
+    co = torch.empty(len(lens), H, ncol, dtype=torch.int64, device=DEV)
+    cn = torch.empty(len(lens), H, ncol, dtype=torch.int32, device=DEV)
+    ind = torch.zeros(T * H * topk, dtype=torch.int32, device=DEV)
+    rows = torch.full((H, T, topk), 12345, dtype=torch.int32, device=DEV)
+    nbytes = _lib.lib.fmb_build_csc_workspace_bytes(len(lens), H, mx, ncol)
+    ws = torch.empty(nbytes, dtype=torch.uint8, device=DEV)
+    _lib.check(_lib.lib.fmb_build_csc_rows(lists.data_ptr(), topk, T * topk, cu.data_ptr(), co.data_ptr(), cn.data_ptr(),
+                                           ind.data_ptr(), rows.data_ptr(), ws.data_ptr(), nbytes, len(lens), H, topk, T, mx, ncol,
+                                           torch.cuda.current_stream().cuda_stream))
+    outside = torch.cat([rows[:, :lead], rows[:, lead + n:]], dim=1)
+    assert torch.equal(outside, torch.full_like(outside, -1))
+
+
+@pytest.mark.parametrize("d,chunk,share", [(64, 64, True), (128, 128, True), (256, 128, True), (128, 128, False)])
+def test_training_step(d, chunk, share, monkeypatch):
+    import flash_moba_b200 as F
+    monkeypatch.setenv("FMB_SHARE_LISTS", "1" if share else "0")      # 0: the attention calls build their own lists
+    torch.manual_seed(chunk + d)
+    lens, H, Hk, topk, pad = [700, 130], 4, 2, 3, 333
+    n, cu = sum(lens), cu_of(lens).to(DEV)
+
+    def step(q, k, v, do):
+        q, k, v = (t.clone().requires_grad_(True) for t in (q, k, v))
+        out = F.flash_moba_varlen_func(q, k, v, cu, cu, max(lens), max(lens), chunk, topk)
+        return [out.detach(), *torch.autograd.grad(out, (q, k, v), do)]
+
+    q, do = (torch.randn(n + pad, H, d, device=DEV).bfloat16() for _ in range(2))
+    k, v = (torch.randn(n, Hk, d, device=DEV).bfloat16() for _ in range(2))
+    want, got = step(q[:n], k, v, do[:n]), step(q, k, v, do)
+    for i, (a, b) in enumerate(zip(want, got)):
+        assert torch.equal(a, b[:n]), i
+        assert torch.equal(b[n:], torch.zeros_like(b[n:])), i
