@@ -268,9 +268,10 @@ __global__ void __launch_bounds__(kDecThreads, DecGeo<D>::CTAS) decode_kernel(De
 #pragma unroll
       for (int j = 0; j < D / 16; ++j) { acc[j][0] *= keep; acc[j][1] *= keep; acc[j][2] *= keep; acc[j][3] *= keep; }
     }
+    const float mref = m > -CUDART_INF_F ? m : 0.f;   // nothing but scores of -inf (no weight) or NaN so far
 #pragma unroll
     for (int kb = 0; kb < KB; ++kb) {
-      const float p0 = exp2f(s[kb][0] - m), p1 = exp2f(s[kb][1] - m);
+      const float p0 = exp2f(s[kb][0] - mref), p1 = exp2f(s[kb][1] - mref);
       l += p0 + p1;
       // P of this thread's value rows: column 0 the rounded value, column 1 what the rounding left
       const float w0 = __shfl_sync(0xffffffffu, p0, 8 * tq), w1 = __shfl_sync(0xffffffffu, p0, 8 * tq + 4);
@@ -317,7 +318,9 @@ __global__ void __launch_bounds__(kDecThreads, DecGeo<D>::CTAS) decode_kernel(De
     if (tq == 0) {                              // columns 0 and 1
 #pragma unroll
       for (int j = 0; j < D / 16; ++j) {
-        const float x = acc[j][0] + acc[j][1], y = acc[j][2] + acc[j][3];
+        // an infinite value makes the hi part infinite, and the lo part infinite the other way or NaN
+        const float x = fabsf(acc[j][0]) < CUDART_INF_F ? acc[j][0] + acc[j][1] : acc[j][0];
+        const float y = fabsf(acc[j][2]) < CUDART_INF_F ? acc[j][2] + acc[j][3] : acc[j][2];
         if constexpr (D == 64) {
           dA[gr * 8 + j] = x;
           dA[gr * 8 + j + 4] = y;
@@ -339,14 +342,13 @@ __global__ void __launch_bounds__(kDecThreads, DecGeo<D>::CTAS) decode_kernel(De
     float mm = -CUDART_INF_F;
     for (int w = 0; w < wph; ++w) mm = fmaxf(mm, M[2 * w]);
     float num = 0.f, den = 0.f;
-    if (mm > -CUDART_INF_F) {
-      for (int w = 0; w < wph; ++w) {
-        const float f = exp2f(M[2 * w] - mm);
-        num = fmaf(f, sAcc[(hr * wph + w) * D + c], num);
-        den = fmaf(f, M[2 * w + 1], den);
-      }
+    for (int w = 0; w < wph; ++w) {
+      const float f = exp2f(M[2 * w] - mm);
+      num = fmaf(f, sAcc[(hr * wph + w) * D + c], num);
+      den = fmaf(f, M[2 * w + 1], den);
     }
-    static_cast<T*>(p.out)[(int64_t)t * p.o_rs + (int64_t)(h0 + hh) * p.o_hs + c] = Elem<T>::from_f(den > 0.f ? num / den : 0.f);
+    // zero only for a row that sees no key (an empty list): NaN in its scores or values stays visible
+    static_cast<T*>(p.out)[(int64_t)t * p.o_rs + (int64_t)(h0 + hh) * p.o_hs + c] = Elem<T>::from_f(sList[hh * topk] >= 0 ? num / den : 0.f);
   }
 }
 

@@ -79,3 +79,62 @@ def test_decode_kernel_ties_and_own_chunk():
     km, cu_km = ops.mean_pool(k.to(DEV), ck.to(DEV), n, chunk)
     got = _decode(q.to(DEV), k.to(DEV), v.to(DEV), km, cu_km, cq.to(DEV), ck.to(DEV), n, topk, chunk, True).cpu().float()
     assert torch.equal(got, torch.full_like(got, (9 + 8 + 7) / 3))
+
+
+def _special(name, q, k, v, own0):
+    """Plants special numbers in keys and values of each row's own chunk (key `own0` on), or in a query."""
+    if name == "nan_q":
+        q[0, 1, 5] = float("nan")
+    elif name == "nan_k":
+        k[own0 + 3, 0, 7] = float("nan")
+    elif name == "nan_v":
+        v[own0 + 3, 0, 7] = float("nan")
+    elif name == "inf_v":
+        v[own0 + 3, 0, 7] = float("inf")
+        v[own0 + 5, 1, 9] = float("-inf")
+    elif name == "inf_k":
+        k[own0 + 3, 0, 7] = float("inf")
+    elif name == "low_k":                          # scores that overflow to -inf for a run of whole groups of keys
+        big = torch.finfo(k.dtype).max
+        for h in range(q.shape[1]):
+            k[own0:own0 + 64, h // (q.shape[1] // k.shape[1])] = -big
+        q.abs_()
+
+
+@pytest.mark.parametrize("d", [64, 128, 256])
+@pytest.mark.parametrize("dtype", ["bf16", "fp16"])
+@pytest.mark.parametrize("name", ["nan_q", "nan_k", "nan_v", "inf_v", "inf_k", "low_k"])
+def test_decode_kernel_special_numbers(name, dtype, d):
+    """NaN and infinities go through as softmax(scores) . V gives them: a row that meets a NaN is NaN, an infinite value with a
+    weight above zero makes its column infinite, keys whose scores are -inf have no weight."""
+    if name == "low_k" and dtype == "fp16":
+        pytest.skip("products of fp16 numbers do not leave the range of fp32")
+    from flash_moba_b200 import ops
+    g = torch.Generator().manual_seed(d)
+    dt = torch.bfloat16 if dtype == "bf16" else torch.float16
+    H, Hk, chunk, topk, n = 4, 2, 128, 3, 1000
+    q, k, v = (torch.randn(m, h, d, generator=g) for m, h in ((1, H), (n, Hk), (n, Hk)))
+    if name == "low_k":
+        q *= 100.0
+    q, k, v = (t.to(dt) for t in (q, k, v))
+    cq, ck = cu_of([1]), cu_of([n])
+    km, cu_km = ops.mean_pool(k.to(DEV), ck.to(DEV), n, chunk)        # centroids before the planted numbers: known lists
+    own0 = (n - 1) // chunk * chunk
+    _special(name, q, k, v, own0)
+    got = _decode(q.to(DEV), k.to(DEV), v.to(DEV), km, cu_km, cq.to(DEV), ck.to(DEV), n, topk, chunk, True).cpu().double()
+    n_km = int(cu_km[-1])
+    idx, _ = O.gate_topk(q.nan_to_num(), km[:n_km].cpu(), cq, ck, cu_km.cpu(), topk, chunk, True)
+    for h in range(H):
+        chunks = [own0 // chunk] if name == "nan_q" and h == 1 else [int(c) for c in idx[0, h] if c >= 0]   # (NaN scores select nothing)
+        keys = torch.cat([torch.arange(c * chunk, min(n, (c + 1) * chunk)) for c in sorted(chunks)])
+        s = (k[keys, h // 2].float() @ q[0, h].float()).double() / math.sqrt(d)
+        p = torch.softmax(s, 0)
+        x = v[keys, h // 2].double()
+        want = torch.where(p.unsqueeze(1) > 0, p.unsqueeze(1) * x, p.unsqueeze(1) * torch.nan_to_num(x, posinf=0, neginf=0)).sum(0)
+        a = got[0, h]
+        assert torch.equal(torch.isnan(a), torch.isnan(want)), h
+        assert torch.equal(torch.isinf(a), torch.isinf(want)) and torch.equal(a[torch.isinf(a)], want[torch.isinf(want)]), h
+        ok = torch.isfinite(want)
+        rel = 2.0 ** -8 if dtype == "bf16" else 2.0 ** -11
+        # (low_k: scores some 100 times larger, and so is the rounding of their fp32 sums: 100 x 2^-24 x sqrt(d) of the weights)
+        assert ((a - want).abs()[ok] <= rel * want.abs()[ok] + (2e-3 if name == "low_k" else 1e-4)).all(), h
