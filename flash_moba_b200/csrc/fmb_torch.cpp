@@ -237,12 +237,13 @@ Pattern build_csc(const Tensor& idx, const Tensor& cu_q, int64_t max_q, int64_t 
 // A pattern that a caller took from flash_topk_varlen_func and hands to flash_moba_attn_varlen_func
 // is recognised by its storage, so that the attention calls on it build no lists of their own.  An
 // entry lives only as long as the pattern's `indices` do (weak references); an in-place write to a
-// pattern tensor changes its version and misses.  At most kKnown entries.
+// pattern tensor changes its version and misses.  Inference tensors have no version, so that a write to
+// one could not be seen: patterns of such tensors are not remembered.  At most kKnown entries.
 struct TensorId {
   const void* ptr = nullptr;
   int64_t numel = 0;
   uint32_t version = 0;
-  explicit TensorId(const Tensor& t) : ptr(t.data_ptr()), numel(t.numel()), version(t.is_inference() ? 0 : t._version()) {}
+  explicit TensorId(const Tensor& t) : ptr(t.data_ptr()), numel(t.numel()), version(t._version()) {}
   TensorId() = default;
   bool operator==(const TensorId& o) const { return ptr == o.ptr && numel == o.numel && version == o.version; }
 };
@@ -264,8 +265,9 @@ std::vector<Known>& known() {
   static auto* v = new std::vector<Known>();      // never destroyed: holds device memory
   return *v;
 }
+bool traceable(const Pattern& p) { return !p.col_offsets.is_inference() && !p.col_nnz.is_inference() && !p.indices.is_inference(); }
 void remember(const Pattern& p) {
-  if (!p.row_slots) return;
+  if (!p.row_slots || !traceable(p)) return;
   std::lock_guard<std::mutex> lock(g_known_mu);
   auto& v = known();
   v.erase(std::remove_if(v.begin(), v.end(), [](const Known& k) { return k.expired(); }), v.end());
@@ -275,6 +277,7 @@ void remember(const Pattern& p) {
 Pattern recall(const Tensor& co, const Tensor& cn, const Tensor& in) {
   Pattern p;
   p.col_offsets = co; p.col_nnz = cn; p.indices = in;
+  if (!traceable(p)) return p;
   std::lock_guard<std::mutex> lock(g_known_mu);
   auto& v = known();
   v.erase(std::remove_if(v.begin(), v.end(), [](const Known& k) { return k.expired(); }), v.end());
