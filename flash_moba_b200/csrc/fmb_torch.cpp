@@ -237,8 +237,9 @@ Pattern build_csc(const Tensor& idx, const Tensor& cu_q, int64_t max_q, int64_t 
 // A pattern that a caller took from flash_topk_varlen_func and hands to flash_moba_attn_varlen_func
 // is recognised by its storage, so that the attention calls on it build no lists of their own.  An
 // entry lives only as long as the pattern's `indices` do (weak references); an in-place write to a
-// pattern tensor changes its version and misses.  Inference tensors have no version, so that a write to
-// one could not be seen: patterns of such tensors are not remembered.  At most kKnown entries.
+// pattern tensor changes its version and misses.  The rows hold places that follow from the sequences'
+// bounds, so these are part of the key.  Inference tensors have no version, so that a write to one could not
+// be seen: patterns of such tensors are not remembered.  At most kKnown entries.
 struct TensorId {
   const void* ptr = nullptr;
   int64_t numel = 0;
@@ -248,16 +249,16 @@ struct TensorId {
   bool operator==(const TensorId& o) const { return ptr == o.ptr && numel == o.numel && version == o.version; }
 };
 struct Known {
-  TensorId id[3];
-  c10::weak_intrusive_ptr<c10::StorageImpl> alive[3];
+  TensorId id[4];
+  c10::weak_intrusive_ptr<c10::StorageImpl> alive[4];
   Tensor row_slots;
   int64_t topk = 0;
-  Known(const Pattern& p)
-      : id{TensorId(p.col_offsets), TensorId(p.col_nnz), TensorId(p.indices)},
+  Known(const Pattern& p, const Tensor& cu_q)
+      : id{TensorId(p.col_offsets), TensorId(p.col_nnz), TensorId(p.indices), TensorId(cu_q)},
         alive{p.col_offsets.storage().getWeakStorageImpl(), p.col_nnz.storage().getWeakStorageImpl(),
-              p.indices.storage().getWeakStorageImpl()},
+              p.indices.storage().getWeakStorageImpl(), cu_q.storage().getWeakStorageImpl()},
         row_slots(*p.row_slots), topk(p.topk) {}
-  bool expired() const { return alive[0].expired() || alive[1].expired() || alive[2].expired(); }
+  bool expired() const { return alive[0].expired() || alive[1].expired() || alive[2].expired() || alive[3].expired(); }
 };
 constexpr size_t kKnown = 4;
 std::mutex g_known_mu;
@@ -265,25 +266,27 @@ std::vector<Known>& known() {
   static auto* v = new std::vector<Known>();      // never destroyed: holds device memory
   return *v;
 }
-bool traceable(const Pattern& p) { return !p.col_offsets.is_inference() && !p.col_nnz.is_inference() && !p.indices.is_inference(); }
-void remember(const Pattern& p) {
-  if (!p.row_slots || !traceable(p)) return;
+bool traceable(const Pattern& p, const Tensor& cu_q) {
+  return !p.col_offsets.is_inference() && !p.col_nnz.is_inference() && !p.indices.is_inference() && !cu_q.is_inference();
+}
+void remember(const Pattern& p, const Tensor& cu_q) {
+  if (!p.row_slots || !traceable(p, cu_q)) return;
   std::lock_guard<std::mutex> lock(g_known_mu);
   auto& v = known();
   v.erase(std::remove_if(v.begin(), v.end(), [](const Known& k) { return k.expired(); }), v.end());
   if (v.size() >= kKnown) v.erase(v.begin());
-  v.emplace_back(p);
+  v.emplace_back(p, cu_q);
 }
-Pattern recall(const Tensor& co, const Tensor& cn, const Tensor& in) {
+Pattern recall(const Tensor& co, const Tensor& cn, const Tensor& in, const Tensor& cu_q) {
   Pattern p;
   p.col_offsets = co; p.col_nnz = cn; p.indices = in;
-  if (!traceable(p)) return p;
+  if (!traceable(p, cu_q)) return p;
   std::lock_guard<std::mutex> lock(g_known_mu);
   auto& v = known();
   v.erase(std::remove_if(v.begin(), v.end(), [](const Known& k) { return k.expired(); }), v.end());
-  const TensorId a(co), b(cn), c(in);
+  const TensorId a(co), b(cn), c(in), d(cu_q);
   for (const Known& k : v)
-    if (k.id[0] == a && k.id[1] == b && k.id[2] == c) {
+    if (k.id[0] == a && k.id[1] == b && k.id[2] == c && k.id[3] == d) {
       p.row_slots = k.row_slots;
       p.topk = k.topk;
       break;
@@ -554,27 +557,27 @@ Tensor try_decode(const Tensor& q0, const Tensor& k0, const Tensor& v0, const Op
 }
 
 using Triple = std::tuple<Tensor, Tensor, Tensor>;
-Triple shown(const Pattern& p) {
-  remember(p);
+Triple shown(const Pattern& p, const Tensor& cu_q) {
+  remember(p, cu_q);
   return {p.col_offsets, p.col_nnz, p.indices};
 }
 
 Triple py_topk_varlen(const Tensor& q, const Tensor& k, const Tensor& cu_q, const Tensor& cu_k, int64_t max_q, int64_t max_k,
                       int64_t topk, int64_t chunk, bool causal) {
-  return shown(moba_pattern(q, k, cu_q, cu_k, max_q, max_k, topk, chunk, causal));
+  return shown(moba_pattern(q, k, cu_q, cu_k, max_q, max_k, topk, chunk, causal), cu_q);
 }
 Triple py_fused_topk(const Tensor& q, const Tensor& km, const Tensor& cu_q, const Tensor& cu_k, const Tensor& cu_km, int64_t max_q,
                      int64_t max_k, int64_t topk, int64_t chunk, bool causal) {
   at::NoGradGuard no_grad;
-  return shown(pattern_from_centroids(fix_last_stride(q), km.contiguous(), cu_q, cu_k, cu_km, max_q, max_k, topk, chunk, causal));
+  return shown(pattern_from_centroids(fix_last_stride(q), km.contiguous(), cu_q, cu_k, cu_km, max_q, max_k, topk, chunk, causal), cu_q);
 }
 Triple py_build_csc(const Tensor& idx, const Tensor& cu_q, int64_t max_q, int64_t ncol, bool keep_rows) {
-  return shown(build_csc(idx, cu_q, max_q, ncol, keep_rows));
+  return shown(build_csc(idx, cu_q, max_q, ncol, keep_rows), cu_q);
 }
 std::tuple<Tensor, Tensor> py_attn_varlen(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& cu_q,
                                           const Tensor& cu_k, int64_t max_q, int64_t max_k, const Tensor& co, const Tensor& cn,
                                           const Tensor& in, int64_t chunk, std::optional<double> scale, bool causal) {
-  return attention(q, k, v, recall(co.contiguous(), cn.contiguous(), in.contiguous()), cu_q, cu_k, max_q, max_k, chunk, scale,
+  return attention(q, k, v, recall(co.contiguous(), cn.contiguous(), in.contiguous(), cu_q), cu_q, cu_k, max_q, max_k, chunk, scale,
                    causal);
 }
 Tensor py_moba_varlen(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& cu_q, const Tensor& cu_k, int64_t max_q,
@@ -597,13 +600,13 @@ std::tuple<Tensor, Tensor, OptTensor> py_attn_fwd(const Tensor& q, const Tensor&
                                                   const Tensor& cn, const Tensor& in, const Tensor& cu_q, const Tensor& cu_k,
                                                   int64_t max_q, int64_t max_k, int64_t chunk, double scale, bool causal,
                                                   const OptTensor& out, const OptTensor& k_begin, const OptTensor& k_end) {
-  return attn_fwd(q, k, v, recall(co, cn, in), cu_q, cu_k, max_q, max_k, chunk, scale, causal, out, k_begin, k_end);
+  return attn_fwd(q, k, v, recall(co, cn, in, cu_q), cu_q, cu_k, max_q, max_k, chunk, scale, causal, out, k_begin, k_end);
 }
 Tensor py_attn_bwd(const Tensor& dout, const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& out, const Tensor& lse,
                    const Tensor& dq, const Tensor& dk, const Tensor& dv, const Tensor& co, const Tensor& cn, const Tensor& in,
                    const Tensor& cu_q, const Tensor& cu_k, int64_t max_q, int64_t max_k, int64_t chunk, double scale, bool causal,
                    const OptTensor& lists) {
-  return attn_bwd(dout, q, k, v, out, lse, dq, dk, dv, recall(co, cn, in), cu_q, cu_k, max_q, max_k, chunk, scale, causal, lists);
+  return attn_bwd(dout, q, k, v, out, lse, dq, dk, dv, recall(co, cn, in, cu_q), cu_q, cu_k, max_q, max_k, chunk, scale, causal, lists);
 }
 
 }  // namespace

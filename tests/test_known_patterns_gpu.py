@@ -39,3 +39,24 @@ def test_edit_in_inference_mode():
         got = _attend(q, k, v, cu, max(lens), pattern)
         want = _attend(q, k, v, cu, max(lens), _copies(pattern))
     assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("inference", [False, True])
+def test_other_sequence_bounds(inference):
+    lens, other = [300, 340], [340, 300]
+    q, k, v = _inputs(lens)
+    cu, cu2 = cu_of(lens).to(DEV), cu_of(other).to(DEV)
+    with torch.inference_mode(inference):
+        pattern = _pattern(q, k, cu, 340)
+        got = _attend(q, k, v, cu2, 340, pattern)
+        want = _attend(q, k, v, cu2, 340, _copies(pattern))
+    assert torch.equal(got, want)
+
+
+def test_bounds_edited_in_place():
+    lens = [300, 340]
+    q, k, v = _inputs(lens)
+    cu = cu_of(lens).to(DEV)
+    pattern = _pattern(q, k, cu, 340)
+    cu[1] = 340
+    assert torch.equal(_attend(q, k, v, cu, 340, pattern), _attend(q, k, v, cu, 340, _copies(pattern)))
