@@ -7,6 +7,7 @@
 // arguments, an autograd Function, two recorded events per attention call, a cache keyed by tuples)
 // needed 0.25 ms per forward call and 0.5-0.6 ms per training step.
 #include <ATen/cuda/CUDAContext.h>
+#include <c10/cuda/CUDACachingAllocator.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <cuda_runtime_api.h>
 #include <torch/csrc/autograd/custom_function.h>
@@ -108,13 +109,17 @@ void drain_status(StatusRing& r, bool block) {
   }
 }
 
+bool capturing() {
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  C10_CUDA_CHECK(cudaStreamIsCapturing((cudaStream_t)current_stream(), &cap));
+  return cap != cudaStreamCaptureStatusNone;
+}
+
 // Claims a slot for the call about to be made; -1: the call's word is not mirrored (checked by
 // synchronising, or the stream is being captured into a graph, whose replays no host code looks at)
 int status_begin(const char* what, const Tensor& q) {
   if (check_status_now()) return -1;
-  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-  C10_CUDA_CHECK(cudaStreamIsCapturing((cudaStream_t)current_stream(), &cap));
-  if (cap != cudaStreamCaptureStatusNone) return -1;
+  if (capturing()) return -1;
   StatusRing& r = ring();
   std::lock_guard<std::mutex> lock(r.mu);
   if (r.words == nullptr) {
@@ -239,7 +244,8 @@ Pattern build_csc(const Tensor& idx, const Tensor& cu_q, int64_t max_q, int64_t 
 // entry lives only as long as the pattern's `indices` do (weak references); an in-place write to a
 // pattern tensor changes its version and misses.  The rows hold places that follow from the sequences'
 // bounds, so these are part of the key.  Inference tensors have no version, so that a write to one could not
-// be seen: patterns of such tensors are not remembered.  At most kKnown entries.
+// be seen: patterns of such tensors are not remembered.  At most kKnown entries, beside those that a captured
+// graph reads: these stay as long as the pattern, which the graph's owner has to keep, does.
 struct TensorId {
   const void* ptr = nullptr;
   int64_t numel = 0;
@@ -253,6 +259,7 @@ struct Known {
   c10::weak_intrusive_ptr<c10::StorageImpl> alive[4];
   Tensor row_slots;
   int64_t topk = 0;
+  bool pinned = false;       // a graph reads row_slots
   Known(const Pattern& p, const Tensor& cu_q)
       : id{TensorId(p.col_offsets), TensorId(p.col_nnz), TensorId(p.indices), TensorId(cu_q)},
         alive{p.col_offsets.storage().getWeakStorageImpl(), p.col_nnz.storage().getWeakStorageImpl(),
@@ -274,7 +281,8 @@ void remember(const Pattern& p, const Tensor& cu_q) {
   std::lock_guard<std::mutex> lock(g_known_mu);
   auto& v = known();
   v.erase(std::remove_if(v.begin(), v.end(), [](const Known& k) { return k.expired(); }), v.end());
-  if (v.size() >= kKnown) v.erase(v.begin());
+  auto spare = [](const Known& k) { return !k.pinned; };
+  if ((size_t)std::count_if(v.begin(), v.end(), spare) >= kKnown) v.erase(std::find_if(v.begin(), v.end(), spare));
   v.emplace_back(p, cu_q);
 }
 Pattern recall(const Tensor& co, const Tensor& cn, const Tensor& in, const Tensor& cu_q) {
@@ -285,8 +293,9 @@ Pattern recall(const Tensor& co, const Tensor& cn, const Tensor& in, const Tenso
   auto& v = known();
   v.erase(std::remove_if(v.begin(), v.end(), [](const Known& k) { return k.expired(); }), v.end());
   const TensorId a(co), b(cn), c(in), d(cu_q);
-  for (const Known& k : v)
+  for (Known& k : v)
     if (k.id[0] == a && k.id[1] == b && k.id[2] == c && k.id[3] == d) {
+      k.pinned = k.pinned || capturing();
       p.row_slots = k.row_slots;
       p.topk = k.topk;
       break;
@@ -311,6 +320,8 @@ bool offer_rows(const Pattern& p, int64_t total_q, int64_t h) {
   if (!share_lists() || !p.row_slots || p.row_slots->numel() != total_q * h * p.topk ||
       p.indices.numel() != p.row_slots->numel())
     return false;
+  // the rows may have been built on another stream; the caller, who never sees them, cannot say so
+  c10::cuda::CUDACachingAllocator::recordStream(p.row_slots->storage().data_ptr(), c10::cuda::getCurrentCUDAStream());
   check(fmb_attn_rows_offer(static_cast<const uint32_t*>(p.row_slots->data_ptr()), total_q, (int)h, (int)p.topk));
   return true;
 }
