@@ -369,6 +369,12 @@ static int check_attn(const char* op, const AttnArgs& a) {
 
 static thread_local const int32_t* g_key_spans[2] = {nullptr, nullptr};
 
+// a call consumes what was offered to it also where it is refused
+struct CallEnd {
+  bool backward;
+  ~CallEnd() { attn_offers_end(backward); }
+};
+
 int fmb_attn_key_spans(const int32_t* k_begin, const int32_t* k_end) {
   FMB_CHECK_ARG((k_begin == nullptr) == (k_end == nullptr), "attn_key_spans: give both arrays or neither");
   g_key_spans[0] = k_begin;
@@ -424,6 +430,7 @@ int fmb_attn_fwd(const void* q, int64_t q_row_stride, int64_t q_head_stride, con
                  size_t workspace_bytes, int batch, int heads, int heads_k, int head_dim, int64_t total_q,
                  int max_seqlen_q, int max_seqlen_k, int chunk, float softmax_scale, int causal, int dtype,
                  fmb_stream_t stream) {
+  const CallEnd end{false};
   AttnArgs a;
   memset(&a, 0, sizeof(a));
   a.q = q; a.k = k; a.v = v; a.o = out;
@@ -464,6 +471,7 @@ int fmb_attn_bwd(const void* dout, int64_t do_row_stride, int64_t do_head_stride
                  size_t workspace_bytes, int batch, int heads, int heads_k, int head_dim, int64_t total_q,
                  int64_t total_k, int max_seqlen_q, int max_seqlen_k, int chunk, float softmax_scale,
                  int causal, int dtype, fmb_stream_t stream) {
+  const CallEnd end{true};
   AttnArgs a;
   memset(&a, 0, sizeof(a));
   a.q = q; a.k = k; a.v = v; a.o = out; a.dout = dout;

@@ -125,6 +125,8 @@ void attn_rows_offer(const uint32_t* row_slots, int64_t total_q, int heads, int 
 // One-shot, per host thread: the next attention call copies its status word to *mirror (memory the
 // device can write and the host can read, e.g. mapped pinned memory) when its main kernels are done.
 void attn_status_mirror(int* mirror);
+// Whatever was offered to this thread's call (rows, mirror; backward: loaded lists) is over, used or not.
+void attn_offers_end(bool backward);
 
 // Builds slot_base and row_ptr / row_pos (CSR transpose of the pass's part of the pattern).
 // Row id = (h - h0)*total_q + token.

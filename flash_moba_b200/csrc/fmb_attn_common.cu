@@ -626,6 +626,12 @@ int attn_lists_load(const AttnArgs& a, const void* src, size_t src_bytes, cudaSt
   return FMB_OK;
 }
 
+void attn_offers_end(bool backward) {
+  g_rows.armed = false;
+  g_mirror = nullptr;
+  if (backward) g_ticket.armed = false;
+}
+
 int launch_attn_bwd(const AttnArgs& a, int engine, cudaStream_t s) {
   AttnWorkspace w = carve_attn_workspace(a.ws, a.ws_bytes, a, 2, false, 0);
   w.mirror = take_mirror();

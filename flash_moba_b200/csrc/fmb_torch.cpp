@@ -137,9 +137,7 @@ int status_begin(const char* what, const Tensor& q) {
   return (int)i;
 }
 void status_end(int ticket, int rc, const Tensor& ws, const char* what) {
-  if (rc != FMB_OK) {                               // what was offered to the call must not reach the next one
-    fmb_attn_status_mirror(nullptr);
-    fmb_attn_rows_offer(nullptr, 0, 0, 0);
+  if (rc != FMB_OK) {
     if (ticket >= 0) ring().words[ticket] = 0;      // nothing will write the slot
     check(rc);
   }
@@ -315,6 +313,16 @@ void check_pattern(const Pattern& p) {
               "moba_col_offsets / moba_col_nnz must both be (batch, heads, ncol)");
 }
 
+// What is offered to the attention call that follows on this thread ends with this scope: an exception between the
+// offer and the call must not leave it to the next call.
+struct Offers {
+  ~Offers() {
+    fmb_attn_status_mirror(nullptr);
+    fmb_attn_rows_offer(nullptr, 0, 0, 0);
+    fmb_attn_key_spans(nullptr, nullptr);
+  }
+};
+
 // offers the pattern builder's rows of this pattern to the attention call that follows on this thread
 bool offer_rows(const Pattern& p, int64_t total_q, int64_t h) {
   if (!share_lists() || !p.row_slots || p.row_slots->numel() != total_q * h * p.topk ||
@@ -375,6 +383,7 @@ std::tuple<Tensor, Tensor, OptTensor> attn_fwd(const Tensor& q, const Tensor& k,
   size_t nbytes = 0;
   Tensor ws = workspace(fmb_attn_fwd_workspace_bytes, q, hk, n_indices, batch, max_k, chunk, &nbytes);
   const bool runs = total_q > 0 && batch > 0;
+  const Offers offers;
   const int ticket = runs ? status_begin("attn_fwd", q) : -1;
   const bool offered = offer_rows(p, total_q, h);
   if (k_begin && k_end)
@@ -421,6 +430,7 @@ Tensor attn_bwd(const Tensor& dout, const Tensor& q, const Tensor& k, const Tens
   size_t nbytes = 0;
   Tensor ws = workspace(fmb_attn_bwd_workspace_bytes, q, hk, n_indices, batch, max_k, chunk, &nbytes);
   const bool runs = total_q > 0 && batch > 0;
+  const Offers offers;
   const int ticket = runs ? status_begin("attn_bwd", q) : -1;
   if (!offer_rows(p, total_q, h) && lists && share_lists()) {
     const int rl = fmb_attn_lists_load(ws.data_ptr(), nbytes, total_q, (int)h, (int)hk, (int)d, n_indices, (int)batch, (int)max_k,

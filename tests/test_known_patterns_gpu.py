@@ -109,3 +109,25 @@ def test_rows_used_under_capture():
     graph.replay()
     torch.cuda.synchronize()
     assert torch.equal(got, want) and len(later) + len(junk) == 22
+
+
+def test_a_refused_call_leaves_nothing_behind():
+    """Rows handed to a call that fails must not reach the next one."""
+    from flash_moba_b200 import _lib
+    lens = [700, 130]
+    q, k, v = _inputs(lens)
+    cu = cu_of(lens).to(DEV)
+    pattern = _pattern(q, k, cu, max(lens))
+    other = _copies(_pattern(k.repeat(1, 2, 1), k, cu, max(lens)))
+    want = _attend(q, k, v, cu, max(lens), other)
+    # a batched tensor has no storage: the call fails between the hand-over and the launch
+    with pytest.raises(RuntimeError):
+        torch.vmap(lambda x: _attend(x, k, v, cu, max(lens), pattern))(q.unsqueeze(0))
+    assert torch.equal(_attend(q, k, v, cu, max(lens), other), want)
+    # the C entry points: refused for its chunk size
+    rows = torch.full((q.shape[1] * q.shape[0] * 3,), -1, dtype=torch.int32, device=DEV)
+    for name in ("fmb_attn_fwd", "fmb_attn_bwd"):
+        _lib.check(_lib.lib.fmb_attn_rows_offer(rows.data_ptr(), q.shape[0], q.shape[1], 3))
+        zeros = [0] * (len(_lib._SIGS[name][1]))
+        assert getattr(_lib.lib, name)(*zeros) != 0
+        assert torch.equal(_attend(q, k, v, cu, max(lens), other), want), name
