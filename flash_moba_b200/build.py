@@ -18,6 +18,7 @@ BUILD = os.path.join(HERE, "_build")
 LIB = os.path.join(HERE, "libflashmoba_b200.so")
 TORCH_EXT = os.path.join(HERE, "_fmb_torch.so")
 TORCH_SRC = os.path.join(CSRC, "fmb_torch.cpp")
+TORCH_HDR = os.path.join(CSRC, "fmb_status_ring.h")
 INCLUDE = os.path.join(os.path.dirname(HERE), "include")
 
 NVCC_FLAGS = [
@@ -41,7 +42,7 @@ def _sources():
 
 
 def _deps_mtime():
-    hdrs = [os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith((".cuh", ".h"))]
+    hdrs = [os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith(".cuh")]
     hdrs += [os.path.join(INCLUDE, f) for f in os.listdir(INCLUDE)]
     return max(os.path.getmtime(h) for h in hdrs)
 
@@ -105,7 +106,7 @@ def build(force: bool = False, verbose: bool = False) -> str:
             raise RuntimeError("link failed:\n" + r.stdout[-4000:])
         if verbose:
             print("linked", LIB)
-    header_t = max(os.path.getmtime(os.path.join(INCLUDE, f)) for f in os.listdir(INCLUDE))
+    header_t = max(os.path.getmtime(f) for f in [os.path.join(INCLUDE, f) for f in os.listdir(INCLUDE)] + [TORCH_HDR])
     if force or not os.path.exists(TORCH_EXT) or os.path.getmtime(TORCH_EXT) < max(os.path.getmtime(TORCH_SRC), header_t):
         _build_torch_ext(os.path.join(BUILD, "fmb_torch.log"))
         if verbose:

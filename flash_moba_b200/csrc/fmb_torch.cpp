@@ -8,21 +8,25 @@
 // needed 0.25 ms per forward call and 0.5-0.6 ms per training step.
 #include <ATen/cuda/CUDAContext.h>
 #include <c10/cuda/CUDACachingAllocator.h>
+#include <c10/cuda/CUDAGraphsC10Utils.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <cuda_runtime_api.h>
 #include <torch/csrc/autograd/custom_function.h>
 #include <torch/extension.h>
 
 #include <algorithm>
+#include <chrono>
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
 #include <mutex>
 #include <optional>
 #include <string>
+#include <thread>
 #include <tuple>
 
 #include "../../include/flash_moba_b200.h"
+#include "fmb_status_ring.h"
 
 namespace {
 
@@ -71,20 +75,15 @@ Tensor bytes_on(const Tensor& like, size_t n) {
 // ---------------------------------------------------------------------------- status words
 // Every attention call leaves a device-side status word: 0, or which bounded wait gave up / 7 = the
 // pattern did not fit the slots.  The library stores it straight into mapped pinned memory
-// (fmb_attn_status_mirror) at the end of the call; the calls that follow look whether it has
-// arrived, without synchronising and without an event: the slot holds kPending until then.  A failure
-// is therefore raised one call late, never silently.  With FMB_CHECK_STATUS=1 every call
-// synchronises and raises at once.
-constexpr int kRing = 256, kPending = -1;
-struct StatusRing {
-  std::mutex mu;
-  volatile int* words = nullptr;
-  const char* what[kRing] = {};
-  int device[kRing] = {};
-  unsigned head = 0, tail = 0;       // next slot to hand out, oldest slot not yet looked at
-};
-StatusRing& ring() {
-  static StatusRing* r = new StatusRing();      // never destroyed: kernels may still write to it at exit
+// (fmb_attn_status_mirror) at the end of the call; the calls that follow look which words have
+// arrived, without synchronising and without an event.  A failure is therefore raised one call late, never
+// silently.  With FMB_CHECK_STATUS=1 every call synchronises and raises at once.
+fmb::StatusRing& ring() {
+  static fmb::StatusRing* r = [] {              // never destroyed: kernels may still write to it at exit
+    void* p = nullptr;
+    C10_CUDA_CHECK(cudaHostAlloc(&p, fmb::StatusRing::kSlots * sizeof(int), cudaHostAllocPortable | cudaHostAllocMapped));
+    return new fmb::StatusRing(static_cast<volatile int*>(p));
+  }();
   return *r;
 }
 
@@ -93,20 +92,9 @@ void raise_for_status(int code, const char* what) {
               ": the pattern does not fit the slots of a pass (overlapping columns, or raise FMB_WORKSPACE_GB)");
   TORCH_CHECK(code == 0, "flash_moba_b200: ", what, ": a bounded device-side wait expired (code ", std::to_string(code), ")");
 }
-
-// looks at the words that have arrived; block: waits for all of them.  Called with the lock held.
-void drain_status(StatusRing& r, bool block) {
-  while (r.tail != r.head) {
-    const unsigned i = r.tail % kRing;
-    if (r.words[i] == kPending) {
-      if (!block) return;
-      c10::cuda::CUDAGuard guard((c10::DeviceIndex)r.device[i]);
-      C10_CUDA_CHECK(cudaDeviceSynchronize());
-    }
-    const int code = r.words[i] == kPending ? 0 : r.words[i];     // still pending: the call launched nothing
-    ++r.tail;
-    raise_for_status(code, r.what[i]);
-  }
+void collect_status() {
+  const fmb::StatusRing::Failure f = ring().collect();
+  raise_for_status(f.code, f.what);
 }
 
 bool capturing() {
@@ -115,45 +103,65 @@ bool capturing() {
   return cap != cudaStreamCaptureStatusNone;
 }
 
-// Claims a slot for the call about to be made; -1: the call's word is not mirrored (checked by
-// synchronising, or the stream is being captured into a graph, whose replays no host code looks at)
-int status_begin(const char* what, const Tensor& q) {
-  if (check_status_now()) return -1;
-  if (capturing()) return -1;
-  StatusRing& r = ring();
-  std::lock_guard<std::mutex> lock(r.mu);
-  if (r.words == nullptr) {
-    void* p = nullptr;
-    C10_CUDA_CHECK(cudaHostAlloc(&p, kRing * sizeof(int), cudaHostAllocPortable | cudaHostAllocMapped));
-    r.words = static_cast<volatile int*>(p);
-  }
-  drain_status(r, r.head - r.tail >= (unsigned)(kRing - 8));
-  const unsigned i = r.head % kRing;
-  r.words[i] = kPending;
-  r.what[i] = what;
-  r.device[i] = q.device().index();
-  ++r.head;
-  check(fmb_attn_status_mirror(const_cast<int*>(r.words) + i));
-  return (int)i;
+// A moment's rest while words are awaited: the words alone, no stream or device is waited for.  After a device
+// error no word will come: the device's stream is asked for one.
+void await_words(int device) {
+  std::this_thread::sleep_for(std::chrono::microseconds(20));
+  c10::cuda::CUDAGuard guard((c10::DeviceIndex)device);
+  if (capturing()) return;
+  c10::cuda::CUDAStreamCaptureModeGuard relaxed(cudaStreamCaptureModeRelaxed);   // (other threads may be capturing)
+  const cudaError_t e = cudaStreamQuery((cudaStream_t)current_stream());
+  if (e != cudaErrorNotReady) C10_CUDA_CHECK(e);
 }
-void status_end(int ticket, int rc, const Tensor& ws, const char* what) {
-  if (rc != FMB_OK) {
-    if (ticket >= 0) ring().words[ticket] = 0;      // nothing will write the slot
-    check(rc);
-  }
-  if (ticket < 0 && check_status_now()) {
-    int code = 0;
-    C10_CUDA_CHECK(cudaMemcpyAsync(&code, ws.data_ptr(), sizeof(int), cudaMemcpyDeviceToHost,
-                                   (cudaStream_t)current_stream()));
-    C10_CUDA_CHECK(cudaStreamSynchronize((cudaStream_t)current_stream()));
-    raise_for_status(code, what);
-  }
-}
+
 void check_pending_status() {
-  StatusRing& r = ring();
-  std::lock_guard<std::mutex> lock(r.mu);
-  drain_status(r, true);
+  const uint64_t claims = ring().claims();
+  for (;;) {
+    collect_status();
+    const int device = ring().outstanding(claims);
+    if (device < 0) return;
+    await_words(device);
+  }
 }
+
+// The status word of the call about to be made.  Not mirrored if it is checked by synchronising, or if the stream is
+// being captured into a graph, whose replays no host code looks at.
+class StatusTicket {
+ public:
+  StatusTicket(const char* what, const Tensor& q, bool runs) : what_(what), runs_(runs) {
+    if (!runs || check_status_now() || capturing()) return;
+    const int device = q.device().index();
+    for (;;) {
+      collect_status();
+      slot_ = ring().claim(what, device);
+      if (slot_ >= 0) break;
+      await_words(device);                      // 256 calls ahead of the GPU
+    }
+    check(fmb_attn_status_mirror(const_cast<int*>(ring().word(slot_))));
+  }
+  ~StatusTicket() {
+    if (slot_ >= 0) ring().withdraw(slot_);     // the call was not made or failed
+  }
+  StatusTicket(const StatusTicket&) = delete;
+  // the call has been made and returned rc
+  void end(int rc, const Tensor& ws) {
+    check(rc);
+    if (slot_ >= 0) {
+      ring().launched(slot_);
+      slot_ = -1;
+    } else if (runs_ && check_status_now()) {
+      int code = 0;
+      C10_CUDA_CHECK(cudaMemcpyAsync(&code, ws.data_ptr(), sizeof(int), cudaMemcpyDeviceToHost, (cudaStream_t)current_stream()));
+      C10_CUDA_CHECK(cudaStreamSynchronize((cudaStream_t)current_stream()));
+      raise_for_status(code, what_);
+    }
+  }
+
+ private:
+  const char* what_;
+  bool runs_;
+  int slot_ = -1;
+};
 
 // ---------------------------------------------------------------------------- stages P, G, O/E/S
 std::tuple<Tensor, Tensor> mean_pool(const Tensor& k, const Tensor& cu_k, int64_t max_k, int64_t chunk) {
@@ -384,7 +392,7 @@ std::tuple<Tensor, Tensor, OptTensor> attn_fwd(const Tensor& q, const Tensor& k,
   Tensor ws = workspace(fmb_attn_fwd_workspace_bytes, q, hk, n_indices, batch, max_k, chunk, &nbytes);
   const bool runs = total_q > 0 && batch > 0;
   const Offers offers;
-  const int ticket = runs ? status_begin("attn_fwd", q) : -1;
+  StatusTicket ticket("attn_fwd", q, runs);
   const bool offered = offer_rows(p, total_q, h);
   if (k_begin && k_end)
     check(fmb_attn_key_spans(static_cast<const int32_t*>(k_begin->data_ptr()), static_cast<const int32_t*>(k_end->data_ptr())));
@@ -394,7 +402,7 @@ std::tuple<Tensor, Tensor, OptTensor> attn_fwd(const Tensor& q, const Tensor& k,
       static_cast<const int64_t*>(p.col_offsets.data_ptr()), static_cast<const int32_t*>(p.col_nnz.data_ptr()),
       static_cast<const int32_t*>(p.indices.data_ptr()), n_indices, cuq, cuk, ws.data_ptr(), nbytes, (int)batch, (int)h, (int)hk,
       (int)d, total_q, (int)max_q, (int)max_k, (int)chunk, (float)scale, causal ? 1 : 0, dtype_code(q), current_stream());
-  if (runs || rc != FMB_OK) status_end(ticket, rc, ws, "attn_fwd");
+  ticket.end(rc, ws);
   OptTensor lists;
   if (share_lists() && n_indices > 0 && runs && !offered) {
     const size_t nlist = fmb_attn_lists_bytes(total_q, (int)h, (int)hk, (int)d, n_indices, (int)batch, (int)max_k, (int)chunk);
@@ -431,7 +439,7 @@ Tensor attn_bwd(const Tensor& dout, const Tensor& q, const Tensor& k, const Tens
   Tensor ws = workspace(fmb_attn_bwd_workspace_bytes, q, hk, n_indices, batch, max_k, chunk, &nbytes);
   const bool runs = total_q > 0 && batch > 0;
   const Offers offers;
-  const int ticket = runs ? status_begin("attn_bwd", q) : -1;
+  StatusTicket ticket("attn_bwd", q, runs);
   if (!offer_rows(p, total_q, h) && lists && share_lists()) {
     const int rl = fmb_attn_lists_load(ws.data_ptr(), nbytes, total_q, (int)h, (int)hk, (int)d, n_indices, (int)batch, (int)max_k,
                                        (int)chunk, lists->data_ptr(), (size_t)lists->numel(), current_stream());
@@ -446,7 +454,7 @@ Tensor attn_bwd(const Tensor& dout, const Tensor& q, const Tensor& k, const Tens
       static_cast<const int32_t*>(p.indices.data_ptr()), n_indices, cuq, cuk, ws.data_ptr(), nbytes, (int)batch, (int)h, (int)hk,
       (int)d, total_q, total_k, (int)max_q, (int)max_k, (int)chunk, (float)scale, causal ? 1 : 0, dtype_code(q),
       current_stream());
-  if (runs || rc != FMB_OK) status_end(ticket, rc, ws, "attn_bwd");
+  ticket.end(rc, ws);
   return softmax_d;
 }
 

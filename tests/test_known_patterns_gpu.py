@@ -62,8 +62,9 @@ def test_bounds_edited_in_place():
     assert torch.equal(_attend(q, k, v, cu, 340, pattern), _attend(q, k, v, cu, 340, _copies(pattern)))
 
 
-def test_rows_used_on_another_stream():
+def test_rows_used_on_another_stream(monkeypatch):
     """The hidden rows stay what they are until the call that reads them is through, whatever the builder's stream does."""
+    monkeypatch.setenv("FMB_CHECK_STATUS", "0")   # (reading the status word back synchronises)
     lens = [3000, 1130]
     q, k, v = _inputs(lens, H=8, Hk=8)
     cu = cu_of(lens).to(DEV)
@@ -73,19 +74,19 @@ def test_rows_used_on_another_stream():
     pattern = _pattern(q, k, cu, max(lens))
     side.wait_stream(torch.cuda.current_stream())
     with torch.cuda.stream(side):
-        torch.cuda._sleep(200_000_000)            # about a tenth of a second
+        torch.cuda._sleep(2_000_000_000)          # about a second
         got = _attend(q, k, v, cu, max(lens), pattern)
     size = pattern[2].numel()
     for t in pattern:
         t.record_stream(side)                     # as the caller of a second stream does
     del pattern
-    later = [_pattern(q, k, cu, max(lens)) for _ in range(5)]
+    later = [_pattern(-q, k, cu, max(lens)) for _ in range(5)]
     junk = [torch.full((size,), -1, dtype=torch.int32, device=DEV) for _ in range(16)]
     torch.cuda.synchronize()
     assert torch.equal(got, want) and len(later) + len(junk) == 21
 
 
-def test_rows_used_under_capture():
+def test_rows_used_under_capture(monkeypatch):
     """A graph that reads the rows of a pattern built before the capture: they live as long as the pattern does."""
     lens = [700, 130]
     q, k, v = _inputs(lens)
@@ -95,14 +96,9 @@ def test_rows_used_under_capture():
     _attend(q, k, v, cu, max(lens), pattern)      # warm-up
     torch.cuda.synchronize()
     graph = torch.cuda.CUDAGraph()
-    import os
-    check = os.environ.pop("FMB_CHECK_STATUS", None)      # (reading the status word back synchronises)
-    try:
-        with torch.cuda.graph(graph):
-            got = _attend(q, k, v, cu, max(lens), pattern)
-    finally:
-        if check is not None:
-            os.environ["FMB_CHECK_STATUS"] = check
+    monkeypatch.setenv("FMB_CHECK_STATUS", "0")   # (reading the status word back synchronises)
+    with torch.cuda.graph(graph):
+        got = _attend(q, k, v, cu, max(lens), pattern)
     later = [_pattern(q, k, cu, max(lens)) for _ in range(6)]
     junk = [torch.full((pattern[2].numel(),), -1, dtype=torch.int32, device=DEV) for _ in range(16)]
     got.zero_()

@@ -17,6 +17,7 @@ import torch
 
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 sys.path.insert(0, ROOT)
+from conftest import cu_of  # noqa: E402
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda"
@@ -115,3 +116,25 @@ def test_attention_sink_column():
     ref = max(float(dvr.abs().max()), float(dkr.abs().max()))
     assert float((dvr - dv[keys, 0].float()).abs().max()) < 0.02 * ref + 2e-2
     assert float((dkr - dk[keys, 0].float()).abs().max()) < 0.02 * ref + 2e-2
+
+
+def test_more_calls_than_status_slots_wait_for_no_other_stream(monkeypatch):
+    """Three hundred calls fill the 256 slots of the status words; an unrelated stream that is busy for about a second is
+    not waited for, neither by a full ring nor by check_pending_status()."""
+    import flash_moba_b200 as F
+    from flash_moba_b200 import ops
+    monkeypatch.setenv("FMB_CHECK_STATUS", "0")
+    q = torch.randn(256, 2, 64, device="cuda").bfloat16()
+    cu = cu_of([256]).cuda()
+    pattern = F.flash_topk_varlen_func(q, q, cu, cu, 256, 256, 2, 64, causal=True)
+    side, busy = torch.cuda.Stream(), torch.cuda.Event()
+    torch.cuda.synchronize()
+    with torch.cuda.stream(side):
+        torch.cuda._sleep(2_000_000_000)
+        busy.record()
+    torch.cuda._sleep(20_000_000)                 # the calls pile up behind this
+    outs = [F.flash_moba_attn_varlen_func(q, q, q, cu, cu, 256, 256, *pattern, 128, 64, causal=True) for _ in range(300)]
+    ops.check_pending_status()
+    assert not busy.query()
+    torch.cuda.synchronize()
+    assert all(torch.equal(o, outs[0]) for o in outs)
