@@ -490,9 +490,12 @@ class MobaAttention : public torch::autograd::Function<MobaAttention> {
     Tensor shown = d == d_og ? out : out.narrow(2, 0, d_og);
     ctx->set_materialize_grads(false);               // no zeros made up for the log-sum-exps' gradient
     if (keep) {
-      ctx->save_for_backward({q, k, v, out, lse, c->cu_q, c->cu_k, c->p.col_offsets, c->p.col_nnz, c->p.indices,
-                              c->p.row_slots.value_or(Tensor()), lists.value_or(Tensor())});
+      ctx->save_for_backward({q, k, v, out, lse, c->cu_q, c->cu_k, c->p.col_offsets, c->p.col_nnz, c->p.indices});
       auto& s = ctx->saved_data;
+      // Which of the two there is depends on what else has been built meanwhile, so they are not saved tensors: a
+      // recomputation has to save what the first pass saved
+      if (c->p.row_slots) s["row_slots"] = *c->p.row_slots;
+      if (lists) s["lists"] = *lists;
       s["geo"] = c10::List<int64_t>({c->max_q, c->max_k, c->chunk, c->p.topk, (int64_t)c->causal, d_og});
       s["scale"] = c->scale;
     }
@@ -504,10 +507,10 @@ class MobaAttention : public torch::autograd::Function<MobaAttention> {
     const Tensor &q = saved[0], &k = saved[1], &v = saved[2];
     Pattern p;
     p.col_offsets = saved[7]; p.col_nnz = saved[8]; p.indices = saved[9];
-    if (saved[10].defined()) p.row_slots = saved[10];
     p.topk = geo[3];
     OptTensor lists;
-    if (saved[11].defined()) lists = saved[11];
+    if (auto it = ctx->saved_data.find("row_slots"); it != ctx->saved_data.end()) p.row_slots = it->second.toTensor();
+    if (auto it = ctx->saved_data.find("lists"); it != ctx->saved_data.end()) lists = it->second.toTensor();
     const int64_t d_og = geo[5], d = q.size(2);
     Tensor dout = g[0].defined() ? pad_to(g[0], d) : at::zeros_like(saved[3]);
     Tensor dq = at::empty_like(q), dk = at::empty_like(k), dv = at::empty_like(v);

@@ -127,3 +127,25 @@ def test_a_refused_call_leaves_nothing_behind():
         zeros = [0] * (len(_lib._SIGS[name][1]))
         assert getattr(_lib.lib, name)(*zeros) != 0
         assert torch.equal(_attend(q, k, v, cu, max(lens), other), want), name
+
+
+def test_checkpointed_layers():
+    """Recomputation saves what the first pass saved, however many patterns were built in between."""
+    from torch.utils.checkpoint import checkpoint
+    lens, layers = [700, 130], 7
+    cu = cu_of(lens).to(DEV)
+    q, k, v = (t.requires_grad_(True) for t in _inputs(lens))
+    patterns = [_pattern(q.detach() * (i + 1), k.detach(), cu, max(lens), topk=2 + i % 3) for i in range(layers)]
+
+    def run(attend):
+        out = sum(attend(q, k, v, cu, max(lens), p) for p in patterns)
+        return torch.autograd.grad(out, (q, k, v), torch.ones_like(out))
+
+    want = run(_attend)
+
+    def recomputed(q, k, v, cu, mx, p):
+        fresh = _pattern(q.detach(), k.detach(), cu, mx)      # a pattern of the layer's own, built again with it
+        return checkpoint(lambda q, k, v: _attend(q, k, v, cu, mx, p) + 0 * _attend(q, k, v, cu, mx, fresh), q, k, v, use_reentrant=False)
+
+    for a, b in zip(want, run(recomputed)):
+        assert torch.equal(a, b)
