@@ -25,12 +25,13 @@ class StatusRing {
   int claim(const char* what, int device) {
     std::lock_guard<std::mutex> lock(mu_);
     for (int n = 0; n < kSlots; ++n) {
-      const int i = (next_ + n) % kSlots;
-      if (slots_[i].state != kFree) continue;
-      next_ = (i + 1) % kSlots;
-      words_[i] = kPending;
-      slots_[i] = Slot{kClaimed, device, what, ++count_};
-      return i;
+      const uint64_t at = head_ + n;
+      Slot& s = slots_[at % kSlots];
+      if (s.state != kFree) continue;
+      head_ = at + 1;
+      words_[at % kSlots] = kPending;
+      s = Slot{kClaimed, device, what, at};
+      return (int)(at % kSlots);
     }
     return -1;
   }
@@ -44,27 +45,30 @@ class StatusRing {
     std::lock_guard<std::mutex> lock(mu_);
     slots_[slot].state = kFree;
   }
-  // frees the slots whose words have arrived, up to the first that reports a failure, which is returned
+  // frees the slots whose words have arrived, in the order of the claims, up to the first that reports a failure,
+  // which is returned
   Failure collect() {
     std::lock_guard<std::mutex> lock(mu_);
-    for (int n = 0; n < kSlots; ++n) {
-      const int i = (next_ + n) % kSlots;               // about the order of the claims
-      if (slots_[i].state != kLaunched || words_[i] == kPending) continue;
-      slots_[i].state = kFree;
-      if (words_[i] != 0) return Failure{words_[i], slots_[i].what};
+    for (; tail_ < head_ && slots_[tail_ % kSlots].state == kFree; ++tail_) {}
+    for (uint64_t at = head_ - tail_ > kSlots ? head_ - kSlots : tail_; at < head_; ++at) {
+      Slot& s = slots_[at % kSlots];
+      const int word = words_[at % kSlots];
+      if (s.state != kLaunched || word == kPending) continue;
+      s.state = kFree;
+      if (word != 0) return Failure{word, s.what};
     }
     return Failure{0, nullptr};
   }
-  // claims so far: what outstanding() is asked about
-  uint64_t claims() {
+  // a bound for outstanding(): the calls made so far
+  uint64_t now() {
     std::lock_guard<std::mutex> lock(mu_);
-    return count_;
+    return head_;
   }
-  // device of a launched call among the first `claims` whose word has not been collected; -1: there is none
-  int outstanding(uint64_t claims) {
+  // device of a launched call from before `bound` whose word has not been collected; -1: there is none
+  int outstanding(uint64_t bound) {
     std::lock_guard<std::mutex> lock(mu_);
     for (const Slot& s : slots_)
-      if (s.state == kLaunched && s.claim <= claims) return s.device;
+      if (s.state == kLaunched && s.at < bound) return s.device;
     return -1;
   }
 
@@ -74,13 +78,12 @@ class StatusRing {
     State state = kFree;
     int device = 0;
     const char* what = nullptr;
-    uint64_t claim = 0;
+    uint64_t at = 0;
   };
   std::mutex mu_;
   volatile int* words_;
   Slot slots_[kSlots];
-  int next_ = 0;
-  uint64_t count_ = 0;
+  uint64_t head_ = 0, tail_ = 0;   // claim number `at` takes slot at % kSlots; no slot in use has a number below tail_
 };
 
 }  // namespace fmb

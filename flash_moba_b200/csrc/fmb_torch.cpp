@@ -115,10 +115,10 @@ void await_words(int device) {
 }
 
 void check_pending_status() {
-  const uint64_t claims = ring().claims();
+  const uint64_t bound = ring().now();
   for (;;) {
     collect_status();
-    const int device = ring().outstanding(claims);
+    const int device = ring().outstanding(bound);
     if (device < 0) return;
     await_words(device);
   }

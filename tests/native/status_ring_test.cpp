@@ -23,7 +23,7 @@ int main() {
     StatusRing r(words);
     const int a = r.claim("a", 0);
     std::thread other([&] {
-      CHECK(1, r.collect().code == 0 && r.outstanding(r.claims()) == -1);
+      CHECK(1, r.collect().code == 0 && r.outstanding(r.now()) == -1);
       std::vector<int> rest;
       for (int i = 1; i < StatusRing::kSlots; ++i) {
         rest.push_back(r.claim("b", 1));
@@ -31,15 +31,15 @@ int main() {
       }
       CHECK(3, r.claim("c", 1) == -1);
       for (int i : rest) { r.launched(i); *r.word(i) = 0; }
-      CHECK(4, r.collect().code == 0 && r.outstanding(r.claims()) == -1);
+      CHECK(4, r.collect().code == 0 && r.outstanding(r.now()) == -1);
     });
     other.join();
     r.launched(a);
-    CHECK(5, r.outstanding(r.claims()) == 0 && r.collect().code == 0);
+    CHECK(5, r.outstanding(r.now()) == 0 && r.collect().code == 0);
     *r.word(a) = 7;
     const StatusRing::Failure f = r.collect();
     CHECK(6, f.code == 7 && f.what[0] == 'a');
-    CHECK(7, r.outstanding(r.claims()) == -1 && r.collect().code == 0);
+    CHECK(7, r.outstanding(r.now()) == -1 && r.collect().code == 0);
   }
   {  // a word that is late holds back no other; a withdrawn slot is free
     StatusRing r(words);
@@ -49,7 +49,7 @@ int main() {
     r.withdraw(none);
     *r.word(bad) = 3;
     CHECK(8, r.collect().code == 3);
-    const uint64_t so_far = r.claims();
+    const uint64_t so_far = r.now();
     for (int i = 1; i < StatusRing::kSlots; ++i) {
       const int s = r.claim("x", 0);
       CHECK(9, s >= 0 && s != late);
@@ -57,7 +57,7 @@ int main() {
     }
     CHECK(10, r.claim("y", 0) == -1);
     *r.word(late) = 0;
-    CHECK(11, r.collect().code == 0 && r.outstanding(so_far) == -1 && r.outstanding(r.claims()) == 0);
+    CHECK(11, r.collect().code == 0 && r.outstanding(so_far) == -1 && r.outstanding(r.now()) == 0);
   }
   {  // several threads: every failure is reported exactly once
     StatusRing r(words);
@@ -79,7 +79,7 @@ int main() {
       });
     for (auto& x : t) x.join();
     take();
-    CHECK(12, sent == got && r.outstanding(r.claims()) == -1);
+    CHECK(12, sent == got && r.outstanding(r.now()) == -1);
   }
   return 0;
 }
