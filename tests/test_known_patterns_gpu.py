@@ -69,6 +69,7 @@ def test_rows_used_on_another_stream(monkeypatch):
     q, k, v = _inputs(lens, H=8, Hk=8)
     cu = cu_of(lens).to(DEV)
     want = _attend(q, k, v, cu, max(lens), _copies(_pattern(q, k, cu, max(lens))))
+    _pattern(-q, k, cu, max(lens)), torch.full((9,), -1, dtype=torch.int32, device=DEV)   # (loading a kernel waits for the GPU)
     side = torch.cuda.Stream()
     torch.cuda.synchronize()
     pattern = _pattern(q, k, cu, max(lens))
@@ -79,7 +80,7 @@ def test_rows_used_on_another_stream(monkeypatch):
     size = pattern[2].numel()
     for t in pattern:
         t.record_stream(side)                     # as the caller of a second stream does
-    del pattern
+    del pattern, t
     later = [_pattern(-q, k, cu, max(lens)) for _ in range(5)]
     junk = [torch.full((size,), -1, dtype=torch.int32, device=DEV) for _ in range(16)]
     torch.cuda.synchronize()
