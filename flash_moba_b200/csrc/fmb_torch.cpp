@@ -557,12 +557,15 @@ Pattern moba_pattern(const Tensor& q0, const Tensor& k0, const Tensor& cu_q, con
   return pattern_from_centroids(q, km, cu_q, cu_k, cu_km, max_q, max_k, topk, chunk, causal);
 }
 
-// A call with few query rows and no gradients to record: one launch for gating and attention
-// (fmb_decode_fwd); undefined where the general path is to run.
+// A call with few query rows and no derivatives to record: one launch for gating and attention
+// (fmb_decode_fwd); undefined where the general path is to run, which also refuses what cannot be (forward-mode
+// derivatives: the autograd node has none).
 Tensor try_decode(const Tensor& q0, const Tensor& k0, const Tensor& v0, const OptTensor& km0, const OptTensor& cu_km0,
                   const Tensor& cu_q, const Tensor& cu_k, int64_t max_k, int64_t topk, int64_t chunk, bool causal) {
   if (at::GradMode::is_enabled() && (q0.requires_grad() || k0.requires_grad() || v0.requires_grad())) return {};
-  if (q0.dim() != 3 || k0.dim() != 3 || v0.dim() != 3 || q0.size(2) % 8 != 0) return {};
+  for (const Tensor* t : {&q0, &k0, &v0})
+    if (t->dim() != 3 || t->_fw_grad(/*level=*/0).defined()) return {};
+  if (q0.size(2) % 8 != 0 || k0.size(2) != q0.size(2) || v0.sizes() != k0.sizes()) return {};
   const int64_t total_q = q0.size(0), h = q0.size(1), d = q0.size(2), hk = k0.size(1), batch = cu_q.numel() - 1;
   if (!fmb_decode_preferred(total_q, k0.size(0), (int)batch, (int)h, (int)hk, (int)d, (int)max_k, (int)topk, (int)chunk)) return {};
   at::NoGradGuard no_grad;
