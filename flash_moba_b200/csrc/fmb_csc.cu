@@ -288,7 +288,7 @@ __global__ void __launch_bounds__(kCscThreads) csc_scatter_kernel(CscParams p) {
     }
     if (p.row_slots != nullptr) {
       uint32_t* out = p.row_slots + ((int64_t)h * p.total_q + seq0 + r0 + tid) * p.topk;
-      if (p.topk == KMAX && gridDim.z == 1) {
+      if (p.topk == KMAX && gridDim.z == 1 && (reinterpret_cast<uintptr_t>(p.row_slots) & 15) == 0) {
 #pragma unroll
         for (int j = 0; j < KMAX; j += 4) *reinterpret_cast<uint4*>(out + j) = make_uint4(at[j], at[j + 1], at[j + 2], at[j + 3]);
       } else {                                                    // a CTA writes the entries of its own columns

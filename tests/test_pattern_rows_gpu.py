@@ -71,3 +71,26 @@ def test_duplicate_ids_count_once():
     got = ops.build_csc(idx.permute(1, 0, 2).contiguous().to(DEV).permute(1, 0, 2), cu.to(DEV), 3, 4)
     for a, b in zip(got, O.build_csc(once, cu, 3, 4)):
         assert torch.equal(a.cpu(), b)
+
+
+@pytest.mark.parametrize("topk", [8, 16])
+def test_row_slots_of_any_alignment(topk):
+    """row_slots is an array of 32-bit numbers that may start anywhere."""
+    from flash_moba_b200 import _lib
+    T, H, ncol = 700, 2, 40
+    g = torch.Generator().manual_seed(topk)
+    lists = torch.rand(H, T, ncol, generator=g).argsort(dim=-1)[..., :topk].to(torch.int32).to(DEV)
+    cu = cu_of([T]).to(DEV)
+    nbytes = _lib.lib.fmb_build_csc_workspace_bytes(1, H, T, ncol)
+    got = []
+    for shift in (0, 1, 2, 3):
+        co, cn = torch.empty(1, H, ncol, dtype=torch.int64, device=DEV), torch.empty(1, H, ncol, dtype=torch.int32, device=DEV)
+        ind, ws = torch.empty(T * H * topk, dtype=torch.int32, device=DEV), torch.empty(nbytes, dtype=torch.uint8, device=DEV)
+        rows = torch.full((H * T * topk + 4,), -7, dtype=torch.int32, device=DEV)
+        _lib.check(_lib.lib.fmb_build_csc_rows(lists.data_ptr(), topk, T * topk, cu.data_ptr(), co.data_ptr(), cn.data_ptr(),
+                                               ind.data_ptr(), rows.data_ptr() + 4 * shift, ws.data_ptr(), nbytes, 1, H, topk, T, T,
+                                               ncol, torch.cuda.current_stream().cuda_stream))
+        n = H * T * topk
+        assert (rows[:shift] == -7).all() and (rows[shift + n:] == -7).all()
+        got.append(rows[shift:shift + n].clone())
+    assert all(torch.equal(x, got[0]) for x in got)
