@@ -32,3 +32,42 @@ def test_forward_mode_is_refused(rows, keys):
                     with pytest.raises((RuntimeError, NotImplementedError)):
                         cache.attend(*args, cq, ck, rows, keys, 2)
     F.flash_moba_varlen_func(q, k, k, cq, ck, rows, keys, 64, 2)     # without tangents: taken
+
+
+@pytest.mark.parametrize("H,Hk,d,chunk,heads_first", [(4, 2, 128, 128, False), (4, 2, 64, 64, False), (16, 2, 64, 64, False), (16, 2, 64, 64, True)])
+def test_rows_that_span_more_than_64_gib(H, Hk, d, chunk, heads_first):
+    """A view of rows that lie far apart: offsets of more than 2^32 units of 16 bytes (16 / 2 heads: items of several heads)."""
+    import flash_moba_b200 as F
+    if torch.cuda.mem_get_info()[0] < 100 << 30:
+        pytest.skip("needs 100 GiB of free device memory")
+    lens, topk = ([1500], 3) if H == 4 else ([63] * 160 + [200] * 5, 2)
+    T = sum(lens)
+    torch.manual_seed(d)
+    base = torch.randn(T, H, d, device=DEV).bfloat16()
+    k, v = (torch.randn(T, Hk, d, device=DEV).bfloat16() for _ in range(2))
+    elements = 36 << 30                                         # 72 GiB
+    buf = torch.empty(elements, dtype=torch.bfloat16, device=DEV)
+    try:
+        rs = (elements - H * d) // T // d * d
+        q = buf.as_strided((T, H, d), (d, elements // H // d * d, 1) if heads_first else (rs, d, 1))
+        assert heads_first or (T - 1) * rs * 2 > 64 << 30
+        q.copy_(base)
+        cu = cu_of(lens).to(DEV)
+        with torch.no_grad():
+            pattern = F.flash_topk_varlen_func(base, k, cu, cu, max(lens), max(lens), topk, chunk, causal=True)
+            args = (k, v, cu, cu, max(lens), max(lens), *pattern, 128, chunk)
+            want = F.flash_moba_attn_varlen_func(base, *args, causal=True, return_attn_probs=True)
+            got = F.flash_moba_attn_varlen_func(q, *args, causal=True, return_attn_probs=True)
+        assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
+        del got
+        from flash_moba_b200 import ops
+        do = torch.randn(T, H, d, device=DEV).bfloat16()
+        grads = []
+        for x in (base, q):
+            g = [torch.empty_like(t) for t in (base, k, v)]
+            ops.attn_bwd(do, x, k, v, want[0], want[1], *g, *pattern, cu, cu, max(lens), max(lens), chunk, d ** -0.5, True)
+            grads.append(g)
+        assert all(torch.equal(a, b) for a, b in zip(*grads))
+    finally:
+        q = buf = None
+        torch.cuda.empty_cache()
