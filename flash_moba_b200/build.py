@@ -61,7 +61,9 @@ def _compile(nvcc, src, obj, log):
 
 def _build_torch_ext(log):
     """_fmb_torch.so: links against the torch libraries of the running interpreter and against
-    libflashmoba_b200.so (found beside it at run time)."""
+    libflashmoba_b200.so (found beside it at run time).  The shared libstdc++ is named: a compiler that has
+    only the static one would give the extension a second copy, whose streams (a number in a TORCH_CHECK message) crash
+    when they meet those of torch's."""
     import sysconfig
 
     import torch
@@ -73,7 +75,7 @@ def _build_torch_ext(log):
     for d in cpp_extension.include_paths() + [sysconfig.get_path("include"), os.path.join(cuda, "include")]:
         cmd += ["-isystem", d]
     cmd += [TORCH_SRC, "-o", TORCH_EXT, "-L", HERE, "-lflashmoba_b200", "-L", torch_lib, "-ltorch_python", "-ltorch",
-            "-ltorch_cpu", "-lc10", "-lc10_cuda", "-L", os.path.join(cuda, "lib64"), "-lcudart", "-Wl,-rpath,$ORIGIN"]
+            "-ltorch_cpu", "-lc10", "-lc10_cuda", "-L", os.path.join(cuda, "lib64"), "-lcudart", "-l:libstdc++.so.6", "-Wl,-rpath,$ORIGIN"]
     r = subprocess.run(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
     with open(log, "w") as f:
         f.write(" ".join(cmd) + "\n" + r.stdout)

@@ -21,7 +21,6 @@
 #include <cstring>
 #include <mutex>
 #include <optional>
-#include <string>
 #include <thread>
 #include <tuple>
 
@@ -33,12 +32,10 @@ namespace {
 using at::Tensor;
 using OptTensor = std::optional<Tensor>;
 
-// (Numbers in messages go through std::to_string: the streams behind TORCH_CHECK may be another C++
-// library's than this file's, and formatting an integer through them has crashed.)
 void check(int rc) {
   if (rc == FMB_OK) return;
   const char* msg = fmb_last_error();
-  if (msg == nullptr || msg[0] == 0) TORCH_CHECK(false, "flash_moba_b200 error ", std::to_string(rc));
+  if (msg == nullptr || msg[0] == 0) TORCH_CHECK(false, "flash_moba_b200 error ", rc);
   TORCH_CHECK(false, msg);
 }
 
@@ -90,7 +87,7 @@ fmb::StatusRing& ring() {
 void raise_for_status(int code, const char* what) {
   TORCH_CHECK(code != 7, "flash_moba_b200: ", what,
               ": the pattern does not fit the slots of a pass (overlapping columns, or raise FMB_WORKSPACE_GB)");
-  TORCH_CHECK(code == 0, "flash_moba_b200: ", what, ": a bounded device-side wait expired (code ", std::to_string(code), ")");
+  TORCH_CHECK(code == 0, "flash_moba_b200: ", what, ": a bounded device-side wait expired (code ", code, ")");
 }
 void collect_status() {
   const fmb::StatusRing::Failure f = ring().collect();
@@ -380,8 +377,8 @@ std::tuple<Tensor, Tensor, OptTensor> attn_fwd(const Tensor& q, const Tensor& k,
   const int64_t total_q = q.size(0), h = q.size(1), d = q.size(2), hk = k.size(1), batch = cu_q.numel() - 1;
   TORCH_CHECK(p.col_offsets.size(0) == batch && p.col_offsets.size(1) == h, "pattern shape does not match (batch, heads)");
   const int64_t ncol = (max_k + chunk - 1) / chunk;
-  TORCH_CHECK(p.col_offsets.size(2) == ncol, "pattern has ", std::to_string(p.col_offsets.size(2)),
-              " columns, expected ceil(max_seqlen_k/lg_block_n) = ", std::to_string(ncol));
+  TORCH_CHECK(p.col_offsets.size(2) == ncol, "pattern has ", p.col_offsets.size(2),
+              " columns, expected ceil(max_seqlen_k/lg_block_n) = ", ncol);
   const int32_t* cuq = i32c(cu_q, "cu_seqlens_q");
   const int32_t* cuk = i32c(cu_k, "cu_seqlens_k");
   c10::cuda::CUDAGuard guard(q.device());
