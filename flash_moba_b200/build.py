@@ -7,6 +7,7 @@ Objects go to flash_moba_b200/_build/, the libraries next to this file, so that 
 libraries travel with a snapshot of the source tree.
 """
 import concurrent.futures
+import importlib.metadata
 import os
 import shutil
 import subprocess
@@ -109,8 +110,13 @@ def build(force: bool = False, verbose: bool = False) -> str:
         if verbose:
             print("linked", LIB)
     header_t = max(os.path.getmtime(f) for f in [os.path.join(INCLUDE, f) for f in os.listdir(INCLUDE)] + [TORCH_HDR])
-    if force or not os.path.exists(TORCH_EXT) or os.path.getmtime(TORCH_EXT) < max(os.path.getmtime(TORCH_SRC), header_t):
+    # the extension holds the layouts of the torch it was compiled against
+    made_for, stamp = f"{sys.version} torch {importlib.metadata.version('torch')}", os.path.join(BUILD, "fmb_torch.made_for")
+    fits = os.path.exists(stamp) and open(stamp).read() == made_for
+    if force or not fits or not os.path.exists(TORCH_EXT) or os.path.getmtime(TORCH_EXT) < max(os.path.getmtime(TORCH_SRC), header_t):
         _build_torch_ext(os.path.join(BUILD, "fmb_torch.log"))
+        with open(stamp, "w") as f:
+            f.write(made_for)
         if verbose:
             print("linked", TORCH_EXT)
     return LIB
