@@ -9,6 +9,7 @@ libraries travel with a snapshot of the source tree.
 import concurrent.futures
 import importlib.metadata
 import os
+import re
 import shutil
 import subprocess
 import sys
@@ -29,6 +30,25 @@ NVCC_FLAGS = [
 # --use_fast_math must not touch the CUDA-core validation engine or the combine kernels'
 # exp/log: those files are built without it.
 PRECISE = {"fmb_attn_simt.cu", "fmb_attn_common.cu", "fmb_gate.cu", "fmb_pool.cu"}
+
+
+# Kernels that hand registers from some warps to others count on the launch's share per thread: (source, kernel, the
+# constant in the source that names it).  A wrong hand-over would never return, so a compiler that allocates
+# another number fails the build (and the launches check it once more).
+REGISTERS = [("fmb_attn_tc.cu", "fwd_main_tc_kernel", "kFwdRegsLaunch"), ("fmb_attn_tc.cu", "bwd_main_tc_kernel", "kBwdRegsLaunch"),
+             ("fmb_attn_tc_wide.cu", "bwd_wide_tc_kernel", "kBwRegsLaunch")]
+
+
+def check_registers(src_name, source, log):
+    """Raises if the compiler's report (-Xptxas -v) on `src_name` shows another number of registers than its text counts on."""
+    for name, kernel, constant in REGISTERS:
+        if name != src_name:
+            continue
+        want = int(re.search(constant + r" = (\d+)", source).group(1))
+        got = [int(n) for entry, n in re.findall(r"Compiling entry function '(\w+)'.*?Used (\d+) registers", log, flags=re.S)
+               if kernel in entry]
+        if not got or any(n != want for n in got):
+            raise RuntimeError(f"{src_name}: {kernel} was built with {got} registers per thread, {constant} = {want} expected")
 
 
 def _nvcc():
@@ -57,6 +77,12 @@ def _compile(nvcc, src, obj, log):
         f.write(" ".join(cmd) + "\n" + r.stdout)
     if r.returncode != 0:
         raise RuntimeError(f"nvcc failed on {src}:\n{r.stdout[-4000:]}")
+    try:
+        with open(src) as f:
+            check_registers(os.path.basename(src), f.read(), r.stdout)
+    except RuntimeError:
+        os.remove(obj)                   # not taken for built by the next run
+        raise
     return obj
 
 

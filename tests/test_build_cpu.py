@@ -1,4 +1,5 @@
-"""What the build leaves behind: one C++ runtime in the process, an extension that fits the running torch."""
+"""What the build leaves behind: one C++ runtime in the process, an extension that fits the running torch, and the
+register counts that the kernels' hand-over of registers counts on."""
 import importlib.metadata
 import importlib.util
 import os
@@ -43,3 +44,16 @@ def test_extension_is_rebuilt_for_another_torch(monkeypatch, tmp_path):
     version[0] = "0.0"
     b.build()
     assert len(built) == 2
+
+
+def test_register_counts_are_checked_at_build_time():
+    b = _build_module()
+    source = open(os.path.join(PKG, "csrc", "fmb_attn_tc.cu")).read()
+    log = "".join(f"ptxas info    : Compiling entry function '_ZN3fmb18{k}I6__halfLi64EEEvPi' for 'sm_100a'\nptxas info    : Used {n} "
+                  "registers, used 1 barriers\n" for k, n in (("fwd_main_tc_kernel", 72), ("bwd_main_tc_kernel", 96), ("other", 40)))
+    b.check_registers("fmb_attn_tc.cu", source, log)
+    with pytest.raises(RuntimeError, match="fwd_main_tc_kernel was built with"):
+        b.check_registers("fmb_attn_tc.cu", source, log.replace("Used 72", "Used 71"))
+    with pytest.raises(RuntimeError, match="bwd_main_tc_kernel was built with"):
+        b.check_registers("fmb_attn_tc.cu", source, log.replace("bwd_main", "bwd_side"))
+    b.check_registers("fmb_gate.cu", "", "")
