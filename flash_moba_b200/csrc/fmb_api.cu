@@ -72,7 +72,7 @@ using namespace fmb;
 
 extern "C" {
 
-int fmb_version(void) { return 100; }
+int fmb_version(void) { return 101; }
 
 const char* fmb_last_error(void) { return error_buffer(); }
 

@@ -10,7 +10,7 @@
  * State the library keeps (everything else lives in the caller's buffers):
  *   - per host thread: the text behind fmb_last_error(); the one-shot offers made with
  *     fmb_attn_rows_offer, fmb_attn_lists_load, fmb_attn_status_mirror and fmb_attn_key_spans,
- *     consumed by that thread's next attention call;
+ *     consumed by that thread's next attention call, also where that call is refused;
  *   - per process: the engine selected with fmb_set_engine, the launch counter and the event
  *     records of fmb_launch_count / fmb_profile_*;
  *   - per device: the gating kernel's status word (fmb_gate_status) and the 8 MiB scratch array
@@ -55,7 +55,9 @@ enum {
   FMB_ERR_TIMEOUT = 5       /* a bounded device-side wait expired              */
 };
 
-/* Library version (major*10000 + minor*100 + patch). */
+/* Library version (major*10000 + minor*100 + patch).
+ * 101: row_slots of fmb_build_csc_rows lists a row's places in ascending order (100: in the order of the
+ *      row's top-k list); fmb_gate_topk_sized, fmb_decode_preferred and fmb_decode_fwd exist. */
 int fmb_version(void);
 
 /* Message of the last failing call made by this thread ("" if none). */

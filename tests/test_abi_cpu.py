@@ -96,3 +96,10 @@ def test_decide_lg_block_m_matches_reference_table():
     assert F.decide_lg_block_m(8, 128, 2048, True) == 128
     assert F.decide_lg_block_m(8, 128, 4096, True) == 256
     assert F.decide_lg_block_m(4, 128, 1024, False) == 128
+
+
+def test_version_says_what_row_slots_holds():
+    """A caller that reads the places of fmb_build_csc_rows by their position in the list can tell the two orders apart."""
+    from flash_moba_b200 import _lib
+    header = open(os.path.join(ROOT, "include", "flash_moba_b200.h")).read()
+    assert _lib.lib.fmb_version() >= 101 and "101: row_slots of fmb_build_csc_rows" in header
