@@ -103,3 +103,15 @@ def test_version_says_what_row_slots_holds():
     from flash_moba_b200 import _lib
     header = open(os.path.join(ROOT, "include", "flash_moba_b200.h")).read()
     assert _lib.lib.fmb_version() >= 101 and "101: row_slots of fmb_build_csc_rows" in header
+
+
+@pytest.mark.parametrize("seqs,keys,rows,preferred", [
+    (16, 16000, 1, 1), (16, 16000, 16, 1), (1, 65001, 1, 1),    # the row-major kernel 56 / 522, 615 / 1222, 19 / 149 us
+    (4, 2000, 4, 1), (4, 2000, 16, 0),                         # 43 / 96 and 140 / 99 us
+    (1, 32768, 32768, 0), (8, 8192, 8192, 0),                  # prompts
+])
+def test_decode_size_rule(seqs, keys, rows, preferred):
+    """Both sides of the line between the row-major kernel and the key-chunk-major ones, at shapes where both were measured
+    (32 / 8 heads, head dim 128, chunk 128, top-k 8)."""
+    from flash_moba_b200 import _lib
+    assert _lib.lib.fmb_decode_preferred(seqs * rows, seqs * keys, seqs, 32, 8, 128, keys, 8, 128) == preferred

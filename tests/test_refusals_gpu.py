@@ -59,7 +59,7 @@ def test_rows_that_span_more_than_64_gib(H, Hk, d, chunk, heads_first):
             want = F.flash_moba_attn_varlen_func(base, *args, causal=True, return_attn_probs=True)
             got = F.flash_moba_attn_varlen_func(q, *args, causal=True, return_attn_probs=True)
         assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
-        del got
+        got = None
         from flash_moba_b200 import ops
         do = torch.randn(T, H, d, device=DEV).bfloat16()
         grads = []
@@ -69,5 +69,5 @@ def test_rows_that_span_more_than_64_gib(H, Hk, d, chunk, heads_first):
             grads.append(g)
         assert all(torch.equal(a, b) for a, b in zip(*grads))
     finally:
-        q = buf = None
+        x = q = buf = args = None
         torch.cuda.empty_cache()
