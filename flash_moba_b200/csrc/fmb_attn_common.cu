@@ -418,55 +418,33 @@ __global__ void __launch_bounds__(kMergeThreads, 3) merge_kernel(const T* __rest
   }
 }
 
-// D[h, t] = sum_d dO.O.  LPR lanes per row, each with one 16-byte load of dO and of O (LPR = d / 8
-// when that is a power of two); LPR = 0 selects the generic warp-per-row form.
+// D[h, t] = sum_d dO.O.  LPR = d / 8 lanes per row, each with one 16-byte load of dO and of O.
 template <typename T, int LPR>
 __global__ void __launch_bounds__(256) dot_do_o_kernel(const T* __restrict__ dout, int64_t do_rs, int64_t do_hs,
                                                        const T* __restrict__ o, int64_t o_rs, int64_t o_hs,
-                                                       float* softmax_d, int64_t total_q, int heads, int d) {
-  using T2 = typename Elem<T>::T2;
+                                                       float* softmax_d, int64_t total_q, int heads) {
   const int lane = threadIdx.x & 31;
   const int64_t wid = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  if (LPR > 0) {
-    constexpr int L = LPR > 0 ? LPR : 32;
-    const int64_t row = wid * (32 / L) + lane / L;
-    float s = 0.f;
-    if (row < total_q * heads) {
-      const int64_t t = row / heads;
-      const int h = (int)(row - t * heads);
-      const int c = (lane % L) * 8;
-      float x[8], y[8];
-      unpack8<T>(ldg_nc_16(dout + t * do_rs + (int64_t)h * do_hs + c), x);
-      unpack8<T>(ldg_nc_16(o + t * o_rs + (int64_t)h * o_hs + c), y);
-#pragma unroll
-      for (int e = 0; e < 8; ++e) s = fmaf(x[e], y[e], s);
-    }
-#pragma unroll
-    for (int o2 = L / 2; o2; o2 >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o2);
-    if (row < total_q * heads && lane % L == 0) {
-      const int64_t t = row / heads;
-      softmax_d[(int64_t)(row - t * heads) * total_q + t] = s;
-    }
-    return;
-  }
-  if (wid >= total_q * heads) return;
-  const int64_t t = wid / heads;
-  const int h = (int)(wid - t * heads);
-  const T* a = dout + t * do_rs + (int64_t)h * do_hs;
-  const T* b = o + t * o_rs + (int64_t)h * o_hs;
+  const int64_t row = wid * (32 / LPR) + lane / LPR;
   float s = 0.f;
-  for (int c = lane * 2; c < d; c += 64) {
-    const float2 x = Elem<T>::to_f2(*reinterpret_cast<const T2*>(a + c));
-    const float2 y = Elem<T>::to_f2(*reinterpret_cast<const T2*>(b + c));
-    s = fmaf(x.x, y.x, s);
-    s = fmaf(x.y, y.y, s);
+  if (row < total_q * heads) {
+    const int64_t t = row / heads;
+    const int h = (int)(row - t * heads);
+    const int c = (lane % LPR) * 8;
+    float x[8], y[8];
+    unpack8<T>(ldg_nc_16(dout + t * do_rs + (int64_t)h * do_hs + c), x);
+    unpack8<T>(ldg_nc_16(o + t * o_rs + (int64_t)h * o_hs + c), y);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) s = fmaf(x[e], y[e], s);
   }
 #pragma unroll
-  for (int o2 = 16; o2; o2 >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o2);
-  if (lane == 0) softmax_d[(int64_t)h * total_q + t] = s;
+  for (int o2 = LPR / 2; o2; o2 >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o2);
+  if (row < total_q * heads && lane % LPR == 0) {
+    const int64_t t = row / heads;
+    softmax_d[(int64_t)(row - t * heads) * total_q + t] = s;
+  }
 }
 
-static int64_t warp_grid(int64_t warps) { return ceil_div64(warps, 8); }
 int sm_count() {
   int dev = 0, n = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0)
@@ -511,13 +489,13 @@ static int dot_do_o_dispatch(const AttnArgs& a, cudaStream_t s) {
   const int64_t rows = a.total_q * a.heads;
   const T* dout = (const T*)a.dout;
   const T* o = (const T*)a.o;
-#define FMB_DOT(LPR_)                                                                                        \
-  dot_do_o_kernel<T, LPR_><<<(unsigned)warp_grid(ceil_div64(rows, LPR_ ? 32 / (LPR_ ? LPR_ : 1) : 1)), 256, 0, s>>>( \
-      dout, a.do_rs, a.do_hs, o, a.o_rs, a.o_hs, a.softmax_d, a.total_q, a.heads, a.d)
+#define FMB_DOT(LPR_)                                                                                              \
+  dot_do_o_kernel<T, LPR_><<<(unsigned)ceil_div64(ceil_div64(rows, 32 / LPR_), 8), 256, 0, s>>>(                     \
+      dout, a.do_rs, a.do_hs, o, a.o_rs, a.o_hs, a.softmax_d, a.total_q, a.heads)
   if (a.d == 128) FMB_DOT(16);
   else if (a.d == 64) FMB_DOT(8);
   else if (a.d == 256) FMB_DOT(32);
-  else FMB_DOT(0);
+  else return fail(FMB_ERR_UNSUPPORTED, "attention: head_dim %d not built (64, 128 or 256)", a.d);
 #undef FMB_DOT
   FMB_LAUNCH_CHECK("dot_do_o_kernel");
   return FMB_OK;

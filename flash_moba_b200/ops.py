@@ -40,12 +40,6 @@ def _i32c(t: torch.Tensor, name: str) -> torch.Tensor:
     return t
 
 
-def _last_contig(t: torch.Tensor, name: str) -> torch.Tensor:
-    if t.stride(-1) != 1:
-        raise RuntimeError(f"{name} must have contiguous last dimension")
-    return t
-
-
 def ptr(t: Optional[torch.Tensor]) -> int:
     return 0 if t is None else t.data_ptr()
 
