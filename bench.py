@@ -565,11 +565,10 @@ def main():
     dom = "bwd_main" if backward else "fwd_main"
     dom_flops = (bwd_f if backward else fwd_f) * (1.0 / world if by_range else h_loc / H)      # rank 0's launch (about, under the range split)
     roof = None
-    # DRAM bytes per (row, chunk) entry of the dominant kernel, from one ncu capture of this build on
-    # 32K tokens x 32 heads (profiles/main_kernels_traffic_32k.md: dram__bytes_read.sum +
-    # dram__bytes_write.sum = 4,759.1 MB over its 8,273,920 entries; the same head-by-head order of
-    # work items as the 64K workload); the traffic is per-entry work (gathered rows in, partial rows
-    # out), so it scales with the entries.
+    # DRAM bytes per (row, chunk) entry of the dominant kernel, from one ncu capture of a 64K-token x 32-head launch
+    # (profiles/main_kernels_traffic_64k.md: dram__bytes_read.sum + dram__bytes_write.sum = 8.91 GB over its
+    # 16,662,528 entries); the traffic is per-entry work (gathered rows in, partial rows out), so it scales with the
+    # entries.
     entry_bytes = {"bwd_main": BWD_MAIN_DRAM_BYTES_PER_ENTRY}.get(dom) if (d == 128 and chunk == 128) else None
     entries = ACC.selected_entries(seqlens, chunk, topk) * h_loc / (world if by_range else 1)
     if kern_ms.get(dom):

@@ -7,13 +7,14 @@
 // (row, chunk) entries, 0.83 ms).  Here a thread-block cluster owns one query row of HG q heads of a kv
 // head and does everything for it, row-major:
 //   1. scores of the row against the centroids of its candidate chunks (fp32), a warp per 32
-//      centroids; each head's scores are collected in the shared memory of one CTA of the cluster
+//      centroids (16 at head dim 256); each head's scores are collected in the shared memory of one CTA of the cluster
 //   2. top-k of each head by one warp (descending score, on equal scores the higher chunk id, the
 //      row's own chunk first under the causal rule: the order of the other gating kernels); the list
 //      goes to every CTA of the cluster
-//   3. attention over the selected chunks, a warp per 32 keys: fp32 scores, online softmax, fp32
+//   3. attention over the selected chunks, a warp per 32 (16) keys: fp32 scores, online softmax, fp32
 //      accumulation; the warps' results meet in the owner CTA's shared memory and are merged in warp
-//      order, so that the result does not depend on timing
+//      order, so that the result does not depend on timing (its last bits do on how many CTAs share a row,
+//      which goes by the number of rows)
 // No pattern, no partials in global memory, no merge launch.  What bounds it: the selected K and V
 // rows, each read once per (row, head) from L2 or HBM.
 //
@@ -25,8 +26,10 @@
 // g and g + 8 (g = lane / 4) and uses them as A fragments as they are, the order of the head dimension
 // inside the product being the same for q.  The values are the A operand of the second product (M =
 // head dim): pairs of key rows are interleaved with byte permutes.  P is used as the sum of two
-// 16-bit numbers (hi in column 0, lo in column 1 of the otherwise unused N side): no rounding of P.
-// All loads of a group (16 KB per warp) are issued before its arithmetic; one CTA of 8 warps per SM.
+// 16-bit numbers (hi in column 0, lo in column 1 of the otherwise unused N side): 16 bits of it in bf16, 22
+// in fp16, where the key-chunk-major kernels keep 8 and 11.
+// All loads of a group (8 KB per warp at d 64, else 16 KB) are issued before its arithmetic; CTAs of 4 warps, four per
+// SM at d 64, else two.
 // Measured (B200, 32 / 8 heads, d 128, chunk 128, top-k 8): see decode_preferred().
 #include <cooperative_groups.h>
 

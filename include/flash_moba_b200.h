@@ -200,9 +200,10 @@ size_t fmb_attn_bwd_workspace_bytes(int64_t total_q, int heads, int heads_k, int
 /* ------------------------------------------------- few query rows: gating + attention in one launch
  * out[row,h] as fmb_attn_fwd gives it for the pattern that fmb_gate_topk + fmb_build_csc would build
  * from the same centroids, without building one: for decoding and short blocks of new rows, where
- * the columns of the pattern hold a row or two each.  The same selection rule; fp32 throughout (no
- * rounding of the probabilities or of partial results), so results agree with fmb_attn_fwd's to the
- * latter's rounding.  km: (km_rows, heads_k, head_dim) contiguous, sequence b's centroids from row
+ * the columns of the pattern hold a row or two each.  The same selection rule; fp32 scores, sums and
+ * partial results, probabilities kept to 16 (bf16) or 22 (fp16) bits, so results agree with
+ * fmb_attn_fwd's, which rounds probabilities and partial results to the I/O type, to the latter's rounding.
+ * The last bits depend on how many rows the call has (more CTAs share a row when there are few).  km: (km_rows, heads_k, head_dim) contiguous, sequence b's centroids from row
  * cu_seqlens_km[b] on.  No gradients (no log-sum-exp is written).  head_dim: any multiple of 8 up to
  * 256; chunk: a multiple of 64; topk <= 64.  Rows of q that belong to no sequence get zeros.
  *

@@ -1,7 +1,7 @@
 """The row-major kernel for few query rows (fmb_decode_fwd: gating and attention in one launch),
 called through the C ABI whatever the size rule says, against the CPU oracle on the same centroids.
 
-Tolerance: scores, probabilities and sums are fp32 and only the result is rounded to the I/O type,
+Tolerance: scores and sums are fp32, probabilities keep at least 16 bits, and only the result is rounded to the I/O type,
 so |x - fp32| <= half a unit in the last place: with p significant bits the unit of a value in
 [2^e, 2^(e+1)) is 2^(e-p+1), so half of it is at most 2^-p of the value (p = 8 in bf16, 11 in fp16);
 plus fp32 summation error over at most 64 * 320 keys of values below 6 (1e-4 absolute covers it)."""
