@@ -264,13 +264,13 @@ __device__ __forceinline__ void cp_async_wait_all() {
   asm volatile("cp.async.wait_group 0;" ::: "memory");
 }
 // 32 rows of NCHUNK*16 bytes gathered by one warp: this lane holds the offset of row `lane` from
-// `base` in units of `unit` bytes (kNoRow = zero fill); tile: the first of the 32 rows (a multiple of 8) in the swizzled tile.  The offsets of four passes
+// `base` in units of UNIT bytes (kNoRow = zero fill); tile: the first of the 32 rows (a multiple of 8) in the swizzled tile.  The offsets of four passes
 // are exchanged before the four copies are issued: shuffles and copies keep their order in the program, and a
 // shuffle's latency in front of every copy held a warp to 92 cycles per copy (5.3 B/clk) whatever else the SM
 // did; measured for whole tiles of 128 rows, B200.  The loop stays rolled: code size counts in these kernels.
 constexpr uint32_t kNoRow = 0xffffffffu;
-template <int NCHUNK>
-__device__ __forceinline__ void gather_rows32(int lane, unsigned char* tile, uint32_t block_stride, const void* base, uint32_t off, uint32_t unit) {
+template <int NCHUNK, int UNIT>
+__device__ __forceinline__ void gather_rows32(int lane, unsigned char* tile, uint32_t block_stride, const void* base, uint32_t off) {
   constexpr int RPP = 32 / NCHUNK;           // rows per pass
   constexpr int GB = 4;                      // copies per turn of the loop
   const int j = lane % NCHUNK, rsub = lane / NCHUNK;
@@ -286,7 +286,7 @@ __device__ __forceinline__ void gather_rows32(int lane, unsigned char* tile, uin
       const int r = (i0 + i) * RPP;          // plus rsub
       const uint32_t d = dst + r * 128 + ((((uint32_t)j & 7) ^ ((r + rsub) & 7)) << 4);
       const bool ok = o[i] != kNoRow;
-      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src + (size_t)(ok ? o[i] : 0u) * unit), "r"(ok ? 16u : 0u)
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src + (size_t)(ok ? o[i] : 0u) * UNIT), "r"(ok ? 16u : 0u)
                    : "memory");
     }
   }

@@ -71,3 +71,27 @@ def test_rows_that_span_more_than_64_gib(H, Hk, d, chunk, heads_first):
     finally:
         x = q = buf = args = None
         torch.cuda.empty_cache()
+
+
+def test_rows_whose_distance_fits_no_unit():
+    """More than 64 GiB apart and no multiple of a head's row: the CUDA-core kernels take the call.  Both engines round
+    probabilities and partial results to 8 bits, at most 2^-8 each of sums of topk parts: 1e-2 in the 2-norm."""
+    import flash_moba_b200 as F
+    if torch.cuda.mem_get_info()[0] < 100 << 30:
+        pytest.skip("needs 100 GiB of free device memory")
+    T, H, d, chunk = 1500, 4, 64, 64
+    torch.manual_seed(5)
+    base = torch.randn(T, H, d, device=DEV).bfloat16()
+    k, v = (torch.randn(T, 2, d, device=DEV).bfloat16() for _ in range(2))
+    buf = torch.empty(36 << 30, dtype=torch.bfloat16, device=DEV)
+    try:
+        q = buf.as_strided((T, H, d), (((36 << 30) - H * d) // T // 8 * 8 // 64 * 64 + 8 - 64, d, 1))
+        q.copy_(base)
+        cu = cu_of([T]).to(DEV)
+        with torch.no_grad():
+            pattern = F.flash_topk_varlen_func(base, k, cu, cu, T, T, 3, chunk, causal=True)
+            want, got = (F.flash_moba_attn_varlen_func(x, k, v, cu, cu, T, T, *pattern, 128, chunk, causal=True).float() for x in (base, q))
+        assert (got - want).norm() <= 1e-2 * want.norm()
+    finally:
+        q = buf = None
+        torch.cuda.empty_cache()
