@@ -1,6 +1,6 @@
 """Patterns of the library's own builder that come back through flash_moba_attn_varlen_func: the row-major view kept beside them
 is used only where it describes the call, lives as long as a kernel may read it, and is not part of what autograd
-saves.  The checker is the same call on copies of the pattern tensors, for which the library builds its own lists."""
+saves.  Compared with the same call on copies of the pattern tensors, for which the library builds its own lists."""
 import pytest
 import torch
 
