@@ -81,13 +81,6 @@ __device__ __forceinline__ void gather_rows16(int lane, unsigned char* tile, uin
   }
 }
 
-// 32 bytes (aligned to 32) in one store: a lane that writes a row of its own then fills whole sectors
-__device__ __forceinline__ void st_global_32(void* dst, uint4 a, uint4 b) {
-  asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(dst), "r"(a.x), "r"(a.y), "r"(a.z), "r"(a.w),
-               "r"(b.x), "r"(b.y), "r"(b.z), "r"(b.w)
-               : "memory");
-}
-
 // ---- forward
 // Work item = key block of one (sequence, several q heads of a kv head); one CTA per item, which walks the 128-row tiles
 // of the heads' columns; 768 threads, warp-specialised:
