@@ -32,6 +32,7 @@ __host__ __device__ __forceinline__ int part_col(int64_t pos, int col, int elems
 // entries over the pass's columns in (b, h, c) order), and a key chunk wider than the kernels'
 // key block KB is handled as nsub = chunk / KB sub-blocks, each with its own plane of `cap`
 // slots: the partial of (entry j of the column, sub-block sb) lives at sb*cap + slot_base + j.
+constexpr int kStatusBytes = 512;   // the workspace's status block: status word, work counter
 struct AttnWorkspace {
   int* status;          // first word: 0, or where a bounded device wait gave up (1-6, 8) / 7 = slot overflow / 9 = misaligned shared memory
   void* part_o;         // nsub*cap*d elements of the I/O dtype (fwd: O partials, bwd: dQ partials)
@@ -136,8 +137,6 @@ int build_row_lists(const AttnArgs& a, const AttnWorkspace& w, const PassParams&
 int launch_fwd_combine(const AttnArgs& a, const AttnWorkspace& w, const PassParams& ps, cudaStream_t s);
 // dq = sum of the row's backward partials (already scaled)
 int launch_bwd_combine(const AttnArgs& a, const AttnWorkspace& w, const PassParams& ps, cudaStream_t s);
-// softmax_d[h, t] = sum_d dout*out
-int launch_dot_do_o(const AttnArgs& a, cudaStream_t s);
 
 // engines: main kernels that produce the partials (and dk/dv in backward)
 int launch_fwd_main_simt(const AttnArgs& a, const AttnWorkspace& w, const PassParams& ps, cudaStream_t s);
