@@ -97,6 +97,7 @@ constexpr int kFwDrainWarp = 8, kFwIssuerWarp = 12, kFwLoadWarp = 16, kFwLoaders
 template <typename T, int C, int D>
 __global__ void __launch_bounds__(kFwThreads, 1) fwd_wide_tc_kernel(WideParams p) {
   static_assert(D == 256 && (C == 64 || C == 128), "head dim 256, key blocks of 64 or 128");
+  follow_on();
   constexpr int NCH = D / 8;                    // 16-byte chunks of a row
   constexpr uint32_t kKBlock = C * 128;         // bytes between 64-element blocks of the K / V tiles
   constexpr uint32_t kQBlock = kM * 128;        // same for the 128-row Q and P tiles
@@ -356,6 +357,7 @@ static_assert(2 * (kBwRegsCompute - kBwRegsLaunch) <= 4 * (kBwRegsLaunch - kBwRe
 template <typename T, int D>
 __global__ void __launch_bounds__(kBwThreads, 1) bwd_wide_tc_kernel(WideParams p) {
   static_assert(D == 256, "two head-dim halves of 128 TMEM lanes");
+  follow_on();
   constexpr int NCH = D / 8;
   constexpr uint32_t kKBlock = kC * 128;
   constexpr uint32_t kQBlock = kM * 128;
@@ -690,7 +692,7 @@ int fwd_wide_launch(const AttnArgs& a, const AttnWorkspace& w, const PassParams&
   const size_t smem = (size_t)2 * C * D * 2 + (size_t)kM * D * 2 + (size_t)kM * C * 2;   // K, V, Q, P
   auto kern = fwd_wide_tc_kernel<T, C, D>;
   FMB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  kern<<<p.items_x * p.items_y * p.items_z, kFwThreads, smem, s>>>(p);
+  FMB_CUDA(launch_follow_on(kern, dim3(p.items_x * p.items_y * p.items_z), dim3(kFwThreads), smem, s, p));
   FMB_LAUNCH_CHECK("fwd_wide_tc_kernel");
   return FMB_OK;
 }
@@ -709,7 +711,7 @@ int bwd_wide_launch(const AttnArgs& a, const AttnWorkspace& w, const PassParams&
   if (regs != kBwRegsLaunch)
     return fail(FMB_ERR_CUDA, "wide-head backward: built with %d registers per thread (%d expected)", regs, kBwRegsLaunch);
   FMB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  kern<<<p.items_x * p.items_y * p.items_z, kBwThreads, smem, s>>>(p);
+  FMB_CUDA(launch_follow_on(kern, dim3(p.items_x * p.items_y * p.items_z), dim3(kBwThreads), smem, s, p));
   FMB_LAUNCH_CHECK("bwd_wide_tc_kernel");
   return FMB_OK;
 }

@@ -87,6 +87,7 @@ __device__ __forceinline__ void csc_load_row(const CscParams& p, const int32_t* 
 // KMAX as for the scatter kernel below.  A chunk that a row names twice counts once.
 template <int KMAX>
 __global__ void __launch_bounds__(kCscThreads) csc_tile_hist_kernel(CscParams p) {
+  follow_on();
   extern __shared__ uint32_t sm[];
   const int bh = blockIdx.x, tile = blockIdx.y, c0 = blockIdx.z * p.cols_per_cta;
   const int b = bh / p.heads, h = bh - b * p.heads;
@@ -130,6 +131,7 @@ __global__ void __launch_bounds__(kCscThreads) csc_tile_hist_kernel(CscParams p)
 
 // grid (b*h, groups of 32 columns): 32 warps, lane = column; the tiles are cut into 32 runs, one per warp
 __global__ void __launch_bounds__(1024) csc_tile_scan_kernel(CscParams p) {
+  follow_on();
   __shared__ int run_sum[32][33];
   const int bh = blockIdx.x, b = bh / p.heads;
   const int ntiles_b = (p.cu_q[b + 1] - p.cu_q[b] + kTileRows - 1) / kTileRows;
@@ -163,6 +165,7 @@ __global__ void __launch_bounds__(1024) csc_tile_scan_kernel(CscParams p) {
 // a thread per entry
 template <int KMAX>
 __global__ void __launch_bounds__(kCscThreads) csc_scatter_kernel(CscParams p) {
+  follow_on();
   extern __shared__ uint32_t sm[];
   __shared__ int64_t warp_sums[kCscThreads / 32];
   const int bh = blockIdx.x, tile = blockIdx.y, c0 = blockIdx.z * p.cols_per_cta;
@@ -351,11 +354,11 @@ int launch_build_csc(const int32_t* topk_idx, int64_t idx_rs, int64_t idx_hs, co
   prof_begin(6, s);
   p.cols_per_cta = min(kMaxHistCols, ncol);
   auto count = topk <= 8 ? csc_tile_hist_kernel<8> : topk <= 16 ? csc_tile_hist_kernel<16> : csc_tile_hist_kernel<0>;
-  count<<<dim3(batch * heads, p.ntiles, ceil_div(ncol, p.cols_per_cta)), kCscThreads,
-                         (size_t)p.cols_per_cta * sizeof(uint32_t), s>>>(p);
+  FMB_CUDA(launch_follow_on(count, dim3(batch * heads, p.ntiles, ceil_div(ncol, p.cols_per_cta)), dim3(kCscThreads),
+                            (size_t)p.cols_per_cta * sizeof(uint32_t), s, p));
   FMB_LAUNCH_CHECK("csc_tile_hist_kernel");
   if (p.scanned) {
-    csc_tile_scan_kernel<<<dim3(batch * heads, ceil_div(ncol, 32)), 1024, 0, s>>>(p);
+    FMB_CUDA(launch_follow_on(csc_tile_scan_kernel, dim3(batch * heads, ceil_div(ncol, 32)), dim3(1024), 0, s, p));
     FMB_LAUNCH_CHECK("csc_tile_scan_kernel");
   }
   p.cols_per_cta = min(kMaxColsPerCta, ncol);
@@ -364,7 +367,7 @@ int launch_build_csc(const int32_t* topk_idx, int64_t idx_rs, int64_t idx_hs, co
   auto scatter = topk <= 8 ? csc_scatter_kernel<8> : topk <= 16 ? csc_scatter_kernel<16> : csc_scatter_kernel<0>;
   // the attribute belongs to the current device: set on every call (cheap, idempotent, thread-safe)
   FMB_CUDA(cudaFuncSetAttribute(scatter, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxColsPerCta * kColBytes));
-  scatter<<<grid, kCscThreads, smem, s>>>(p);
+  FMB_CUDA(launch_follow_on(scatter, grid, dim3(kCscThreads), smem, s, p));
   prof_end(6, s);
   FMB_LAUNCH_CHECK("csc_scatter_kernel");
   return FMB_OK;

@@ -704,6 +704,7 @@ __global__ void __launch_bounds__(kSelThreads, D <= 128 ? 2 : 1)
 gate_select_kernel(GateParams p, const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_km,
                    int batch, int row_tiles, FastDiv by_chunk) {
   using namespace tc;
+  follow_on();
   constexpr uint32_t kQTile = kGateM * D * 2, kKTile = kSelN * D * 2;
   constexpr int CAP = sel_cap<KMAX>();                   // queue entries per thread
   constexpr int STEP = KMAX == 8 ? 8 : 4;                // scores between two looks at the queue's length
@@ -1059,7 +1060,7 @@ static int gate_select_launch(const GateParams& p, const CUtensorMap& mq, const 
   const int row_tiles = ceil_div(max_q, kGateM);
   const int64_t items = (int64_t)row_tiles * p.heads * batch;
   const int64_t ctas = (int64_t)sm_count() * (D <= 128 ? 2 : 1);
-  kern<<<(unsigned)(items < ctas ? items : ctas), kSelThreads, smem, s>>>(p, mq, mk, batch, row_tiles, fd);
+  FMB_CUDA(launch_follow_on(kern, dim3((unsigned)(items < ctas ? items : ctas)), dim3(kSelThreads), smem, s, p, mq, mk, batch, row_tiles, fd));
   FMB_LAUNCH_CHECK("gate_select_kernel");
   return FMB_OK;
 }

@@ -54,6 +54,7 @@ mean_pool_kernel(const T* __restrict__ k, int64_t row_stride, int64_t head_strid
                  const int32_t* __restrict__ cu_k, int32_t* cu_km,
                  T* __restrict__ km, int heads_k, int d, int chunk) {
   constexpr int RPI = 32 / LPR;
+  follow_on();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int n = blockIdx.x * kPoolWarps + warp;  // chunk of this sequence
   const int hk = blockIdx.y, b = blockIdx.z;
