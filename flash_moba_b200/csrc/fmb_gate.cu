@@ -702,7 +702,7 @@ constexpr int kSelSeqs = 64;         // sequences whose bounds are kept in share
 template <typename T, int D, int KMAX>
 __global__ void __launch_bounds__(kSelThreads, D <= 128 ? 2 : 1)
 gate_select_kernel(GateParams p, const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_km,
-                   int batch, int row_tiles, FastDiv by_chunk) {
+                   int batch, int row_tiles, FastDiv by_chunk, FastDiv by_tile, FastDiv by_heads) {
   using namespace tc;
   follow_on();
   constexpr uint32_t kQTile = kGateM * D * 2, kKTile = kSelN * D * 2;
@@ -742,7 +742,7 @@ gate_select_kernel(GateParams p, const __grid_constant__ CUtensorMap map_q, cons
   const int per_tile = p.heads * batch, n_items = row_tiles * per_tile;
   struct Item { int h, r0, q0, rows, shift, km0, nchunks, nt; };
   auto decode = [&](int item, Item& I) -> bool {
-    const int x = item / per_tile, y = item - x * per_tile, b = y / p.heads;
+    const int x = fast_div(item, by_tile), y = item - x * per_tile, b = fast_div(y, by_heads);
     int len_k, km1;
     I.h = y - b * p.heads;
     I.r0 = (row_tiles - 1 - x) * kGateM;
@@ -1050,17 +1050,21 @@ static int gate_select_launch(const GateParams& p, const CUtensorMap& mq, const 
   constexpr int kCap = sel_cap<KMAX>();
   const size_t smem = 1024 + (size_t)kGateM * D * 2 + (size_t)kSelRing * kSelN * D * 2 + (size_t)kCap * 256 * 8;
   static_assert(2 * KMAX * 32 * 4 <= kCap * 64 * 8, "a pair's exchange area fits its queues");
-  FastDiv fd{0, 0, (uint32_t)p.chunk};
-  if (p.chunk > 1) {                   // 2^(32 + shift) / chunk rounded up, shift = ceil(log2(chunk)) - 1
-    while ((2u << fd.shift) < fd.d) ++fd.shift;
-    fd.mul = (uint32_t)((((uint64_t)1 << (32 + fd.shift)) + fd.d - 1) / fd.d);
-  }
+  auto divider = [](int d) {
+    FastDiv fd{0, 0, (uint32_t)d};
+    if (d > 1) {                       // 2^(32 + shift) / d rounded up, shift = ceil(log2(d)) - 1
+      while ((2u << fd.shift) < fd.d) ++fd.shift;
+      fd.mul = (uint32_t)((((uint64_t)1 << (32 + fd.shift)) + fd.d - 1) / fd.d);
+    }
+    return fd;
+  };
   auto kern = gate_select_kernel<T, D, KMAX>;
   FMB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   const int row_tiles = ceil_div(max_q, kGateM);
   const int64_t items = (int64_t)row_tiles * p.heads * batch;
   const int64_t ctas = (int64_t)sm_count() * (D <= 128 ? 2 : 1);
-  FMB_CUDA(launch_follow_on(kern, dim3((unsigned)(items < ctas ? items : ctas)), dim3(kSelThreads), smem, s, p, mq, mk, batch, row_tiles, fd));
+  FMB_CUDA(launch_follow_on(kern, dim3((unsigned)(items < ctas ? items : ctas)), dim3(kSelThreads), smem, s, p, mq, mk, batch, row_tiles,
+                            divider(p.chunk), divider(p.heads * batch), divider(p.heads)));
   FMB_LAUNCH_CHECK("gate_select_kernel");
   return FMB_OK;
 }
