@@ -18,9 +18,12 @@
 //                  order (row_slots): the row-major view of the pattern that the attention kernels' merge
 //                  needs, so that an attention call on this pattern builds no lists of its own.
 // Measured (B200, three kernels with bitmap walks before / now): 64K tokens x 32 heads, 512 columns 297 / 192 us; 32K x 16
-// 71 / 45; 317K tokens, lists of 16 2.19 / 1.63 ms; 512K x 4 heads, 2,048 columns 1.49 / 0.84 ms.
+// 71 / 45; 317K tokens, lists of 16 2.19 / 1.63 ms; 512K x 4 heads, 2,048 columns 1.49 / 0.84 ms.  The scatter with its counts per 32
+// rows laid out column by column (stores of a warp eight to a bank) and 64-bit scans / row group by row group and 32-bit scans:
+// 64K 143 / 129 us, 317K 1.32 / 1.23 ms, 512K 0.80 / 0.71 ms.
 // HBM bound.  Algorithmic bytes: 4*nnz read + 4*nnz written + 12*B*H*ncol.
 #include <mutex>
+#include <type_traits>
 
 #include "fmb_common.cuh"
 
@@ -167,7 +170,9 @@ template <int KMAX>
 __global__ void __launch_bounds__(kCscThreads) csc_scatter_kernel(CscParams p) {
   follow_on();
   extern __shared__ uint32_t sm[];
-  __shared__ int64_t warp_sums[kCscThreads / 32];
+  // places inside a (b, h)'s region: fewer than 65,535 tiles of 512 rows, of lists of up to 16, fit 32 bits
+  using Off = typename std::conditional<(KMAX > 0), int, int64_t>::type;
+  __shared__ Off warp_sums[kCscThreads / 32];
   const int bh = blockIdx.x, tile = blockIdx.y, c0 = blockIdx.z * p.cols_per_cta;
   const int b = bh / p.heads, h = bh - b * p.heads;
   const int lead = p.cu_q[0], seq0 = p.cu_q[b], len_q = p.cu_q[b + 1] - seq0;
@@ -176,7 +181,7 @@ __global__ void __launch_bounds__(kCscThreads) csc_scatter_kernel(CscParams p) {
   const int ncols = min(p.cols_per_cta, p.ncol - c0);
   const int ntiles_b = (len_q + kTileRows - 1) / kTileRows;
   uint32_t* bm = sm;                                              // [ncols][kBmStride] bit (row) of every column
-  uint16_t* before = reinterpret_cast<uint16_t*>(bm + ncols * kBmStride);   // [ncols][kTileWords] rows ahead of each 32
+  uint16_t* before = reinterpret_cast<uint16_t*>(bm + ncols * kBmStride);   // [kTileWords][ncols] rows ahead of each 32
   uint32_t* base = reinterpret_cast<uint32_t*>(before + ncols * kTileWords);   // [ncols] first place of the tile's entries
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int64_t region = ((int64_t)seq0 * p.heads + (int64_t)len_q * h) * p.topk;   // first place of this (b, h) in `indices`
@@ -184,7 +189,7 @@ __global__ void __launch_bounds__(kCscThreads) csc_scatter_kernel(CscParams p) {
 
   // ---- column offsets (places inside the region) and this tile's cursor in every column
   const int32_t* hist = p.hist + (int64_t)bh * p.ntiles * p.ncol;
-  int64_t carry = 0;
+  Off carry = 0;
   for (int g0 = 0; g0 < p.ncol; g0 += kCscThreads) {
     const int c = g0 + tid;
     int nnz = 0, cursor = 0;
@@ -201,23 +206,23 @@ __global__ void __launch_bounds__(kCscThreads) csc_scatter_kernel(CscParams p) {
         }
       }
     }
-    int64_t x = nnz;
+    Off x = nnz;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-      const int64_t y = __shfl_up_sync(0xffffffffu, x, o);
+      const Off y = __shfl_up_sync(0xffffffffu, x, o);
       if (lane >= o) x += y;
     }
     if (lane == 31) warp_sums[warp] = x;
     __syncthreads();
-    int64_t ahead = carry, total = 0;
+    Off ahead = carry, total = 0;
 #pragma unroll
     for (int w = 0; w < kCscThreads / 32; ++w) {
-      const int64_t y = warp_sums[w];
+      const Off y = warp_sums[w];
       ahead += w < warp ? y : 0;
       total += y;
     }
     if (c < p.ncol) {
-      const int64_t off = ahead + x - nnz;
+      const Off off = ahead + x - nnz;
       if (c >= c0 && c < c0 + ncols) base[c - c0] = (uint32_t)(off + cursor);
       if (tile == 0 && blockIdx.z == 0) {
         p.col_offsets[(int64_t)bh * p.ncol + c] = region + off;
@@ -265,7 +270,7 @@ __global__ void __launch_bounds__(kCscThreads) csc_scatter_kernel(CscParams p) {
     int run = 0;
 #pragma unroll
     for (int w = 0; w < kTileWords; ++w) {
-      before[c * kTileWords + w] = (uint16_t)run;
+      before[w * ncols + c] = (uint16_t)run;             // (neighbouring lanes, neighbouring places: no bank conflicts)
       run += __popc(bm[c * kBmStride + w]);
     }
   }
@@ -273,7 +278,7 @@ __global__ void __launch_bounds__(kCscThreads) csc_scatter_kernel(CscParams p) {
 
   // ---- places: first place of the column's entries in this tile, plus its rows ahead of this one
   auto place = [&](int c, int r) {
-    return base[c] + before[c * kTileWords + (r >> 5)] + (uint32_t)__popc(bm[c * kBmStride + (r >> 5)] & ((1u << (r & 31)) - 1u));
+    return base[c] + before[(r >> 5) * ncols + c] + (uint32_t)__popc(bm[c * kBmStride + (r >> 5)] & ((1u << (r & 31)) - 1u));
   };
   if constexpr (KMAX > 0) {
     if (tid >= rows) return;
