@@ -17,10 +17,12 @@
 namespace fmb {
 
 // Partial rows are stored with their 16-byte chunks permuted: chunk c of the pair at position
-// `pos` sits at chunk (c ^ (pos & 7)).  The tensor-core kernels stage a tile of partial rows
+// `pos` sits at chunk (c ^ (pos & 7)).  The backward kernel stages a tile of partial rows
 // in shared memory before one bulk copy per warp; with this permutation the 32 lanes of a
 // warp (consecutive positions) write their rows without bank conflicts, and the linear copy
-// preserves it.  Writers and the merge kernel use part_col() for the element index.
+// preserves it.  The kernels that write a row per lane straight from registers, 32 bytes a store, need it too: without
+// it all lanes would write the same quarter of their 128-byte lines at a time (64K tokens x 32 heads, forward 1.60 / 1.93 ms
+// with / without).  Writers and the merge kernel use part_col() for the element index.
 __host__ __device__ __forceinline__ int part_col(int64_t pos, int col, int elems_per_chunk) {
   const int chunk = col / elems_per_chunk;
   return ((chunk ^ (int)(pos & 7)) * elems_per_chunk) + (col % elems_per_chunk);

@@ -28,7 +28,7 @@ static size_t layout(AttnWorkspace& w, void* base, const AttnArgs& a, size_t par
   const int64_t rows = a.total_q * nh;
   const int64_t ncols = (int64_t)a.batch * nh * a.ncol;
   w.status = static_cast<int*>(take(kStatusBytes));
-  // the partials are stored 32 bytes at a time (head dim 256): a caller's workspace may start on any 16-byte boundary
+  // the partials are stored 32 bytes at a time: a caller's workspace may start on any 16-byte boundary
   off += base ? (32 - (reinterpret_cast<uintptr_t>(base) + off) % 32) % 32 : 32;
   w.part_o = take((size_t)w.nsub * w.cap * a.d * part_elem_bytes);
   w.part_lse = static_cast<float*>(take(with_lse ? (size_t)w.nsub * w.cap * sizeof(float) : 0));
