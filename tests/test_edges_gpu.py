@@ -60,6 +60,7 @@ def test_dot_of_gradient_and_output(T, H, d):
     ([37, 1], [8000, 5000], 16, 16, 4),            # hundreds of items of one short tile
     ([130, 70], [4100, 3000], 32, 8, 5),           # several heads to an item
     ([129, 64, 300], [129, 64, 300], 8, 8, 3),     # rows at the mask's edges, tiles of one row
+    ([700, 300], [30000, 11000], 16, 16, 8),       # up to 69 items of one tile per CTA, one after the other
 ])
 def test_forward_of_short_items(lens_q, lens_k, H, Hk, topk, chunk, d):
     """Tolerance: inputs of 8 significant bits, probabilities and every chunk's part of a row rounded to them, at most 2^-8 each, of

@@ -1,0 +1,69 @@
+"""The forward kernel's ring of item descriptions against the roles that read it: the waits of the kernel as rules over
+counts, one reader held up as long as they allow while everyone else goes on, and how far the scout publishes
+meanwhile.  (A ring that is too short shows on a GPU only if a warp is late by several GEMMs.)"""
+import os
+import random
+import re
+
+import pytest
+
+from conftest import ROOT
+
+SOURCE = open(os.path.join(ROOT, "flash_moba_b200", "csrc", "fmb_attn_tc.cu")).read()
+
+
+def _constant(name):
+    return int(re.search(r"constexpr int %s = (\d+);" % name, SOURCE).group(1))
+
+
+def _published_while(role, held, tiles_of, NK, NB, G):
+    """Last item published while `role` never gets past tile (V: item) `held`."""
+    item = [i for i, n in enumerate(tiles_of) for _ in range(n)]
+    last = [i + 1 == len(item) or item[i + 1] != item[i] for i in range(len(item))]
+    end = {i: t for t, i in enumerate(item)}              # an item's last tile
+    T, N = len(item), len(tiles_of)
+    pub, kst, vst = [False] * N, [False] * N, [False] * N
+    full, S, ready, PV, tfree, done = ([False] * T for _ in range(6))
+    pub[0] = True
+    moved = True
+    while moved:
+        moved = False
+
+        def step(a, i, cond):
+            nonlocal moved
+            if not a[i] and cond:
+                a[i] = moved = True
+
+        for n in range(N):
+            step(kst, n, pub[n] and (n < NK or S[end[n - NK]]))
+            if n + 1 < N:
+                step(pub, n + 1, kst[n])
+            step(vst, n, pub[n] and (n == 0 or (vst[n - 1] and PV[end[n - 1]])) and not (role == "v" and n > held))
+        for t in range(T):
+            prev = t < G
+            step(full, t, pub[item[t]] and (prev or full[t - G]) and (t < NB or (full[t - NB] and PV[t - NB]))
+                 and not (role == "loader" and t > held and (t - held) % G == 0))
+            step(S, t, kst[item[t]] and full[t] and (t == 0 or S[t - 1]) and (prev or tfree[t - G]))
+            step(ready, t, S[t] and (prev or done[t - G]))
+            step(PV, t, ready[t] and vst[item[t]] and (t == 0 or PV[t - 1]))
+            step(tfree, t, PV[t])
+            step(done, t, tfree[t] and not (role == "group" and t == held))
+    assert last[-1]
+    # the held reader has the items behind its own still to look up
+    first_needed = (held if role == "v" else item[held]) + 1
+    return max(i for i in range(N) if pub[i]) - first_needed + 1
+
+
+@pytest.mark.parametrize("NK", [1, 2])
+@pytest.mark.parametrize("NB", [5, 6, 8])
+def test_no_item_is_overwritten_before_its_readers_are_through(NK, NB):
+    G, ring = _constant("kFwdGroups"), _constant("kFwdRing")
+    rng = random.Random(NK * 10 + NB)
+    streams = [[1] * 40] + [[rng.choice((1, 1, 1, 2, 5)) for _ in range(40)] for _ in range(10)]
+    need = {role: max(_published_while(role, held, s, NK, NB, G) for s in streams for held in (8, 9, 10, 11))
+            for role in ("group", "loader", "v")}
+    assert max(need.values()) <= ring, need
+
+
+def test_kernel_asserts_the_same_bound():
+    assert "static_assert(kFwdRing >= NK + 8" in SOURCE
