@@ -426,8 +426,8 @@ __global__ void __launch_bounds__(kMergeThreads, 3) merge_kernel(const T* __rest
 // (6.3 TB/s), four 204 us; d 256, 16K tokens x 16 heads 53 / 35 us.
 constexpr int kDotRows = 2;
 template <typename T, int LPR>
-__global__ void __launch_bounds__(256) dot_do_o_kernel(const T* __restrict__ dout, int64_t do_rs, int64_t do_hs,
-                                                       const T* __restrict__ o, int64_t o_rs, int64_t o_hs,
+__global__ void __launch_bounds__(256) dot_do_o_kernel(const T* dout, int64_t do_rs, int64_t do_hs,
+                                                       const T* o, int64_t o_rs, int64_t o_hs,
                                                        float* softmax_d, int64_t total_q, int heads, int* status) {
   constexpr int RPW = 32 / LPR;                  // rows of a warp at a time
   follow_on();
@@ -444,8 +444,8 @@ __global__ void __launch_bounds__(256) dot_do_o_kernel(const T* __restrict__ dou
     a[i] = b[i] = make_uint4(0, 0, 0, 0);
     dst[i] = nullptr;
     if (t < total_q) {
-      a[i] = ldg_nc_16(dout + t * do_rs + (int64_t)h * do_hs + c);
-      b[i] = ldg_nc_16(o + t * o_rs + (int64_t)h * o_hs + c);
+      a[i] = ldg_16(dout + t * do_rs + (int64_t)h * do_hs + c);
+      b[i] = ldg_16(o + t * o_rs + (int64_t)h * o_hs + c);
       dst[i] = softmax_d + (int64_t)h * total_q + t;
     }
     for (h += RPW; h >= heads; h -= heads) ++t;

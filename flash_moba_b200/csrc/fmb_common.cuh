@@ -88,9 +88,19 @@ __device__ __forceinline__ uint4 pack8(const float* f) {
   return u;
 }
 
+// Data that nobody writes while the kernel exists: ordinary launches only (see follow_on())
 __device__ __forceinline__ uint4 ldg_nc_16(const void* p) {
   uint4 r;
   asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];"
+               : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w)
+               : "l"(p));
+  return r;
+}
+
+// The same load without that promise, for kernels that are brought up while the one before still writes.  (Measured, .nc / this one: no difference)
+__device__ __forceinline__ uint4 ldg_16(const void* p) {
+  uint4 r;
+  asm volatile("ld.global.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];"
                : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w)
                : "l"(p));
   return r;
@@ -100,7 +110,8 @@ __device__ __forceinline__ uint4 ldg_nc_16(const void* p) {
 // Most kernels of a step are launched with programmatic stream serialization: a kernel's CTAs may be brought up while the
 // kernel before is still running, so that the launch is not waited for.  Every such kernel begins with follow_on(): it waits
 // until the kernel before has completed, its writes included, before it touches memory, and lets the one behind it be
-// brought up in turn (which happens when all of its own CTAs have been).  Ordinary launches: the pool kernel, which opens a
+// brought up in turn (which happens when all of its own CTAs have been).  As it exists while that kernel still writes, it uses no
+// non-coherent loads (.nc, const __restrict__), which are for data that is constant as long as the kernel exists.  Ordinary launches: the pool kernel, which opens a
 // call (its CTAs waiting beside the call before: the pattern of 32K tokens x 16 heads 170 -> 177 us), and the merges (see there).
 // Measured (B200, ordinary launches throughout / these): 9K tokens x 12 heads, d 64, a training step 334 / 318 us; the
 // pattern of 32K tokens x 16 heads 178 / 170 us; 3.6K new rows behind 66K cached keys 285 / 270 us; 16K tokens x 16 heads, d 256

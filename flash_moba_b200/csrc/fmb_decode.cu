@@ -99,7 +99,7 @@ __device__ __forceinline__ void dec_load_k(uint4 (&u)[DecGeo<D>::KB][2][DecGeo<D
       const char* row = base + (int64_t)r * row_bytes + t * 16;
 #pragma unroll
       for (int i = 0; i < DecGeo<D>::KC; ++i)
-        u[kb][half][i] = (r < rows && t + 4 * i < nch) ? ldg_nc_16(row + i * 64) : make_uint4(0, 0, 0, 0);
+        u[kb][half][i] = (r < rows && t + 4 * i < nch) ? ldg_16(row + i * 64) : make_uint4(0, 0, 0, 0);
     }
   }
 }
@@ -159,7 +159,7 @@ __global__ void __launch_bounds__(kDecThreads, DecGeo<D>::CTAS) decode_kernel(De
   auto load_q = [&](uint4 (&q)[KC], int h, bool ok) {
     const T* row = static_cast<const T*>(p.q) + (int64_t)t * p.q_rs + (int64_t)(h0 + h) * p.q_hs + tq * 8;
 #pragma unroll
-    for (int i = 0; i < KC; ++i) q[i] = (ok && tq + 4 * i < nch) ? ldg_nc_16(row + i * 32) : make_uint4(0, 0, 0, 0);
+    for (int i = 0; i < KC; ++i) q[i] = (ok && tq + 4 * i < nch) ? ldg_16(row + i * 32) : make_uint4(0, 0, 0, 0);
   };
   const int my_warp = rank * kDecWarps + warp, n_warps = S * kDecWarps;
 
@@ -258,7 +258,7 @@ __global__ void __launch_bounds__(kDecThreads, DecGeo<D>::CTAS) decode_kernel(De
           const int r = kb * 16 + 2 * tq + (x & 1) + (x >> 1) * 8;
 #pragma unroll
           for (int i = 0; i < VC; ++i)
-            uv[kb][x][i] = (r < rows && gr + 8 * i < nch) ? ldg_nc_16(vb + (int64_t)r * v_row + i * 128) : make_uint4(0, 0, 0, 0);
+            uv[kb][x][i] = (r < rows && gr + 8 * i < nch) ? ldg_16(vb + (int64_t)r * v_row + i * 128) : make_uint4(0, 0, 0, 0);
         }
     }
     float s[KB][2], mx = -CUDART_INF_F;

@@ -61,12 +61,12 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int* s
 }
 
 // ---- a load that is issued where it is written
-// A plain load of read-only data may be moved by the compiler down to its first use (it does so
+// A plain load may be moved by the compiler down to its first use (it does so
 // under register pressure), which turns a prefetch into a full-latency stall.  This is a volatile
 // asm statement: it keeps its place among the other volatile statements (barrier waits).
 __device__ __forceinline__ int ldg_s32_here(const int* ptr) {
   int v;
-  asm volatile("ld.global.nc.s32 %0, [%1];" : "=r"(v) : "l"(ptr));
+  asm volatile("ld.global.s32 %0, [%1];" : "=r"(v) : "l"(ptr));
   return v;
 }
 
