@@ -67,3 +67,18 @@ def test_no_item_is_overwritten_before_its_readers_are_through(NK, NB):
 
 def test_kernel_asserts_the_same_bound():
     assert "static_assert(kFwdRing >= NK + 8" in SOURCE
+
+
+def test_a_wait_that_runs_out_does_so_for_the_whole_warp():
+    """Behind a wait stand shuffles and __syncwarp(): lanes that gave up must not leave the others there."""
+    code = re.sub(r"//[^\n]*", "", SOURCE)
+    kernel = code[code.index("fwd_main_tc_kernel(TcParams p"):code.index("struct BwdItem")]
+    waits = [s for s in re.split(r"[;{}]", kernel) if "mbar_wait(" in s]
+    assert len(waits) >= 6
+    for s in waits:
+        assert "__all_sync(0xffffffffu, mbar_wait(" in " ".join(s.split()) or "bar_info" in s, s
+    # descriptions: the answer is voted on where it is asked for
+    asked = [m.end() for m in re.finditer(r"const int total = item_total\(n\);", kernel)]
+    assert len(asked) == 3 and kernel.count("item_total(n)") == 3
+    for at in asked:
+        assert "__all_sync(0xffffffffu, total >= 0);" in kernel[at:at + 80]
