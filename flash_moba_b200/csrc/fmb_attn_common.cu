@@ -510,8 +510,8 @@ static int dot_do_o_dispatch(const AttnArgs& a, int* status, cudaStream_t s) {
   const T* dout = (const T*)a.dout;
   const T* o = (const T*)a.o;
 #define FMB_DOT(LPR_)                                                                                                \
-  FMB_CUDA(launch_follow_on(dot_do_o_kernel<T, LPR_>, dim3((unsigned)ceil_div64(rows, 8 * (32 / LPR_) * kDotRows)), dim3(256), 0, s, \
-                            dout, a.do_rs, a.do_hs, o, a.o_rs, a.o_hs, a.softmax_d, a.total_q, a.heads, status))
+  launch_follow_on(dot_do_o_kernel<T, LPR_>, dim3((unsigned)ceil_div64(rows, 8 * (32 / LPR_) * kDotRows)), dim3(256), 0, s, \
+                   dout, a.do_rs, a.do_hs, o, a.o_rs, a.o_hs, a.softmax_d, a.total_q, a.heads, status)
   if (a.d == 128) FMB_DOT(16);
   else if (a.d == 64) FMB_DOT(8);
   else if (a.d == 256) FMB_DOT(32);
@@ -587,7 +587,8 @@ int launch_attn_fwd(const AttnArgs& a, int engine, cudaStream_t s) {
   int rc = check_pass_sizes("attn_fwd", a, w, w.bytes);
   if (rc) return rc;
   const bool rows_given = take_rows(a, w);
-  FMB_CUDA(launch_follow_on(clear_status_kernel, dim3(1), dim3(kStatusBytes / 4), 0, s, w.status));   // in place of a memset, which would wait its turn and make the kernel behind wait; counted as little as one
+  launch_follow_on(clear_status_kernel, dim3(1), dim3(kStatusBytes / 4), 0, s, w.status);
+  FMB_CUDA(cudaGetLastError());   // in place of a memset, which would wait its turn and make the kernel behind wait; counted as little as one
   for (int h0 = 0; h0 < a.heads; h0 += w.nh) {
     const PassParams ps = make_pass(a, w, h0, min(w.nh, a.heads - h0));
     if (!rows_given && (rc = build_row_lists(a, w, ps, s))) return rc;

@@ -692,7 +692,7 @@ int fwd_wide_launch(const AttnArgs& a, const AttnWorkspace& w, const PassParams&
   const size_t smem = (size_t)2 * C * D * 2 + (size_t)kM * D * 2 + (size_t)kM * C * 2;   // K, V, Q, P
   auto kern = fwd_wide_tc_kernel<T, C, D>;
   FMB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  FMB_CUDA(launch_follow_on(kern, dim3(p.items_x * p.items_y * p.items_z), dim3(kFwThreads), smem, s, p));
+  launch_follow_on(kern, dim3(p.items_x * p.items_y * p.items_z), dim3(kFwThreads), smem, s, p);
   FMB_LAUNCH_CHECK("fwd_wide_tc_kernel");
   return FMB_OK;
 }
@@ -711,7 +711,7 @@ int bwd_wide_launch(const AttnArgs& a, const AttnWorkspace& w, const PassParams&
   if (regs != kBwRegsLaunch)
     return fail(FMB_ERR_CUDA, "wide-head backward: built with %d registers per thread (%d expected)", regs, kBwRegsLaunch);
   FMB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  FMB_CUDA(launch_follow_on(kern, dim3(p.items_x * p.items_y * p.items_z), dim3(kBwThreads), smem, s, p));
+  launch_follow_on(kern, dim3(p.items_x * p.items_y * p.items_z), dim3(kBwThreads), smem, s, p);
   FMB_LAUNCH_CHECK("bwd_wide_tc_kernel");
   return FMB_OK;
 }

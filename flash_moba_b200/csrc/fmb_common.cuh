@@ -32,8 +32,10 @@ void prof_end(int kind, cudaStream_t s);
 #define FMB_CUDA(call)                                                                  \
   do {                                                                                  \
     cudaError_t e_ = (call);                                                            \
-    if (e_ != cudaSuccess)                                                              \
+    if (e_ != cudaSuccess) {                                                            \
+      (void)cudaGetLastError();   /* reported here, and not by the next call's check */ \
       return ::fmb::fail(FMB_ERR_CUDA, "%s failed: %s", #call, cudaGetErrorString(e_)); \
+    }                                                                                   \
   } while (0)
 
 #define FMB_LAUNCH_CHECK(name)                                                           \
@@ -120,8 +122,9 @@ __device__ __forceinline__ void follow_on() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
+// (a launch that fails leaves its error to the FMB_LAUNCH_CHECK behind it, as <<<>>> does)
 template <typename... P, typename... A>
-cudaError_t launch_follow_on(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A&&... args) {
+void launch_follow_on(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A&&... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = block;
@@ -132,7 +135,7 @@ cudaError_t launch_follow_on(void (*kern)(P...), dim3 grid, dim3 block, size_t s
   at[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
   cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
+  (void)cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
 }
 
 __host__ __device__ __forceinline__ int ceil_div(int a, int b) { return (a + b - 1) / b; }

@@ -359,11 +359,11 @@ int launch_build_csc(const int32_t* topk_idx, int64_t idx_rs, int64_t idx_hs, co
   prof_begin(6, s);
   p.cols_per_cta = min(kMaxHistCols, ncol);
   auto count = topk <= 8 ? csc_tile_hist_kernel<8> : topk <= 16 ? csc_tile_hist_kernel<16> : csc_tile_hist_kernel<0>;
-  FMB_CUDA(launch_follow_on(count, dim3(batch * heads, p.ntiles, ceil_div(ncol, p.cols_per_cta)), dim3(kCscThreads),
-                            (size_t)p.cols_per_cta * sizeof(uint32_t), s, p));
+  launch_follow_on(count, dim3(batch * heads, p.ntiles, ceil_div(ncol, p.cols_per_cta)), dim3(kCscThreads),
+                   (size_t)p.cols_per_cta * sizeof(uint32_t), s, p);
   FMB_LAUNCH_CHECK("csc_tile_hist_kernel");
   if (p.scanned) {
-    FMB_CUDA(launch_follow_on(csc_tile_scan_kernel, dim3(batch * heads, ceil_div(ncol, 32)), dim3(1024), 0, s, p));
+    launch_follow_on(csc_tile_scan_kernel, dim3(batch * heads, ceil_div(ncol, 32)), dim3(1024), 0, s, p);
     FMB_LAUNCH_CHECK("csc_tile_scan_kernel");
   }
   p.cols_per_cta = min(kMaxColsPerCta, ncol);
@@ -372,7 +372,7 @@ int launch_build_csc(const int32_t* topk_idx, int64_t idx_rs, int64_t idx_hs, co
   auto scatter = topk <= 8 ? csc_scatter_kernel<8> : topk <= 16 ? csc_scatter_kernel<16> : csc_scatter_kernel<0>;
   // the attribute belongs to the current device: set on every call (cheap, idempotent, thread-safe)
   FMB_CUDA(cudaFuncSetAttribute(scatter, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxColsPerCta * kColBytes));
-  FMB_CUDA(launch_follow_on(scatter, grid, dim3(kCscThreads), smem, s, p));
+  launch_follow_on(scatter, grid, dim3(kCscThreads), smem, s, p);
   prof_end(6, s);
   FMB_LAUNCH_CHECK("csc_scatter_kernel");
   return FMB_OK;

@@ -436,7 +436,7 @@ static int decode_launch(const DecodeParams& p, const DecodeShape& sh, int64_t t
   at[0].val.clusterDim.z = 1;
   cfg.attrs = at;
   cfg.numAttrs = sh.S <= 2 ? 2 : 1;
-  FMB_CUDA(cudaLaunchKernelEx(&cfg, kern, p));
+  (void)cudaLaunchKernelEx(&cfg, kern, p);
   FMB_LAUNCH_CHECK("decode_kernel");
   return FMB_OK;
 }

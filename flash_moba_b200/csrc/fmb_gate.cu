@@ -1063,8 +1063,8 @@ static int gate_select_launch(const GateParams& p, const CUtensorMap& mq, const 
   const int row_tiles = ceil_div(max_q, kGateM);
   const int64_t items = (int64_t)row_tiles * p.heads * batch;
   const int64_t ctas = (int64_t)sm_count() * (D <= 128 ? 2 : 1);
-  FMB_CUDA(launch_follow_on(kern, dim3((unsigned)(items < ctas ? items : ctas)), dim3(kSelThreads), smem, s, p, mq, mk, batch, row_tiles,
-                            divider(p.chunk), divider(p.heads * batch), divider(p.heads)));
+  launch_follow_on(kern, dim3((unsigned)(items < ctas ? items : ctas)), dim3(kSelThreads), smem, s, p, mq, mk, batch, row_tiles,
+                   divider(p.chunk), divider(p.heads * batch), divider(p.heads));
   FMB_LAUNCH_CHECK("gate_select_kernel");
   return FMB_OK;
 }

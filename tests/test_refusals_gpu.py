@@ -95,3 +95,22 @@ def test_rows_whose_distance_fits_no_unit():
     finally:
         q = buf = None
         torch.cuda.empty_cache()
+
+
+def test_a_launch_that_fails_leaves_no_error_behind():
+    """The runtime keeps a thread's last error until it is asked for: a refused call must not make the next one, of this library or
+    of torch, report it.  (More column groups than a grid may have: the runtime refuses the launch, nothing runs.)"""
+    import ctypes
+
+    from flash_moba_b200 import _lib, ops
+    cudart = ctypes.CDLL("libcudart.so.12")
+    some = torch.zeros(4096, dtype=torch.int64, device=DEV)
+    ncol = 8192 * 65536                                  # 65536 groups of the histogram's 8192 columns
+    rc = _lib.lib.fmb_build_csc(*[some.data_ptr(), 1, 1] + [some.data_ptr()] * 5, 4 * ncol + 256, 1, 1, 1, 16, ncol,
+                                torch.cuda.current_stream().cuda_stream)
+    assert rc != 0
+    assert cudart.cudaPeekAtLastError() == 0
+    assert b"csc_tile_hist_kernel" in _lib.lib.fmb_last_error()
+    k = torch.ones(100, 2, 64, device=DEV, dtype=torch.bfloat16)
+    km, _ = ops.mean_pool(k, torch.tensor([0, 100], dtype=torch.int32, device=DEV), 100, 64)
+    assert (km[:2] == 1).all()
