@@ -3,8 +3,8 @@
 // Replaces the reference's Triton kernel (flash_moba/triton_mean_pool.py:41-109) and its
 // host prologue (:134-142).  HBM bound: reads K once (T*Hk*d*2 bytes), writes one row per
 // chunk.  One warp owns one (chunk, kv head): lanes cover the head dimension with 16-byte
-// loads, several rows per iteration, sixteen independent loads in flight per lane, fp32
-// accumulation, one shuffle reduction at the end.
+// loads, several rows at a time, a turn's loads independent of one another, fp32 accumulation,
+// one shuffle reduction at the end.
 #include "fmb_common.cuh"
 
 namespace fmb {
@@ -37,9 +37,22 @@ int launch_chunk_offsets(const int32_t* cu_k, int batch, int chunk, int32_t* cu_
 }
 
 constexpr int kPoolWarps = 4;
-// Loads in flight per lane.  Measured (B200, 4 / 16): 32K tokens x 16 heads, d 128 27 / 24 us (134 MB), 64K x 32 92 / 90 us, 512K x
-// 4 heads, chunk 256 102 / 93 us, 317K x 8 heads, chunk 64 115 / 107 us, 3K x 8 heads, d 64 6.0 / 5.1 us
-constexpr int kPoolDepth = 16;
+// A turn: N rows of a lane are requested, then added in their order (so that the sum does not depend on N); ALL false: rows at or
+// past `rows` count as zeros, which changes no bit of a sum that starts at +0.
+template <typename T, int RPI, int N, bool ALL>
+__device__ __forceinline__ void pool_turn(float (&acc)[8], const T* base, int64_t row_stride, int r, int rows) {
+  uint4 u[N];
+#pragma unroll
+  for (int x = 0; x < N; ++x)
+    u[x] = ALL || r + x * RPI < rows ? ldg_nc_16(base + (int64_t)(r + x * RPI) * row_stride) : make_uint4(0, 0, 0, 0);
+#pragma unroll
+  for (int x = 0; x < N; ++x) {
+    float f[8];
+    unpack8<T>(u[x], f);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) acc[i] += f[i];
+  }
+}
 
 // batches up to this many sequences have their chunk offsets computed inside the pool kernel
 // (every warp sums the chunk counts of the sequences before its own: two rounds of loads at most)
@@ -48,7 +61,7 @@ constexpr int kPoolInlineOffsets = 64;
 // LPR = lanes per row (power of two >= d/8), RPI = rows per warp iteration = 32 / LPR.
 // OFFS: cu_km is an OUTPUT: the warp derives its sequence's first centroid row from cu_k itself and
 // the first warp of every sequence publishes it (no separate offsets launch).
-template <typename T, int LPR, bool OFFS, int DEPTH>
+template <typename T, int LPR, bool OFFS>
 __global__ void __launch_bounds__(kPoolWarps * 32)
 mean_pool_kernel(const T* __restrict__ k, int64_t row_stride, int64_t head_stride,
                  const int32_t* __restrict__ cu_k, int32_t* cu_km,
@@ -91,21 +104,25 @@ mean_pool_kernel(const T* __restrict__ k, int64_t row_stride, int64_t head_strid
   const T* base = k + (int64_t)(seq0 + row0) * row_stride + (int64_t)hk * head_stride + col * 8;
   if (col_ok) {
     int r = sub;
-    auto add = [&](const uint4& u) {
-      float f[8];
-      unpack8<T>(u, f);
-#pragma unroll
-      for (int i = 0; i < 8; ++i) acc[i] += f[i];
-    };
-    // DEPTH independent 16-byte loads in flight per lane; the order of the sum does not depend on it
-    for (; r + (DEPTH - 1) * RPI < rows; r += DEPTH * RPI) {
-      uint4 u[DEPTH];
-#pragma unroll
-      for (int x = 0; x < DEPTH; ++x) u[x] = ldg_nc_16(base + (int64_t)(r + x * RPI) * row_stride);
-#pragma unroll
-      for (int x = 0; x < DEPTH; ++x) add(u[x]);
+    // Sixteen rows a turn (of which the compiler keeps as many in flight as its 44 - 62 registers hold), the rest of a long
+    // chunk by eights; chunks of fewer rows per lane, the short last ones among them, step down.  Measured (B200; turns of 4 and
+    // single rows / of 16 and single rows / these): 32K tokens x 16 heads, d 128, chunk 128 25.4 / 22.1 / 21.2 us (134 MB), 64K
+    // x 32 82.7 / 78.5 / 77.9, 512K x 4, chunk 256 90.9 / 83.3 / 82.0; 16 ragged sequences, d 64, chunk 64 15.0 / 12.9 / 12.4,
+    // chunk 16 18.4 / 18.6 / 16.1, d 256 16.5 / 20.5 / 16.7; sequences that end in 57 to 63 rows 8.4 / 10.0 / 5.4
+    if (rows >= 16 * RPI) {
+      for (; r + 15 * RPI < rows; r += 16 * RPI) pool_turn<T, RPI, 16, true>(acc, base, row_stride, r, rows);
+      for (; r < rows; r += 8 * RPI) pool_turn<T, RPI, 8, false>(acc, base, row_stride, r, rows);
+    } else {
+      if (r + 7 * RPI < rows) {
+        pool_turn<T, RPI, 8, true>(acc, base, row_stride, r, rows);
+        r += 8 * RPI;
+      }
+      if (r + 3 * RPI < rows) {
+        pool_turn<T, RPI, 4, true>(acc, base, row_stride, r, rows);
+        r += 4 * RPI;
+      }
+      if (r < rows) pool_turn<T, RPI, 4, false>(acc, base, row_stride, r, rows);
     }
-    for (; r < rows; r += RPI) add(ldg_nc_16(base + (int64_t)r * row_stride));
   }
   // reduce the RPI partial rows (lanes with equal `col`)
 #pragma unroll
@@ -134,7 +151,7 @@ static int pool_dispatch(const void* k, int64_t rs, int64_t hs, const int32_t* c
   T* kmp = static_cast<T*>(km);
 #define FMB_POOL(L)                                                                                              \
   do {                                                                                                           \
-    auto kern = offsets ? mean_pool_kernel<T, L, true, kPoolDepth> : mean_pool_kernel<T, L, false, kPoolDepth>;    \
+    auto kern = offsets ? mean_pool_kernel<T, L, true> : mean_pool_kernel<T, L, false>;                            \
     kern<<<grid, block, 0, s>>>(kp, rs, hs, cu_k, cu_km, kmp, heads_k, d, chunk);                                  \
   } while (0)
   if (lanes <= 1) FMB_POOL(1);

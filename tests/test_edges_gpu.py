@@ -36,6 +36,31 @@ def test_pool_row_counts(d, chunk):
     assert int(cu_km[-1]) == row
 
 
+@pytest.mark.parametrize("d", [8, 32, 64, 96, 256])
+@pytest.mark.parametrize("chunk", [16, 64, 80, 320])
+def test_pool_sums_in_row_order(d, chunk):
+    """However many rows are requested at a time: a lane adds its rows (every 32 / lanes-per-row th) in their order in fp32, then the
+    lanes' sums meet pairwise.  The same bits."""
+    from flash_moba_b200 import ops
+    lens = [1, 3, 15, 16, 17, 57, 61, 63, 64, 79, 81, 130, 255, 319, 321]
+    k = torch.randn(sum(lens), 2, d, generator=torch.Generator().manual_seed(d)).bfloat16()
+    km, _ = ops.mean_pool(k.to(DEV), cu_of(lens).to(DEV), max(lens), chunk)
+    rpi = 32 // (1 << (d // 8 - 1).bit_length())
+    at, row = 0, 0
+    for n in lens:
+        for c in range(0, n, chunk):
+            x = k[at + c:at + min(n, c + chunk)].float()
+            parts = [torch.zeros_like(x[0]) for _ in range(rpi)]
+            for i in range(len(x)):
+                parts[i % rpi] = parts[i % rpi] + x[i]
+            while len(parts) > 1:
+                parts = [a + b for a, b in zip(parts[::2], parts[1::2])]
+            want = (parts[0] * (torch.ones(()) / len(x))).bfloat16()
+            assert torch.equal(km[row].cpu(), want), (n, c)
+            row += 1
+        at += n
+
+
 @pytest.mark.parametrize("H", [1, 2, 3, 7, 12])
 @pytest.mark.parametrize("T,d", [(1, 64), (129, 64), (65, 128), (33, 256)])
 def test_dot_of_gradient_and_output(T, H, d):
