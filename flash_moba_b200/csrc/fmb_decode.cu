@@ -425,9 +425,11 @@ static int decode_launch(const DecodeParams& p, const DecodeShape& sh, int64_t t
   cfg.dynamicSmemBytes = sh.smem;
   cfg.stream = s;
   cudaLaunchAttribute at[2];
-  // Brought up beside the kernel before it (see follow_on()) where clusters are small; clusters of eight CTAs, placed around
-  // those that still run, pile up on fewer SMs.  Measured back to back, without / with: 16 rows (clusters of two)
-  // 55.0 / 53.2 us, one row (of eight) 18.5 / 25.0 us
+  // Brought up beside the kernel before it (see follow_on()), but for clusters of eight CTAs: placed around those of a call
+  // that still runs they pile up on fewer SMs.  Measured, without / with, back to back; between elementwise kernels of torch
+  // (32 / 8 heads): d 128, 32 rows (no clusters) 94.2 / 92.1; 94.3 / 91.1 us, 16 rows (of two) 56.0 / 54.4; 56.0 / 54.2, 8 rows (of
+  // four) 34.8 / 32.8; 35.8 / 32.8, 4 rows (of four) 22.6 / 21.3; 23.6 / 22.0, one row (of eight) 18.5 / 25.7; 18.6 / 15.4;
+  // d 64, 8 rows 22.5 / 20.2; 23.2 / 20.2, d 256, 4 rows 37.0 / 35.5; 37.7 / 35.9
   at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at[1].val.programmaticStreamSerializationAllowed = 1;
   at[0].id = cudaLaunchAttributeClusterDimension;
@@ -435,7 +437,7 @@ static int decode_launch(const DecodeParams& p, const DecodeShape& sh, int64_t t
   at[0].val.clusterDim.y = 1;
   at[0].val.clusterDim.z = 1;
   cfg.attrs = at;
-  cfg.numAttrs = sh.S <= 2 ? 2 : 1;
+  cfg.numAttrs = sh.S <= 4 ? 2 : 1;
   (void)cudaLaunchKernelEx(&cfg, kern, p);
   FMB_LAUNCH_CHECK("decode_kernel");
   return FMB_OK;
