@@ -587,8 +587,10 @@ int launch_attn_fwd(const AttnArgs& a, int engine, cudaStream_t s) {
   int rc = check_pass_sizes("attn_fwd", a, w, w.bytes);
   if (rc) return rc;
   const bool rows_given = take_rows(a, w);
+  // A kernel in place of a memset, which would wait its turn and make the kernel behind wait (a training step of 3K tokens x
+  // 8 heads, d 64 107.2 / 103.2 us, 3.6K new rows behind 66K cached keys 280 / 266 us with the memset / with it).  The backward's dO.O does it on the way.
   launch_follow_on(clear_status_kernel, dim3(1), dim3(kStatusBytes / 4), 0, s, w.status);
-  FMB_CUDA(cudaGetLastError());   // in place of a memset, which would wait its turn and make the kernel behind wait; counted as little as one
+  FMB_LAUNCH_CHECK("clear_status_kernel");
   for (int h0 = 0; h0 < a.heads; h0 += w.nh) {
     const PassParams ps = make_pass(a, w, h0, min(w.nh, a.heads - h0));
     if (!rows_given && (rc = build_row_lists(a, w, ps, s))) return rc;

@@ -2,7 +2,7 @@
 // pattern -> attention hand-over, the autograd node.  Everything below it is the C ABI
 // (include/flash_moba_b200.h); nothing here computes on tensors.
 //
-// Why native: a step is ten kernel launches, and at small sizes (a few thousand tokens, a decode
+// Why native: a step is eleven kernel launches, and at small sizes (a few thousand tokens, a decode
 // step) the kernels need 0.06-0.15 ms while the same host path in Python (ctypes calls of forty
 // arguments, an autograd Function, two recorded events per attention call, a cache keyed by tuples)
 // needed 0.25 ms per forward call and 0.5-0.6 ms per training step.

@@ -568,7 +568,7 @@ def test_lists_of_a_caller_built_pattern_and_launch_counts(monkeypatch):
     got_copy, n_copy = attn(copy)
     for a, b in zip(got_own, got_copy):
         assert torch.equal(a, b)
-    assert n_own == 5, n_own                          # forward main + combine, dO.O, backward main + combine
+    assert n_own == 6, n_own                          # status block, forward main + combine, dO.O, backward main + combine
     assert n_own < n_copy
     monkeypatch.setenv("FMB_SHARE_LISTS", "0")
     got_off, n_off = attn(copy)
