@@ -1,6 +1,6 @@
-"""Kernels at the sizes where their loops and rings can go wrong: rows of a chunk around the pool's sixteen loads in flight,
+"""Kernels at the sizes where their loops and rings can go wrong: rows of a chunk around the pool's turns of sixteen, eight and four,
 rows of the dO.O kernel whose (token, head) is found by counting, forward items of a single tile that follow one another
-through the K and V buffers, tiles whose rows stand at the edge of the causal mask, equal scores in one lane's and in
+through the K and V buffers, backward items of one and of seven tiles, tiles whose rows stand at the edge of the causal mask, equal scores in one lane's and in
 several lanes' candidates of the decode kernel."""
 import os
 import sys
@@ -109,10 +109,29 @@ def test_forward_of_short_items(lens_q, lens_k, H, Hk, topk, chunk, d):
     assert diff.norm() <= 4 * 2.0 ** -9 * want.norm()
 
 
+@pytest.mark.parametrize("chunk", [64, 128])
+@pytest.mark.parametrize("tiles", [1, 7])
+def test_backward_of_items_of_few_tiles(tiles, chunk):
+    """Head dim 64, where the backward kernel has three Q buffers and three (64-key blocks) or two (128) dO buffers: items of one tile
+    leave the ring of buffers turned by one for the next item, items of seven go around it more than twice.  Every row
+    sees every chunk of its sequence.  Error bars: those of the other attention tests."""
+    from test_kernels_gpu import _attn_check
+    g = torch.Generator().manual_seed(chunk)
+    H = 12 if tiles == 1 else 4
+    lens = [1 + i % chunk for i in range(0, 120 * 7, 7)] if tiles == 1 else [7 * 128] * 16
+    ncol = -(-max(lens) // chunk)
+    q, k, v, do = (torch.randn(sum(lens), H, 64, generator=g).bfloat16() for _ in range(4))
+    mask = torch.ones(len(lens), H, max(lens), ncol, dtype=torch.bool)
+    for b, n in enumerate(lens):
+        mask[b, :, n:] = False
+        mask[b, :, :, -(-n // chunk):] = False
+    _attn_check(q, k, v, do, cu_of(lens), cu_of(lens), mask, chunk, False, 1)
+
+
 @pytest.mark.parametrize("n_chunks,topk", [(2, 8), (31, 4), (33, 8), (64, 8), (65, 5), (100, 16), (200, 33)])
 def test_decode_selection_of_equal_scores(n_chunks, topk):
-    """Keys alike inside a chunk and of a few values only: the centroids are exact, most scores tie (zeros of either sign among
-    them), and any other choice of chunks gives another result.  Tolerance as for the decode kernel: half a unit of the
+    """Keys alike inside a chunk and of a few values only: the centroids are exact, most scores tie (at zero among others; all zeros are +0,
+    as the pool and the products start their sums from it), and any other choice of chunks gives another result.  Tolerance as for the decode kernel: half a unit of the
     result's type (2^-8 of it) + fp32 sums."""
     from flash_moba_b200 import ops
     from test_decode_gpu import _decode
@@ -121,7 +140,7 @@ def test_decode_selection_of_equal_scores(n_chunks, topk):
     n = n_chunks * chunk - 5
     q = torch.randint(-1, 2, (2, H, d), generator=g).bfloat16() * 0.5
     few = torch.randint(-1, 2, (3, Hk, d), generator=g).bfloat16()
-    few[0] = -0.0                                     # a third of the chunks scores zero, of whatever sign
+    few[0] = -0.0                                     # a third of the chunks scores zero
     k = few[torch.randint(0, 3, (n_chunks,), generator=g)].repeat_interleave(chunk, 0)[:n].contiguous()
     v = torch.randn(n, Hk, d, generator=g).bfloat16()
     cq, ck = cu_of([2]), cu_of([n])
