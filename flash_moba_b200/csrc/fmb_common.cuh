@@ -114,7 +114,9 @@ __device__ __forceinline__ uint4 ldg_16(const void* p) {
 // until the kernel before has completed, its writes included, before it touches memory, and lets the one behind it be
 // brought up in turn (which happens when all of its own CTAs have been).  As it exists while that kernel still writes, it uses no
 // non-coherent loads (.nc, const __restrict__), which are for data that is constant as long as the kernel exists.  Ordinary launches: the pool kernel, which opens a
-// call (its CTAs waiting beside the call before: the pattern of 32K tokens x 16 heads 170 -> 177 us), and the merges (see there).
+// call (its CTAs waiting beside the call before: the pattern of 32K tokens x 16 heads 170 -> 177 us), the merges and decode
+// calls with clusters of eight (see there), and what is launched with <<<>>> besides: chunk offsets, the older gating kernels, slot
+// and row lists, the CUDA-core engine, the self tests.  The pool and the merges call follow_on() too: the kernel behind them comes early.
 // Measured (B200, ordinary launches throughout / these): 9K tokens x 12 heads, d 64, a training step 334 / 318 us; the
 // pattern of 32K tokens x 16 heads 178 / 170 us; 3.6K new rows behind 66K cached keys 285 / 270 us; 16K tokens x 16 heads, d 256
 // 2.54 / 2.52 ms; long steps the same.

@@ -198,7 +198,7 @@ __global__ void __launch_bounds__(kDecThreads, DecGeo<D>::CTAS) decode_kernel(De
       j = 1;
     }
     // Every lane knows the best of its candidates (n = lane, lane + 32, ...); a round takes the best of the lanes' and only
-    // the lane it came from looks for its next.  Scores as ordered integers (+0 and -0 alike), 0: none.  (With a scan of all
+    // the lane it came from looks for its next.  Scores as ordered integers (+0 and -0 alike, though no sum that starts at +0 is -0), 0: none.  (With a scan of all
     // candidates and ten shuffles in every round: one row of 32 heads and 65,001 keys 17.7 us, 16 rows of 16
     // sequences 54.6; now 16.3 and 52.7)
     uint32_t best;
