@@ -813,6 +813,8 @@ gate_select_kernel(GateParams p, const __grid_constant__ CUtensorMap map_q, cons
         gs += steps;
         ++qn;
       }
+      // nobody waits for the last tiles' bar_kfree: their arrivals land before the CTA's shared memory is given up
+      if (ok && qn > 0) mbar_wait(&bar_qfree, (qn - 1) & 1, &g_gate_status, 2);
     }
   } else {
     // =============================================================== selection

@@ -75,10 +75,20 @@ def test_a_wait_that_runs_out_does_so_for_the_whole_warp():
     kernel = code[code.index("fwd_main_tc_kernel(TcParams p"):code.index("struct BwdItem")]
     waits = [s for s in re.split(r"[;{}]", kernel) if "mbar_wait(" in s]
     assert len(waits) >= 6
-    for s in waits:
-        assert "__all_sync(0xffffffffu, mbar_wait(" in " ".join(s.split()) or "bar_info" in s, s
+    for s in waits:                               # (the issuer is a single thread)
+        assert "__all_sync(0xffffffffu, mbar_wait(" in " ".join(s.split()) or "bar_info" in s or "(np - 1) & 1" in s, s
     # descriptions: the answer is voted on where it is asked for
     asked = [m.end() for m in re.finditer(r"const int total = item_total\(n\);", kernel)]
     assert len(asked) == 3 and kernel.count("item_total(n)") == 3
     for at in asked:
         assert "__all_sync(0xffffffffu, total >= 0);" in kernel[at:at + 80]
+
+
+@pytest.mark.parametrize("name,kernel,last", [("fmb_attn_tc.cu", "fwd_main_tc_kernel(TcParams p", "bar_fin, (np - 1) & 1"),
+                                              ("fmb_gate.cu", "gate_select_kernel(GateParams p", "bar_qfree, (qn - 1) & 1")])
+def test_the_last_commit_lands_before_the_cta_ends(name, kernel, last):
+    """A commit arrives on a barrier in the CTA's shared memory when its MMAs have completed, whether or not anyone waits for it."""
+    code = open(os.path.join(ROOT, "flash_moba_b200", "csrc", name)).read()
+    code = code[code.index(kernel):]
+    code = code[:code.index("tmem_dealloc(")]
+    assert code.rindex("mbar_wait(&" + last) > code.rindex("umma_commit(")
