@@ -605,24 +605,30 @@ __global__ void __launch_bounds__(128 * NQ) gate_topk_tc_kernel(GateParams p) {
 //            Group maxima are different candidates' scores, so the k-th largest of them is a floor no
 //            member of the row's top-k lies under; only some 9 scores of a row (k = 8) reach it;
 //   sweep 2  appends the scores that reach the floor to a short queue in shared memory (predicated
-//            stores, no branch).  A candidate's place in the list is then the number of the row's
-//            candidates ahead of it, counted by comparing all with all; the two threads of a row share
-//            the row's candidates evenly, however they were distributed over the columns.
+//            stores, no branch).  Each of a row's two threads then sorts its own queue: 32-bit keys, the upper 26 bits of the
+//            score and the entry's place in the queues, through a network of min / max pairs; the first thread merges the
+//            two lists and writes the row's.  Neighbours that agree in those 26 bits are compared exactly and exchanged; where
+//            more than two agree, or the last place and what was dropped (masses of equal scores), the pair of warps
+//            takes the long way: a candidate's place is the number of the row's candidates ahead of it, counted by comparing
+//            all with all.
 // The score tiles of sweep 2 are those of sweep 1, still in TMEM, for up to 256 candidates; beyond that the
 // products are computed again (the tensor pipe is idle otherwise).  A queue that runs full (masses of
 // equal scores) is cut down to its k best, the last of which then is the floor.
-// Persistent CTAs, two per SM.  Warp 8 loads Q and the centroid tiles by TMA and issues the MMAs, running
+// Persistent CTAs, two per SM.  Warp 8 loads Q and the centroid tiles by TMA, warp 9 issues the MMAs, both running
 // ahead into the next item (row tile, head, sequence) while warps 0-7 (two threads per row, alternate halves of a
-// tile's columns) are still in sweep 2: with a CTA per item, start-up and Q's way from HBM were a third of its time.
-// Measured (B200, d 128, the kernel above / this one): 64K tokens, 32 heads, chunk 128, top-k 8 1.02 / 0.65 ms;
-// 8 x 8K tokens 0.58 / 0.28 ms; 32K tokens, 16 heads 185 / 104 us; 317K tokens in 16 sequences, chunk 64, top-k 16
-// 7.4 / 3.7 ms; d 256, 16K tokens, 16 heads 141 / 59 us.  Now: 15,500 instructions per row tile and head at 61 % issue
-// (fixed-latency dependencies and the shared min / max pipe), 30 instructions per score.
+// tile's columns) are still in sweep 2: with a CTA per item, start-up and Q's way from HBM were a third of its time.  With one
+// thread for loads and MMAs a centroid tile was requested only when the MMAs before it had been issued, one tile in flight at a
+// time: 1 us a step, which is what long sequences took (64K tokens, 32 heads 605 / 549 us with one / two warps).
+// Measured (B200, d 128; the kernel above / two sweeps, all compared with all / sorted keys): 64K tokens, 32 heads, chunk 128, top-k 8
+// 1020 / 605 / 492 us; 8 x 8K tokens 580 / 256 / 198; 32K tokens, 16 heads 185 / 97 / 83; 317K tokens in 16 sequences, chunk 64, top-k 16
+// 7400 / 3430 / 3290; 512K tokens, 4 heads, chunk 256, top-k 16 - / 2106 / 1982; d 64, 9K tokens, 12 heads, no mask - / 31 / 23.
+// What bounds it now: instructions at 60 % issue (32K tokens: 1,600 a warp and row tile; the min / max pipe is busy for 58 %), at
+// 64K also the MMAs (128 x 64 x 16: 52 cycles, of which A's and B's way from shared memory takes 48).
 // ---------------------------------------------------------------------------------------
 constexpr int kSelN = 64;            // centroids per score tile
 constexpr int kSelBufs = 4;          // score tiles in TMEM
 constexpr int kSelRing = 2;          // centroid tiles in shared memory
-constexpr int kSelThreads = 256 + 32;
+constexpr int kSelThreads = 256 + 64;  // selection, loads, MMAs
 
 // descending sorting networks on registers: 8 values in 19 compare-exchanges; 16 as two sorted eights
 // and a bitonic merge
@@ -631,7 +637,13 @@ __device__ __forceinline__ void sel_ce(float& a, float& b) {
   a = hi;
   b = lo;
 }
-__device__ __forceinline__ void sel_sort8(float* x) {
+__device__ __forceinline__ void sel_ce(uint32_t& a, uint32_t& b) {
+  const uint32_t hi = max(a, b), lo = min(a, b);
+  a = hi;
+  b = lo;
+}
+template <typename V>
+__device__ __forceinline__ void sel_sort8(V* x) {
   sel_ce(x[0], x[1]); sel_ce(x[2], x[3]); sel_ce(x[4], x[5]); sel_ce(x[6], x[7]);
   sel_ce(x[0], x[2]); sel_ce(x[1], x[3]); sel_ce(x[4], x[6]); sel_ce(x[5], x[7]);
   sel_ce(x[1], x[2]); sel_ce(x[5], x[6]); sel_ce(x[0], x[4]); sel_ce(x[3], x[7]);
@@ -641,16 +653,16 @@ __device__ __forceinline__ void sel_sort8(float* x) {
   sel_ce(x[3], x[4]);
 }
 // x bitonic -> descending
-template <int N>
-__device__ __forceinline__ void sel_bitonic(float* x) {
+template <int N, typename V>
+__device__ __forceinline__ void sel_bitonic(V* x) {
 #pragma unroll
   for (int o = N / 2; o; o >>= 1)
 #pragma unroll
     for (int i = 0; i < N; ++i)
       if ((i & o) == 0) sel_ce(x[i], x[i + o]);
 }
-template <int N>
-__device__ __forceinline__ void sel_sort(float* x) {
+template <int N, typename V>
+__device__ __forceinline__ void sel_sort(V* x) {
   if constexpr (N == 8) {
     sel_sort8(x);
   } else {
@@ -693,9 +705,9 @@ __device__ __forceinline__ int fast_div(int n, const FastDiv& f) {
 }
 
 // Queue entries per thread: what two CTAs per SM leave room for.  A row has some 9 (k = 8) or 19 (k = 16)
-// candidates, a thread half of them on average; more than 12 or 18 in one thread's queue are rare (with room
-// for 16 the queues ran full all the time: 0.82 ms instead of 0.65 at 64K).
-template <int KMAX> __host__ __device__ constexpr int sel_cap() { return KMAX == 8 ? 20 : 22; }
+// candidates, a thread half of them on average; more than 12 or 15 in one thread's queue are rare (with room
+// for 16 the queues of k = 8 ran full all the time: 0.82 ms instead of 0.65 at 64K).
+template <int KMAX> __host__ __device__ constexpr int sel_cap() { return KMAX == 8 ? 20 : 19; }
 
 constexpr int kSelSeqs = 64;         // sequences whose bounds are kept in shared memory
 
@@ -708,20 +720,26 @@ gate_select_kernel(GateParams p, const __grid_constant__ CUtensorMap map_q, cons
   constexpr uint32_t kQTile = kGateM * D * 2, kKTile = kSelN * D * 2;
   constexpr int CAP = sel_cap<KMAX>();                   // queue entries per thread
   constexpr int STEP = KMAX == 8 ? 8 : 4;                // scores between two looks at the queue's length
-  constexpr int OWN = KMAX == 8 ? 6 : 12;                // candidates of a row that each of its two threads ranks at a time
-  extern __shared__ unsigned char smem_raw[];
+  constexpr int OWN = KMAX == 8 ? 6 : 12;                // the long way: candidates of a row that each of its two threads ranks at a time
+  extern __shared__ __align__(1024) unsigned char smem_raw[];
   __shared__ uint64_t bar_q, bar_qfree, bar_kfull[kSelRing], bar_kfree[kSelRing], bar_tfull[kSelBufs], bar_tfree[kSelBufs];
   __shared__ uint32_t tmem_base_s;
-  __shared__ int sCount[256];
+  __shared__ uint8_t sCount[256];
   __shared__ int sCu[3][kSelSeqs + 1];
-  unsigned char* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
-  unsigned char* sQ = smem;
+  // (no room for padding: the base is aligned as declared, checked here)
+  if ((smem_u32(smem_raw) & 1023u) != 0) {
+    if (threadIdx.x == 0) atomicCAS(&g_gate_status, 0, 9);
+    return;
+  }
+  unsigned char* sQ = smem_raw;
   unsigned char* sKM = sQ + kQTile;
   unsigned char* sQueue = sKM + kSelRing * kKTile;       // per warp pair [CAP][64] (score, chunk); also the pair's exchange area
+  uint32_t* sKeys = reinterpret_cast<uint32_t*>(sQueue + CAP * 256 * 8);   // per warp pair [KMAX + 1][32] sorted keys of the rows' second threads
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int topk = p.topk;
   const bool small_batch = batch <= kSelSeqs;
+  const bool vec_out = (reinterpret_cast<uintptr_t>(p.topk_idx) & 15) == 0 && (p.t_hs & 3) == 0;
   if (small_batch)
     for (int i = tid; i <= batch; i += kSelThreads) { sCu[0][i] = p.cu_q[i]; sCu[1][i] = p.cu_k[i]; sCu[2][i] = p.cu_km[i]; }
   if (warp == 0) tmem_alloc(&tmem_base_s, kSelBufs * kSelN);
@@ -766,10 +784,8 @@ gate_select_kernel(GateParams p, const __grid_constant__ CUtensorMap map_q, cons
   };
 
   if (warp == 8) {
-    // =============================================================== loads and MMAs
+    // =============================================================== loads
     if (lane == 0) {
-      constexpr uint32_t idesc = make_idesc(FmtOf<T>::v, kGateM, kSelN, 0, 0);
-      const uint32_t hi = desc_hi_sw128(1024), q_km = desc_lo_sw128(smem_u32(sQ), 16);
       const int group = p.heads / p.heads_k;
       uint32_t gs = 0, qn = 0;                           // steps and items with candidates so far
       bool ok = true;
@@ -778,24 +794,39 @@ gate_select_kernel(GateParams p, const __grid_constant__ CUtensorMap map_q, cons
         Item I;
         if (!decode(item, I) || I.nt == 0) continue;
         const int nt = I.nt, steps = nt <= kSelBufs ? nt : 2 * nt, hk = I.h / group;
-        auto load_km = [&](int s) {                      // centroid tile of step s into its ring slot
-          const uint32_t n = gs + s, slot = n % kSelRing;
-          if (n >= kSelRing) ok = ok && mbar_wait(&bar_kfree[slot], (n / kSelRing - 1) & 1, &g_gate_status, 2);
-          if (!ok) return;
-          const int row = I.km0 + (s < nt ? s : s - nt) * kSelN;
-          mbar_expect_tx(&bar_kfull[slot], kKTile);
-#pragma unroll
-          for (int hb = 0; hb < D / 64; ++hb)
-            tma_load_3d(sKM + slot * kKTile + hb * (kSelN * 128), &map_km, hb * 64, hk, row, &bar_kfull[slot]);
-        };
         if (qn > 0) ok = mbar_wait(&bar_qfree, (qn - 1) & 1, &g_gate_status, 2);   // the last item's MMAs have read Q
         if (!ok) break;
         mbar_expect_tx(&bar_q, kQTile);
 #pragma unroll
         for (int hb = 0; hb < D / 64; ++hb) tma_load_3d(sQ + hb * (kGateM * 128), &map_q, hb * 64, I.h, I.q0 + I.r0, &bar_q);
-        load_km(0);
-        if (steps > 1) load_km(1);
-        ok = ok && mbar_wait(&bar_q, qn & 1, &g_gate_status, 2);
+#pragma unroll 1
+        for (int s = 0; s < steps && ok; ++s) {          // centroid tiles, each as soon as its ring slot is free
+          const uint32_t n = gs + s, slot = n % kSelRing;
+          if (n >= kSelRing) ok = mbar_wait(&bar_kfree[slot], (n / kSelRing - 1) & 1, &g_gate_status, 2);
+          if (!ok) break;
+          const int row = I.km0 + (s < nt ? s : s - nt) * kSelN;
+          mbar_expect_tx(&bar_kfull[slot], kKTile);
+#pragma unroll
+          for (int hb = 0; hb < D / 64; ++hb)
+            tma_load_3d(sKM + slot * kKTile + hb * (kSelN * 128), &map_km, hb * 64, hk, row, &bar_kfull[slot]);
+        }
+        gs += steps;
+        ++qn;
+      }
+    }
+  } else if (warp == 9) {
+    // =============================================================== MMAs
+    if (lane == 0) {
+      constexpr uint32_t idesc = make_idesc(FmtOf<T>::v, kGateM, kSelN, 0, 0);
+      const uint32_t hi = desc_hi_sw128(1024), q_km = desc_lo_sw128(smem_u32(sQ), 16);
+      uint32_t gs = 0, qn = 0;
+      bool ok = true;
+#pragma unroll 1
+      for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
+        Item I;
+        if (!decode(item, I) || I.nt == 0) continue;
+        const int steps = I.nt <= kSelBufs ? I.nt : 2 * I.nt;
+        ok = mbar_wait(&bar_q, qn & 1, &g_gate_status, 2);
 #pragma unroll 1
         for (int s = 0; s < steps && ok; ++s) {
           const uint32_t n = gs + s, slot = n % kSelRing, buf = n % kSelBufs;
@@ -807,7 +838,6 @@ gate_select_kernel(GateParams p, const __grid_constant__ CUtensorMap map_q, cons
                             desc_lo_sw128(smem_u32(sKM) + slot * kKTile, 16), hi, 2, (kSelN * 128) >> 4, idesc, 0);
           umma_commit(&bar_tfull[buf]);
           umma_commit(&bar_kfree[slot]);
-          if (s >= 1 && s + 1 < steps) load_km(s + 1);   // into the slot of the step before this one
         }
         umma_commit(&bar_qfree);
         gs += steps;
@@ -935,8 +965,106 @@ gate_select_kernel(GateParams p, const __grid_constant__ CUtensorMap map_q, cons
       }
       gs += resident ? nt : 2 * nt;
       const int cnt = (q_next - q_first) / 512;
-      sCount[tid] = cnt;
-      bar_sync(pair, 64);                                // both queues are complete
+      sCount[tid] = (uint8_t)cnt;
+      // ---- the list, short way: 32-bit keys of the score's upper bits and the candidate's place in its queue, sorted by each
+      // thread for its own queue; the first thread of a row merges the two lists
+      uint32_t key[KMAX], dropped = 0;                   // dropped: the largest key that is in no list any more
+#pragma unroll
+      for (int j = 0; j < KMAX; ++j) {
+        const uint32_t k = (score_to_ordered(queue[j * 64].x) & ~63u) | (uint32_t)(qd * 32 + j);
+        key[j] = j < cnt ? k : 0u;
+      }
+      sel_sort<KMAX>(key);
+      for (int j = KMAX; __any_sync(0xffffffffu, j < cnt); ++j) {
+        const uint32_t k = (score_to_ordered(queue[min(j, CAP - 1) * 64].x) & ~63u) | (uint32_t)(qd * 32 + j);
+        uint32_t x = j < cnt ? k : 0u;
+#pragma unroll
+        for (int i = 0; i < KMAX; ++i) sel_ce(key[i], x);
+        dropped = max(dropped, x);
+      }
+      uint32_t* keys = sKeys + (warp & 3) * ((KMAX + 1) * 32) + lane;
+      if (qd == 1) {
+#pragma unroll
+        for (int j = 0; j < KMAX; ++j) keys[j * 32] = key[j];
+        keys[KMAX * 32] = dropped;
+      }
+      bar_sync(pair, 64);                                // both queues are complete, the second thread's list is there
+      const int first_place = own ? 1 : 0;
+      bool close = false;
+      auto candidate = [&](uint32_t k) { return reinterpret_cast<const float2*>(mine) + (k & 31u) * 64 + (k & 32u) + lane; };
+      if (qd == 0) {
+        uint32_t low = max(dropped, keys[KMAX * 32]);
+#pragma unroll
+        for (int j = 0; j < KMAX; ++j) {
+          const uint32_t o = keys[(KMAX - 1 - j) * 32];
+          low = max(low, min(key[j], o));
+          key[j] = max(key[j], o);
+        }
+        sel_bitonic<KMAX>(key);
+        // neighbours that may agree in the bits that the keys hold
+        uint32_t gap = ~0u;
+#pragma unroll
+        for (int j = 0; j + 1 < KMAX; ++j) gap = min(gap, key[j] - key[j + 1]);
+        if (need == KMAX) gap = min(gap, key[KMAX - 1] - low);
+        if (__any_sync(0xffffffffu, gap < 64u)) {
+          uint32_t near = 0;
+#pragma unroll
+          for (int j = 0; j + 1 < KMAX; ++j) near |= key[j] - key[j + 1] < 64u ? 1u << j : 0u;
+          const int c = min(KMAX, cnt + (int)sCount[tid ^ 128]);
+          near &= (1u << max(c - 1, 0)) - 1u;
+          if (low != 0u && key[KMAX - 1] - low < 64u) near |= 1u << (KMAX - 1);
+          close = (near & (near >> 1)) != 0 || (need == KMAX && (near >> (KMAX - 1)) != 0);
+          // pairs are put right one by one, anything more is left to the long way below
+#pragma unroll
+          for (int j = 0; j < KMAX; ++j) keys[j * 32] = key[j];
+          for (near &= (1u << (KMAX - 1)) - 1u; near != 0 && !close; near &= near - 1) {
+            uint32_t* pair_at = keys + (__ffs(near) - 1) * 32;
+            const uint32_t x = pair_at[0], y = pair_at[32];
+            if (sel_key(*candidate(y)) > sel_key(*candidate(x))) {
+              pair_at[0] = y;
+              pair_at[32] = x;
+            }
+          }
+#pragma unroll
+          for (int j = 0; j < KMAX; ++j) key[j] = keys[j * 32];
+        }
+        const int64_t row_at = (int64_t)(I.q0 + I.r0 + lt) * p.t_rs + (int64_t)I.h * p.t_hs;
+        if (row_ok) {
+          int id[KMAX];
+#pragma unroll
+          for (int j = 0; j < KMAX; ++j) {
+            id[j] = key[j] != 0u ? __float_as_int(candidate(key[j])->y) : -1;
+          }
+          if (topk == KMAX && p.t_rs == KMAX && vec_out) {
+            int4* dst = reinterpret_cast<int4*>(p.topk_idx + row_at);
+#pragma unroll
+            for (int j = 0; j < KMAX; j += 4) {
+              int4 x;
+              x.x = own ? (j == 0 ? pos_chunk : id[j > 0 ? j - 1 : 0]) : id[j];
+              x.y = own ? id[j] : id[j + 1];
+              x.z = own ? id[j + 1] : id[j + 2];
+              x.w = own ? id[j + 2] : id[j + 3];
+              dst[j / 4] = x;
+            }
+          } else {
+            if (own) p.topk_idx[row_at] = pos_chunk;
+#pragma unroll
+            for (int j = 0; j < KMAX; ++j)
+              if (j + first_place < topk) p.topk_idx[row_at + j + first_place] = id[j];
+          }
+          if (p.topk_val) {
+            if (own) p.topk_val[row_at] = CUDART_INF_F;
+#pragma unroll
+            for (int j = 0; j < KMAX; ++j) {
+              if (j + first_place < topk) p.topk_val[row_at + j + first_place] = key[j] != 0u ? candidate(key[j])->x : -CUDART_INF_F;
+            }
+          }
+        }
+      }
+      if (bar_and(pair, 64, good && !close)) continue;   // the pair goes on, or leaves, together; its areas are free
+      good = bar_and(pair, 64, good);
+      if (!good) break;
+      // ---- the list, long way: exact comparisons of all with all
       {
         // ---- ranks: this thread takes every second one of the row's candidates
         const int other = sCount[tid ^ 128];
@@ -1050,7 +1178,7 @@ static int gate_tc_pick(const GateParams& p, int batch, int max_q, cudaStream_t 
 template <typename T, int D, int KMAX>
 static int gate_select_launch(const GateParams& p, const CUtensorMap& mq, const CUtensorMap& mk, int batch, int max_q, cudaStream_t s) {
   constexpr int kCap = sel_cap<KMAX>();
-  const size_t smem = 1024 + (size_t)kGateM * D * 2 + (size_t)kSelRing * kSelN * D * 2 + (size_t)kCap * 256 * 8;
+  const size_t smem = (size_t)kGateM * D * 2 + (size_t)kSelRing * kSelN * D * 2 + (size_t)kCap * 256 * 8 + (size_t)4 * (KMAX + 1) * 32 * 4;
   static_assert(2 * KMAX * 32 * 4 <= kCap * 64 * 8, "a pair's exchange area fits its queues");
   auto divider = [](int d) {
     FastDiv fd{0, 0, (uint32_t)d};

@@ -44,3 +44,26 @@ def test_gate_select_exact(lens_q, lens_k, H, Hk, d, topk, causal, spread):
         ref_idx, ref_val = O.gate_topk(q, km, cq, ck, ck, topk, 1, causal)
         assert torch.equal(idx.cpu(), ref_idx)
         assert val is None or torch.equal(val.cpu(), ref_val)
+
+
+@pytest.mark.parametrize("topk,causal,n_values", [(8, True, 400), (8, False, 400), (16, True, 300), (16, False, 60), (5, True, 40), (12, False, 500), (8, True, 12), (16, True, 20)])
+def test_scores_that_differ_in_their_last_bits(topk, causal, n_values):
+    """Lists are put in order by the upper 26 bits of the scores first.  Here a score is an integer of six or seven bits plus 0 to 3 times
+    2**-15, exact in fp32: among the integers' repetitions are equal scores, pairs that differ below those bits, and more than two of a kind."""
+    from flash_moba_b200 import ops
+    g = torch.Generator().manual_seed(topk + n_values)
+    lens_q, lens_k, H, Hk, d = [200, 77], [260, 333], 2, 1, 128
+    q = torch.zeros(sum(lens_q), H, d)
+    q[..., 0], q[..., 5] = 1.0, 2.0 ** -15
+    sign = torch.randint(0, 2, (sum(lens_q), H), generator=g) * 2 - 1
+    q[..., 0] *= sign
+    km = torch.zeros(sum(lens_k), Hk, d)
+    # (an integer of up to eight bits is exact in bf16)
+    km[..., 0] = torch.randint(0, n_values, (sum(lens_k), Hk), generator=g).remainder(127).float() + 1
+    km[..., 5] = torch.randint(0, 4, (sum(lens_k), Hk), generator=g).float()
+    q, km = q.bfloat16(), km.bfloat16()
+    cq, ck = cu_of(lens_q), cu_of(lens_k)
+    idx, val = ops.gate_topk(q.to(DEV), km.to(DEV), cq.to(DEV), ck.to(DEV), ck.to(DEV), max(lens_q), max(lens_k), topk, 1, causal,
+                             return_values=True)
+    ref_idx, ref_val = O.gate_topk(q, km, cq, ck, ck, topk, 1, causal)
+    assert torch.equal(idx.cpu(), ref_idx) and torch.equal(val.cpu(), ref_val)
