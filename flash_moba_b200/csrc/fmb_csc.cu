@@ -13,15 +13,20 @@
 //   3. scatter   : the column offsets (a scan over col_nnz, repeated by every CTA: a few hundred numbers);
 //                  a bitmap (column x row) of the tile in shared memory with a running count per 32 rows, from
 //                  which every entry's place in its column follows directly: columns come out ascending,
-//                  bit-exact and run-to-run deterministic, entries are written where the row stands.
+//                  bit-exact and run-to-run deterministic.  Lists of up to 16 are put in order column by column in shared
+//                  memory first, so that a warp's stores fill whole sectors of a few columns instead of 4 bytes in each of 32.
 //                  On request the same thread also writes the row's places in `indices`, in ascending
 //                  order (row_slots): the row-major view of the pattern that the attention kernels' merge
 //                  needs, so that an attention call on this pattern builds no lists of its own.
 // Measured (B200, three kernels with bitmap walks before / now): 64K tokens x 32 heads, 512 columns 297 / 192 us; 32K x 16
 // 71 / 45; 317K tokens, lists of 16 2.19 / 1.63 ms; 512K x 4 heads, 2,048 columns 1.49 / 0.84 ms.  The scatter with its counts per 32
 // rows laid out column by column (stores of a warp eight to a bank) and 64-bit scans / row group by row group and 32-bit scans:
-// 64K 143 / 129 us, 317K 1.32 / 1.23 ms, 512K 0.80 / 0.71 ms.
-// HBM bound.  Algorithmic bytes: 4*nnz read + 4*nnz written + 12*B*H*ncol.
+// 64K 143 / 129 us, 317K 1.32 / 1.23 ms, 512K 0.80 / 0.71 ms.  Entries stored by the row's thread, lists read behind the scan, a
+// bitonic network per row in the histogram too / in column order, read ahead of it, networks of 19 exchanges and none in the
+// histogram of distinct lists, all three kernels: 64K 158 / 142 us, 32K x 16 39 / 36, d 64, 9K x 12 13.8 / 11.8, 8 x 8K 127 / 127 (of 64 columns; stores
+// by the row's thread 123), 317K 1450 / 1190, 512K 636 / 598.  (Three CTAs per SM with 40 registers: 64K 143, 8 x 8K 117, but 9K x 12 14.8.)
+// What bounds it: the scatter's instructions (1,300 a warp of 32 rows before, 60 % issue) and its shared-memory accesses at random columns
+// (65 - 75 % of the wavefronts); HBM 11 - 25 %.  Algorithmic bytes: 4*nnz read + 4*nnz written + 12*B*H*ncol.
 #include <mutex>
 #include <type_traits>
 
@@ -34,8 +39,12 @@ constexpr int kTileWords = kTileRows / 32;     // bitmap words per column
 constexpr int kBmStride = kTileWords + 1;      // padded: conflict-free column walks
 constexpr int kMaxHistCols = 8192;             // columns per CTA of the histogram (32 KB of counters)
 constexpr int kMaxColsPerCta = 1024;           // columns per CTA of the scatter
-constexpr int kColBytes = kBmStride * 4 + kTileWords * 2 + 4;   // shared memory of the scatter per column
+constexpr int kColBytes = kBmStride * 4 + kTileWords * 2 + 8;   // shared memory of the scatter per column
 constexpr int kCscThreads = 512;
+// shared memory of the scatter: the columns' arrays; the tile's entries (lists of up to `kmax`) take the place of all but the cursors
+constexpr size_t scatter_bytes(int ncols, int kmax) {
+  return (size_t)ncols * 8 + ((size_t)ncols * (kColBytes - 8) > (size_t)kTileRows * kmax * 4 ? (size_t)ncols * (kColBytes - 8) : (size_t)kTileRows * kmax * 4);
+}
 
 struct CscParams {
   const int32_t* topk_idx; int64_t idx_rs, idx_hs;   // element strides of (row, head)
@@ -48,23 +57,34 @@ struct CscParams {
   int scanned;                                        // 1: hist holds cursors (tile_scan has run), 0: counts
 };
 
-// ascending sorting networks on 8 and 16 ids
+// ascending sorting networks on 8 and 16 ids: 19 compare-exchanges; two sorted eights and a bitonic merge
 __device__ __forceinline__ void csc_ce(int& a, int& b) {
   const int lo = min(a, b), hi = max(a, b);
   a = lo;
   b = hi;
 }
+__device__ __forceinline__ void csc_sort8(int* x) {
+  csc_ce(x[0], x[1]); csc_ce(x[2], x[3]); csc_ce(x[4], x[5]); csc_ce(x[6], x[7]);
+  csc_ce(x[0], x[2]); csc_ce(x[1], x[3]); csc_ce(x[4], x[6]); csc_ce(x[5], x[7]);
+  csc_ce(x[1], x[2]); csc_ce(x[5], x[6]); csc_ce(x[0], x[4]); csc_ce(x[3], x[7]);
+  csc_ce(x[1], x[5]); csc_ce(x[2], x[6]);
+  csc_ce(x[1], x[4]); csc_ce(x[3], x[6]);
+  csc_ce(x[2], x[4]); csc_ce(x[3], x[5]);
+  csc_ce(x[3], x[4]);
+}
 template <int N>
 __device__ __forceinline__ void csc_sort(int* x) {
 #pragma unroll
-  for (int k = 2; k <= N; k <<= 1)
+  for (int i = 0; i < N; i += 8) csc_sort8(x + i);
+  if constexpr (N == 16) {
 #pragma unroll
-    for (int j = k >> 1; j >= 1; j >>= 1)
+    for (int i = 0; i < 8; ++i) csc_ce(x[i], x[15 - i]);
 #pragma unroll
-      for (int i = 0; i < N; ++i) {
-        const int l = j == (k >> 1) ? (i ^ (k - 1)) : (i ^ j);
-        if (l > i) csc_ce(x[i], x[l]);
-      }
+    for (int o = 4; o; o >>= 1)
+#pragma unroll
+      for (int i = 0; i < 16; ++i)
+        if ((i & o) == 0) csc_ce(x[i], x[i + o]);
+  }
 }
 
 constexpr int kCscNone = 0x7fffffff;
@@ -106,17 +126,21 @@ __global__ void __launch_bounds__(kCscThreads) csc_tile_hist_kernel(CscParams p)
   __syncthreads();
   const int32_t* src = p.topk_idx + (int64_t)(seq0 + r0) * p.idx_rs + (int64_t)h * p.idx_hs;
   auto count = [&](int c) {
-    c -= c0;
-    if (c >= 0 && c < ncols) atomicAdd(&sm[c], 1u);
+    if ((uint32_t)(c - c0) < (uint32_t)ncols) atomicAdd(&sm[c - c0], 1u);
   };
   if constexpr (KMAX > 0) {
     if ((int)threadIdx.x < rows) {
       int id[KMAX];
       csc_load_row<KMAX>(p, src, threadIdx.x, id);
-      csc_sort<KMAX>(id);
+      if (p.row_slots != nullptr) {                               // (asked for only with lists that name a chunk once)
 #pragma unroll
-      for (int j = 0; j < KMAX; ++j)
-        if (id[j] != kCscNone && (j == 0 || id[j] != id[j > 0 ? j - 1 : 0])) count(id[j]);
+        for (int j = 0; j < KMAX; ++j) count(id[j]);
+      } else {
+        csc_sort<KMAX>(id);
+#pragma unroll
+        for (int j = 0; j < KMAX; ++j)
+          if (j == 0 || id[j] != id[j > 0 ? j - 1 : 0]) count(id[j]);
+      }
     }
   } else {
     for (int e = threadIdx.x; e < rows * p.topk; e += kCscThreads) {
@@ -167,9 +191,9 @@ __global__ void __launch_bounds__(1024) csc_tile_scan_kernel(CscParams p) {
 // KMAX: 8 or 16: lists of at most that many ids are sorted in registers by one thread per row; 0: any length,
 // a thread per entry
 template <int KMAX>
-__global__ void __launch_bounds__(kCscThreads) csc_scatter_kernel(CscParams p) {
+__global__ void __launch_bounds__(kCscThreads, 2) csc_scatter_kernel(CscParams p) {
   follow_on();
-  extern __shared__ uint32_t sm[];
+  extern __shared__ __align__(16) uint32_t sm[];
   // places inside a (b, h)'s region: fewer than 65,535 tiles of 512 rows, of lists of up to 16, fit 32 bits
   using Off = typename std::conditional<(KMAX > 0), int, int64_t>::type;
   __shared__ Off warp_sums[kCscThreads / 32];
@@ -180,16 +204,50 @@ __global__ void __launch_bounds__(kCscThreads) csc_scatter_kernel(CscParams p) {
   if (rows <= 0 && tile > 0) return;            // (the first tile of an empty sequence still writes its columns)
   const int ncols = min(p.cols_per_cta, p.ncol - c0);
   const int ntiles_b = (len_q + kTileRows - 1) / kTileRows;
-  uint32_t* bm = sm;                                              // [ncols][kBmStride] bit (row) of every column
+  // [ncols] x: first of the column's entries among the tile's (column by column), y: from there to their places in the region
+  uint2* base = reinterpret_cast<uint2*>(sm);
+  uint32_t* bm = sm + ncols * 2;                                  // [ncols][kBmStride] bit (row) of every column
   uint16_t* before = reinterpret_cast<uint16_t*>(bm + ncols * kBmStride);   // [kTileWords][ncols] rows ahead of each 32
-  uint32_t* base = reinterpret_cast<uint32_t*>(before + ncols * kTileWords);   // [ncols] first place of the tile's entries
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int64_t region = ((int64_t)seq0 * p.heads + (int64_t)len_q * h) * p.topk;   // first place of this (b, h) in `indices`
-  for (int i = tid; i < ncols * kBmStride; i += kCscThreads) bm[i] = 0u;
+  {
+    uint4* zero = reinterpret_cast<uint4*>(sm);                   // (the cursors as well: they are written further down)
+    const int n = (ncols * (2 + kBmStride) + 3) / 4;              // (at most 12 bytes into `before`)
+    for (int i = tid; i < n; i += kCscThreads) zero[i] = make_uint4(0u, 0u, 0u, 0u);
+  }
+  // the row's list, on its way while the columns are looked up
+  const int32_t* src = p.topk_idx + (int64_t)(seq0 + r0) * p.idx_rs + (int64_t)h * p.idx_hs;
+  static_assert(kTileRows == kCscThreads, "a thread per row");
+  int id[KMAX > 0 ? KMAX : 1];
+  if constexpr (KMAX > 0) {
+    if (tid < rows) csc_load_row<KMAX>(p, src, tid, id);
+  }
 
   // ---- column offsets (places inside the region) and this tile's cursor in every column
   const int32_t* hist = p.hist + (int64_t)bh * p.ntiles * p.ncol;
-  Off carry = 0;
+  // exclusive sum over the CTA's threads; `total`: of all
+  auto scan = [&](Off x, Off& total) {
+    const Off own = x;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const Off y = __shfl_up_sync(0xffffffffu, x, o);
+      if (lane >= o) x += y;
+    }
+    if (lane == 31) warp_sums[warp] = x;
+    __syncthreads();
+    constexpr int W = kCscThreads / 32;
+    Off sums = warp_sums[lane % W];
+#pragma unroll
+    for (int o = 1; o < W; o <<= 1) {
+      const Off y = __shfl_up_sync(0xffffffffu, sums, o, W);
+      if (lane % W >= o) sums += y;
+    }
+    total = __shfl_sync(0xffffffffu, sums, W - 1);
+    const Off ahead = __shfl_sync(0xffffffffu, sums, max(warp - 1, 0));
+    __syncthreads();
+    return (warp > 0 ? ahead : 0) + x - own;
+  };
+  Off carry = 0, total;
   for (int g0 = 0; g0 < p.ncol; g0 += kCscThreads) {
     const int c = g0 + tid;
     int nnz = 0, cursor = 0;
@@ -206,31 +264,15 @@ __global__ void __launch_bounds__(kCscThreads) csc_scatter_kernel(CscParams p) {
         }
       }
     }
-    Off x = nnz;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const Off y = __shfl_up_sync(0xffffffffu, x, o);
-      if (lane >= o) x += y;
-    }
-    if (lane == 31) warp_sums[warp] = x;
-    __syncthreads();
-    Off ahead = carry, total = 0;
-#pragma unroll
-    for (int w = 0; w < kCscThreads / 32; ++w) {
-      const Off y = warp_sums[w];
-      ahead += w < warp ? y : 0;
-      total += y;
-    }
+    const Off off = carry + scan(nnz, total);
     if (c < p.ncol) {
-      const Off off = ahead + x - nnz;
-      if (c >= c0 && c < c0 + ncols) base[c - c0] = (uint32_t)(off + cursor);
+      if (c >= c0 && c < c0 + ncols) base[c - c0].y = (uint32_t)(off + cursor);
       if (tile == 0 && blockIdx.z == 0) {
         p.col_offsets[(int64_t)bh * p.ncol + c] = region + off;
         if (!p.scanned) p.col_nnz[(int64_t)bh * p.ncol + c] = nnz;
       }
     }
     carry += total;
-    __syncthreads();
   }
   // the unused tail of the region stays zero, as in the reference's zero-initialised buffer
   // (csrc/flash_topk/flash_topk_api.cpp:217); its tiles share it
@@ -247,16 +289,12 @@ __global__ void __launch_bounds__(kCscThreads) csc_scatter_kernel(CscParams p) {
   if (rows <= 0) return;
 
   // ---- bitmap of the tile
-  const int32_t* src = p.topk_idx + (int64_t)(seq0 + r0) * p.idx_rs + (int64_t)h * p.idx_hs;
-  static_assert(kTileRows == kCscThreads, "a thread per row");
-  int id[KMAX > 0 ? KMAX : 1];
   if constexpr (KMAX > 0) {
     if (tid < rows) {
-      csc_load_row<KMAX>(p, src, tid, id);
 #pragma unroll
       for (int j = 0; j < KMAX; ++j) {
         const int c = id[j] - c0;
-        if (c >= 0 && c < ncols) atomicOr(&bm[c * kBmStride + (tid >> 5)], 1u << (tid & 31));
+        if ((uint32_t)c < (uint32_t)ncols) atomicOr(&bm[c * kBmStride + warp], 1u << lane);
       }
     }
   } else {
@@ -266,44 +304,66 @@ __global__ void __launch_bounds__(kCscThreads) csc_scatter_kernel(CscParams p) {
     }
   }
   __syncthreads();
-  for (int c = tid; c < ncols; c += kCscThreads) {
+  int entries = 0;                                                // of the tile, in this CTA's columns
+  for (int g0 = 0; g0 < ncols; g0 += kCscThreads) {
+    const int c = g0 + tid;
     int run = 0;
+    if (c < ncols) {
 #pragma unroll
-    for (int w = 0; w < kTileWords; ++w) {
-      before[w * ncols + c] = (uint16_t)run;             // (neighbouring lanes, neighbouring places: no bank conflicts)
-      run += __popc(bm[c * kBmStride + w]);
+      for (int w = 0; w < kTileWords; ++w) {
+        before[w * ncols + c] = (uint16_t)run;           // (neighbouring lanes, neighbouring places: no bank conflicts)
+        run += __popc(bm[c * kBmStride + w]);
+      }
     }
+    const int first = entries + (int)scan(run, total);
+    if (c < ncols) base[c] = make_uint2((uint32_t)first, base[c].y - (uint32_t)first);
+    entries += (int)total;
   }
   __syncthreads();
 
-  // ---- places: first place of the column's entries in this tile, plus its rows ahead of this one
+  // ---- places: first of the column's entries in this tile, plus its rows ahead of this one
   auto place = [&](int c, int r) {
-    return base[c] + before[(r >> 5) * ncols + c] + (uint32_t)__popc(bm[c * kBmStride + (r >> 5)] & ((1u << (r & 31)) - 1u));
+    return before[(r >> 5) * ncols + c] + (uint32_t)__popc(bm[c * kBmStride + (r >> 5)] & ((1u << (r & 31)) - 1u));
   };
   if constexpr (KMAX > 0) {
-    if (tid >= rows) return;
-    if (p.row_slots != nullptr) csc_sort<KMAX>(id);               // ascending columns are ascending places
-    uint32_t at[KMAX];
+    uint32_t local[KMAX];                                         // place among the tile's entries
+    if (tid < rows) {
+      if (p.row_slots != nullptr) csc_sort<KMAX>(id);             // ascending columns are ascending places
+      uint32_t at[KMAX];
 #pragma unroll
-    for (int j = 0; j < KMAX; ++j) {
-      const int c = id[j] - c0;
-      at[j] = 0xffffffffu;
-      if (c >= 0 && c < ncols) {
-        const uint32_t x = place(c, tid);
-        p.indices[region + x] = r0 + tid;
-        at[j] = (uint32_t)region + x;                             // (row_slots are kept for fewer than 2^32 entries only)
+      for (int j = 0; j < KMAX; ++j) {
+        const int c = id[j] - c0;
+        at[j] = local[j] = 0xffffffffu;
+        if ((uint32_t)c < (uint32_t)ncols) {
+          const uint2 f = base[c];
+          local[j] = f.x + place(c, tid);
+          at[j] = (uint32_t)region + local[j] + f.y;              // (row_slots are kept for fewer than 2^32 entries only)
+        }
+      }
+      if (p.row_slots != nullptr) {
+        uint32_t* out = p.row_slots + ((int64_t)h * p.total_q + seq0 + r0 + tid) * p.topk;
+        if (p.topk == KMAX && gridDim.z == 1 && (reinterpret_cast<uintptr_t>(p.row_slots) & 15) == 0) {
+#pragma unroll
+          for (int j = 0; j < KMAX; j += 4) *reinterpret_cast<uint4*>(out + j) = make_uint4(at[j], at[j + 1], at[j + 2], at[j + 3]);
+        } else {                                                  // a CTA writes the entries of its own columns
+#pragma unroll
+          for (int j = 0; j < KMAX; ++j)
+            if (j < p.topk && (at[j] != 0xffffffffu || (id[j] == kCscNone && blockIdx.z == 0))) out[j] = at[j];
+        }
       }
     }
-    if (p.row_slots != nullptr) {
-      uint32_t* out = p.row_slots + ((int64_t)h * p.total_q + seq0 + r0 + tid) * p.topk;
-      if (p.topk == KMAX && gridDim.z == 1 && (reinterpret_cast<uintptr_t>(p.row_slots) & 15) == 0) {
+    __syncthreads();                                              // the bitmap is done with: its place takes the entries
+    uint32_t* entry = bm;                                         // column and row of every entry, column by column
+    if (tid < rows) {
 #pragma unroll
-        for (int j = 0; j < KMAX; j += 4) *reinterpret_cast<uint4*>(out + j) = make_uint4(at[j], at[j + 1], at[j + 2], at[j + 3]);
-      } else {                                                    // a CTA writes the entries of its own columns
-#pragma unroll
-        for (int j = 0; j < KMAX; ++j)
-          if (j < p.topk && (at[j] != 0xffffffffu || (id[j] == kCscNone && blockIdx.z == 0))) out[j] = at[j];
-      }
+      for (int j = 0; j < KMAX; ++j)
+        if (local[j] != 0xffffffffu) entry[local[j]] = (uint32_t)(id[j] - c0) << 16 | (uint32_t)tid;
+    }
+    __syncthreads();
+    int32_t* into = p.indices + region;
+    for (int i = tid; i < entries; i += kCscThreads) {
+      const uint32_t e = entry[i];
+      into[i + base[e >> 16].y] = r0 + (int)(e & 0xffffu);
     }
   } else {
     uint32_t* out = p.row_slots ? p.row_slots + ((int64_t)h * p.total_q + seq0 + r0) * p.topk : nullptr;
@@ -316,7 +376,7 @@ __global__ void __launch_bounds__(kCscThreads) csc_scatter_kernel(CscParams p) {
       const bool here = used && c >= 0 && c < ncols;
       uint32_t x = 0;
       if (here) {
-        x = place(c, r);
+        x = base[c].x + place(c, r) + base[c].y;
         p.indices[region + x] = r0 + r;
       }
       if (out != nullptr && (here || (!used && blockIdx.z == 0))) {
@@ -368,10 +428,11 @@ int launch_build_csc(const int32_t* topk_idx, int64_t idx_rs, int64_t idx_hs, co
   }
   p.cols_per_cta = min(kMaxColsPerCta, ncol);
   const dim3 grid(batch * heads, p.ntiles, ceil_div(ncol, p.cols_per_cta));
-  const size_t smem = (size_t)p.cols_per_cta * kColBytes;
+  const int kmax = topk <= 8 ? 8 : topk <= 16 ? 16 : 0;
+  const size_t smem = scatter_bytes(p.cols_per_cta, kmax);
   auto scatter = topk <= 8 ? csc_scatter_kernel<8> : topk <= 16 ? csc_scatter_kernel<16> : csc_scatter_kernel<0>;
   // the attribute belongs to the current device: set on every call (cheap, idempotent, thread-safe)
-  FMB_CUDA(cudaFuncSetAttribute(scatter, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxColsPerCta * kColBytes));
+  FMB_CUDA(cudaFuncSetAttribute(scatter, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)scatter_bytes(kMaxColsPerCta, kmax)));
   launch_follow_on(scatter, grid, dim3(kCscThreads), smem, s, p);
   prof_end(6, s);
   FMB_LAUNCH_CHECK("csc_scatter_kernel");
