@@ -16,16 +16,13 @@
 
 namespace fmb {
 
-// Partial rows are stored with their 16-byte chunks permuted: chunk c of the pair at position
-// `pos` sits at chunk (c ^ (pos & 7)).  The backward kernel stages a tile of partial rows
-// in shared memory before one bulk copy per warp; with this permutation the 32 lanes of a
-// warp (consecutive positions) write their rows without bank conflicts, and the linear copy
-// preserves it.  The kernels that write a row per lane straight from registers, 32 bytes a store, need it too: without
-// it all lanes would write the same quarter of their 128-byte lines at a time (64K tokens x 32 heads, forward 1.60 / 1.93 ms
-// with / without).  Writers and the merge kernel use part_col() for the element index.
-__host__ __device__ __forceinline__ int part_col(int64_t pos, int col, int elems_per_chunk) {
-  const int chunk = col / elems_per_chunk;
-  return ((chunk ^ (int)(pos & 7)) * elems_per_chunk) + (col % elems_per_chunk);
+// How a partial row is stored: inside every 64 columns, column 8 j + 2 i + e (i = 0 .. 3, e = 0 or 1) is element 16 i + 2 j + e.
+// This is the order in which a TMEM load of 16 lanes x 64 columns (tmem_ld_16x64) spreads a row over four threads: each of them
+// has 32 contiguous bytes of it, and a warp's store fills eight whole 128-byte lines.  With a row per thread, 32 bytes a store, every
+// lane went to a line of its own: 857 data-pipe cycles a tile of 128 rows instead of 256, in a forward whose data pipe was busy for 85 %
+// of the time (operands of the MMAs 34 %).  The merge puts a row back in order, once for all its partials.
+__host__ __device__ __forceinline__ int part_col(int col) {
+  return (col & ~63) | ((col >> 1) & 3) << 4 | ((col >> 3) & 7) << 1 | (col & 1);
 }
 
 // A call is processed in one or more PASSES over ranges of query heads [h0, h0+nh), so that the

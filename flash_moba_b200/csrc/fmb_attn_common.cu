@@ -359,7 +359,7 @@ __global__ void __launch_bounds__(kMergeThreads, 3) merge_kernel(const T* __rest
         if (sk == kNoSlot) {
           x[k] = make_uint4(0, 0, 0, 0);
         } else {
-          x[k] = ldg_nc_16(part + ((int64_t)sb * c.cap + sk) * D + ((gl ^ (int)(sk & 7)) * 8));
+          x[k] = ldg_nc_16(part + ((int64_t)sb * c.cap + sk) * D + gl * 8);
         }
       }
     };
@@ -405,16 +405,31 @@ __global__ void __launch_bounds__(kMergeThreads, 3) merge_kernel(const T* __rest
       }
     }
     if (FWD) l_n = lse_of(slot_of(next), 0);
+    if (FWD) {
+      const float inv = ssum > 0.f ? 1.f / ssum : 0.f;
+#pragma unroll
+      for (int e = 0; e < 8; ++e) acc[e] *= inv;
+    }
+    // from the order of a partial row (part_col): lane gl has columns 8 (4 (gl & 1) + k) + (gl & 6) and the next one of its 64, k = 0 .. 3;
+    // an exchange among the four lanes of the same parity gives it eight neighbouring ones
+    uint4 u = pack8<T>(acc);
+    {
+      const bool odd = gl & 2, high = gl & 4;
+      const uint32_t a = __shfl_xor_sync(0xffffffffu, odd ? u.x : u.y, 2), b = __shfl_xor_sync(0xffffffffu, odd ? u.z : u.w, 2);
+      if (odd) { u.x = a; u.z = b; }
+      else { u.y = a; u.w = b; }
+      const uint32_t e = __shfl_xor_sync(0xffffffffu, high ? u.x : u.z, 4), f = __shfl_xor_sync(0xffffffffu, high ? u.y : u.w, 4);
+      if (high) { u.x = e; u.y = f; }
+      else { u.z = e; u.w = f; }
+    }
     if (rid < n_rows) {
       const int hr = (int)(rid / c.total_q);
       const int64_t t = rid - (int64_t)hr * c.total_q;
       if (FWD) {
-        const float inv = ssum > 0.f ? 1.f / ssum : 0.f;
-#pragma unroll
-        for (int e = 0; e < 8; ++e) acc[e] *= inv;
         if (gl == 0) lse[(int64_t)c.h0 * c.total_q + rid] = ssum > 0.f ? m + logf(ssum) : CUDART_INF_F;
       }
-      *reinterpret_cast<uint4*>(out + t * rs + (int64_t)(c.h0 + hr) * hs + gl * 8) = pack8<T>(acc);
+      const int chunk = (gl & ~7) | (gl & 1) << 2 | ((gl >> 1) & 3);
+      *reinterpret_cast<uint4*>(out + t * rs + (int64_t)(c.h0 + hr) * hs + chunk * 8) = u;
     }
   }
 }

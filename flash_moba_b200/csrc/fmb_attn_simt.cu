@@ -203,7 +203,7 @@ __global__ void __launch_bounds__(kSimtThreads) fwd_main_simt_kernel(SimtParams 
         const int64_t slot = slot0 + t0 + m;
         T* dst = part_o + (plane + slot) * D;
 #pragma unroll
-        for (int x = 0; x < TD; ++x) dst[part_col(slot, tx * TD + x, 8)] = Elem<T>::from_f(o[i][x] * inv);
+        for (int x = 0; x < TD; ++x) dst[part_col(tx * TD + x)] = Elem<T>::from_f(o[i][x] * inv);
       }
     }
   }
@@ -353,7 +353,7 @@ __global__ void __launch_bounds__(kSimtThreads) bwd_main_simt_kernel(SimtParams 
             const int64_t slot = slot0 + t0 + m;
             T* dst = part_dq + (plane + slot) * D;
 #pragma unroll
-            for (int j = 0; j < TD; ++j) dst[part_col(slot, tx * TD + j, 8)] = Elem<T>::from_f(dq[i][j] * p.scale);
+            for (int j = 0; j < TD; ++j) dst[part_col(tx * TD + j)] = Elem<T>::from_f(dq[i][j] * p.scale);
           }
         }
       }

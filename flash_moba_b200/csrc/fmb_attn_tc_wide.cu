@@ -243,34 +243,34 @@ __global__ void __launch_bounds__(kFwThreads, 1) fwd_wide_tc_kernel(WideParams p
     uint32_t g = 0;
 #pragma unroll 1
     for (Tile t = first(); t.valid && good; advance(t), ++g) {
-      const bool mine = lt < t.nnz - t.t0;
-      const int64_t slot = plane + t.slot + t.t0 + lt;
-      const int key = (int)(slot & 7);
-      T* dst = part_o + slot * D;
+      const int row = (warp & 3) * 32 + (lane >> 2), left = t.nnz - t.t0 - row;
+      T* dst = part_o + (plane + t.slot + t.t0 + row) * D + (lane & 3) * 16;
       if (!(good = wait_all(&bar_pready[g & 1], g >> 1, 4))) break;   // (for 1 / l)
-      const float inv = sInv[g & 1][lt];
-      // ---- normalised partial O of row `lt`; 16-byte chunks permuted like every partial, a 32-byte store takes a pair
-      // of neighbouring chunks
+      float inv[4];                    // (at once: the group's next tile but one replaces them)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) inv[i] = sInv[g & 1][row + i * 8];
+      // ---- normalised partial O, halves of the head dim, 16 rows of the warp at a time: a thread has a quarter of a line of
+      // two rows (part_col)
 #pragma unroll 1
-      for (int q4 = 0; q4 < D / 32; ++q4) {
-        if ((q4 & 3) == 0) {
-          if (!(good = wait_all(&bar_o[g & 1][q4 >> 2], g >> 1, 4))) break;
-          tc_fence_after_sync();
-        }
-        float o[32];
-        tmem_ld32(tO + at + q4 * 32, o);
-        tmem_ld_wait();
-        if ((q4 & 3) == 3) {
-          tc_fence_before_sync();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(&bar_ofree[q4 >> 2]);
-        }
-#pragma unroll
-        for (int e = 0; e < 32; ++e) o[e] *= inv;
-#pragma unroll
-        for (int jj = 0; jj < 4; jj += 2) {
-          const uint4 u = pack8<T>(o + jj * 8), v = pack8<T>(o + jj * 8 + 8);
-          if (mine) st_global_32(dst + ((((q4 * 4 + jj) ^ key) & ~1) << 3), (key & 1) ? v : u, (key & 1) ? u : v);
+      for (int hh = 0; hh < 2; ++hh) {
+        if (!(good = wait_all(&bar_o[g & 1][hh], g >> 1, 4))) break;
+        tc_fence_after_sync();
+#pragma unroll 1
+        for (int r16 = 0; r16 < 32; r16 += 16) {
+          const float ia = r16 ? inv[2] : inv[0], ib = r16 ? inv[3] : inv[1];
+#pragma unroll 1
+          for (int c = hh * 128; c < hh * 128 + 128; c += 64) {
+            float o[32];
+            tmem_ld_16x64(tO + at + ((uint32_t)r16 << 16) + c, o);
+            tmem_ld_wait();
+            if (r16 == 16 && (c & 64)) {
+              tc_fence_before_sync();
+              __syncwarp();
+              if (lane == 0) mbar_arrive(&bar_ofree[hh]);
+            }
+            if (left > r16) store_part<T>(dst + r16 * D + c, o, ia);
+            if (left > r16 + 8) store_part<T>(dst + (r16 + 8) * D + c, o + 2, ib);
+          }
         }
       }
     }
@@ -555,33 +555,28 @@ __global__ void __launch_bounds__(kBwThreads, 1) bwd_wide_tc_kernel(WideParams p
     uint32_t g = 0;
 #pragma unroll 1
     for (Tile t = first(); t.valid && good; advance(t), ++g) {
-      const bool mine = lt < t.nnz - t.t0;
-      const int64_t slot = plane + t.slot + t.t0 + lt;
-      const int key = (int)(slot & 7);
-      T* dst = part_dq + slot * D;
-      // ---- dQ partial of row `lt`: scaled, rounded, 16-byte chunks permuted like every partial; a 32-byte store takes
-      // a pair of neighbouring chunks
+      const int row = (warp & 3) * 32 + (lane >> 2), left = t.nnz - t.t0 - row;
+      T* dst = part_dq + (plane + t.slot + t.t0 + row) * D + (lane & 3) * 16;
+      // ---- dQ partial: scaled, rounded, halves of the head dim, 16 rows of the warp at a time: a thread has a quarter of a
+      // line of two rows (part_col)
 #pragma unroll 1
       for (int hh = 0; hh < 2; ++hh) {
         if (!(good = wait_all(&bar_dq[hh], g, 4))) break;
         tc_fence_after_sync();
 #pragma unroll 1
-        for (int i2 = 0; i2 < 4; ++i2) {
-          float o[32];
-          tmem_ld32(tdQ + at + i2 * 32, o);
-          tmem_ld_wait();
-          if (i2 == 3) {
-            tc_fence_before_sync();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&bar_dqfree);
-          }
-#pragma unroll
-          for (int e = 0; e < 32; ++e) o[e] *= p.scale;
-#pragma unroll
-          for (int jj = 0; jj < 4; jj += 2) {
-            const uint4 u = pack8<T>(o + jj * 8), v = pack8<T>(o + jj * 8 + 8);
-            const int ch = hh * 16 + i2 * 4 + jj;
-            if (mine) st_global_32(dst + (((ch ^ key) & ~1) << 3), (key & 1) ? v : u, (key & 1) ? u : v);
+        for (int r16 = 0; r16 < 32; r16 += 16) {
+#pragma unroll 1
+          for (int c = 0; c < 128; c += 64) {
+            float o[32];
+            tmem_ld_16x64(tdQ + at + ((uint32_t)r16 << 16) + c, o);
+            tmem_ld_wait();
+            if (r16 == 16 && c == 64) {
+              tc_fence_before_sync();
+              __syncwarp();
+              if (lane == 0) mbar_arrive(&bar_dqfree);
+            }
+            if (left > r16) store_part<T>(dst + r16 * D + hh * 128 + c, o, p.scale);
+            if (left > r16 + 8) store_part<T>(dst + (r16 + 8) * D + hh * 128 + c, o + 2, p.scale);
           }
         }
       }

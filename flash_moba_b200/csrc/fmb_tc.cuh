@@ -146,6 +146,22 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float* v) {
       : "r"(taddr)
       : "memory");
 }
+// 16 lanes x 64 consecutive fp32 columns: thread t of the warp gets, of lane t / 4 and of lane t / 4 + 8, columns 8 j + 2 (t % 4) and the
+// next one, j = 0 .. 7: v[4 j], v[4 j + 1] and v[4 j + 2], v[4 j + 3].  (The lane in `taddr`: a multiple of 16.)
+__device__ __forceinline__ void tmem_ld_16x64(uint32_t taddr, float* v) {
+  uint32_t* r = reinterpret_cast<uint32_t*>(v);
+  asm volatile(
+      "tcgen05.ld.sync.aligned.16x256b.x8.b32 "
+      "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
+      "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+        "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]),
+        "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]),
+        "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]),
+        "=r"(r[30]), "=r"(r[31])
+      : "r"(taddr)
+      : "memory");
+}
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
 // ---- shared-memory matrix descriptors (128-byte swizzle) ------------------------------
@@ -337,6 +353,20 @@ __device__ __forceinline__ void st_global_32(void* dst, uint4 a, uint4 b) {
   asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(dst), "r"(a.x), "r"(a.y), "r"(a.z), "r"(a.w),
                "r"(b.x), "r"(b.y), "r"(b.z), "r"(b.w)
                : "memory");
+}
+
+// a thread's quarter of a partial row's line, as tmem_ld_16x64 gives it: values 4 j and 4 j + 1, times `f`
+template <typename T>
+__device__ __forceinline__ void store_part(T* dst, const float* o, float f) {
+  const float2 f2 = make_float2(f, f);
+  float x[16];
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    const float2 y = mul_f32x2(make_float2(o[4 * j], o[4 * j + 1]), f2);
+    x[2 * j] = y.x;
+    x[2 * j + 1] = y.y;
+  }
+  st_global_32(dst, pack8<T>(x), pack8<T>(x + 8));
 }
 
 // ---- bulk (TMA, non-tensor) shared -> global stores -----------------------------------
