@@ -375,11 +375,15 @@ static DecodeShape decode_shape(int64_t total_q, int heads, int heads_k, int d, 
   static_assert(kDecWarps == 4, "4, 2 or 1 heads per cluster");
   r.hg = group % 4 == 0 ? 4 : group % 2 == 0 ? 2 : 1;
   // With few rows: fewer heads per cluster and clusters of more CTAs, until the device is full or a
-  // warp would be left without a group of keys.
+  // warp would be left without a group of keys; of eight CTAs only where with four a warp would have four groups or more: clusters of
+  // eight find their places later, and are no longer brought up early (below).  Measured, eight / four, one row: 32 / 8 heads, d 128, top-k 8,
+  // 65,001 keys 15.8 / 13.1 us, 4,000 keys 13.8 / 11.6; 16 / 4 heads, d 64 11.2 / 10.0; two rows, 16 / 8 heads, chunk 64, top-k 16 19.5 / 16.7 (two
+  // groups a warp with four CTAs, all of them); 8 heads, chunk 256, top-k 8 (four groups) 13.0 / 13.7; 32 / 16 heads, d 64, chunk 256, top-k 16
+  // (eight) 17.7 / 20.2.
   const int64_t want = 148 * (d <= 64 ? DecGeo<64>::CTAS : DecGeo<128>::CTAS);
   while (r.hg > 1 && total_q * (heads / r.hg) * 8 < want) r.hg /= 2;
   r.S = 1;
-  while (r.S < 8 && total_q * (heads / r.hg) * r.S * 2 <= want && (int64_t)r.hg * topk * (chunk / keys) >= 2 * r.S * kDecWarps)
+  while (r.S < 8 && total_q * (heads / r.hg) * r.S * 2 <= want && (int64_t)r.hg * topk * (chunk / keys) >= (r.S < 4 ? 2 : 4) * r.S * kDecWarps)
     r.S *= 2;
   r.ncap = (max_k + chunk - 1) / chunk;
   if (r.ncap < 1) r.ncap = 1;

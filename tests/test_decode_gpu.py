@@ -37,7 +37,8 @@ def _decode(q, k, v, km, cu_km, cq, ck, mk, topk, chunk, causal):
 @pytest.mark.parametrize("causal", [True, False])
 @pytest.mark.parametrize("lens_q,lens_k,H,Hk,d,chunk,topk,dtype", [
     ([1], [1], 4, 2, 128, 64, 4, "bf16"),                                  # a single key
-    ([1], [5000], 8, 2, 128, 128, 8, "bf16"),                              # one row: clusters of several CTAs
+    ([1], [5000], 8, 2, 128, 128, 8, "bf16"),                              # one row: clusters of four CTAs
+    ([1], [9000], 8, 8, 128, 256, 8, "bf16"),                              # of eight: 64 groups of keys for a head
     ([1, 1, 1], [64, 65, 1279], 4, 4, 64, 64, 3, "fp16"),                  # chunk boundaries
     ([1] * 40, [300 + 37 * i for i in range(40)], 16, 2, 128, 128, 8, "bf16"),   # more rows than CTAs: no cluster
     ([3, 1, 0, 7], [700, 1, 50, 2000], 6, 2, 128, 64, 5, "fp16"),          # three heads per kv head, an empty block
