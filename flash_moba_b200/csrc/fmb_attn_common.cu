@@ -290,6 +290,21 @@ constexpr uint32_t kNoSlot = 0xffffffffu;
 constexpr int kMergeThreads = 256;
 constexpr int kMergeBatch = 8;      // partial rows in flight per row
 
+// From the order of a partial row (part_col) to a row's own: lane gl has columns 8 (4 (gl & 1) + k) + (gl & 6) and the next one of its
+// 64, k = 0 .. 3; an exchange among the four lanes of the same parity gives it eight neighbouring ones, 16-byte chunk
+// merged_place() of the row
+__device__ __forceinline__ uint4 merged_chunk(uint4 u, int gl) {
+  const bool odd = gl & 2, high = gl & 4;
+  const uint32_t a = __shfl_xor_sync(0xffffffffu, odd ? u.x : u.y, 2), b = __shfl_xor_sync(0xffffffffu, odd ? u.z : u.w, 2);
+  if (odd) { u.x = a; u.z = b; }
+  else { u.y = a; u.w = b; }
+  const uint32_t e = __shfl_xor_sync(0xffffffffu, high ? u.x : u.z, 4), f = __shfl_xor_sync(0xffffffffu, high ? u.y : u.w, 4);
+  if (high) { u.x = e; u.y = f; }
+  else { u.z = e; u.w = f; }
+  return u;
+}
+__device__ __forceinline__ int merged_place(int gl) { return (gl & ~7) | (gl & 1) << 2 | ((gl >> 1) & 3); }
+
 // Row lists are in ascending slot order (the pattern builder writes them so; sort_rows_kernel puts the
 // lists of other patterns in order), so a row's partials are taken as they come: D/8 lanes per
 // (head, token) row, one 16-byte chunk of every partial each, eight partials requested before anything
@@ -410,28 +425,107 @@ __global__ void __launch_bounds__(kMergeThreads, 3) merge_kernel(const T* __rest
 #pragma unroll
       for (int e = 0; e < 8; ++e) acc[e] *= inv;
     }
-    // from the order of a partial row (part_col): lane gl has columns 8 (4 (gl & 1) + k) + (gl & 6) and the next one of its 64, k = 0 .. 3;
-    // an exchange among the four lanes of the same parity gives it eight neighbouring ones
-    uint4 u = pack8<T>(acc);
-    {
-      const bool odd = gl & 2, high = gl & 4;
-      const uint32_t a = __shfl_xor_sync(0xffffffffu, odd ? u.x : u.y, 2), b = __shfl_xor_sync(0xffffffffu, odd ? u.z : u.w, 2);
-      if (odd) { u.x = a; u.z = b; }
-      else { u.y = a; u.w = b; }
-      const uint32_t e = __shfl_xor_sync(0xffffffffu, high ? u.x : u.z, 4), f = __shfl_xor_sync(0xffffffffu, high ? u.y : u.w, 4);
-      if (high) { u.x = e; u.y = f; }
-      else { u.z = e; u.w = f; }
-    }
+    const uint4 u = merged_chunk(pack8<T>(acc), gl);
     if (rid < n_rows) {
       const int hr = (int)(rid / c.total_q);
       const int64_t t = rid - (int64_t)hr * c.total_q;
       if (FWD) {
         if (gl == 0) lse[(int64_t)c.h0 * c.total_q + rid] = ssum > 0.f ? m + logf(ssum) : CUDART_INF_F;
       }
-      const int chunk = (gl & ~7) | (gl & 1) << 2 | ((gl >> 1) & 3);
-      *reinterpret_cast<uint4*>(out + t * rs + (int64_t)(c.h0 + hr) * hs + chunk * 8) = u;
+      *reinterpret_cast<uint4*>(out + t * rs + (int64_t)(c.h0 + hr) * hs + merged_place(gl) * 8) = u;
     }
   }
+}
+
+// The same merge for the builder's own lists of up to eight places, in one plane: the partials come by cp.async through a lane's own
+// places in shared memory, the next row's requested before this one's are waited for, so that a warp has up to 8 KB on the way and
+// the registers of one row.  Same sums in the same order.  Bound: HBM, 6.2 - 6.5 TB/s of partials at 64K tokens x 32 heads.
+constexpr int kMergeStages = 2, kMergeStage = 32 * kMergeBatch * 16, kMergeSmem = kMergeThreads / 32 * kMergeStages * kMergeStage;
+template <typename T, int D, bool FWD>
+__global__ void __launch_bounds__(kMergeThreads, 3) merge_staged_kernel(const T* part, const float* part_lse, MergeParams c, T* out, int64_t rs,
+                                                                     int64_t hs, float* lse) {
+  constexpr int LPR = D / 8, RPW = 32 / LPR;
+  follow_on();
+  if (c.mirror != nullptr && blockIdx.x == 0 && threadIdx.x == 0) *c.mirror = *c.status;   // (the main kernel has completed)
+  extern __shared__ __align__(16) unsigned char merge_smem[];
+  const int lane = threadIdx.x & 31, gl = lane % LPR;
+  const uint32_t mine = (uint32_t)__cvta_generic_to_shared(merge_smem) + (threadIdx.x >> 5) * (kMergeStages * kMergeStage) + lane * 16;
+  const int64_t n_rows = c.total_q * c.nh, stride = (int64_t)gridDim.x * (kMergeThreads / 32) * RPW;
+  int64_t row = ((int64_t)blockIdx.x * (kMergeThreads / 32) + (threadIdx.x >> 5)) * RPW + lane / LPR;
+  int64_t t;
+  T* to;
+  {
+    const int64_t h = row / c.total_q;
+    t = row - h * c.total_q;
+    to = out + (c.h0 + h) * hs + merged_place(gl) * 8;
+  }
+  auto fetch = [&](int64_t r) { return r < n_rows && gl < c.fixed_k ? c.row_pos[r * c.fixed_k + gl] : kNoSlot; };
+  // a place's content -> slot of the pass (kNoSlot also for what is none)
+  auto slot_of = [&](uint32_t x) {
+    const uint32_t at = x - (uint32_t)c.slot_shift;
+    return x != kNoSlot && at < c.cap ? at : kNoSlot;
+  };
+  auto request = [&](uint32_t s, uint32_t stage) {
+#pragma unroll
+    for (int k = 0; k < kMergeBatch; ++k) {
+      const uint32_t sk = __shfl_sync(0xffffffffu, s, k, LPR);
+      const bool ok = sk != kNoSlot;
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(mine + stage * kMergeStage + k * 512),
+                   "l"(part + (int64_t)(ok ? sk : 0u) * D + gl * 8), "r"(ok ? 16u : 0u) : "memory");
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  auto lse_of = [&](uint32_t s) { return FWD && s != kNoSlot ? part_lse[s] : -CUDART_INF_F; };
+  uint32_t slot = slot_of(fetch(row));
+  float l = lse_of(slot);
+  request(slot, 0);
+  uint32_t next = fetch(row + stride), stage = 0;
+#pragma unroll 1
+  for (int64_t first = row - lane / LPR; first < n_rows; first += stride, row += stride) {
+    const uint32_t s1 = slot_of(next);
+    const float l1 = lse_of(s1);
+    request(s1, stage ^ 1u);
+    next = fetch(row + 2 * stride);
+    float w = 1.f, m = l, ssum = 0.f, acc[8];
+    if (FWD) {
+#pragma unroll
+      for (int o = kMergeBatch / 2; o; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));   // (lanes 0 - 7 of the row hold its list)
+      w = slot != kNoSlot && m > -CUDART_INF_F ? __expf(l - m) : 0.f;
+    }
+#pragma unroll
+    for (int e = 0; e < 8; ++e) acc[e] = 0.f;
+    asm volatile("cp.async.wait_group 1;" ::: "memory");   // (a lane reads back what it copied itself)
+#pragma unroll
+    for (int k = 0; k < kMergeBatch; ++k) {
+      uint4 x;
+      asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
+                   : "=r"(x.x), "=r"(x.y), "=r"(x.z), "=r"(x.w) : "r"(mine + stage * kMergeStage + k * 512) : "memory");
+      float f[8];
+      unpack8<T>(x, f);
+      if (FWD) {
+        const float wk = __shfl_sync(0xffffffffu, w, k, LPR);
+        ssum += wk;
+#pragma unroll
+        for (int e = 0; e < 8; ++e) acc[e] = fmaf(wk, f[e], acc[e]);
+      } else {
+#pragma unroll
+        for (int e = 0; e < 8; ++e) acc[e] += f[e];
+      }
+    }
+    if (FWD) {
+      const float inv = ssum > 0.f ? 1.f / ssum : 0.f;
+#pragma unroll
+      for (int e = 0; e < 8; ++e) acc[e] *= inv;
+      if (gl == 0 && row < n_rows) lse[(int64_t)c.h0 * c.total_q + row] = ssum > 0.f ? m + logf(ssum) : CUDART_INF_F;
+    }
+    const uint4 u = merged_chunk(pack8<T>(acc), gl);
+    if (row < n_rows) *reinterpret_cast<uint4*>(to + t * rs) = u;
+    for (t += stride; t >= c.total_q; t -= c.total_q) to += hs;
+    slot = s1;
+    l = l1;
+    stage ^= 1u;
+  }
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
 }
 
 // D[h, t] = sum_d dO.O.  LPR = d / 8 lanes per row, each with one 16-byte load of dO and of O.  A thread's kDotRows rows are
@@ -498,6 +592,21 @@ static int merge_launch(const AttnArgs& a, const AttnWorkspace& w, const PassPar
   // persistent CTAs, as many as are resident
   const int64_t ctas = ceil_div64(a.total_q * ps.nh, (kMergeThreads / 32) * (32 / (D / 8))), most = (int64_t)sm_count() * 3;
   const unsigned grid = (unsigned)(ctas < most ? ctas : most);
+  // Where the staged kernel is the better one: head dims of 128 and more; dQ, whose merge has less to do per row, from half a gigabyte of
+  // partials on.  Measured, from registers / staged, us: 64K tokens x 32 heads, d 128, top-k 8 828 / 780 forward, 790 / 750 backward; 8 x 8K 805 / 738
+  // and 751 / 723; 32K x 16 213 / 207 and 202 / 202; 3.6K x 32 (235 MB) 51.7 / 47.6 and 43.5 / 47; d 64, 32K x 16 111 / 113 and 109 / 110.  Lists of 16, or
+  // of two planes, with a staged kernel of several steps a row: 317K tokens 6.97 / 7.66 ms, 512K x 4 2.95 / 3.23.
+  if constexpr (D >= 128) {
+    if (c.fixed_k > 0 && c.fixed_k <= kMergeBatch && c.nsub == 1 &&
+        (FWD || a.total_q * ps.nh * c.fixed_k * D * (int64_t)sizeof(T) >= (int64_t)1 << 29)) {
+      auto kern = merge_staged_kernel<T, D, FWD>;
+      FMB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kMergeSmem));
+      if (FWD) kern<<<grid, kMergeThreads, kMergeSmem, s>>>((const T*)w.part_o, w.part_lse, c, (T*)const_cast<void*>(a.o), a.o_rs, a.o_hs, a.lse);
+      else kern<<<grid, kMergeThreads, kMergeSmem, s>>>((const T*)w.part_o, nullptr, c, (T*)a.dq, a.dq_rs, a.dq_hs, nullptr);
+      FMB_LAUNCH_CHECK("merge_staged_kernel");
+      return FMB_OK;
+    }
+  }
   // An ordinary launch: brought up early, on whatever SMs the kernel before leaves first, the CTAs would spread unevenly, and each
   // has its fixed share of the rows (64K tokens x 32 heads: a step 4 % slower)
   if (FWD) merge_kernel<T, D, true><<<grid, kMergeThreads, 0, s>>>((const T*)w.part_o, w.part_lse, c, (T*)const_cast<void*>(a.o), a.o_rs, a.o_hs, a.lse);
