@@ -150,3 +150,29 @@ def test_checkpointed_layers():
 
     for a, b in zip(want, run(recomputed)):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("lens,H,Hk,d,chunk,topk", [
+    ([1], 3, 1, 128, 128, 1),                     # three rows of one place in all: most warps have none
+    ([5, 0, 2], 300, 300, 128, 64, 8),            # a warp's next row is many heads further
+    ([517], 8, 2, 256, 128, 7),
+    ([130, 259], 6, 6, 128, 128, 8),
+    ([400], 4, 4, 128, 256, 4),                   # two planes: not staged
+    ([300], 4, 4, 128, 64, 9),                    # nine places: not staged
+])
+def test_rows_merged_from_their_own_lists(lens, H, Hk, d, chunk, topk):
+    """The merge of the builder's lists (up to eight places: staged in shared memory) against that of lists the call builds itself, bit
+    for bit: same partials, same order of the sums.  Rows of no sequence (q is longer than its sequences) included."""
+    import flash_moba_b200 as F
+    q, k, v = _inputs(lens, H, Hk, d, seed=len(lens) + topk)
+    pad = torch.randn(3, H, d, device=DEV).bfloat16()
+    q = torch.cat([q, pad])
+    cu, mx = cu_of(lens).to(DEV), max(lens)
+    outs = []
+    for copies in (False, True):
+        x = [t.detach().clone().requires_grad_(True) for t in (q, k, v)]
+        pattern = F.flash_topk_varlen_func(x[0].detach(), x[1].detach(), cu, cu, mx, mx, topk, chunk, causal=True)
+        o = F.flash_moba_attn_varlen_func(*x, cu, cu, mx, mx, *(_copies(pattern) if copies else pattern), 128, chunk, causal=True)
+        outs.append((o,) + torch.autograd.grad(o, x, torch.ones_like(o)))
+    for a, b in zip(*outs):
+        assert torch.isfinite(a).all() and torch.equal(a, b)
