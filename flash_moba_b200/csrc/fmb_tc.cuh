@@ -348,7 +348,7 @@ __device__ __forceinline__ float2 mul_f32x2(float2 a, float2 b) {
   return d;
 }
 
-// ---- 32 bytes (aligned to 32) in one store: a lane that writes a row of its own then fills whole sectors
+// ---- 32 bytes (aligned to 32) in one store: a whole sector
 __device__ __forceinline__ void st_global_32(void* dst, uint4 a, uint4 b) {
   asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(dst), "r"(a.x), "r"(a.y), "r"(a.z), "r"(a.w),
                "r"(b.x), "r"(b.y), "r"(b.z), "r"(b.w)
