@@ -22,9 +22,10 @@
 // 71 / 45; 317K tokens, lists of 16 2.19 / 1.63 ms; 512K x 4 heads, 2,048 columns 1.49 / 0.84 ms.  The scatter with its counts per 32
 // rows laid out column by column (stores of a warp eight to a bank) and 64-bit scans / row group by row group and 32-bit scans:
 // 64K 143 / 129 us, 317K 1.32 / 1.23 ms, 512K 0.80 / 0.71 ms.  Entries stored by the row's thread, lists read behind the scan, a
-// bitonic network per row in the histogram too / in column order, read ahead of it, networks of 19 exchanges and none in the
-// histogram of distinct lists, all three kernels: 64K 158 / 142 us, 32K x 16 39 / 36, d 64, 9K x 12 13.8 / 11.8, 8 x 8K 127 / 127 (of 64 columns; stores
-// by the row's thread 123), 317K 1450 / 1190, 512K 636 / 598.  (Three CTAs per SM with 40 registers: 64K 143, 8 x 8K 117, but 9K x 12 14.8.)
+// bitonic network per row / in column order, read ahead of it, networks of 19 exchanges, all three kernels: 64K 159 / 146 us,
+// 32K x 16 39.5 / 37.3, d 64, 9K x 12 13.8 / 12.5, 8 x 8K 128 / 130 (of 64 columns, where stores by the row's thread are 4 us less), 317K 1460 / 1231, 512K
+// 642 / 607.  (Three CTAs per SM with 40 registers: 64K 1 % more, 8 x 8K 8 % less, but 9K x 12 20 % more.  A histogram that trusts the lists to be distinct would
+// save 3 %; a chunk that is named twice counts once instead.)
 // What bounds it: the scatter's instructions (1,300 a warp of 32 rows before, 60 % issue) and its shared-memory accesses at random columns
 // (65 - 75 % of the wavefronts); HBM 11 - 25 %.  Algorithmic bytes: 4*nnz read + 4*nnz written + 12*B*H*ncol.
 #include <mutex>
@@ -132,15 +133,10 @@ __global__ void __launch_bounds__(kCscThreads) csc_tile_hist_kernel(CscParams p)
     if ((int)threadIdx.x < rows) {
       int id[KMAX];
       csc_load_row<KMAX>(p, src, threadIdx.x, id);
-      if (p.row_slots != nullptr) {                               // (asked for only with lists that name a chunk once)
+      csc_sort<KMAX>(id);
 #pragma unroll
-        for (int j = 0; j < KMAX; ++j) count(id[j]);
-      } else {
-        csc_sort<KMAX>(id);
-#pragma unroll
-        for (int j = 0; j < KMAX; ++j)
-          if (j == 0 || id[j] != id[j > 0 ? j - 1 : 0]) count(id[j]);
-      }
+      for (int j = 0; j < KMAX; ++j)
+        if (j == 0 || id[j] != id[j > 0 ? j - 1 : 0]) count(id[j]);
     }
   } else {
     for (int e = threadIdx.x; e < rows * p.topk; e += kCscThreads) {
