@@ -719,6 +719,7 @@ gate_select_kernel(GateParams p, const __grid_constant__ CUtensorMap map_q, cons
   follow_on();
   constexpr uint32_t kQTile = kGateM * D * 2, kKTile = kSelN * D * 2;
   constexpr int CAP = sel_cap<KMAX>();                   // queue entries per thread
+  constexpr bool kByEight = KMAX == 8;                   // see mask8
   constexpr int STEP = KMAX == 8 ? 8 : 4;                // scores between two looks at the queue's length
   constexpr int OWN = KMAX == 8 ? 6 : 12;                // the long way: candidates of a row that each of its two threads ranks at a time
   extern __shared__ __align__(1024) unsigned char smem_raw[];
@@ -869,9 +870,9 @@ gate_select_kernel(GateParams p, const __grid_constant__ CUtensorMap map_q, cons
       if (!row_ok) nlim = 0;
       const bool own = p.causal && row_ok && pos >= 0 && I.nchunks > 0;
       const int need = topk - (own ? 1 : 0);
-      const int nlim_warp = __reduce_max_sync(0xffffffffu, nlim);
+      const int nlim_warp = __reduce_max_sync(0xffffffffu, nlim), nlim_all = __reduce_min_sync(0xffffffffu, nlim);
 
-      // this thread's 32 scores of score tile s; columns at or past the row's limit read as -inf
+      // this thread's 32 scores of score tile s
       auto fetch = [&](uint32_t n, int s, bool wait, bool release, float (&v)[32]) {
         const int buf = n % kSelBufs;
         if (wait && good) good = mbar_wait(&bar_tfull[buf], (n / kSelBufs) & 1, &g_gate_status, 1);
@@ -886,9 +887,19 @@ gate_select_kernel(GateParams p, const __grid_constant__ CUtensorMap map_q, cons
           if (lane == 0) mbar_arrive(&bar_tfree[buf]);
         }
         const int left = nlim - (s * kSelN + qd * 16);
-        if (__any_sync(0xffffffffu, left < 48)) {
+        if (!kByEight && __any_sync(0xffffffffu, left < 48)) {
 #pragma unroll
           for (int j = 0; j < 32; ++j) v[j] = j + (j & 16) < left ? v[j] : -CUDART_INF_F;
+        }
+      };
+      // Columns at or past a row's limit read as -inf.  Lists of eight: eight columns at a time, those past every row of the warp are left
+      // out, those before every row's limit need no mask (chunks and row tiles mostly end together, so that one group of an
+      // item does).  Lists of 16 mask whole tiles: their code is too long as it is.  Measured, whole tiles / by eight: 8 x 8K tokens x 32 heads
+      // 198.8 / 185.7 us, 32K x 16 83.0 / 82.0, d 64, 9K x 12 23.0 / 22.2, 64K x 32 493.8 / 497.6; lists of 16, 317K 3297 / 3396, 512K x 4 1990 / 2064
+      auto mask8 = [&](float* v, int first) {
+        if (first + 8 > nlim_all) {
+#pragma unroll
+          for (int j = 0; j < 8; ++j) v[j] = first + j < nlim ? v[j] : -CUDART_INF_F;
         }
       };
       // ---- sweep 1: the KMAX largest group maxima of this thread's columns
@@ -903,8 +914,20 @@ gate_select_kernel(GateParams p, const __grid_constant__ CUtensorMap map_q, cons
         for (int s = 0; s < nt; ++s) {
           float v[32];
           fetch(gs + s, s, true, !resident, v);
+          const int nb = s * kSelN + qd * 16;
+          if (!kByEight || nb + 48 <= nlim_all) {
 #pragma unroll
-          for (int j = 0; j < 32; ++j) gm[j % KMAX] = fmaxf(gm[j % KMAX], v[j]);   // (fmaxf drops NaN operands)
+            for (int j = 0; j < 32; ++j) gm[j % KMAX] = fmaxf(gm[j % KMAX], v[j]);   // (fmaxf drops NaN operands)
+          } else {
+#pragma unroll
+            for (int js = 0; js < 32; js += 8) {
+              const int first = nb + js + (js & 16);
+              if (first >= nlim_warp) break;             // warp-uniform
+              mask8(v + js, first);
+#pragma unroll
+              for (int j = js; j < js + 8; ++j) gm[j % KMAX] = fmaxf(gm[j % KMAX], v[j]);
+            }
+          }
           if (++since == period || s + 1 == nt) {
             since = 0;
             sel_sort<KMAX>(gm);
@@ -942,6 +965,7 @@ gate_select_kernel(GateParams p, const __grid_constant__ CUtensorMap map_q, cons
 #pragma unroll
         for (int js = 0; js < 32; js += STEP) {
           if (nb + js + (js & 16) >= nlim_warp) break;   // warp-uniform
+          if (kByEight) mask8(v + js, nb + js + (js & 16));
           if (__any_sync(0xffffffffu, q_next > q_first + (CAP - STEP) * 512)) {
             const int cnt = (q_next - q_first) / 512;
             if (cnt > need) {
