@@ -610,7 +610,7 @@ __global__ void __launch_bounds__(128 * NQ) gate_topk_tc_kernel(GateParams p) {
 //            two lists and writes the row's.  Neighbours that agree in those 26 bits are compared exactly and exchanged; where
 //            more than two agree, or the last place and what was dropped (masses of equal scores), the pair of warps
 //            takes the long way: a candidate's place is the number of the row's candidates ahead of it, counted by comparing
-//            all with all.
+//            all with all (out of line: with that code in the kernel 64K tokens took 495 instead of 471 us, lists of 16 3 % more).
 // The score tiles of sweep 2 are those of sweep 1, still in TMEM, for up to 256 candidates; beyond that the
 // products are computed again (the tensor pipe is idle otherwise).  A queue that runs full (masses of
 // equal scores) is cut down to its k best, the last of which then is the floor.
@@ -620,10 +620,11 @@ __global__ void __launch_bounds__(128 * NQ) gate_topk_tc_kernel(GateParams p) {
 // thread for loads and MMAs a centroid tile was requested only when the MMAs before it had been issued, one tile in flight at a
 // time: 1 us a step, which is what long sequences took (64K tokens, 32 heads 605 / 549 us with one / two warps).
 // Measured (B200, d 128; the kernel above / two sweeps, all compared with all / sorted keys): 64K tokens, 32 heads, chunk 128, top-k 8
-// 1020 / 605 / 492 us; 8 x 8K tokens 580 / 256 / 198; 32K tokens, 16 heads 185 / 97 / 83; 317K tokens in 16 sequences, chunk 64, top-k 16
-// 7400 / 3430 / 3290; 512K tokens, 4 heads, chunk 256, top-k 16 - / 2106 / 1982; d 64, 9K tokens, 12 heads, no mask - / 31 / 23.
-// What bounds it now: instructions at 60 % issue (32K tokens: 1,600 a warp and row tile; the min / max pipe is busy for 58 %), at
-// 64K also the MMAs (128 x 64 x 16: 52 cycles, of which A's and B's way from shared memory takes 48).
+// 1020 / 605 / 471 us; 8 x 8K tokens 580 / 256 / 178; 32K tokens, 16 heads 185 / 97 / 78; 317K tokens in 16 sequences, chunk 64, top-k 16
+// 7400 / 3430 / 3206; 512K tokens, 4 heads, chunk 256, top-k 16 - / 2106 / 1965; d 64, 9K tokens, 12 heads, no mask - / 31 / 22.  (All scores
+// equal, the long way throughout: 16K tokens, 8 heads 84 / 91 us, top-k 16 197 / 229.)
+// What bounds it now: instructions at 60 % issue (32K tokens: 1,900 a warp and row tile before, 1,600 with sorted keys; the min / max pipe is busy
+// for 58 %), fetching them where lists are of 16, at 64K also the MMAs (128 x 64 x 16: 52 cycles, of which A's and B's way from shared memory takes 48).
 // ---------------------------------------------------------------------------------------
 constexpr int kSelN = 64;            // centroids per score tile
 constexpr int kSelBufs = 4;          // score tiles in TMEM
@@ -695,6 +696,45 @@ __device__ __noinline__ void sel_compact(float2* queue, int cnt, int keep) {
   }
 }
 
+// A row's list by exact comparisons of all candidates with all: the place of a candidate is the number of those ahead of it.  The queues of the
+// row's two threads start at `queue` and 32 entries behind it, c0 and c - c0 entries; a thread ranks every second candidate from `first` on and
+// writes what is among the first `topk`.  By whole warps; rare and long like sel_compact, so that the kernel's own code stays small (inlined: see
+// gate_select_kernel).
+constexpr int kSelOwn = 6;
+__device__ __noinline__ void sel_rank_all(const float2* queue, int c0, int c, int first, int places, int topk, int32_t* out, float* val) {
+  const int most = __reduce_max_sync(0xffffffffu, c);
+#pragma unroll 1
+  for (; first < most; first += 2 * kSelOwn) {
+    uint64_t key[kSelOwn];
+    int rank[kSelOwn];
+#pragma unroll
+    for (int m = 0; m < kSelOwn; ++m) {
+      const int i = first + 2 * m;
+      rank[m] = topk;
+      key[m] = ~0ull;
+      if (i < c) {
+        key[m] = sel_key(queue[i < c0 ? i * 64 : (i - c0) * 64 + 32]);
+        rank[m] = places;
+      }
+    }
+    const float2* at = queue;
+    for (int i = 0; i < most; ++i) {
+      if (i == c0) at = queue + 32;
+      const uint64_t k = i < c ? sel_key(*at) : 0ull;
+      at += 64;
+#pragma unroll
+      for (int m = 0; m < kSelOwn; ++m) rank[m] += k > key[m] ? 1 : 0;
+    }
+#pragma unroll
+    for (int m = 0; m < kSelOwn; ++m) {
+      if (rank[m] < topk) {
+        out[rank[m]] = (int)(uint32_t)key[m];
+        if (val) val[rank[m]] = ordered_to_score((uint32_t)(key[m] >> 32));
+      }
+    }
+  }
+}
+
 // n / d for 0 <= n < 2^31: one multiplication with a reciprocal from the host, rounded up, which is exact
 // for these n (d = 1 is its own case)
 struct FastDiv {
@@ -721,7 +761,6 @@ gate_select_kernel(GateParams p, const __grid_constant__ CUtensorMap map_q, cons
   constexpr int CAP = sel_cap<KMAX>();                   // queue entries per thread
   constexpr bool kByEight = KMAX == 8;                   // see mask8
   constexpr int STEP = KMAX == 8 ? 8 : 4;                // scores between two looks at the queue's length
-  constexpr int OWN = KMAX == 8 ? 6 : 12;                // the long way: candidates of a row that each of its two threads ranks at a time
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   __shared__ uint64_t bar_q, bar_qfree, bar_kfull[kSelRing], bar_kfree[kSelRing], bar_tfull[kSelBufs], bar_tfree[kSelBufs];
   __shared__ uint32_t tmem_base_s;
@@ -1088,70 +1127,20 @@ gate_select_kernel(GateParams p, const __grid_constant__ CUtensorMap map_q, cons
       if (bar_and(pair, 64, good && !close)) continue;   // the pair goes on, or leaves, together; its areas are free
       good = bar_and(pair, 64, good);
       if (!good) break;
-      // ---- the list, long way: exact comparisons of all with all
+      // ---- the list, long way
       {
-        // ---- ranks: this thread takes every second one of the row's candidates
-        const int other = sCount[tid ^ 128];
-        const float2* q_lo = reinterpret_cast<const float2*>(mine) + lane;
-        const int c0 = qd == 0 ? cnt : other, c = cnt + other;
-        const int most = __reduce_max_sync(0xffffffffu, c);      // (the same for both warps of the pair)
-        const bool staged = most <= 2 * OWN && p.t_rs == topk;   // one round, and the pair's lists are contiguous in memory
-        int* sOut = reinterpret_cast<int*>(mine) + lane * topk;
+        const int other = sCount[tid ^ 128], c = cnt + other;
         const int64_t row_at = (int64_t)(I.q0 + I.r0 + lt) * p.t_rs + (int64_t)I.h * p.t_hs;
-        int* out = staged ? sOut : p.topk_idx + row_at;
         float* val = p.topk_val ? p.topk_val + row_at : nullptr;
-#pragma unroll 1
-        for (int first = qd; first < most; first += 2 * OWN) {
-          uint64_t key[OWN];
-          int rank[OWN];
-#pragma unroll
-          for (int m = 0; m < OWN; ++m) {
-            const int i = first + 2 * m;
-            rank[m] = topk;
-            key[m] = ~0ull;
-            if (i < c) {
-              key[m] = sel_key(q_lo[i < c0 ? i * 64 : (i - c0) * 64 + 32]);
-              rank[m] = own ? 1 : 0;
-            }
-          }
-          const float2* at = q_lo;
-          for (int i = 0; i < most; ++i) {
-            if (i == c0) at = q_lo + 32;
-            const uint64_t k = i < c ? sel_key(*at) : 0ull;
-            at += 64;
-#pragma unroll
-            for (int m = 0; m < OWN; ++m) rank[m] += k > key[m] ? 1 : 0;
-          }
-          if (staged) bar_sync(pair, 64);                // both have read the queues: their place takes the lists
-#pragma unroll
-          for (int m = 0; m < OWN; ++m) {
-            if (rank[m] < topk) {
-              out[rank[m]] = (int)(uint32_t)key[m];
-              if (val) val[rank[m]] = ordered_to_score((uint32_t)(key[m] >> 32));
-            }
-          }
-        }
-        if (staged && qd >= most) bar_sync(pair, 64);    // (most is 0, or 1 for the second thread: no round above)
+        sel_rank_all(reinterpret_cast<const float2*>(mine) + lane, qd == 0 ? cnt : other, c, qd, first_place, topk, p.topk_idx + row_at, val);
         if (qd == 0 && row_ok) {                         // the row's own chunk first, nothing after the last candidate
           if (own) {
-            out[0] = pos_chunk;
+            p.topk_idx[row_at] = pos_chunk;
             if (val) val[0] = CUDART_INF_F;
           }
-          for (int j = c + (own ? 1 : 0); j < topk; ++j) {
-            out[j] = -1;
+          for (int j = c + first_place; j < topk; ++j) {
+            p.topk_idx[row_at + j] = -1;
             if (val) val[j] = -CUDART_INF_F;
-          }
-        }
-        if (staged) {
-          bar_sync(pair, 64);                            // the pair's 32 lists are complete
-          const int first = (warp & 3) * 32, n_out = max(0, min(32, I.rows - first)) * topk;
-          int32_t* dst = p.topk_idx + (int64_t)(I.q0 + I.r0 + first) * p.t_rs + (int64_t)I.h * p.t_hs;
-          const int* src = reinterpret_cast<const int*>(mine);
-          if ((topk & 3) == 0 && (reinterpret_cast<uintptr_t>(dst) & 15) == 0) {
-            for (int i = qd * 32 + lane; i < n_out / 4; i += 64)
-              reinterpret_cast<int4*>(dst)[i] = reinterpret_cast<const int4*>(src)[i];
-          } else {
-            for (int i = qd * 32 + lane; i < n_out; i += 64) dst[i] = src[i];
           }
         }
       }
