@@ -621,8 +621,8 @@ __global__ void __launch_bounds__(128 * NQ) gate_topk_tc_kernel(GateParams p) {
 // time: 1 us a step, which is what long sequences took (64K tokens, 32 heads 605 / 549 us with one / two warps).
 // Measured (B200, d 128; the kernel above / two sweeps, all compared with all / sorted keys): 64K tokens, 32 heads, chunk 128, top-k 8
 // 1020 / 605 / 471 us; 8 x 8K tokens 580 / 256 / 178; 32K tokens, 16 heads 185 / 97 / 78; 317K tokens in 16 sequences, chunk 64, top-k 16
-// 7400 / 3430 / 3206; 512K tokens, 4 heads, chunk 256, top-k 16 - / 2106 / 1965; d 64, 9K tokens, 12 heads, no mask - / 31 / 22.  (All scores
-// equal, the long way throughout: 16K tokens, 8 heads 84 / 91 us, top-k 16 197 / 229.)
+// 7400 / 3430 / 2946; 512K tokens, 4 heads, chunk 256, top-k 16 - / 2106 / 1850; d 64, 9K tokens, 12 heads, no mask - / 31 / 22.  (All scores
+// equal, the long way throughout: 16K tokens, 8 heads 84 / 91 us, top-k 16 198 / 221.)
 // What bounds it now: instructions at 60 % issue (32K tokens: 1,900 a warp and row tile before, 1,600 with sorted keys; the min / max pipe is busy
 // for 58 %), fetching them where lists are of 16, at 64K also the MMAs (128 x 64 x 16: 52 cycles, of which A's and B's way from shared memory takes 48).
 // ---------------------------------------------------------------------------------------
@@ -696,6 +696,25 @@ __device__ __noinline__ void sel_compact(float2* queue, int cnt, int keep) {
   }
 }
 
+// Four scores, of columns col ... col + 3, for a thread's queue of `cnt` of `cap` entries, for warps in which four more may be too many for
+// some thread: one score at a time, queues cut down (as above) whenever one of the warp is full.  Returns entries and floor.  (Cut down inside the
+// kernel, as lists of eight are: 317K tokens, lists of 16 3210 us, this way 2946; 512K 1963 / 1850: less code to fetch.)
+__device__ __noinline__ float2 sel_append4(float2* queue, int cnt, int cap, int keep, float thr, float4 v, int col) {
+  for (int j = 0; j < 4; ++j) {
+    if (__any_sync(0xffffffffu, cnt == cap)) {
+      if (cnt > keep) {
+        sel_compact(queue, cnt, keep);
+        cnt = keep;
+        thr = fmaxf(thr, queue[(keep - 1) * 64].x);
+      }
+      __syncwarp();
+    }
+    if (v.x >= thr) queue[cnt++ * 64] = make_float2(v.x, __int_as_float(col + j));
+    v = make_float4(v.y, v.z, v.w, v.x);
+  }
+  return make_float2(__int_as_float(cnt), thr);
+}
+
 // A row's list by exact comparisons of all candidates with all: the place of a candidate is the number of those ahead of it.  The queues of the
 // row's two threads start at `queue` and 32 entries behind it, c0 and c - c0 entries; a thread ranks every second candidate from `first` on and
 // writes what is among the first `topk`.  By whole warps; rare and long like sel_compact, so that the kernel's own code stays small (inlined: see
@@ -745,9 +764,12 @@ __device__ __forceinline__ int fast_div(int n, const FastDiv& f) {
 }
 
 // Queue entries per thread: what two CTAs per SM leave room for.  A row has some 9 (k = 8) or 19 (k = 16)
-// candidates, a thread half of them on average; more than 12 or 15 in one thread's queue are rare (with room
-// for 16 the queues of k = 8 ran full all the time: 0.82 ms instead of 0.65 at 64K).
+// candidates, a thread half of them on average; more than 12 or 15 in one thread's queue are rare where scores are independent (with
+// room for 16 the queues of k = 8 ran full all the time: 0.82 ms instead of 0.65 at 64K), not where neighbouring chunks score alike or equal.
 template <int KMAX> __host__ __device__ constexpr int sel_cap() { return KMAX == 8 ? 20 : 19; }
+// Scores between two looks at the queues' lengths, after which no queue has more than CAP - STEP entries, or `need` of them where that is more.  A
+// full list of 16 and four scores do not fit: sel_append4.
+template <int KMAX> __host__ __device__ constexpr int sel_step() { return KMAX == 8 ? 8 : 4; }
 
 constexpr int kSelSeqs = 64;         // sequences whose bounds are kept in shared memory
 
@@ -760,7 +782,9 @@ gate_select_kernel(GateParams p, const __grid_constant__ CUtensorMap map_q, cons
   constexpr uint32_t kQTile = kGateM * D * 2, kKTile = kSelN * D * 2;
   constexpr int CAP = sel_cap<KMAX>();                   // queue entries per thread
   constexpr bool kByEight = KMAX == 8;                   // see mask8
-  constexpr int STEP = KMAX == 8 ? 8 : 4;                // scores between two looks at the queue's length
+  constexpr int STEP = sel_step<KMAX>();                 // scores between two looks at the queue's length
+  constexpr bool kOneByOne = KMAX + STEP > CAP;          // a queue that has been cut has no room for a step's scores
+  static_assert(KMAX < CAP && CAP <= 32 && (!kOneByOne || STEP == 4), "a queue that has been cut has room; places have five bits; sel_append4");
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   __shared__ uint64_t bar_q, bar_qfree, bar_kfull[kSelRing], bar_kfree[kSelRing], bar_tfull[kSelBufs], bar_tfree[kSelBufs];
   __shared__ uint32_t tmem_base_s;
@@ -1007,6 +1031,12 @@ gate_select_kernel(GateParams p, const __grid_constant__ CUtensorMap map_q, cons
           if (kByEight) mask8(v + js, nb + js + (js & 16));
           if (__any_sync(0xffffffffu, q_next > q_first + (CAP - STEP) * 512)) {
             const int cnt = (q_next - q_first) / 512;
+            if constexpr (kOneByOne) {
+              const float2 x = sel_append4(queue, cnt, CAP, need, thr, make_float4(v[js], v[js + 1], v[js + 2], v[js + 3]), nb + js + (js & 16));
+              q_next = q_first + __float_as_int(x.x) * 512;
+              thr = x.y;
+              continue;
+            }
             if (cnt > need) {
               sel_compact(queue, cnt, need);
               q_next = q_first + need * 512;
@@ -1039,7 +1069,7 @@ gate_select_kernel(GateParams p, const __grid_constant__ CUtensorMap map_q, cons
       }
       sel_sort<KMAX>(key);
       for (int j = KMAX; __any_sync(0xffffffffu, j < cnt); ++j) {
-        const uint32_t k = (score_to_ordered(queue[min(j, CAP - 1) * 64].x) & ~63u) | (uint32_t)(qd * 32 + j);
+        const uint32_t k = (score_to_ordered(queue[j * 64].x) & ~63u) | (uint32_t)(qd * 32 + j);
         uint32_t x = j < cnt ? k : 0u;
 #pragma unroll
         for (int i = 0; i < KMAX; ++i) sel_ce(key[i], x);

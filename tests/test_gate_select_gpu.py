@@ -67,3 +67,46 @@ def test_scores_that_differ_in_their_last_bits(topk, causal, n_values):
                              return_values=True)
     ref_idx, ref_val = O.gate_topk(q, km, cq, ck, ck, topk, 1, causal)
     assert torch.equal(idx.cpu(), ref_idx) and torch.equal(val.cpu(), ref_val)
+
+
+def _scores(kind, n, rng):
+    """Integer scores of n candidates, exact in bf16."""
+    if kind == "equal":
+        return torch.full((n,), 3.0)
+    if kind == "ascending":                          # block by block of 16
+        return (torch.arange(n) // 16).float()
+    if kind == "smooth":                             # neighbouring chunks score alike, few values
+        return torch.randint(-1, 2, (n,), generator=rng).cumsum(0).clamp(-200, 200).float()
+    assert kind == "one share"                       # the best are all in the columns of one of a row's two threads
+    best = torch.arange(n) % 32 < 16
+    return torch.where(best, torch.randint(60, 64, (n,), generator=rng), torch.randint(0, 50, (n,), generator=rng)).float()
+
+
+@pytest.mark.parametrize("kind", ["equal", "ascending", "smooth", "one share"])
+@pytest.mark.parametrize("d,topk,causal,lens_k", [
+    (128, 16, False, [36, 700]), (64, 16, False, [65, 256]), (256, 16, False, [257, 300]),
+    (128, 16, False, [600, 320]), (128, 15, False, [129, 420]), (128, 16, True, [700, 300]),
+    (128, 8, False, [40, 610]), (64, 8, True, [300, 200]), (128, 9, False, [500, 64]),
+])
+def test_queues_that_run_full(kind, d, topk, causal, lens_k):
+    """More candidates than a queue has room for, in row tiles whose 128 rows all have some, so that every warp pair's queues are in use:
+    zero and repeated keys, padding rows, scores that are smooth from chunk to chunk.  The lists are the oracle's, each time."""
+    from flash_moba_b200 import ops
+    g = torch.Generator().manual_seed(d + topk + lens_k[0])
+    lens_q, H, Hk = [200, 130], 4, 2
+    q = torch.zeros(sum(lens_q), H, d)
+    q[..., 3] = torch.randint(0, 2, (sum(lens_q), H), generator=g).float() * 2 - 1      # the scores, or their negatives
+    q[torch.rand(sum(lens_q), generator=g) < 0.2] = 0.0                                 # rows without any preference
+    km = torch.zeros(sum(lens_k), Hk, d)
+    at = 0
+    for n in lens_k:
+        for h in range(Hk):
+            km[at:at + n, h, 3] = _scores(kind, n, g)
+        at += n
+    q, km = q.bfloat16(), km.bfloat16()
+    cq, ck = cu_of(lens_q), cu_of(lens_k)
+    ref_idx, ref_val = O.gate_topk(q, km, cq, ck, ck, topk, 1, causal)
+    for _ in range(3):
+        idx, val = ops.gate_topk(q.to(DEV), km.to(DEV), cq.to(DEV), ck.to(DEV), ck.to(DEV), max(lens_q), max(lens_k), topk, 1, causal,
+                                 return_values=True)
+        assert torch.equal(idx.cpu(), ref_idx) and torch.equal(val.cpu(), ref_val)
