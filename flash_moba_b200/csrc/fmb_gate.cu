@@ -772,6 +772,7 @@ template <int KMAX> __host__ __device__ constexpr int sel_cap() { return KMAX ==
 template <int KMAX> __host__ __device__ constexpr int sel_step() { return KMAX == 8 ? 8 : 4; }
 
 constexpr int kSelSeqs = 64;         // sequences whose bounds are kept in shared memory
+constexpr size_t kSelStatic = 1280;  // at least what the kernel declares in static shared memory
 
 template <typename T, int D, int KMAX>
 __global__ void __launch_bounds__(kSelThreads, D <= 128 ? 2 : 1)
@@ -785,17 +786,13 @@ gate_select_kernel(GateParams p, const __grid_constant__ CUtensorMap map_q, cons
   constexpr int STEP = sel_step<KMAX>();                 // scores between two looks at the queue's length
   constexpr bool kOneByOne = KMAX + STEP > CAP;          // a queue that has been cut has no room for a step's scores
   static_assert(KMAX < CAP && CAP <= 32 && (!kOneByOne || STEP == 4), "a queue that has been cut has room; places have five bits; sel_append4");
-  extern __shared__ __align__(1024) unsigned char smem_raw[];
+  extern __shared__ unsigned char smem_raw[];
   __shared__ uint64_t bar_q, bar_qfree, bar_kfull[kSelRing], bar_kfree[kSelRing], bar_tfull[kSelBufs], bar_tfree[kSelBufs];
   __shared__ uint32_t tmem_base_s;
   __shared__ uint8_t sCount[256];
   __shared__ int sCu[3][kSelSeqs + 1];
-  // (no room for padding: the base is aligned as declared, checked here)
-  if ((smem_u32(smem_raw) & 1023u) != 0) {
-    if (threadIdx.x == 0) atomicCAS(&g_gate_status, 0, 9);
-    return;
-  }
-  unsigned char* sQ = smem_raw;
+  static_assert((2 + 2 * kSelRing + 2 * kSelBufs) * 8 + 4 + sizeof(sCount) + sizeof(sCu) + 64 <= kSelStatic, "see gate_select_launch");
+  unsigned char* sQ = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
   unsigned char* sKM = sQ + kQTile;
   unsigned char* sQueue = sKM + kSelRing * kKTile;       // per warp pair [CAP][64] (score, chunk); also the pair's exchange area
   uint32_t* sKeys = reinterpret_cast<uint32_t*>(sQueue + CAP * 256 * 8);   // per warp pair [KMAX + 1][32] sorted keys of the rows' second threads
@@ -1221,7 +1218,8 @@ static int gate_tc_pick(const GateParams& p, int batch, int max_q, cudaStream_t 
 template <typename T, int D, int KMAX>
 static int gate_select_launch(const GateParams& p, const CUtensorMap& mq, const CUtensorMap& mk, int batch, int max_q, cudaStream_t s) {
   constexpr int kCap = sel_cap<KMAX>();
-  const size_t smem = (size_t)kGateM * D * 2 + (size_t)kSelRing * kSelN * D * 2 + (size_t)kCap * 256 * 8 + (size_t)4 * (KMAX + 1) * 32 * 4;
+  constexpr size_t smem = 1024 + (size_t)kGateM * D * 2 + (size_t)kSelRing * kSelN * D * 2 + (size_t)kCap * 256 * 8 + (size_t)4 * (KMAX + 1) * 32 * 4;
+  static_assert(D > 128 || 2 * (smem + kSelStatic + 1024) <= 228 * 1024, "two CTAs per SM, each with 1 KB that the system takes");
   static_assert(2 * KMAX * 32 * 4 <= kCap * 64 * 8, "a pair's exchange area fits its queues");
   auto divider = [](int d) {
     FastDiv fd{0, 0, (uint32_t)d};

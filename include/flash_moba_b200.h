@@ -282,7 +282,7 @@ int fmb_gate_engine(int head_dim, int topk);
 
 /* Synchronising read of the gating kernel's device-side status word of the current device into
  * *host_status: 0 = ok, non-zero = a bounded wait expired in some gating launch since the last
- * read (9: the kernel's shared memory was not aligned as declared and nothing was written).  The word is cleared by the read.  Returns FMB_ERR_TIMEOUT when it was non-zero. */
+ * read.  The word is cleared by the read.  Returns FMB_ERR_TIMEOUT when it was non-zero. */
 int fmb_gate_status(int* host_status);
 
 /* Synchronising read of the status word that fmb_attn_fwd / fmb_attn_bwd left in the first 4

@@ -46,3 +46,11 @@ def test_no_queue_outgrows_its_room(kmax):
                 cut = [s[:quiet] + [0] * (-quiet % step) + s[quiet:] for s in streams]
                 cut = [s[:len(s) // step * step] for s in cut]
                 assert _longest(cut, cap, step, need, one_by_one) <= cap, (need, density, quiet)
+
+
+def test_every_cta_writes_its_lists():
+    """The lists' memory is not initialised, and the status word is read on request only: a CTA that leaves before it has written
+    its lists would hand what the memory held before to the pattern builder."""
+    code = re.sub(r"//[^\n]*", "", SOURCE[SOURCE.index("\ngate_select_kernel(GateParams p"):])
+    code = code[:code.index("tmem_dealloc(")]
+    assert re.findall(r"\breturn\b *;", code) == []
