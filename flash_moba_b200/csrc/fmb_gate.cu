@@ -621,8 +621,9 @@ __global__ void __launch_bounds__(128 * NQ) gate_topk_tc_kernel(GateParams p) {
 // time: 1 us a step, which is what long sequences took (64K tokens, 32 heads 605 / 549 us with one / two warps).
 // Measured (B200, d 128; the kernel above / two sweeps, all compared with all / sorted keys): 64K tokens, 32 heads, chunk 128, top-k 8
 // 1020 / 605 / 471 us; 8 x 8K tokens 580 / 256 / 178; 32K tokens, 16 heads 185 / 97 / 78; 317K tokens in 16 sequences, chunk 64, top-k 16
-// 7400 / 3430 / 2946; 512K tokens, 4 heads, chunk 256, top-k 16 - / 2106 / 1850; d 64, 9K tokens, 12 heads, no mask - / 31 / 22.  (All scores
-// equal, the long way throughout: 16K tokens, 8 heads 84 / 91 us, top-k 16 198 / 221.)
+// 7400 / 3430 / 2914; 512K tokens, 4 heads, chunk 256, top-k 16 - / 2106 / 1821; d 64, 9K tokens, 12 heads, no mask - / 31 / 22.  All scores
+// equal, the long way throughout: 16K tokens, 8 heads 84 / 88 us, top-k 16 198 / 130; no mask 161 / 166 and 440 / 247.  Scores that are smooth from chunk
+// to chunk (correlation 0.95): 32K tokens, 16 heads 111 / 92, chunk 64, top-k 16 304 / 293, no mask 512 / 447.
 // What bounds it now: instructions at 60 % issue (32K tokens: 1,900 a warp and row tile before, 1,600 with sorted keys; the min / max pipe is busy
 // for 58 %), fetching them where lists are of 16, at 64K also the MMAs (128 x 64 x 16: 52 cycles, of which A's and B's way from shared memory takes 48).
 // ---------------------------------------------------------------------------------------
@@ -684,15 +685,36 @@ __device__ __forceinline__ uint64_t sel_key(float2 c) { return ((uint64_t)score_
 // kept out of line.
 __device__ __noinline__ void sel_compact(float2* queue, int cnt, int keep) {
   for (int i = 0; i < keep; ++i) {
+    float2 x = queue[i * 64];
+    const float2 first = x;
     int best = i;
-    uint64_t kb = sel_key(queue[i * 64]);
+    uint64_t kb = sel_key(x);
+#pragma unroll 4
     for (int j = i + 1; j < cnt; ++j) {
-      const uint64_t kj = sel_key(queue[j * 64]);
-      if (kj > kb) { kb = kj; best = j; }
+      const float2 y = queue[j * 64];
+      const uint64_t kj = sel_key(y);
+      if (kj > kb) { kb = kj; best = j; x = y; }
     }
-    const float2 x = queue[i * 64];
-    queue[i * 64] = queue[best * 64];
-    queue[best * 64] = x;
+    queue[i * 64] = x;
+    queue[best * 64] = first;
+  }
+}
+// The same for lists of 16, of which few have to go: the worst are taken out one by one; returns the score of the worst that stays.  (16K tokens,
+// 8 heads, top-k 16, no mask, all scores equal, the best put in order / the worst taken out: 561 / 252 us.  Lists of eight, where more have to go
+// than stay, 91 / 104.)
+__device__ __noinline__ float sel_cut(float2* queue, int cnt, int keep) {
+  for (;; --cnt) {
+    int worst = 0;
+    float2 w = queue[0];
+    uint64_t kw = sel_key(w);
+#pragma unroll 4
+    for (int j = 1; j < cnt; ++j) {
+      const float2 x = queue[j * 64];
+      const uint64_t kj = sel_key(x);
+      if (kj < kw) { kw = kj; worst = j; w = x; }
+    }
+    if (cnt <= keep) return w.x;
+    queue[worst * 64] = queue[(cnt - 1) * 64];
   }
 }
 
@@ -703,9 +725,8 @@ __device__ __noinline__ float2 sel_append4(float2* queue, int cnt, int cap, int 
   for (int j = 0; j < 4; ++j) {
     if (__any_sync(0xffffffffu, cnt == cap)) {
       if (cnt > keep) {
-        sel_compact(queue, cnt, keep);
+        thr = fmaxf(thr, sel_cut(queue, cnt, keep));
         cnt = keep;
-        thr = fmaxf(thr, queue[(keep - 1) * 64].x);
       }
       __syncwarp();
     }
@@ -719,7 +740,7 @@ __device__ __noinline__ float2 sel_append4(float2* queue, int cnt, int cap, int 
 // row's two threads start at `queue` and 32 entries behind it, c0 and c - c0 entries; a thread ranks every second candidate from `first` on and
 // writes what is among the first `topk`.  By whole warps; rare and long like sel_compact, so that the kernel's own code stays small (inlined: see
 // gate_select_kernel).
-constexpr int kSelOwn = 6;
+constexpr int kSelOwn = 8;
 __device__ __noinline__ void sel_rank_all(const float2* queue, int c0, int c, int first, int places, int topk, int32_t* out, float* val) {
   const int most = __reduce_max_sync(0xffffffffu, c);
 #pragma unroll 1
