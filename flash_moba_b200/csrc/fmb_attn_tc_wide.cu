@@ -237,7 +237,6 @@ __global__ void __launch_bounds__(kFwThreads, 1) fwd_wide_tc_kernel(WideParams p
   } else if (warp >= kFwDrainWarp) {
     // =============================================================== drain warps
     const uint32_t at = (uint32_t)((warp & 3) * 32) << 16;
-    const int lt = tid & (kM - 1);
     T* part_o = static_cast<T*>(p.part_o);
     bool good = true;
     uint32_t g = 0;
@@ -550,7 +549,6 @@ __global__ void __launch_bounds__(kBwThreads, 1) bwd_wide_tc_kernel(WideParams p
     // =============================================================== drain warps
     reg_dec<kBwRegsOther>();
     const uint32_t at = (uint32_t)((warp & 3) * 32) << 16;
-    const int lt = tid & (kM - 1);
     bool good = true;
     uint32_t g = 0;
 #pragma unroll 1

@@ -169,7 +169,6 @@ __global__ void __launch_bounds__(kGateThreads) gate_topk_kernel(GateParams p) {
   const int rows = min(kGateM, len_q - r0);
   const int hk = h / (p.heads / p.heads_k);
   const int shift = len_k - len_q;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int topk = p.topk;
 
   // initial lists: empty, or the row's own chunk pinned at rank 0 under the causal rule

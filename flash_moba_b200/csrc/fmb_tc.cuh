@@ -369,15 +369,9 @@ __device__ __forceinline__ void store_part(T* dst, const float* o, float f) {
   st_global_32(dst, pack8<T>(x), pack8<T>(x + 8));
 }
 
-// ---- bulk (TMA, non-tensor) shared -> global stores -----------------------------------
-// 16-byte aligned addresses, size a multiple of 16.  The issuing thread commits its copies
-// as a group and must wait for the group's READS before the shared-memory source is reused
-// (or the CTA exits).
-__device__ __forceinline__ void bulk_store(void* gdst, const void* ssrc, uint32_t bytes) {
-  asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(gdst), "r"(smem_u32(ssrc)),
-               "r"(bytes)
-               : "memory");
-}
+// ---- groups of TMA shared -> global stores ---------------------------------------------
+// The issuing thread commits its stores as a group and must wait for the group's READS before the
+// shared-memory source is reused (or the CTA exits).
 __device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
 __device__ __forceinline__ void bulk_wait_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
 
