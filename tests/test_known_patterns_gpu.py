@@ -154,15 +154,17 @@ def test_checkpointed_layers():
 
 @pytest.mark.parametrize("lens,H,Hk,d,chunk,topk", [
     ([1], 3, 1, 128, 128, 1),                     # three rows of one place in all: most warps have none
-    ([5, 0, 2], 300, 300, 128, 64, 8),            # a warp's next row is many heads further
+    ([5, 0, 2], 2400, 2400, 128, 64, 8),          # a warp's next row is hundreds of heads further, three turns of 148 SMs
+    ([70, 0, 201], 300, 300, 128, 64, 8),         # eleven turns, rows of one to four places
     ([517], 8, 2, 256, 128, 7),
     ([130, 259], 6, 6, 128, 128, 8),
     ([400], 4, 4, 128, 256, 4),                   # two planes: not staged
     ([300], 4, 4, 128, 64, 9),                    # nine places: not staged
 ])
 def test_rows_merged_from_their_own_lists(lens, H, Hk, d, chunk, topk):
-    """The merge of the builder's lists (up to eight places: staged in shared memory) against that of lists the call builds itself, bit
-    for bit: same partials, same order of the sums.  Rows of no sequence (q is longer than its sequences) included."""
+    """The merge of the builder's lists (up to eight places: O staged in shared memory, dQ not for so few partials) against that of
+    lists the call builds itself, bit for bit: same partials, same order of the sums.  Rows of no sequence (q is longer than its
+    sequences) included."""
     import flash_moba_b200 as F
     q, k, v = _inputs(lens, H, Hk, d, seed=len(lens) + topk)
     pad = torch.randn(3, H, d, device=DEV).bfloat16()
@@ -173,6 +175,28 @@ def test_rows_merged_from_their_own_lists(lens, H, Hk, d, chunk, topk):
         x = [t.detach().clone().requires_grad_(True) for t in (q, k, v)]
         pattern = F.flash_topk_varlen_func(x[0].detach(), x[1].detach(), cu, cu, mx, mx, topk, chunk, causal=True)
         o = F.flash_moba_attn_varlen_func(*x, cu, cu, mx, mx, *(_copies(pattern) if copies else pattern), 128, chunk, causal=True)
+        outs.append((o,) + torch.autograd.grad(o, x, torch.ones_like(o)))
+    for a, b in zip(*outs):
+        assert torch.isfinite(a).all() and torch.equal(a, b)
+
+
+@pytest.mark.parametrize("lens,H,Hk,d,topk", [
+    ([8189], 32, 8, 128, 8),                      # the fewest partials whose dQ is staged: 512 MiB, three rows of no sequence
+    ([2500, 1, 4099, 2000], 32, 8, 128, 8),
+    ([4701], 32, 4, 256, 7),
+])
+def test_dq_merged_from_its_own_lists(lens, H, Hk, d, topk):
+    """As above where there are enough partials for dQ's merge to be staged too."""
+    import flash_moba_b200 as F
+    assert (sum(lens) + 3) * H * topk * d * 2 >= 1 << 29
+    q, k, v = _inputs(lens, H, Hk, d, seed=d)
+    q = torch.cat([q, torch.randn(3, H, d, device=DEV).bfloat16()])
+    cu, mx = cu_of(lens).to(DEV), max(lens)
+    outs = []
+    for copies in (False, True):
+        x = [t.detach().clone().requires_grad_(True) for t in (q, k, v)]
+        pattern = F.flash_topk_varlen_func(x[0].detach(), x[1].detach(), cu, cu, mx, mx, topk, 128, causal=True)
+        o = F.flash_moba_attn_varlen_func(*x, cu, cu, mx, mx, *(_copies(pattern) if copies else pattern), 128, 128, causal=True)
         outs.append((o,) + torch.autograd.grad(o, x, torch.ones_like(o)))
     for a, b in zip(*outs):
         assert torch.isfinite(a).all() and torch.equal(a, b)
