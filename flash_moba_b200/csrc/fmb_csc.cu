@@ -23,8 +23,7 @@
 // rows laid out column by column (stores of a warp eight to a bank) and 64-bit scans / row group by row group and 32-bit scans:
 // 64K 143 / 129 us, 317K 1.32 / 1.23 ms, 512K 0.80 / 0.71 ms.  Entries stored by the row's thread, lists read behind the scan, a
 // bitonic network per row / in column order, read ahead of it, networks of 19 exchanges, all three kernels: 64K 159 / 146 us,
-// 32K x 16 39.5 / 37.3, d 64, 9K x 12 13.8 / 12.5, 8 x 8K 128 / 130 (of 64 columns, where stores by the row's thread are 4 us less), 317K 1460 / 1231, 512K
-// 642 / 607.  (Three CTAs per SM with 40 registers: 64K 1 % more, 8 x 8K 8 % less, but 9K x 12 20 % more.  A histogram that trusts the lists to be distinct would
+// 32K x 16 39.5 / 37.3, d 64, 9K x 12 13.8 / 12.5, 8 x 8K 128 / 130, 317K 1460 / 1231, 512K 642 / 607.  (Three CTAs per SM with 40 registers: 64K 1 % more, 8 x 8K 8 % less, but 9K x 12 20 % more.  A histogram that trusts the lists to be distinct would
 // save 3 %; a chunk that is named twice counts once instead.)
 // What bounds it: the scatter's instructions (1,300 a warp of 32 rows before, 60 % issue) and its shared-memory accesses at random columns
 // (65 - 75 % of the wavefronts); HBM 11 - 25 %.  Algorithmic bytes: 4*nnz read + 4*nnz written + 12*B*H*ncol.
@@ -42,6 +41,11 @@ constexpr int kMaxHistCols = 8192;             // columns per CTA of the histogr
 constexpr int kMaxColsPerCta = 1024;           // columns per CTA of the scatter
 constexpr int kColBytes = kBmStride * 4 + kTileWords * 2 + 8;   // shared memory of the scatter per column
 constexpr int kCscThreads = 512;
+// Up to this many columns the row's thread stores the entries: a warp's 32 rows then put eight (lists of eight) or more into a column's
+// sectors at once, and putting them in order costs more than it saves.  Measured, three kernels, by the row's thread / in order, us: 16
+// columns, 128 x 2K tokens x 16 heads 224 / 242; 32 columns, 16 x 4K x 32 118 / 125, lists of 16 102 / 109, without a causal mask 46.4 / 45.4;
+// 64 columns, 8 x 8K x 32 127 / 130, without a mask, 16 x 4K x 12 52 / 47, 4 x 4K 18.4 / 16.7.
+constexpr int kDirectCols = 32;
 // shared memory of the scatter: the columns' arrays; the tile's entries (lists of up to `kmax`) take the place of all but the cursors
 constexpr size_t scatter_bytes(int ncols, int kmax) {
   return (size_t)ncols * 8 + ((size_t)ncols * (kColBytes - 8) > (size_t)kTileRows * kmax * 4 ? (size_t)ncols * (kColBytes - 8) : (size_t)kTileRows * kmax * 4);
@@ -323,6 +327,8 @@ __global__ void __launch_bounds__(kCscThreads, 2) csc_scatter_kernel(CscParams p
   };
   if constexpr (KMAX > 0) {
     uint32_t local[KMAX];                                         // place among the tile's entries
+    int32_t* into = p.indices + region;
+    const bool direct = ncols <= kDirectCols;                     // (CTA-uniform)
     if (tid < rows) {
       if (p.row_slots != nullptr) csc_sort<KMAX>(id);             // ascending columns are ascending places
       uint32_t at[KMAX];
@@ -334,6 +340,7 @@ __global__ void __launch_bounds__(kCscThreads, 2) csc_scatter_kernel(CscParams p
           const uint2 f = base[c];
           local[j] = f.x + place(c, tid);
           at[j] = (uint32_t)region + local[j] + f.y;              // (row_slots are kept for fewer than 2^32 entries only)
+          if (direct) into[local[j] + f.y] = r0 + tid;
         }
       }
       if (p.row_slots != nullptr) {
@@ -348,6 +355,7 @@ __global__ void __launch_bounds__(kCscThreads, 2) csc_scatter_kernel(CscParams p
         }
       }
     }
+    if (direct) return;
     __syncthreads();                                              // the bitmap is done with: its place takes the entries
     uint32_t* entry = bm;                                         // column and row of every entry, column by column
     if (tid < rows) {
@@ -356,7 +364,6 @@ __global__ void __launch_bounds__(kCscThreads, 2) csc_scatter_kernel(CscParams p
         if (local[j] != 0xffffffffu) entry[local[j]] = (uint32_t)(id[j] - c0) << 16 | (uint32_t)tid;
     }
     __syncthreads();
-    int32_t* into = p.indices + region;
     for (int i = tid; i < entries; i += kCscThreads) {
       const uint32_t e = entry[i];
       into[i + base[e >> 16].y] = r0 + (int)(e & 0xffffu);

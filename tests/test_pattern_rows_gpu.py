@@ -20,6 +20,7 @@ DEV = "cuda"
 @pytest.mark.parametrize("lens,H,topk,ncol", [
     ([512, 1, 513], 2, 8, 40), ([8192], 1, 8, 64), ([8193, 700, 0, 9000], 2, 3, 1024), ([8200], 1, 16, 1025),
     ([1500], 2, 12, 2100), ([600, 40], 2, 20, 1030), ([9000], 1, 17, 70), ([100], 3, 1, 1),
+    ([513, 700], 2, 8, 32), ([513, 700], 2, 8, 33), ([1100], 2, 16, 32), ([1100], 2, 13, 33), ([900], 2, 4, 1030),   # stored by the row, in order
 ])
 def test_row_slots_and_columns(lens, H, topk, ncol):
     from flash_moba_b200 import _lib
