@@ -592,8 +592,11 @@ static int merge_launch(const AttnArgs& a, const AttnWorkspace& w, const PassPar
   // persistent CTAs, as many as are resident
   const int64_t ctas = ceil_div64(a.total_q * ps.nh, (kMergeThreads / 32) * (32 / (D / 8))), most = (int64_t)sm_count() * 3;
   const unsigned grid = (unsigned)(ctas < most ? ctas : most);
-  // Where the staged kernel is the better one: head dims of 128 and more; dQ, whose merge has less to do per row, from half a gigabyte of
-  // partials on.  Measured, from registers / staged, us: 64K tokens x 32 heads, d 128, top-k 8 828 / 780 forward, 790 / 750 backward; 8 x 8K 805 / 738
+  // Where the staged kernel is the better one: head dims of 128 and more; dQ, whose merge has less to do per row, from about a gigabyte of
+  // partials on where lists are of eight, far earlier where they are shorter (a row's places are a smaller part of its work); the line lies
+  // where lists of eight lose little.  dQ, from registers / staged, us: top-k 8, 234 MB 43.4 / 45.7, 402 MB 74.5 / 78.5, 537 MB 101 / 103, 671 MB
+  // 125 / 127, 1.07 GB 201 / 199; d 256, 524 MB 167 / 166, 1.07 GB 344 / 342; top-k 6, 402 MB 81 / 78, 537 MB 106 / 105; top-k 4, 268 MB 74 / 64, 537
+  // MB 141 / 114, 1.07 GB 281 / 219.  All: 64K tokens x 32 heads, d 128, top-k 8 828 / 780 forward, 790 / 750 backward; 8 x 8K 805 / 738
   // and 751 / 723; 32K x 16 213 / 207 and 202 / 202; 3.6K x 32 (235 MB) 51.7 / 47.6 and 43.5 / 47; d 64, 32K x 16 111 / 113 and 109 / 110.  Lists of 16, or
   // of two planes, with a staged kernel of several steps a row: 317K tokens 6.97 / 7.66 ms, 512K x 4 2.95 / 3.23.
   if constexpr (D >= 128) {

@@ -430,10 +430,12 @@ static int decode_launch(const DecodeParams& p, const DecodeShape& sh, int64_t t
   cfg.stream = s;
   cudaLaunchAttribute at[2];
   // Brought up beside the kernel before it (see follow_on()), but for clusters of eight CTAs: placed around those of a call
-  // that still runs they pile up on fewer SMs.  Measured, without / with, back to back; between elementwise kernels of torch
+  // that still runs they may pile up on fewer SMs.  Measured, without / with, back to back; between elementwise kernels of torch
   // (32 / 8 heads): d 128, 32 rows (no clusters) 94.2 / 92.1; 94.3 / 91.1 us, 16 rows (of two) 56.0 / 54.4; 56.0 / 54.2, 8 rows (of
-  // four) 34.8 / 32.8; 35.8 / 32.8, 4 rows (of four) 22.6 / 21.3; 23.6 / 22.0, one row (of eight) 18.5 / 25.7; 18.6 / 15.4;
-  // d 64, 8 rows 22.5 / 20.2; 23.2 / 20.2, d 256, 4 rows 37.0 / 35.5; 37.7 / 35.9
+  // four) 34.8 / 32.8; 35.8 / 32.8, 4 rows (of four) 22.6 / 21.3; 23.6 / 22.0, one row (of four) and 65,001 keys 13.1 / 13.1; 12.8 / 12.7,
+  // 4,000 keys 12.1 / 11.7; 11.7 / 11.4; d 64, 8 rows 22.5 / 20.2; 23.2 / 20.2, d 256, 4 rows 37.0 / 35.5; 37.7 / 35.9.  Of eight: one
+  // row and 65,001 keys, when it was split that far, 18.5 / 25.7; 18.6 / 15.4; 8 heads, chunk 256, one row 13.1 / 12.6; 12.8 / 12.5;
+  // 32 / 16 heads, d 64, chunk 256, top-k 16, one row 17.7 / 18.0; 17.5 / 17.3
   at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at[1].val.programmaticStreamSerializationAllowed = 1;
   at[0].id = cudaLaunchAttributeClusterDimension;
