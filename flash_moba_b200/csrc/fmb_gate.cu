@@ -620,9 +620,9 @@ __global__ void __launch_bounds__(128 * NQ) gate_topk_tc_kernel(GateParams p) {
 // time: 1 us a step, which is what long sequences took (64K tokens, 32 heads 605 / 549 us with one / two warps).
 // Measured (B200, d 128; the kernel above / two sweeps, all compared with all / sorted keys): 64K tokens, 32 heads, chunk 128, top-k 8
 // 1020 / 605 / 471 us; 8 x 8K tokens 580 / 256 / 178; 32K tokens, 16 heads 185 / 97 / 78; 317K tokens in 16 sequences, chunk 64, top-k 16
-// 7400 / 3430 / 2914; 512K tokens, 4 heads, chunk 256, top-k 16 - / 2106 / 1821; d 64, 9K tokens, 12 heads, no mask - / 31 / 22.  All scores
+// 7400 / 3430 / 2928; 512K tokens, 4 heads, chunk 256, top-k 16 - / 2106 / 1824; d 64, 9K tokens, 12 heads, no mask - / 31 / 22.  All scores
 // equal, the long way throughout: 16K tokens, 8 heads 84 / 88 us, top-k 16 198 / 130; no mask 161 / 166 and 440 / 247.  Scores that are smooth from chunk
-// to chunk (correlation 0.95): 32K tokens, 16 heads 111 / 92, chunk 64, top-k 16 304 / 293, no mask 512 / 447.
+// to chunk (correlation 0.95): 32K tokens, 16 heads 111 / 92, chunk 64, top-k 16 304 / 300, no mask 512 / 454.
 // What bounds it now: instructions at 60 % issue (32K tokens: 1,900 a warp and row tile before, 1,600 with sorted keys; the min / max pipe is busy
 // for 58 %), fetching them where lists are of 16, at 64K also the MMAs (128 x 64 x 16: 52 cycles, of which A's and B's way from shared memory takes 48).
 // ---------------------------------------------------------------------------------------
@@ -1111,12 +1111,13 @@ gate_select_kernel(GateParams p, const __grid_constant__ CUtensorMap map_q, cons
           key[j] = max(key[j], o);
         }
         sel_bitonic<KMAX>(key);
-        // neighbours that may agree in the bits that the keys hold
+        // neighbours that may agree in the bits that the keys hold (less one: keys differ, but for the empty ones, which do not count:
+        // with them 8 x 8K tokens, top-k 4 / 12 took 177 / 365 us instead of 173 / 351)
         uint32_t gap = ~0u;
 #pragma unroll
-        for (int j = 0; j + 1 < KMAX; ++j) gap = min(gap, key[j] - key[j + 1]);
-        if (need == KMAX) gap = min(gap, key[KMAX - 1] - low);
-        if (__any_sync(0xffffffffu, gap < 64u)) {
+        for (int j = 0; j + 1 < KMAX; ++j) gap = min(gap, key[j] - key[j + 1] - 1u);
+        if (need == KMAX) gap = min(gap, key[KMAX - 1] - low - 1u);
+        if (__any_sync(0xffffffffu, gap < 63u)) {
           uint32_t near = 0;
 #pragma unroll
           for (int j = 0; j + 1 < KMAX; ++j) near |= key[j] - key[j + 1] < 64u ? 1u << j : 0u;
