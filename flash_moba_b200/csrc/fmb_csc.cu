@@ -25,8 +25,8 @@
 // bitonic network per row / in column order, read ahead of it, networks of 19 exchanges, all three kernels: 64K 159 / 146 us,
 // 32K x 16 39.5 / 37.3, d 64, 9K x 12 13.8 / 12.5, 8 x 8K 128 / 130, 317K 1460 / 1231, 512K 642 / 607.  (Three CTAs per SM with 40 registers: 64K 1 % more, 8 x 8K 8 % less, but 9K x 12 20 % more.  A histogram that trusts the lists to be distinct would
 // save 3 %; a chunk that is named twice counts once instead.)
-// What bounds it: the scatter's instructions (1,300 a warp of 32 rows before, 60 % issue) and its shared-memory accesses at random columns
-// (65 - 75 % of the wavefronts); HBM 11 - 25 %.  Algorithmic bytes: 4*nnz read + 4*nnz written + 12*B*H*ncol.
+// What bounds it: the scatter's instructions (1,070 a warp of 32 rows, 57 % issue) and its shared-memory accesses at random columns
+// (two thirds to four fifths of the wavefronts); HBM 8 - 25 %.  Algorithmic bytes: 4*nnz read + 4*nnz written + 12*B*H*ncol.
 #include <mutex>
 #include <type_traits>
 
