@@ -279,6 +279,13 @@ __device__ __forceinline__ void cp_async_wait_all() {
   asm volatile("cp.async.commit_group;" ::: "memory");
   asm volatile("cp.async.wait_group 0;" ::: "memory");
 }
+// This thread's copies so far, once they have landed, arrive once at `bar` (which counts a whole warp as 32): the warp goes on to its next tile
+// meanwhile.  Whoever waits for the barrier makes the copies (generic proxy) visible to the MMAs with fence_async_smem().
+// Measured, warps that waited for their copies and arrived themselves / this: backward of 317K tokens, 32 / 8 heads, chunk 64 25.7 / 24.3 ms
+// (a warp with 64 rows of 256 bytes took about as long for a tile as the tile's GEMMs), training steps of 64K x 32 heads 8.01 / 7.92 ms
+__device__ __forceinline__ void cp_async_arrive(uint64_t* bar) {
+  asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
 // 32 rows of NCHUNK*16 bytes gathered by one warp: this lane holds the offset of row `lane` from
 // `base` in units of UNIT bytes (kNoRow = zero fill); tile: the first of the 32 rows (a multiple of 8) in the swizzled tile.  The offsets of four passes
 // are exchanged before the four copies are issued: shuffles and copies keep their order in the program, and a
