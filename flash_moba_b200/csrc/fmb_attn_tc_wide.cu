@@ -204,7 +204,7 @@ __global__ void __launch_bounds__(kFwThreads, 1) fwd_wide_tc_kernel(WideParams p
     }
   } else if (warp >= kFwIssuerWarp) {
     // =============================================================== MMA issuer
-    if (warp == kFwIssuerWarp && lane == 0) {
+    if (warp == kFwIssuerWarp && elect_one()) {
       constexpr uint32_t idesc_s = make_idesc(FmtOf<T>::v, kM, C, 0, 0);
       constexpr uint32_t idesc_o = make_idesc(FmtOf<T>::v, kM, 128, 0, 1);
       const uint32_t hi = desc_hi_sw128(1024);

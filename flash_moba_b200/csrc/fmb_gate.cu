@@ -897,7 +897,7 @@ gate_select_kernel(GateParams p, const __grid_constant__ CUtensorMap map_q, cons
     }
   } else if (warp == 9) {
     // =============================================================== MMAs
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr uint32_t idesc = make_idesc(FmtOf<T>::v, kGateM, kSelN, 0, 0);
       const uint32_t hi = desc_hi_sw128(1024), q_km = desc_lo_sw128(smem_u32(sQ), 16);
       uint32_t gs = 0, qn = 0;
