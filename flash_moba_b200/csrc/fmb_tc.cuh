@@ -305,26 +305,46 @@ __device__ __forceinline__ void cp_async_arrive(uint64_t* bar) {
 // are exchanged before the four copies are issued: shuffles and copies keep their order in the program, and a
 // shuffle's latency in front of every copy held a warp to 92 cycles per copy (5.3 B/clk) whatever else the SM
 // did; measured for whole tiles of 128 rows, B200.  The loop stays rolled: code size counts in these kernels.
+// A warp whose rows are all there (every tile but a column's last) copies without tests, three or four instructions a copy.  With a test in
+// every copy / this: 317K tokens, chunk 64, backward 23.3 / 22.4 ms; 64K x 32 heads, forward 1.65 / 1.61 ms.  Head dim 256 has no use for
+// it (and no registers).
 constexpr uint32_t kNoRow = 0xffffffffu;
 template <int NCHUNK, int UNIT>
 __device__ __forceinline__ void gather_rows32(int lane, unsigned char* tile, uint32_t block_stride, const void* base, uint32_t off) {
   constexpr int RPP = 32 / NCHUNK;           // rows per pass
   constexpr int GB = 4;                      // copies per turn of the loop
   const int j = lane % NCHUNK, rsub = lane / NCHUNK;
-  const uint32_t dst = smem_u32(tile + (j >> 3) * block_stride) + rsub * 128;
   const char* src = static_cast<const char*>(base) + j * 16;
+  uint32_t dst[GB];                          // of the first turn; a turn's rows are a multiple of 8: the swizzle is the same in every turn
+#pragma unroll
+  for (int i = 0; i < GB; ++i) {
+    const int r = i * RPP + rsub;
+    dst[i] = smem_u32(tile + (j >> 3) * block_stride) + r * 128 + ((((uint32_t)j ^ r) & 7) << 4);
+  }
+  static_assert(GB * RPP % 8 == 0, "whole groups of eight rows per turn");
+  if (NCHUNK < 32 && __all_sync(0xffffffffu, off != kNoRow)) {
 #pragma unroll 1
-  for (int i0 = 0; i0 < NCHUNK; i0 += GB) {
-    uint32_t o[GB];
+    for (int i0 = 0; i0 < NCHUNK; i0 += GB) {
+      uint32_t o[GB];
 #pragma unroll
-    for (int i = 0; i < GB; ++i) o[i] = __shfl_sync(0xffffffffu, off, (i0 + i) * RPP + rsub);
+      for (int i = 0; i < GB; ++i) o[i] = __shfl_sync(0xffffffffu, off, i0 * RPP + i * RPP + rsub);
 #pragma unroll
-    for (int i = 0; i < GB; ++i) {
-      const int r = (i0 + i) * RPP;          // plus rsub
-      const uint32_t d = dst + r * 128 + ((((uint32_t)j & 7) ^ ((r + rsub) & 7)) << 4);
-      const bool ok = o[i] != kNoRow;
-      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src + (size_t)(ok ? o[i] : 0u) * UNIT), "r"(ok ? 16u : 0u)
-                   : "memory");
+      for (int i = 0; i < GB; ++i) {
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst[i]), "l"(src + (size_t)o[i] * UNIT) : "memory");
+        dst[i] += GB * RPP * 128;
+      }
+    }
+  } else {
+#pragma unroll 1
+    for (int i0 = 0; i0 < NCHUNK; i0 += GB) {
+#pragma unroll
+      for (int i = 0; i < GB; ++i) {
+        const uint32_t o = __shfl_sync(0xffffffffu, off, i0 * RPP + i * RPP + rsub);
+        const bool ok = o != kNoRow;
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst[i]), "l"(src + (size_t)(ok ? o : 0u) * UNIT), "r"(ok ? 16u : 0u)
+                     : "memory");
+        dst[i] += GB * RPP * 128;
+      }
     }
   }
 }
