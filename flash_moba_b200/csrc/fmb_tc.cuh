@@ -410,11 +410,12 @@ __device__ __forceinline__ void store_part(T* dst, const float* o, float f) {
   st_global_32(dst, pack8<T>(x), pack8<T>(x + 8));
 }
 
-// ---- groups of TMA shared -> global stores ---------------------------------------------
-// The issuing thread commits its stores as a group and must wait for the group's READS before the
-// shared-memory source is reused (or the CTA exits).
-__device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
-__device__ __forceinline__ void bulk_wait_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
+// 8x8 matrix of 16-bit numbers, a row in four threads (two columns each): transposed
+__device__ __forceinline__ uint32_t movmatrix_trans(uint32_t a) {
+  uint32_t d;
+  asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(d) : "r"(a));
+  return d;
+}
 
 template <typename T> struct FmtOf;
 template <> struct FmtOf<__nv_bfloat16> { static constexpr int v = 1; };
