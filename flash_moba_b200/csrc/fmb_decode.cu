@@ -44,6 +44,7 @@ namespace cg = cooperative_groups;
 
 constexpr int kDecThreads = 128, kDecWarps = kDecThreads / 32;
 constexpr float kLog2eDec = 1.4426950408889634f;
+constexpr int kDecHeld = 16;   // candidates of a lane that are kept in registers while a list is made
 
 struct DecodeParams {
   const void *q, *k, *v, *km;
@@ -198,30 +199,58 @@ __global__ void __launch_bounds__(kDecThreads, DecGeo<D>::CTAS) decode_kernel(De
       j = 1;
     }
     // Every lane knows the best of its candidates (n = lane, lane + 32, ...); a round takes the best of the lanes' and only
-    // the lane it came from looks for its next.  Scores as ordered integers (+0 and -0 alike, though no sum that starts at +0 is -0), 0: none.  (With a scan of all
-    // candidates and ten shuffles in every round: one row of 32 heads and 65,001 keys 17.7 us, 16 rows of 16
-    // sequences 54.6; now 16.3 and 52.7)
-    uint32_t best;
-    int at;
-    auto look = [&] {
-      float m = -CUDART_INF_F;
-      at = -1;
-      for (int n = lane; n < ncand; n += 32) {
-        const float x = sc[n];
-        if (x >= m && x > -CUDART_INF_F) { m = x; at = n; }       // ascending n: the higher id on equal scores
-      }
-      const uint32_t u = __float_as_uint(m + 0.f);
-      best = at < 0 ? 0u : (u & 0x80000000u) ? ~u : (u | 0x80000000u);
+    // the lane it came from looks for its next.  Scores as ordered integers (+0 and -0 alike, though no sum that starts at +0 is -0), 0: none
+    // (-inf, NaN).  Up to kDecHeld candidates a lane are held in registers, for a look at all of them takes a round as long as the reductions; more
+    // are looked up in shared memory.  (With a scan of all candidates and ten shuffles in every round: one row of 32 heads
+    // and 65,001 keys 17.7 us, 16 rows of 16 sequences 54.6; looks in shared memory 16.3 and 52.7.  Since then, looks in shared
+    // memory / in registers: one row 14.6 / 13.7, two of 16,000 keys 14.8 / 14.5, 16 54.0 / 53.7, d 64, eight rows 19.8 / 19.35)
+    auto ordered = [](float x) {
+      const uint32_t u = __float_as_uint(x + 0.f);
+      return !(x > -CUDART_INF_F) ? 0u : (u & 0x80000000u) ? ~u : (u | 0x80000000u);
     };
-    look();
-    for (; j < topk; ++j) {
-      const uint32_t top = __reduce_max_sync(0xffffffffu, best);
-      const int pick = __reduce_max_sync(0xffffffffu, best == top ? at : -1);
-      if (pick >= 0 && pick == at) {
-        sc[at] = -CUDART_INF_F;                                   // taken
-        look();
+    auto rounds = [&](auto look, auto take) {
+      uint32_t best;
+      int at;
+      look(best, at);
+      for (; j < topk; ++j) {
+        const uint32_t top = __reduce_max_sync(0xffffffffu, best);
+        const int pick = __reduce_max_sync(0xffffffffu, best == top ? at : -1);
+        if (pick >= 0 && pick == at) {
+          take(at);
+          look(best, at);
+        }
+        if (lane < S) cluster.map_shared_rank(sList, lane)[h * topk + j] = pick;
       }
-      if (lane < S) cluster.map_shared_rank(sList, lane)[h * topk + j] = pick;
+    };
+    if (ncand <= 32 * kDecHeld) {
+      uint32_t u[kDecHeld];
+#pragma unroll
+      for (int i = 0; i < kDecHeld; ++i) u[i] = lane + 32 * i < ncand ? ordered(sc[lane + 32 * i]) : 0u;
+      rounds(
+          [&](uint32_t& best, int& at) {
+            best = 0u;
+            at = 0;
+#pragma unroll
+            for (int i = 0; i < kDecHeld; ++i)
+              if (u[i] >= best) { best = u[i]; at = lane + 32 * i; }   // ascending n: the higher id on equal scores
+            if (best == 0u) at = -1;
+          },
+          [&](int at) {
+#pragma unroll
+            for (int i = 0; i < kDecHeld; ++i)
+              if (at == lane + 32 * i) u[i] = 0u;
+          });
+    } else {
+      rounds(
+          [&](uint32_t& best, int& at) {
+            best = 0u;
+            at = -1;
+            for (int n = lane; n < ncand; n += 32) {
+              const uint32_t x = ordered(sc[n]);
+              if (x >= best && x != 0u) { best = x; at = n; }
+            }
+          },
+          [&](int at) { sc[at] = -CUDART_INF_F; });
     }
   }
   cluster.sync();
