@@ -58,13 +58,29 @@ __device__ __forceinline__ WideItem wide_item(const WideParams& p) {
 }
 
 // 16 rows of NCHUNK*16 bytes gathered by one warp: lanes 0-15 (and again 16-31) hold the rows' numbers (-1 = zero fill);
-// see gather_rows32()
-template <int NCHUNK, typename T>
+// see gather_rows32().  FULL: without tests where all rows are there (backward 1,140 / 1,090 us at 16,389 tokens, 16 / 4 heads; the forward, where
+// the code is longer than what it saves, 102 / 107 us at 16,892 tokens, 2 heads)
+template <int NCHUNK, bool FULL, typename T>
 __device__ __forceinline__ void gather_rows16(int lane, unsigned char* tile, uint32_t block_stride, const T* base, int64_t rs, int row) {
   static_assert(NCHUNK == 32, "a warp copies a row at a time");
   constexpr int GB = 4;                         // copies per turn of the loop
   const uint32_t dst = smem_u32(tile + (lane >> 3) * block_stride);
   const T* src = base + lane * 8;
+  if (FULL && __all_sync(0xffffffffu, row >= 0)) {   // every tile but a column's last
+#pragma unroll 1
+    for (int i0 = 0; i0 < 16; i0 += GB) {
+      int o[GB];
+#pragma unroll
+      for (int i = 0; i < GB; ++i) o[i] = __shfl_sync(0xffffffffu, row, i0 + i);
+#pragma unroll
+      for (int i = 0; i < GB; ++i) {
+        const int r = i0 + i;
+        const uint32_t d = dst + r * 128 + ((((uint32_t)lane & 7) ^ (r & 7)) << 4);
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src + (int64_t)o[i] * rs) : "memory");
+      }
+    }
+    return;
+  }
 #pragma unroll 1
   for (int i0 = 0; i0 < 16; i0 += GB) {
     int o[GB];
@@ -196,7 +212,7 @@ __global__ void __launch_bounds__(kFwThreads, 1) fwd_wide_tc_kernel(WideParams p
       advance(t);
       raw = entry(t);                           // the next tile's, in flight meanwhile
       if (g > 0 && !wait_all(&bar_s[(g - 1) & 1], (g - 1) >> 1, 5)) break;   // S of the tile before has read the Q tile
-      gather_rows16<NCH>(lane, sQ + row0 * 128, kQBlock, qbase, p.q_rs, r);
+      gather_rows16<NCH, false>(lane, sQ + row0 * 128, kQBlock, qbase, p.q_rs, r);
       cp_async_wait_all();
       fence_async_smem();                       // the copies are generic-proxy writes; the MMAs read through the async proxy
       __syncwarp();
@@ -348,6 +364,8 @@ __global__ void __launch_bounds__(kFwThreads, 1) fwd_wide_tc_kernel(WideParams p
 // read the tile before have completed: dK^T += Q^T.dS is issued first (Q is what the next tile starts with), dV^T += dO^T.P
 // behind it, then dQ, whose two halves share 128 TMEM columns: the second is issued behind the next tile's dP.
 // What bounds it is that cycle: gather of Q, S, P (dP beside it), dS, dK.
+// Q's copies and dO's arrive on their own, and the issuing thread tests its barriers (16,389 tokens, 16 / 4 heads, us: Q announced behind dO's issue,
+// waits / this 1,150 / 1,090; with an elected thread 1,120).
 constexpr int kBwDrainWarp = 8, kBwIssuerWarp = 12, kBwLoadWarp = 16, kBwLoaders = 8, kBwThreads = 768;
 // registers per thread: launched with 80 (65536 / 768 rounded down to a multiple of 8)
 constexpr int kBwRegsLaunch = 80, kBwRegsCompute = 112, kBwRegsOther = 64;
@@ -398,7 +416,7 @@ __global__ void __launch_bounds__(kBwThreads, 1) bwd_wide_tc_kernel(WideParams p
 
   if (warp == 0) tmem_alloc(&tmem_base_s, 512);
   if (tid == 0) {
-    mbar_init(&bar_fullq, kBwLoaders); mbar_init(&bar_fulldo, kBwLoaders);   // one arrival per loader warp
+    mbar_init(&bar_fullq, kBwLoaders * 33); mbar_init(&bar_fulldo, kBwLoaders * 32);   // one arrival per thread of the loader warps, and one per warp
     mbar_init(&bar_s, 1); mbar_init(&bar_p, 1); mbar_init(&bar_dk, 1); mbar_init(&bar_dv, 1);
     mbar_init(&bar_dq[0], 1); mbar_init(&bar_dq[1], 1); mbar_init(&bar_fin, 1);
     mbar_init(&bar_ds, 8);                      // one arrival per compute warp
@@ -470,20 +488,14 @@ __global__ void __launch_bounds__(kBwThreads, 1) bwd_wide_tc_kernel(WideParams p
       raw = entry(t);                           // the next tile's, in flight meanwhile
       // dK of the tile before has read the Q tile (and, before that, the compute warps the row data)
       if (g > 0 && !wait_all(&bar_dk, g - 1, 5)) break;
-      gather_rows16<NCH>(lane, sQ + row0 * 128, kQBlock, qbase, p.q_rs, r);
-      asm volatile("cp.async.commit_group;" ::: "memory");
       if (lane < 16) { sRow[i] = r; sLse[i] = l; sDsum[i] = dd; }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&bar_fullq);             // (for the row data)
+      gather_rows16<NCH, true>(lane, sQ + row0 * 128, kQBlock, qbase, p.q_rs, r);
+      cp_async_arrive(&bar_fullq);                        // Q does not wait for dO
       if (g > 0 && !wait_all(&bar_dv, g - 1, 5)) break;   // dV has read the dO tile
-      gather_rows16<NCH>(lane, sdO + row0 * 128, kQBlock, obase, p.do_rs, r);
-      asm volatile("cp.async.commit_group;" ::: "memory");
-      asm volatile("cp.async.wait_group 1;" ::: "memory");
-      fence_async_smem();                       // the copies are generic-proxy writes; the MMAs read through the async proxy
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&bar_fullq);
-      asm volatile("cp.async.wait_group 0;" ::: "memory");
-      fence_async_smem();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&bar_fulldo);
+      gather_rows16<NCH, true>(lane, sdO + row0 * 128, kQBlock, obase, p.do_rs, r);
+      cp_async_arrive(&bar_fulldo);
     }
     cp_async_wait_all();
   } else if (warp >= kBwIssuerWarp) {
@@ -504,7 +516,7 @@ __global__ void __launch_bounds__(kBwThreads, 1) bwd_wide_tc_kernel(WideParams p
       bool ok = true;
       // the second dQ half of tile g, once the first has been read out
       auto dq_second = [&] {
-        if (!mbar_wait(&bar_dqfree, 0, p.status, 6)) return false;   // phase 2 g: the first half of tile g
+        if (!mbar_spin(&bar_dqfree, 0, p.status, 6)) return false;   // phase 2 g: the first half of tile g
         tc_fence_after_sync();
         umma_gemm<kC / 16>(tdQ, ds_km, hi, 2, 0, k_mn + (2 * kKBlock >> 4), hi, 128, 512, idesc_dq, 0);
         umma_commit(&bar_dq[1]);
@@ -514,18 +526,20 @@ __global__ void __launch_bounds__(kBwThreads, 1) bwd_wide_tc_kernel(WideParams p
       for (uint32_t g = 0; g <= ntiles && ok; ++g) {
         if (g < ntiles) {
           // S(g) and dP(g): their columns were read before dS(g - 1) was ready
-          if (!(ok = mbar_wait(&bar_fullq, g & 1, p.status, 6))) break;
+          if (!(ok = mbar_spin(&bar_fullq, g & 1, p.status, 6))) break;
+          fence_async_smem();                   // the gathers are generic-proxy writes; the MMAs read through the async proxy
           tc_fence_after_sync();
           umma_gemm<D / 16>(tS, q_km, hi, 2, kQBlock >> 4, k_km, hi, 2, kKBlock >> 4, idesc_s, 0);
           umma_commit(&bar_s);
-          if (!(ok = mbar_wait(&bar_fulldo, g & 1, p.status, 6))) break;
+          if (!(ok = mbar_spin(&bar_fulldo, g & 1, p.status, 6))) break;
+          fence_async_smem();
           tc_fence_after_sync();
           umma_gemm<D / 16>(tdP, do_km, hi, 2, kQBlock >> 4, v_km, hi, 2, kKBlock >> 4, idesc_s, 0);
           umma_commit(&bar_p);
         }
         if (g > 0 && !(ok = dq_second())) break;
         if (g == ntiles) break;
-        if (!(ok = mbar_wait(&bar_ds, g & 1, p.status, 6))) break;
+        if (!(ok = mbar_spin(&bar_ds, g & 1, p.status, 6))) break;
         tc_fence_after_sync();
         const uint32_t acc = g > 0 ? 1u : 0u;   // the item's first tile starts the accumulators
         // dK^T[half] += Q^T.dS, dV^T[half] += dO^T.P : M = 128 head-dim columns, N = keys, K = the rows
@@ -538,7 +552,7 @@ __global__ void __launch_bounds__(kBwThreads, 1) bwd_wide_tc_kernel(WideParams p
           umma_gemm<kM / 16>(tdV + hh * 64, do_mn + hh * (2 * kQBlock >> 4), hi, 128, 512, p_mn, hi, 128, 512, idesc_t, acc);
         umma_commit(&bar_dv);
         // first half of dQ = dS.K, once the second half of the tile before has been read out (phase 2 g - 1 of bar_dqfree)
-        if (g > 0 && !(ok = mbar_wait(&bar_dqfree, 1, p.status, 6))) break;
+        if (g > 0 && !(ok = mbar_spin(&bar_dqfree, 1, p.status, 6))) break;
         tc_fence_after_sync();
         umma_gemm<kC / 16>(tdQ, ds_km, hi, 2, 0, k_mn, hi, 128, 512, idesc_dq, 0);
         umma_commit(&bar_dq[0]);

@@ -60,6 +60,18 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int* s
   return false;
 }
 
+// The same, by tests in turn, for the thread that issues MMAs: 55 cycles each, where a try_wait that has to wait wakes up late (backward, 3K tokens
+// x 8 heads, d 64 45 / 40 us, 64K x 32 heads, d 128 3.52 / 3.46 ms).  Not for warps that compute: they take issue slots from the others
+// (forward 1 - 5 % slower).
+__device__ __forceinline__ bool mbar_spin(uint64_t* bar, uint32_t parity, int* status, int where) {
+#pragma unroll 1
+  for (uint32_t i = 0; i < (kSpinLimit << 7); ++i) {   // half a second as well
+    if (mbar_test(bar, parity)) return true;
+  }
+  if (status) atomicCAS(status, 0, where);
+  return false;
+}
+
 // ---- a load that is issued where it is written
 // A plain load may be moved by the compiler down to its first use (it does so
 // under register pressure), which turns a prefetch into a full-latency stall.  This is a volatile
