@@ -429,6 +429,12 @@ __device__ __forceinline__ uint32_t movmatrix_trans(uint32_t a) {
   return d;
 }
 
+// ---- groups of TMA shared -> global stores ---------------------------------------------
+// The issuing thread commits its stores as a group and must wait for the group's READS before the
+// shared-memory source is reused (or the CTA exits).
+__device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
+__device__ __forceinline__ void bulk_wait_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
+
 template <typename T> struct FmtOf;
 template <> struct FmtOf<__nv_bfloat16> { static constexpr int v = 1; };
 template <> struct FmtOf<__half> { static constexpr int v = 0; };
