@@ -34,8 +34,6 @@
 
 namespace fmb {
 
-int sm_count();                                // SMs of the current device
-
 constexpr int kTileRows = 512;                 // query rows per tile
 constexpr int kTileWords = kTileRows / 32;     // bitmap words per column
 constexpr int kBmStride = kTileWords + 1;      // padded: conflict-free column walks
@@ -48,13 +46,8 @@ constexpr int kCscThreads = 512;
 // columns, 128 x 2K tokens x 16 heads 224 / 242; 32 columns, 16 x 4K x 32 118 / 125, lists of 16 102 / 109, without a causal mask 46.4 / 45.4;
 // 64 columns, 8 x 8K x 32 127 / 130, without a mask, 16 x 4K x 12 52 / 47, 4 x 4K 18.4 / 16.7.
 constexpr int kDirectCols = 32;
-// Sequences of up to this many tiles, if all tiles have a place on the GPU at once: every scatter CTA counts the tiles of its (b, h) itself instead of
-// waiting for a launch that does.  Measured, both kernels / one, us: four sequences of 512, 16 heads 6.95 / 6.03, eight of 500, top-k 16 9.65 / 7.6, two of
-// 2,000, top-k 8 10.3 / 9.6, 1K tokens x 8 heads 7.06 / 6.27; 1K and 2K tokens, 8 heads, lists of four in places of eight 7.0 / 7.55, but a launch
-// less for the host, which such calls wait for (the whole pattern 23.2 / 20.5 us to enqueue).  With up to twice as many tiles as SMs 12.5 / 13.5
-constexpr int kOwnTiles = 4;
 // shared memory of the scatter: the columns' arrays; the tile's entries (lists of up to `kmax`) take the place of all but the cursors
-__host__ __device__ constexpr size_t scatter_bytes(int ncols, int kmax) {
+constexpr size_t scatter_bytes(int ncols, int kmax) {
   return (size_t)ncols * 8 + ((size_t)ncols * (kColBytes - 8) > (size_t)kTileRows * kmax * 4 ? (size_t)ncols * (kColBytes - 8) : (size_t)kTileRows * kmax * 4);
 }
 
@@ -66,7 +59,7 @@ struct CscParams {
   uint32_t* row_slots;                                // optional: [(h*total_q + token)*topk + ...], ascending, 0xffffffff = no entry
   int64_t total_q;
   int batch, heads, topk, ncol, ntiles, cols_per_cta;
-  int scanned;                                        // 1: hist holds cursors (tile_scan has run), 0: counts, 2: nothing (see kOwnTiles)
+  int scanned;                                        // 1: hist holds cursors (tile_scan has run), 0: counts
 };
 
 // ascending sorting networks on 8 and 16 ids: 19 compare-exchanges; two sorted eights and a bitonic merge
@@ -197,7 +190,7 @@ __global__ void __launch_bounds__(1024) csc_tile_scan_kernel(CscParams p) {
 
 // KMAX: 8 or 16: lists of at most that many ids are sorted in registers by one thread per row; 0: any length,
 // a thread per entry
-// OWN: see kOwnTiles
+// OWN: a sequence is one tile: its columns are the tile's, nobody has counted them before
 template <int KMAX, bool OWN>
 __global__ void __launch_bounds__(kCscThreads, 2) csc_scatter_kernel(CscParams p) {
   follow_on();
@@ -231,28 +224,6 @@ __global__ void __launch_bounds__(kCscThreads, 2) csc_scatter_kernel(CscParams p
     if (tid < rows) csc_load_row<KMAX>(p, src, tid, id);
   }
 
-  // ---- entries per column of the whole (b, h), and above them (<< 16) of the tiles before this one
-  uint32_t* own = OWN ? sm + scatter_bytes(ncols, KMAX) / 4 : nullptr;   // [ncol] (a single group of columns)
-  if constexpr (OWN) {
-    {
-      for (int c = tid; c < ncols; c += kCscThreads) own[c] = 0u;
-      __syncthreads();
-      const int32_t* all = p.topk_idx + (int64_t)seq0 * p.idx_rs + (int64_t)h * p.idx_hs;
-#pragma unroll 1
-      for (int r = tid; r < min(len_q, kOwnTiles * kTileRows); r += kCscThreads) {
-        int x[KMAX];
-        csc_load_row<KMAX>(p, all, r, x);
-        csc_sort<KMAX>(x);
-        const uint32_t one = r < r0 ? 0x10001u : 1u;
-#pragma unroll
-        for (int j = 0; j < KMAX; ++j)
-          if (x[j] != kCscNone && (j == 0 || x[j] != x[j > 0 ? j - 1 : 0])) atomicAdd(&own[x[j]], one);
-      }
-      __syncthreads();
-    }
-  }
-
-  // ---- column offsets (places inside the region) and this tile's cursor in every column
   const int32_t* hist = p.hist + (int64_t)bh * p.ntiles * p.ncol;
   // exclusive sum over the CTA's threads; `total`: of all
   auto scan = [&](Off x, Off& total) {
@@ -276,15 +247,17 @@ __global__ void __launch_bounds__(kCscThreads, 2) csc_scatter_kernel(CscParams p
     __syncthreads();
     return (warp > 0 ? ahead : 0) + x - own;
   };
+  auto put_column = [&](int c, int64_t off, int nnz) {
+    p.col_offsets[(int64_t)bh * p.ncol + c] = region + off;
+    if (OWN || !p.scanned) p.col_nnz[(int64_t)bh * p.ncol + c] = nnz;
+  };
+  // ---- column offsets (places inside the region) and this tile's cursor in every column
   Off carry = 0, total;
-  for (int g0 = 0; g0 < p.ncol; g0 += kCscThreads) {
+  for (int g0 = 0; !OWN && g0 < p.ncol; g0 += kCscThreads) {
     const int c = g0 + tid;
     int nnz = 0, cursor = 0;
     if (c < p.ncol) {
-      if (OWN) {
-        nnz = (int)(own[c] & 0xffffu);
-        cursor = (int)(own[c] >> 16);
-      } else if (p.scanned) {
+      if (p.scanned) {
         nnz = p.col_nnz[(int64_t)bh * p.ncol + c];
         cursor = tile < ntiles_b ? hist[(int64_t)tile * p.ncol + c] : 0;
       } else {
@@ -299,18 +272,18 @@ __global__ void __launch_bounds__(kCscThreads, 2) csc_scatter_kernel(CscParams p
     const Off off = carry + scan(nnz, total);
     if (c < p.ncol) {
       if (c >= c0 && c < c0 + ncols) base[c - c0].y = (uint32_t)(off + cursor);
-      if (tile == 0 && blockIdx.z == 0) {
-        p.col_offsets[(int64_t)bh * p.ncol + c] = region + off;
-        if (OWN || !p.scanned) p.col_nnz[(int64_t)bh * p.ncol + c] = nnz;
-      }
+      if (tile == 0 && blockIdx.z == 0) put_column(c, off, nnz);
     }
     carry += total;
   }
   // the unused tail of the region stays zero, as in the reference's zero-initialised buffer
   // (csrc/flash_topk/flash_topk_api.cpp:217); its tiles share it
-  if (blockIdx.z == 0 && ntiles_b > 0)
-    for (int64_t i = carry + (int64_t)tile * kCscThreads + tid; i < (int64_t)len_q * p.topk; i += (int64_t)ntiles_b * kCscThreads)
-      p.indices[region + i] = 0;
+  auto clear_tail = [&](int64_t used) {
+    if (blockIdx.z == 0 && ntiles_b > 0)
+      for (int64_t i = used + (int64_t)tile * kCscThreads + tid; i < (int64_t)len_q * p.topk; i += (int64_t)ntiles_b * kCscThreads)
+        p.indices[region + i] = 0;
+  };
+  if (!OWN) clear_tail(carry);
   // rows of no sequence (q padded to a fixed size): their lists are empty.  The merge goes over all rows of q
   if (p.row_slots != nullptr && b == p.batch - 1 && blockIdx.z == 0 && (lead > 0 || seq0 + len_q < p.total_q)) {
     uint32_t* lists = p.row_slots + (int64_t)h * p.total_q * p.topk;
@@ -318,9 +291,10 @@ __global__ void __launch_bounds__(kCscThreads, 2) csc_scatter_kernel(CscParams p
     for (int64_t i = first; i < (int64_t)lead * p.topk; i += step) lists[i] = 0xffffffffu;
     for (int64_t i = (int64_t)(seq0 + len_q) * p.topk + first; i < p.total_q * p.topk; i += step) lists[i] = 0xffffffffu;
   }
-  if (rows <= 0) return;
+  if (!OWN && rows <= 0) return;
 
   // ---- bitmap of the tile
+  if (OWN) __syncthreads();                                       // (it has been cleared: otherwise a scan has come in between)
   if constexpr (KMAX > 0) {
     if (tid < rows) {
 #pragma unroll
@@ -348,10 +322,13 @@ __global__ void __launch_bounds__(kCscThreads, 2) csc_scatter_kernel(CscParams p
       }
     }
     const int first = entries + (int)scan(run, total);
-    if (c < ncols) base[c] = make_uint2((uint32_t)first, base[c].y - (uint32_t)first);
+    if (OWN && c < ncols) put_column(c, first, run);
+    if (c < ncols) base[c] = make_uint2((uint32_t)first, OWN ? 0u : base[c].y - (uint32_t)first);
     entries += (int)total;
   }
   __syncthreads();
+  if (OWN) clear_tail(entries);
+  if (OWN && rows <= 0) return;
 
   // ---- places: first of the column's entries in this tile, plus its rows ahead of this one
   auto place = [&](int c, int r) {
@@ -451,27 +428,31 @@ int launch_build_csc(const int32_t* topk_idx, int64_t idx_rs, int64_t idx_hs, co
   // few tiles: their scatter CTAs add up the counts of the tiles before their own (at most 16 numbers per
   // column) instead of waiting for one more launch
   p.scanned = p.ntiles > 16 ? 1 : 0;
-  if (topk <= 16 && p.ntiles <= kOwnTiles && ncol <= kMaxColsPerCta && (int64_t)batch * heads * p.ntiles <= sm_count()) p.scanned = 2;
+  // A tile a sequence: the scatter's bitmap has the columns' entries anyway, nobody counts them ahead of it.  Both kernels / the scatter alone, us: four
+  // sequences of 512, 16 heads 7.26 / 4.59, eight of 500, lists of 16 14.55 / 6.97, one of 200, 4 heads 5.94 / 3.69; the whole pattern of 64 of 500, 16
+  // heads 95.1 / 87.3, of 200 of 120 102.9 / 84.4.  Two to four tiles, two kernels / scatter CTAs that each count all tiles of their (b, h): 1K and
+  // 2K tokens, 8 heads, lists of four 7.2 / 8.3, of eight 8.1 / 11.2, of 16 12.4 / 20.0 (the whole pattern 27.2 / 44.7)
+  const bool own = topk <= 16 && p.ntiles == 1 && ncol <= kMaxColsPerCta;
   prof_begin(6, s);
-  if (p.scanned != 2) {
+  if (!own) {
     p.cols_per_cta = min(kMaxHistCols, ncol);
     auto count = topk <= 8 ? csc_tile_hist_kernel<8> : topk <= 16 ? csc_tile_hist_kernel<16> : csc_tile_hist_kernel<0>;
     launch_follow_on(count, dim3(batch * heads, p.ntiles, ceil_div(ncol, p.cols_per_cta)), dim3(kCscThreads),
                      (size_t)p.cols_per_cta * sizeof(uint32_t), s, p);
     FMB_LAUNCH_CHECK("csc_tile_hist_kernel");
   }
-  if (p.scanned == 1) {
+  if (p.scanned) {
     launch_follow_on(csc_tile_scan_kernel, dim3(batch * heads, ceil_div(ncol, 32)), dim3(1024), 0, s, p);
     FMB_LAUNCH_CHECK("csc_tile_scan_kernel");
   }
   p.cols_per_cta = min(kMaxColsPerCta, ncol);
   const dim3 grid(batch * heads, p.ntiles, ceil_div(ncol, p.cols_per_cta));
   const int kmax = topk <= 8 ? 8 : topk <= 16 ? 16 : 0;
-  const size_t smem = scatter_bytes(p.cols_per_cta, kmax) + (p.scanned == 2 ? (size_t)ncol * 4 : 0);
-  auto scatter = p.scanned == 2 ? (topk <= 8 ? csc_scatter_kernel<8, true> : csc_scatter_kernel<16, true>)
+  const size_t smem = scatter_bytes(p.cols_per_cta, kmax);
+  auto scatter = own ? (topk <= 8 ? csc_scatter_kernel<8, true> : csc_scatter_kernel<16, true>)
                : topk <= 8 ? csc_scatter_kernel<8, false> : topk <= 16 ? csc_scatter_kernel<16, false> : csc_scatter_kernel<0, false>;
   // the attribute belongs to the current device: set on every call (cheap, idempotent, thread-safe)
-  FMB_CUDA(cudaFuncSetAttribute(scatter, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(scatter_bytes(kMaxColsPerCta, kmax) + kMaxColsPerCta * 4)));
+  FMB_CUDA(cudaFuncSetAttribute(scatter, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)scatter_bytes(kMaxColsPerCta, kmax)));
   launch_follow_on(scatter, grid, dim3(kCscThreads), smem, s, p);
   prof_end(6, s);
   FMB_LAUNCH_CHECK("csc_scatter_kernel");
