@@ -35,6 +35,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <type_traits>
 
 #include "fmb_common.cuh"
 
@@ -44,7 +45,11 @@ namespace cg = cooperative_groups;
 
 constexpr int kDecThreads = 128, kDecWarps = kDecThreads / 32;
 constexpr float kLog2eDec = 1.4426950408889634f;
-constexpr int kDecHeld = 16;   // candidates of a lane that are kept in registers while a list is made
+// Candidates of a lane that are kept in registers while a list is made: up to kDecFew if all lists are that short, else up to kDecHeld (every look
+// goes over all places, used or not).  One row, us, all looked up in shared memory / 16 / 4 or 16: 2 chunks 7.7 / 8.0 / 7.4, d 64, 20 chunks
+// 7.3 / 7.4 / 7.0; two rows, 125 chunks 14.6 / 14.3 / 13.4.  With 8 in place of 4: 235 chunks 12.0 / 11.4, but 125 13.4 / 13.8 and 8 8.6 / 8.8;
+// with 24 in place of 16: 703 chunks 13.4 / 12.5, but 508 12.3 / 12.8 and 313 10.7 / 11.5
+constexpr int kDecFew = 4, kDecHeld = 16;
 
 struct DecodeParams {
   const void *q, *k, *v, *km;
@@ -200,8 +205,8 @@ __global__ void __launch_bounds__(kDecThreads, DecGeo<D>::CTAS) decode_kernel(De
     }
     // Every lane knows the best of its candidates (n = lane, lane + 32, ...); a round takes the best of the lanes' and only
     // the lane it came from looks for its next.  Scores as ordered integers (+0 and -0 alike, though no sum that starts at +0 is -0), 0: none
-    // (-inf, NaN).  Up to kDecHeld candidates a lane are held in registers, for a look at all of them takes a round as long as the reductions; more
-    // are looked up in shared memory.  (With a scan of all candidates and ten shuffles in every round: one row of 32 heads
+    // (-inf, NaN).  Up to kDecHeld candidates a lane are held in registers, for a look in shared memory at all of them takes a round as long as the reductions;
+    // more are looked up there.  (With a scan of all candidates and ten shuffles in every round: one row of 32 heads
     // and 65,001 keys 17.7 us, 16 rows of 16 sequences 54.6; looks in shared memory 16.3 and 52.7.  Since then, looks in shared
     // memory / in registers: one row 14.6 / 13.7, two of 16,000 keys 14.8 / 14.5, 16 54.0 / 53.7, d 64, eight rows 19.8 / 19.35.
     // Looks in shared memory compare floats and make an integer of the best one only: with one made of every score, one row
@@ -224,24 +229,30 @@ __global__ void __launch_bounds__(kDecThreads, DecGeo<D>::CTAS) decode_kernel(De
         if (lane < S) cluster.map_shared_rank(sList, lane)[h * topk + j] = pick;
       }
     };
-    if (ncand <= 32 * kDecHeld) {
-      uint32_t u[kDecHeld];
+    auto held = [&](auto most) {
+      constexpr int N = decltype(most)::value;
+      uint32_t u[N];
 #pragma unroll
-      for (int i = 0; i < kDecHeld; ++i) u[i] = lane + 32 * i < ncand ? ordered(sc[lane + 32 * i]) : 0u;
+      for (int i = 0; i < N; ++i) u[i] = lane + 32 * i < ncand ? ordered(sc[lane + 32 * i]) : 0u;
       rounds(
           [&](uint32_t& best, int& at) {
             best = 0u;
             at = 0;
 #pragma unroll
-            for (int i = 0; i < kDecHeld; ++i)
+            for (int i = 0; i < N; ++i)
               if (u[i] >= best) { best = u[i]; at = lane + 32 * i; }   // ascending n: the higher id on equal scores
             if (best == 0u) at = -1;
           },
           [&](int at) {
 #pragma unroll
-            for (int i = 0; i < kDecHeld; ++i)
+            for (int i = 0; i < N; ++i)
               if (at == lane + 32 * i) u[i] = 0u;
           });
+    };
+    if (ncand <= 32 * kDecFew) {
+      held(std::integral_constant<int, kDecFew>{});
+    } else if (ncand <= 32 * kDecHeld) {
+      held(std::integral_constant<int, kDecHeld>{});
     } else {
       rounds(
           [&](uint32_t& best, int& at) {

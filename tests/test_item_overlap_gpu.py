@@ -67,3 +67,9 @@ def test_forward_items_of_ragged_batches(chunk, d):
 def test_decode_selection_around_the_held_candidates(n_chunks, topk):
     """Rows of n_chunks chunks have n_chunks - 1 candidates; 512 are held in registers."""
     edges.test_decode_selection_of_equal_scores(n_chunks, topk)
+
+
+@pytest.mark.parametrize("n_chunks,topk", [(128, 8), (129, 16), (130, 8), (257, 33)])
+def test_decode_selection_around_few_candidates(n_chunks, topk):
+    """Up to 128 candidates a list are held four a lane, more sixteen a lane."""
+    edges.test_decode_selection_of_equal_scores(n_chunks, topk)
