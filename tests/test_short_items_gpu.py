@@ -40,3 +40,27 @@ def test_many_short_sequences_forward(chunk, d, H, Hk):
     dev = [t.to(DEV) for t in (q, k, v)]
     runs = [F.flash_moba_attn_varlen_func(*dev, cu.to(DEV), cu.to(DEV), max(lens), max(lens), *pattern, 128, chunk, causal=True) for _ in range(3)]
     assert torch.equal(runs[0], runs[1]) and torch.equal(runs[0], runs[2])
+
+
+@pytest.mark.parametrize("H,Hk", [(8, 8), (16, 4)])
+@pytest.mark.parametrize("d", [64, 128, 256])
+@pytest.mark.parametrize("chunk", [64, 128])
+def test_many_short_sequences_backward(chunk, d, H, Hk):
+    """Keys that no row selects have gradients of exactly zero, and two runs agree to the bit."""
+    from flash_moba_b200 import ops
+    from test_kernels_gpu import _attn_check
+    lens, cu, q, k, v, do, mask = _batch(H, Hk, d, chunk)
+    _attn_check(q, k, v, do, cu, cu, mask, chunk, True, 1)
+    pattern = [t.to(DEV) for t in O.mask_to_csc(mask, cu, cu, chunk)[:3]]
+    dev = [t.to(DEV) for t in (q, k, v, do, cu)]
+    geo = (*pattern, dev[4], dev[4], max(lens), max(lens), chunk, d ** -0.5, True)
+    out, lse = ops.attn_fwd(*dev[:3], *geo)
+    runs = []
+    for _ in range(2):
+        grads = [torch.full_like(t, 7.0) for t in dev[:3]]
+        ops.attn_bwd(dev[3], *dev[:3], out, lse, *grads, *geo)
+        runs.append(grads)
+    assert all(torch.equal(a, b) for a, b in zip(*runs))
+    for i in range(0, len(lens), 3):
+        rows = slice(int(cu[i]) + chunk, int(cu[i + 1]))
+        assert not runs[0][1][rows].any() and not runs[0][2][rows].any()
