@@ -44,6 +44,7 @@ _SIGS = {
     "fmb_attn_status_mirror": (i32, [c_ptr]),
     "fmb_attn_key_spans": (i32, [c_ptr, c_ptr]),
     "fmb_selftest_wait_expiry": (i32, [c_ptr, c_ptr, c_ptr]),
+    "fmb_selftest_spin_expiry": (i32, [c_ptr, c_ptr, c_ptr]),
     "fmb_selftest_umma": (i32, [c_ptr, c_ptr, c_ptr, i32, i32, c_ptr, c_ptr]),
     "fmb_launch_count": (ctypes.c_ulonglong, []),
     "fmb_profile_enable": (i32, [i32]),

@@ -167,7 +167,12 @@ int fmb_attn_status_mirror(int* mirror) {
 
 int fmb_selftest_wait_expiry(int* status, unsigned long long* elapsed_ns, fmb_stream_t stream) {
   FMB_CHECK_ARG(status && elapsed_ns, "selftest_wait_expiry: null pointer");
-  return launch_selftest_wait_expiry(status, elapsed_ns, (cudaStream_t)stream);
+  return launch_selftest_wait_expiry(false, status, elapsed_ns, (cudaStream_t)stream);
+}
+
+int fmb_selftest_spin_expiry(int* status, unsigned long long* elapsed_ns, fmb_stream_t stream) {
+  FMB_CHECK_ARG(status && elapsed_ns, "selftest_spin_expiry: null pointer");
+  return launch_selftest_wait_expiry(true, status, elapsed_ns, (cudaStream_t)stream);
 }
 
 int fmb_chunk_offsets(const int32_t* cu_seqlens_k, int batch, int chunk, int32_t* cu_seqlens_km,

@@ -101,11 +101,20 @@ def selftest_umma(a: torch.Tensor, b: torch.Tensor, b_mn_major: bool) -> torch.T
 def selftest_wait_expiry(device=None) -> Tuple[int, float]:
     """Runs the library's bounded wait on an mbarrier nobody arrives at (see fmb_selftest_wait_expiry).
     Returns (status code written by the kernel, seconds the wait lasted before it gave up)."""
+    return _expire(lib.fmb_selftest_wait_expiry, device)
+
+
+def selftest_spin_expiry(device=None) -> Tuple[int, float]:
+    """The same of the wait of the threads that issue the backward's MMAs (see fmb_selftest_spin_expiry)."""
+    return _expire(lib.fmb_selftest_spin_expiry, device)
+
+
+def _expire(call, device) -> Tuple[int, float]:
     dev = torch.device("cuda", torch.cuda.current_device()) if device is None else torch.device(device)
     with torch.cuda.device(dev):
         status = torch.full((1,), -1, dtype=torch.int32, device=dev)
         ns = torch.zeros((1,), dtype=torch.int64, device=dev)
-        check(lib.fmb_selftest_wait_expiry(ptr(status), ptr(ns), _stream()))
+        check(call(ptr(status), ptr(ns), _stream()))
         torch.cuda.synchronize(dev)
     return int(status.item()), int(ns.item()) * 1e-9
 

@@ -305,6 +305,9 @@ int fmb_selftest_umma(const void* a, const void* b, float* d, int b_mn_major, in
  * Nothing else runs in the kernel, so no copy or MMA is in flight when it gives up. */
 int fmb_selftest_wait_expiry(int* status, unsigned long long* elapsed_ns, fmb_stream_t stream);
 
+/* The same of the bounded wait of the threads that issue the backward's MMAs, which tests the mbarrier in turn: code 6. */
+int fmb_selftest_spin_expiry(int* status, unsigned long long* elapsed_ns, fmb_stream_t stream);
+
 /* Optional hand-over of the pattern's slot and row lists (the CSR transpose that both attention
  * calls build in their workspace) from a forward call to the backward call of the same pattern.
  * No counterpart in the reference, whose kernels walk the pattern query-block-major and need no

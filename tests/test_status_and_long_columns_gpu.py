@@ -35,6 +35,19 @@ def test_bounded_wait_gives_up_and_reports():
     assert torch.allclose(d, a.float() @ a.float().T, atol=0.5, rtol=2e-2)
 
 
+def test_issuing_threads_wait_gives_up_and_reports():
+    """Bounds as for the other wait, and about as long as that one."""
+    from flash_moba_b200 import ops
+    code, seconds = ops.selftest_spin_expiry()
+    assert code == 6
+    assert 0.05 < seconds < 30.0, seconds
+    assert seconds < 2 * ops.selftest_wait_expiry()[1], seconds
+    print(f"bounded wait of an issuing thread gave up after {seconds:.3f} s")
+    a = torch.randn(128, 128, device=DEV).bfloat16()
+    d = ops.selftest_umma(a, a, False)
+    assert torch.allclose(d, a.float() @ a.float().T, atol=0.5, rtol=2e-2)
+
+
 def _overlapping_pattern(T, H, ncol):
     # two columns that both claim all T places of `indices`
     ind = torch.arange(T, dtype=torch.int32, device=DEV).repeat(H)
