@@ -45,7 +45,7 @@ namespace cg = cooperative_groups;
 
 constexpr int kDecThreads = 128, kDecWarps = kDecThreads / 32;
 constexpr float kLog2eDec = 1.4426950408889634f;
-// Candidates of a lane that are kept in registers while a list is made: up to kDecFew if all lists are that short, else up to kDecHeld (every look
+// Candidates of a lane that are kept in registers while a list is made: four of them for rows of up to 128 candidates, else sixteen (every look
 // goes over all places, used or not).  One row, us, all looked up in shared memory / 16 / 4 or 16: 2 chunks 7.7 / 8.0 / 7.4, d 64, 20 chunks
 // 7.3 / 7.4 / 7.0; two rows, 125 chunks 14.6 / 14.3 / 13.4.  With 8 in place of 4: 235 chunks 12.0 / 11.4, but 125 13.4 / 13.8 and 8 8.6 / 8.8;
 // with 24 in place of 16: 703 chunks 13.4 / 12.5, but 508 12.3 / 12.8 and 313 10.7 / 11.5

@@ -64,7 +64,7 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int* s
   return false;
 }
 
-// The same, by tests in turn, for the thread that issues MMAs: 55 cycles each, where a try_wait that has to wait wakes up late (backward, 3K tokens
+// The same, by tests in turn, for the thread that issues MMAs: one that succeeds takes 55 cycles, where a try_wait that has to wait wakes up late (backward, 3K tokens
 // x 8 heads, d 64 45 / 40 us, 64K x 32 heads, d 128 3.52 / 3.46 ms).  Not for warps that compute: they take issue slots from the others
 // (forward 1 - 5 % slower).
 __device__ __forceinline__ bool mbar_spin(uint64_t* bar, uint32_t parity, int* status, int where) {
@@ -317,13 +317,14 @@ __device__ __forceinline__ void cp_async_arrive(uint64_t* bar) {
   asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
 // 32 rows of NCHUNK*16 bytes gathered by one warp: this lane holds the offset of row `lane` from
-// `base` in units of UNIT bytes (kNoRow = zero fill); tile: the first of the 32 rows (a multiple of 8) in the swizzled tile.  The offsets of four passes
-// are exchanged before the four copies are issued: shuffles and copies keep their order in the program, and a
-// shuffle's latency in front of every copy held a warp to 92 cycles per copy (5.3 B/clk) whatever else the SM
-// did; measured for whole tiles of 128 rows, B200.  The loop stays rolled: code size counts in these kernels.
+// `base` in units of UNIT bytes (kNoRow = zero fill); tile: the first of the 32 rows (a multiple of 8) in the swizzled tile.  The loop stays
+// rolled: code size counts in these kernels.
 // A warp whose rows are all there (every tile but a column's last) copies without tests, three or four instructions a copy.  With a test in
-// every copy / this: 317K tokens, chunk 64, backward 23.3 / 22.4 ms; 64K x 32 heads, forward 1.65 / 1.61 ms.  Head dim 256 has no use for
-// it (and no registers).
+// every copy / this: 317K tokens, chunk 64, backward 23.3 / 22.4 ms; 64K x 32 heads, forward 1.65 / 1.61 ms.  The offsets of four passes are exchanged
+// before the four copies are issued: shuffles and copies keep their order in the program, and a shuffle's latency in front of every copy held a
+// warp to 92 cycles per copy (5.3 B/clk) whatever else the SM did; measured for whole tiles of 128 rows, B200.  A column's last tile exchanges one offset
+// a copy, which is shorter; four at a time there, us: 64 sequences of 100 tokens, 16 heads, forward 72.5 / 72.5, backward 101.4 / 100.9, 200 of 37,
+// d 64 47.3 / 47.8 and 72.4 / 72.4, 100 rows behind 16K keys, d 64, backward 724 / 735.
 constexpr uint32_t kNoRow = 0xffffffffu;
 template <int NCHUNK, int UNIT>
 __device__ __forceinline__ void gather_rows32(int lane, unsigned char* tile, uint32_t block_stride, const void* base, uint32_t off) {
@@ -338,7 +339,7 @@ __device__ __forceinline__ void gather_rows32(int lane, unsigned char* tile, uin
     dst[i] = smem_u32(tile + (j >> 3) * block_stride) + r * 128 + ((((uint32_t)j ^ r) & 7) << 4);
   }
   static_assert(GB * RPP % 8 == 0, "whole groups of eight rows per turn");
-  if (NCHUNK < 32 && __all_sync(0xffffffffu, off != kNoRow)) {
+  if (__all_sync(0xffffffffu, off != kNoRow)) {
 #pragma unroll 1
     for (int i0 = 0; i0 < NCHUNK; i0 += GB) {
       uint32_t o[GB];
